@@ -1,8 +1,9 @@
-// Depthwise 3x3 convolution (stride 1 or 2, channel count a multiple of 32) as a
+// Depthwise 3x3 and 5x5 convolution (stride 1 or 2, any channel count) as a
 // persistent, TMA-fed, HBM-bound kernel.
 //
 // One block per SM slot walks a list of tiles. A tile is th x tw output pixels of
-// one image for a slab of 32 channels; tw is the map's width when that is at most 32
+// one image for a slab of 32 channels (16 where 32 would leave much of the last slab
+// empty; channels past the tensor arrive as zeros and are not stored); tw is the map's width when that is at most 32
 // (so 19- and 10-wide maps are covered without ragged column tiles), else 32 or 16. Its input window, halo included, is ONE TMA
 // box [IH rows][IW cols][32 channels]; pixels outside the image arrive as zeros,
 // which is the convolution's padding. A ring of two to four shared-memory stages: while
@@ -13,6 +14,8 @@
 // window down RPG output rows of it; 8 lanes cover one pixel's 128 bytes, so
 // shared-memory reads are conflict-free. The 32 pixel slots of a block are split into
 // 32 / tw row groups.
+// Widths that are no multiple of 32 channels, and 5x5 windows, ran on kernels that fetch every
+// tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 25 us here (16 us floor).
 #include <cstdlib>
 
 #include "tc_common.cuh"
@@ -34,14 +37,17 @@ struct DwTiles {
     long total;
 };
 
-template <int S, int RPG>
-__global__ void __launch_bounds__(256)
-dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict__ w, const float* __restrict__ bias,
+// KS: window size. CB: float4s of a channel slab (8 = 32 channels, 4 = 16). A 5x5 window keeps its 25 taps
+// in registers too (100 of them), which leaves one block per SM: eight warps with 4-row accumulators are
+// enough to keep the copies ahead of the multiplies.
+template <int KS, int S, int RPG, int CB>
+__global__ void __launch_bounds__(256, KS == 3 ? 2 : 1)
+dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict__ w, const float* __restrict__ bias,
                  float4* __restrict__ y, const ConvArgs a, const DwTiles tl, int* err_flag) {
-    constexpr int CB = 8;                          // float4s (32 channels) per tile
-    constexpr int ROWS_IN = (RPG - 1) * S + 3;
+    constexpr int ROWS_IN = (RPG - 1) * S + KS;
     const int TW = tl.tw, TH = tl.th, IW = tl.iw;
     const uint32_t kTileBytes = (uint32_t)(tl.ih * tl.iw * CB * 16);
+    const uint32_t pitch = (kTileBytes + 127u) & ~127u;      // TMA destinations are 128-byte aligned
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kDwMaxStages];
 
@@ -71,7 +77,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
         const int ty = (int)(t % (unsigned)tl.tiles_y); t /= (unsigned)tl.tiles_y;
         const int n = (int)t;
         mbar_expect_tx(&bar_full[stage], kTileBytes);
-        tma_load_4d(base + (uint32_t)stage * kTileBytes, &tmX, &bar_full[stage], cb * 32, tx * TW * S - a.pad,
+        tma_load_4d(base + (uint32_t)stage * pitch, &tmX, &bar_full[stage], cb * CB * 4, tx * TW * S - a.pad,
                     ty * TH * S - a.pad, n);
     };
 
@@ -84,7 +90,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
     long it = 0;
     int stage = 0;
     uint32_t phase = 0;
-    float4 wk[9];
+    float4 wk[KS * KS];
     float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
     int loaded_cb = -1;
     for (long tile = blockIdx.x; tile < tl.total; tile += gridDim.x, ++it) {
@@ -104,9 +110,14 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
         // count every tile of a block has the same slab, and they are loaded once
         if (cb != loaded_cb) {
 #pragma unroll
-            for (int k = 0; k < 9; ++k) wk[k] = w[k * (a.Kp >> 2) + cq];
+            for (int k = 0; k < KS * KS; ++k) wk[k] = cq < (a.Kp >> 2) ? w[k * (a.Kp >> 2) + cq] : make_float4(0.f, 0.f, 0.f, 0.f);
             bv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (a.has_bias) bv = make_float4(bias[cq * 4], bias[cq * 4 + 1], bias[cq * 4 + 2], bias[cq * 4 + 3]);
+            if (a.has_bias) {                          // bias holds exactly K floats
+                if (cq * 4 + 0 < a.K) bv.x = bias[cq * 4 + 0];
+                if (cq * 4 + 1 < a.K) bv.y = bias[cq * 4 + 1];
+                if (cq * 4 + 2 < a.K) bv.z = bias[cq * 4 + 2];
+                if (cq * 4 + 3 < a.K) bv.w = bias[cq * 4 + 3];
+            }
             loaded_cb = cb;
         }
 
@@ -118,7 +129,7 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
             }
             break;   // uniform: every thread waits on the same barrier with the same bound
         }
-        const float4* tile_s = stage0 + (size_t)stage * (kTileBytes / 16);
+        const float4* tile_s = stage0 + (size_t)stage * (pitch / 16);
         if (active) {
         float4 acc[RPG];
 #pragma unroll
@@ -126,16 +137,16 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
         const int row0 = rg * RPG * S;
 #pragma unroll
         for (int r = 0; r < ROWS_IN; ++r) {
-            float4 v[3];
+            float4 v[KS];
 #pragma unroll
-            for (int kx = 0; kx < 3; ++kx) v[kx] = tile_s[((row0 + r) * IW + col * S + kx) * CB + c];
+            for (int kx = 0; kx < KS; ++kx) v[kx] = tile_s[((row0 + r) * IW + col * S + kx) * CB + c];
 #pragma unroll
             for (int o = 0; o < RPG; ++o) {
                 const int ky = r - o * S;
-                if (ky < 0 || ky > 2) continue;
+                if (ky < 0 || ky >= KS) continue;
 #pragma unroll
-                for (int kx = 0; kx < 3; ++kx) {
-                    const float4 f = wk[ky * 3 + kx];
+                for (int kx = 0; kx < KS; ++kx) {
+                    const float4 f = wk[ky * KS + kx];
                     acc[o].x = fmaf(f.x, v[kx].x, acc[o].x);
                     acc[o].y = fmaf(f.y, v[kx].y, acc[o].y);
                     acc[o].z = fmaf(f.z, v[kx].z, acc[o].z);
@@ -144,12 +155,18 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
             }
         }
         const int ox = tx * TW + col;
-        if (ox < a.Wo) {
+        if (ox < a.Wo && cq < (a.Kp >> 2)) {
 #pragma unroll
             for (int o = 0; o < RPG; ++o) {
                 const int oy = ty * TH + rg * RPG + o;
                 if (oy >= a.Ho) continue;
-                y[(((long)n * a.Ho + oy) * a.Wo + ox) * out_q + off_q + cq] = apply_act4(acc[o], a.act, a.lo, a.hi);
+                float4 r = apply_act4(acc[o], a.act, a.lo, a.hi);
+                if (cq * 4 + 4 > a.K) {                // lanes past K stay zero
+                    if (cq * 4 + 1 >= a.K) r.y = 0.f;
+                    if (cq * 4 + 2 >= a.K) r.z = 0.f;
+                    r.w = 0.f;
+                }
+                y[(((long)n * a.Ho + oy) * a.Wo + ox) * out_q + off_q + cq] = r;
             }
         }
         }
@@ -158,43 +175,51 @@ dw3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restri
     }
 }
 
-template <int S, int RPG>
+template <int KS, int S, int RPG, int CB>
 int launch(const ConvArgs& a, const DwTiles& shape, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
     CUtensorMap mX;
-    const cuuint64_t dims[4] = {(cuuint64_t)a.C, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
+    const cuuint64_t dims[4] = {(cuuint64_t)a.Kp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
     const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
-    const cuuint32_t box[4] = {32, (cuuint32_t)shape.iw, (cuuint32_t)shape.ih, 1};
+    const cuuint32_t box[4] = {CB * 4, (cuuint32_t)shape.iw, (cuuint32_t)shape.ih, 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     if (!make_map_sw(CU_TENSOR_MAP_SWIZZLE_NONE, &mX, x, 4, dims, str, box, es)) return OGLE_ERR_CUDA;
     DwTiles tl = shape;
     tl.tiles_x = (a.Wo + tl.tw - 1) / tl.tw;
     tl.tiles_y = (a.Ho + tl.th - 1) / tl.th;
-    tl.cblocks = a.K / 32;
+    tl.cblocks = (a.Kp + CB * 4 - 1) / (CB * 4);
     tl.total = (long)tl.tiles_x * tl.tiles_y * tl.cblocks * a.N;
-    const size_t smem = (size_t)tl.stages * tl.ih * tl.iw * 8 * 16 + 128;
+    const size_t smem = (size_t)tl.stages * (((size_t)tl.ih * tl.iw * CB * 16 + 127) / 128 * 128) + 128;
     static thread_local int attr_device = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(dw3x3_tma_kernel<S, RPG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(dw_tma_kernel<KS, S, RPG, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmemMax);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
     }
     if (tl.total > 0x7fffffffL) return OGLE_ERR_UNSUPPORTED;
-    long blocks = (long)kNumSMs * 2;
+    long blocks = (long)kNumSMs * (KS == 3 ? 2 : 1);
     // a multiple of the channel-slab count: block b then always works on slab b % cblocks
     if (tl.cblocks <= blocks) blocks -= blocks % tl.cblocks;
     if (blocks > tl.total) blocks = tl.total;
-    launch_overlapped(dw3x3_tma_kernel<S, RPG>, dim3((unsigned)blocks), dim3(256), smem, s, mX, reinterpret_cast<const float4*>(w),
+    launch_overlapped(dw_tma_kernel<KS, S, RPG, CB>, dim3((unsigned)blocks), dim3(256), smem, s, mX, reinterpret_cast<const float4*>(w),
                       bias, reinterpret_cast<float4*>(y), a, tl, error_flag_ptr());
     return finish_launch();
+}
+
+// Float4s of a channel slab: 32 channels, or 16 where slabs of 32 would compute over a sixth more channels than
+// slabs of 16 do (a slab's empty lanes cost shared memory and issue slots, not traffic).
+int slab_quads(const ConvArgs& a) {
+    const int full = (a.Kp + 31) / 32 * 32, half = (a.Kp + 15) / 16 * 16;
+    return 6 * full <= 7 * half ? 8 : 4;
 }
 
 // Tile shape for a map: full-width tiles when the map is at most 16 wide, equal parts up to 48; the rows per
 // thread (one of the compiled RPG values) that leaves the fewest idle output rows.
 // Returns the chosen RPG, or 0 when no shape fits two stages in kDwSmemMax.
 int choose_shape(const ConvArgs& a, DwTiles* t) {
-    const int S = a.stride;
+    const int S = a.stride, KS = a.kernel, CB = slab_quads(a);
+    const int slots = 256 / CB;                      // output pixels a block computes at once
     int tw = a.Wo <= 32 ? a.Wo : (S == 1 ? 32 : 16);
     // Widths that would leave many of the 32 pixel slots of a block idle are cut into equal parts
     // (measured at batch 256: 19 -> 2 x 10 is 6 % faster, 38 -> 3 x 13 is 18 % faster than 32 + 6)
@@ -202,30 +227,31 @@ int choose_shape(const ConvArgs& a, DwTiles* t) {
     else if (a.Wo > 32 && a.Wo <= 48) tw = (a.Wo + 2) / 3;
     if (const char* e = getenv("OGLE_DW_TW")) { const int v = atoi(e); if (v >= 1 && v <= 32) tw = v < a.Wo ? v : a.Wo; }
     const int force_rpg = getenv("OGLE_DW_RPG") ? atoi(getenv("OGLE_DW_RPG")) : 0;
-    const int groups = 32 / tw;
-    static const int kRpg1[] = {10, 8, 7, 5, 4, 2}, kRpg2[] = {7, 5, 4, 2};
-    const int* cand = S == 1 ? kRpg1 : kRpg2;
-    const int ncand = S == 1 ? 6 : 4;
+    const int groups = slots / tw;
+    static const int kRpg1[] = {10, 8, 7, 5, 4, 2}, kRpg2[] = {7, 5, 4, 2}, kRpg5[] = {4, 2};
+    const int* cand = KS == 5 ? kRpg5 : (S == 1 ? kRpg1 : kRpg2);
+    const int ncand = KS == 5 ? 2 : (S == 1 ? 6 : 4);
     int best = 0;
     long best_cost = -1;
     for (int i = 0; i < ncand; ++i) {
         const int rpg = cand[i], th = rpg * groups;
         if (force_rpg && rpg != force_rpg) continue;
-        const int iw = (tw - 1) * S + 3, ih = (th - 1) * S + 3;
+        const int iw = (tw - 1) * S + KS, ih = (th - 1) * S + KS;
         if (iw > 256 || ih > 256) continue;
-        if (2 * (size_t)ih * iw * 128 + 128 > (size_t)kDwSmemMax) continue;
+        const size_t tile = ((size_t)ih * iw * CB * 16 + 127) / 128 * 128;
+        if (2 * tile + 128 > (size_t)kDwSmemMax) continue;
         const long tiles_y = (a.Ho + th - 1) / th;
         // rows computed (idle ones included) plus a charge per tile for its halo rows
-        long cost = tiles_y * (th * S + 2);
-        // a single channel slab (32 channels): neighbouring blocks then work on neighbouring
+        long cost = tiles_y * (th * S + KS - 1);
+        // a single channel slab: neighbouring blocks then work on neighbouring
         // tiles of the same rows, and a ring of three shallower tiles measured 20 % faster
         // than two deep ones on the 150x150 map
-        if (a.K == 32 && 3 * (size_t)ih * iw * 128 + 128 > (size_t)kDwSmemMax) cost *= 2;
+        if (a.Kp <= CB * 4 && 3 * tile + 128 > (size_t)kDwSmemMax) cost *= 2;
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost; best = rpg;
             t->tw = tw; t->th = th; t->row_groups = groups; t->iw = iw; t->ih = ih;
             // as many tiles in flight as fit: HBM latency x bandwidth needs ~90 KB per SM
-            int st = (int)((size_t)(kDwSmemMax - 128) / ((size_t)ih * iw * 128));
+            int st = (int)((size_t)(kDwSmemMax - 128) / tile);
             t->stages = st > kDwMaxStages ? kDwMaxStages : st;
         }
     }
@@ -235,34 +261,43 @@ int choose_shape(const ConvArgs& a, DwTiles* t) {
 }  // namespace
 
 bool dw_tma_supported(const ConvArgs& a) {
-    if (!(a.kernel == 3 && a.dil == 1 && a.pad <= 1 && (a.stride == 1 || a.stride == 2) && a.K % 32 == 0 && a.C == a.K &&
-          a.Wo >= 8 && a.Ho >= 4 && encode_fn() != nullptr))
+    if (!((a.kernel == 3 || a.kernel == 5) && a.dil == 1 && a.pad <= a.kernel / 2 && (a.stride == 1 || a.stride == 2) &&
+          a.C == a.K && a.Wo >= 8 && a.Ho >= 4 && encode_fn() != nullptr))
         return false;
     DwTiles t;
     return choose_shape(a, &t) != 0;
 }
 
-int launch_dw_tma(const ConvArgs& a, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
+template <int CB>
+static int launch_slab(const ConvArgs& a, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
     DwTiles t = {};
     const int rpg = choose_shape(a, &t);
+    if (a.kernel == 5) {
+        if (a.stride == 1) return rpg == 4 ? launch<5, 1, 4, CB>(a, t, x, w, bias, y, s) : launch<5, 1, 2, CB>(a, t, x, w, bias, y, s);
+        return rpg == 4 ? launch<5, 2, 4, CB>(a, t, x, w, bias, y, s) : launch<5, 2, 2, CB>(a, t, x, w, bias, y, s);
+    }
     if (a.stride == 1) {
         switch (rpg) {
-            case 10: return launch<1, 10>(a, t, x, w, bias, y, s);
-            case 8: return launch<1, 8>(a, t, x, w, bias, y, s);
-            case 7: return launch<1, 7>(a, t, x, w, bias, y, s);
-            case 5: return launch<1, 5>(a, t, x, w, bias, y, s);
-            case 4: return launch<1, 4>(a, t, x, w, bias, y, s);
-            case 2: return launch<1, 2>(a, t, x, w, bias, y, s);
+            case 10: return launch<3, 1, 10, CB>(a, t, x, w, bias, y, s);
+            case 8: return launch<3, 1, 8, CB>(a, t, x, w, bias, y, s);
+            case 7: return launch<3, 1, 7, CB>(a, t, x, w, bias, y, s);
+            case 5: return launch<3, 1, 5, CB>(a, t, x, w, bias, y, s);
+            case 4: return launch<3, 1, 4, CB>(a, t, x, w, bias, y, s);
+            case 2: return launch<3, 1, 2, CB>(a, t, x, w, bias, y, s);
         }
     } else {
         switch (rpg) {
-            case 7: return launch<2, 7>(a, t, x, w, bias, y, s);
-            case 5: return launch<2, 5>(a, t, x, w, bias, y, s);
-            case 4: return launch<2, 4>(a, t, x, w, bias, y, s);
-            case 2: return launch<2, 2>(a, t, x, w, bias, y, s);
+            case 7: return launch<3, 2, 7, CB>(a, t, x, w, bias, y, s);
+            case 5: return launch<3, 2, 5, CB>(a, t, x, w, bias, y, s);
+            case 4: return launch<3, 2, 4, CB>(a, t, x, w, bias, y, s);
+            case 2: return launch<3, 2, 2, CB>(a, t, x, w, bias, y, s);
         }
     }
     return OGLE_ERR_UNSUPPORTED;
+}
+
+int launch_dw_tma(const ConvArgs& a, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
+    return slab_quads(a) == 8 ? launch_slab<8>(a, x, w, bias, y, s) : launch_slab<4>(a, x, w, bias, y, s);
 }
 
 }  // namespace ogle
