@@ -375,6 +375,11 @@ typedef struct {
 int ogle_cuda_ssd_detect(const OgleDetectParams* p, const float* logits, const float* boxes,
                          float* out_score, int* out_anchor, int* out_class, float* out_box,
                          int* out_count, ogle_stream_t stream);
+/* ogle_cuda_ssd_decode followed by ogle_cuda_ssd_detect in one pass: pred [N][A][4] deltas and anchors [A][4] instead
+ * of boxes. Only the boxes of selected anchors are decoded, by the same arithmetic. */
+int ogle_cuda_ssd_decode_detect(const OgleDetectParams* p, const float* logits, const float* pred, const float* anchors,
+                                const float variances[4], float* out_score, int* out_anchor, int* out_class,
+                                float* out_box, int* out_count, ogle_stream_t stream);
 
 #ifdef __cplusplus
 }

@@ -104,6 +104,7 @@ CUDA_SYMBOLS = {
     "ogle_cuda_reshape_placed": (C.c_int, [_vp, _vp, C.c_long, C.c_int, C.c_int, C.c_long, C.c_long, _vp]),
     "ogle_cuda_ssd_decode": (C.c_int, [_vp, _vp, _vp, C.c_int, C.c_int, C.POINTER(C.c_float), _vp]),
     "ogle_cuda_ssd_detect": (C.c_int, [C.POINTER(DetectParams)] + [_vp] * 8),
+    "ogle_cuda_ssd_decode_detect": (C.c_int, [C.POINTER(DetectParams), _vp, _vp, _vp, C.POINTER(C.c_float)] + [_vp] * 6),
 }
 
 _cuda = None

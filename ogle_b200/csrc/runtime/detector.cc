@@ -33,8 +33,6 @@ Detector::Detector(const DetectorOptions& options, Context* context) : options_(
 }
 
 void Detector::Release() {
-    if (boxes_) cudaFree(boxes_);
-    boxes_ = nullptr;
     for (Slot& s : slots_) {
         if (s.stage) cudaFree(s.stage);
         if (s.bytes) cudaFree(s.bytes);
@@ -70,7 +68,6 @@ void Detector::Allocate(int N, int H, int W) {
     counts_per_image_ = L.counts_per_image;
     off_anchor_ = L.anchor; off_cls_ = L.cls; off_box_ = L.box; off_count_ = L.count;
     out_bytes_ = L.total;
-    OGLE_RT_CUDA(cudaMalloc(&boxes_, size_t(N) * num_anchors_ * 16));
     for (int i = 0; i < kDepth; ++i) {
         Slot& s = slots_[i];
         OGLE_RT_CUDA(cudaMalloc(&s.stage, stage_bytes));
@@ -254,12 +251,9 @@ void Detector::PostProcess(Slot& slot, int N, int H, int W, const OgleImageDesc*
     Tensor* anchors = session_->FindTensorByName(options_.output_names[2]);
     OGLE_CHECK(cls_logits && box_preds && anchors);
     OGLE_CHECK_EQ(cls_logits->shape()[0], N);
-    // detector.cc:242-258: GPU box decode into a cached tensor
-    Tensor decoded(IntList{N, num_anchors_, 4}, dlxnet::TensorProto::ANY4, boxes_);
-    Tensor anchors2d(IntList{num_anchors_, 4}, dlxnet::TensorProto::ANY4, anchors->device<float>());
+    // detector.cc:242-258 (box decode) and 150-228 (selection) in one pass on the device
     OGLE_CHECK_EQ(anchors->num_elements(), size_t(num_anchors_) * 4);
-    functor::SSDBBoxDecoder()(context_, box_preds, &anchors2d, &decoded, options_.variances);
-    // detector.cc:150-228 on the device
+    OGLE_CHECK_EQ(options_.variances.size(), 4u);
     OgleDetectParams p;
     std::memset(&p, 0, sizeof(p));
     p.N = N; p.A = num_anchors_; p.C = num_classes_;
@@ -273,10 +267,11 @@ void Detector::PostProcess(Slot& slot, int N, int H, int W, const OgleImageDesc*
     // this slot's output buffer must have been copied out by its previous user
     OGLE_RT_CUDA(cudaStreamWaitEvent(compute, E(slot.ev_d2h), 0));
     char* d = static_cast<char*>(slot.out_dev);
-    OGLE_CUDA_OK(ogle_cuda_ssd_detect(&p, cls_logits->device<float>(), boxes_, reinterpret_cast<float*>(d),
-                                      reinterpret_cast<int*>(d + off_anchor_), reinterpret_cast<int*>(d + off_cls_),
-                                      reinterpret_cast<float*>(d + off_box_), reinterpret_cast<int*>(d + off_count_),
-                                      context_->stream()));
+    OGLE_CUDA_OK(ogle_cuda_ssd_decode_detect(&p, cls_logits->device<float>(), box_preds->device<float>(), anchors->device<float>(),
+                                             options_.variances.data(), reinterpret_cast<float*>(d),
+                                             reinterpret_cast<int*>(d + off_anchor_), reinterpret_cast<int*>(d + off_cls_),
+                                             reinterpret_cast<float*>(d + off_box_), reinterpret_cast<int*>(d + off_count_),
+                                             context_->stream()));
     OGLE_RT_CUDA(cudaEventRecord(E(slot.ev_done), compute));
 }
 

@@ -107,7 +107,6 @@ private:
     Context* context_;
     std::unique_ptr<FBOSession> session_;
     int num_classes_ = 0, num_anchors_ = 0, batch_ = 0, rows_ = 0, counts_per_image_ = 0;
-    float* boxes_ = nullptr;          // decoded [N][A][4]
     Slot slots_[kDepth];
     int next_slot_ = 0;
     std::vector<int> pending_;

@@ -1,0 +1,113 @@
+"""Kernels at the sizes where their tilings, remainders and fallbacks change, against the oracle.
+
+Bounds: data movement and batchnorm bit-exact; sums of n fp32 products 1e-5 + 1e-5|ref| (tests of the same kernels
+at ordinary sizes use the same); selections exact wherever the oracle's scores are not tied within fp32 rounding.
+"""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(__file__))
+from test_ops_gpu import _check_per_class, close  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("channels", [5, 8, 16, 20, 36, 48, 144, 389])
+@pytest.mark.parametrize("kernel,stride,size", [(3, 1, (19, 33)), (3, 2, (38, 21)), (5, 1, (12, 40)), (5, 2, (31, 17)), (3, 1, (4, 8))])
+def test_depthwise_any_width(oracle_port, channels, kernel, stride, size):
+    """Channel slabs of 32 and 16 with a ragged last one, lanes past the width, 3x3 and 5x5 windows; a clip whose
+    lower bound must not lift the padded lanes."""
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(channels * 10 + kernel)
+    x = rng.standard_normal((2,) + size + (channels,), dtype=np.float32)
+    w = rng.standard_normal((channels, 1, kernel, kernel), dtype=np.float32) * np.float32(0.3)
+    b = rng.standard_normal(channels, dtype=np.float32)
+    case = dict(op="conv2d", x=x, w=w, bias=b, stride=stride, pad=kernel // 2, dilation=1, group=channels, act=1, lo=0.5, hi=6.0)
+    close(run_case_cuda(case), oracle_port.conv2d(x, w, b, stride, kernel // 2, 1, channels, 1, 0.5, 6.0))
+
+
+@pytest.mark.parametrize("channels", [1, 6, 12, 20, 129, 1028])
+def test_batchnorm_any_width_is_exact(oracle_port, channels):
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(channels)
+    x = rng.standard_normal((3, 7, 11, channels), dtype=np.float32)
+    g, b, m = (rng.standard_normal(channels, dtype=np.float32) for _ in range(3))
+    v = rng.random(channels, dtype=np.float32) + np.float32(0.1)
+    got = run_case_cuda(dict(op="batchnorm", x=x, gamma=g, beta=b, mean=m, var=v, eps=1e-5))
+    assert np.array_equal(got, oracle_port.batchnorm(x, g, b, m, v, 1e-5))
+
+
+@pytest.mark.parametrize("widths", [(3, 5), (1, 1, 1, 1, 1), (8, 4, 2), (6, 8), (130, 7, 33)])
+def test_concat_ragged_channels_is_exact(widths):
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(sum(widths))
+    xs = [rng.random((2, 5, 9, w), dtype=np.float32) for w in widths]
+    assert np.array_equal(run_case_cuda(dict(op="concat", xs=xs, axis=3)), np.concatenate(xs, axis=3))
+
+
+def test_average_pool_divides_exactly(oracle_port):
+    """3x3 stride 2 averages at both signs, zeros, tiny and huge values: the quotient of the window's sum by 9 is the
+    correctly rounded one (a window that holds one value and zeros has no summation order)."""
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(5)
+    x = np.zeros((1, 64, 64, 8), np.float32)
+    # odd positions: each window 2i..2i+2 holds exactly one of them (even ones would put four values in a window, whose
+    # sum depends on their order)
+    x[:, 1::2, 1::2] = (rng.standard_normal((1, 32, 32, 8)) * 10.0 ** rng.uniform(-44, 38, (1, 32, 32, 8))).astype(np.float32)
+    got = run_case_cuda(dict(op="pool", x=x, kernel=3, stride=2, pad=0, type_=1))
+    assert np.array_equal(got[0, :, :, :], oracle_port.pool(x, 3, 2, 0, 1)[0])
+
+
+@pytest.mark.parametrize("anchors,classes,top_k,spread", [
+    (1917, 21, 200, 2.0),       # the benchmark's decoder
+    (1917, 21, 200, 1e-3),      # all scores within a fraction of a bin
+    (1917, 21, 200, 0.0),       # all scores equal: index order
+    (1920, 3, 256, 5.0),        # scores crowd at 0 and 1
+    (31, 2, 100, 1.0),          # fewer anchors than results
+    (4001, 30, 37, 1.0),        # scores of a few classes at a time, ragged anchor count
+    (1001, 40, 5, 1.0),         # rows of logits that are not kept in registers
+])
+def test_detect_selection_edges(oracle_port, anchors, classes, top_k, spread):
+    rng = np.random.default_rng(anchors + classes)
+    logits = (rng.standard_normal((2, anchors, classes)) * spread).astype(np.float32)
+    boxes = rng.random((2, anchors, 4), dtype=np.float32)
+    for thr in (0.01, 0.0, 0.3):
+        _check_per_class(oracle_port, logits, boxes, thr, top_k, (classes + 3) // 4 * 4)
+
+
+@pytest.mark.parametrize("anchors,classes,spread,thr", [(1917, 2, 3.0, 0.3), (1917, 21, 1e-3, 0.01), (333, 5, 0.0, 0.1), (40, 33, 2.0, -1.0)])
+def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
+    """The reference detector's rule, decoded by the caller and decoded on the way, over the same edges."""
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    rng = np.random.default_rng(anchors + classes)
+    N, K = 3, 100
+    logits = torch.zeros((N, anchors, ops.up4(classes)))
+    logits[..., :classes] = torch.from_numpy((rng.standard_normal((N, anchors, classes)) * spread).astype(np.float32))
+    logits = logits.cuda()
+    pred = ops.dense_to_device(rng.standard_normal((N, anchors, 4), dtype=np.float32) * np.float32(0.5))
+    priors = ops.dense_to_device(np.concatenate([rng.random((anchors, 2)), rng.random((anchors, 2)) * 0.3 + 0.05], 1))
+    boxes = ops.ssd_decode(pred, priors)
+    out = ops.ssd_detect(logits, boxes, classes, 0, thr, K, 0.45, 300, 300)
+    p = _lib.DetectParams()
+    p.N, p.A, p.C, p.logit_stride, p.mode = N, anchors, classes, logits.shape[-1], 0
+    p.score_thr, p.top_k, p.nms_thr, p.image_w, p.image_h = thr, K, 0.45, 300, 300
+    fused = [torch.empty_like(t) for t in out]
+    var = (C.c_float * 4)(0.1, 0.1, 0.2, 0.2)
+    assert _lib.cuda_lib().ogle_cuda_ssd_decode_detect(C.byref(p), ops._p(logits), ops._p(pred), ops._p(priors), var,
+                                                       *[C.c_void_p(t.data_ptr()) for t in fused], ops._stream()) == 0
+    for a, b in zip(out, fused):
+        assert torch.equal(a, b)
+    score, anchor, cls, box, count = [t.cpu().numpy() for t in out]
+    for n in range(N):
+        ref = oracle_port.detect(boxes[n].cpu().numpy(), logits[n, :, :classes].cpu().numpy(), 300, 300, thr, K, 0.45)
+        k = len(ref["anchor"])
+        assert count[n] == k
+        assert np.abs(score[n, :k] - ref["score"]).max(initial=0) <= 2e-6
+        if spread != 1e-3:         # (scores that differ by less than their rounding may change places)
+            assert np.array_equal(anchor[n, :k], ref["anchor"]) and np.array_equal(box[n, :k].astype(np.int32), ref["rect"])
+        assert (anchor[n, k:] == -1).all()
