@@ -3,9 +3,9 @@
 //     thread owns a float4 of channels for a 2x2 patch of output pixels so the
 //     overlapping input rows are reused from registers;
 //   - grouped (non-depthwise) direct convolution: scalar, rarely used;
-//   - dense implicit GEMM for group == 1 in OGLE_MATH_FP32 mode and for layers
-//     whose reduction is too short for the tensor-core pipeline (the RGB stem).
-#include "conv_args.cuh"
+// and the dispatch of the dense ones that the tensor cores do not serve (OGLE_MATH_FP32 mode, too few input
+// channels) to the small-channel kernel (conv_stem.cu) or the implicit GEMM (igemm.cu).
+#include "igemm.cuh"
 
 namespace ogle {
 
@@ -164,150 +164,6 @@ __global__ void grouped_kernel(const float* __restrict__ x, const float* __restr
     }
 }
 
-// ------------------------------------------------------- dense implicit GEMM
-// D[m][k] = sum_r A[m][r] * B[r][k]; m = output pixel, r = (tap, channel),
-// A gathered from the NHWC4 input with zero fill outside the image,
-// B = tap-major packed filter [taps*Cp][Kp].
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-conv_igemm_kernel(const float* __restrict__ x, const float* __restrict__ wp,
-                  const float* __restrict__ bias, float* __restrict__ y, ConvArgs a) {
-    constexpr int BK = 16;
-    constexpr int NT = (BM / TM) * (BN / TN);
-    constexpr int A_LD = BM * (BK / 4) / NT;       // float4 loads of A per thread per tile
-    constexpr int B_F4 = BK * BN / 4;              // float4s in a B tile
-    constexpr int B_LD = (B_F4 + NT - 1) / NT;
-    static_assert(BM * (BK / 4) % NT == 0, "A tile must divide over the threads");
-    static_assert(TM % 4 == 0 && TN == 4, "register tile shape");
-
-    __shared__ __align__(16) float As[2][BK][BM + 4];
-    __shared__ __align__(16) float Bs[2][BK][BN];
-
-    const int tid = threadIdx.x;
-    const long m0 = (long)blockIdx.x * BM;
-    const int n0 = blockIdx.y * BN;
-    const int R = a.kernel * a.kernel * a.Cp;   // reduction length, multiple of 4
-    const int ntiles = (R + BK - 1) / BK;
-
-    // per-thread A rows (fixed for the whole reduction)
-    int a_row[A_LD], a_kq[A_LD], a_iy0[A_LD], a_ix0[A_LD];
-    long a_img[A_LD];
-    bool a_ok[A_LD];
-#pragma unroll
-    for (int j = 0; j < A_LD; ++j) {
-        const int idx = tid + j * NT;
-        a_row[j] = idx >> 2;
-        a_kq[j] = idx & 3;
-        const long m = m0 + a_row[j];
-        a_ok[j] = m < a.M;
-        const long mm = a_ok[j] ? m : 0;
-        const int ox = int(mm % a.Wo);
-        const long t = mm / a.Wo;
-        const int oy = int(t % a.Ho);
-        const long n = t / a.Ho;
-        a_iy0[j] = oy * a.stride - a.pad;
-        a_ix0[j] = ox * a.stride - a.pad;
-        a_img[j] = n * a.H;
-    }
-
-    float4 ra[A_LD], rb[B_LD];
-    auto load_tile = [&](int kt) {
-#pragma unroll
-        for (int j = 0; j < A_LD; ++j) {
-            const int r = kt * BK + a_kq[j] * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (a_ok[j] && r < R) {
-                const int tap = r / a.Cp, c = r - tap * a.Cp;
-                const int ky = tap / a.kernel, kx = tap - ky * a.kernel;
-                const int iy = a_iy0[j] + ky * a.dil, ix = a_ix0[j] + kx * a.dil;
-                if (iy >= 0 && iy < a.H && ix >= 0 && ix < a.W && c < a.Cs)
-                    v = *reinterpret_cast<const float4*>(x + ((a_img[j] + iy) * a.W + ix) * a.Cs + c);
-            }
-            ra[j] = v;
-        }
-#pragma unroll
-        for (int j = 0; j < B_LD; ++j) {
-            const int idx = tid + j * NT;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (idx < B_F4) {
-                const int kr = idx / (BN / 4), nc = (idx % (BN / 4)) * 4;
-                const int r = kt * BK + kr;
-                if (r < R && n0 + nc < a.Kp)
-                    v = *reinterpret_cast<const float4*>(wp + (long)r * a.Kp + n0 + nc);
-            }
-            rb[j] = v;
-        }
-    };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-        for (int j = 0; j < A_LD; ++j) {
-            const int k = a_kq[j] * 4;
-            As[buf][k + 0][a_row[j]] = ra[j].x;
-            As[buf][k + 1][a_row[j]] = ra[j].y;
-            As[buf][k + 2][a_row[j]] = ra[j].z;
-            As[buf][k + 3][a_row[j]] = ra[j].w;
-        }
-#pragma unroll
-        for (int j = 0; j < B_LD; ++j) {
-            const int idx = tid + j * NT;
-            if (idx < B_F4) {
-                const int kr = idx / (BN / 4), nc = (idx % (BN / 4)) * 4;
-                *reinterpret_cast<float4*>(&Bs[buf][kr][nc]) = rb[j];
-            }
-        }
-    };
-
-    const int ty = tid / (BN / TN), tx = tid % (BN / TN);
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
-    load_tile(0);
-    store_tile(0);
-    __syncthreads();
-    for (int kt = 0; kt < ntiles; ++kt) {
-        const int buf = kt & 1;
-        if (kt + 1 < ntiles) load_tile(kt + 1);
-#pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            float av[TM];
-#pragma unroll
-            for (int i = 0; i < TM; i += 4) {
-                const float4 t4 = *reinterpret_cast<const float4*>(&As[buf][k][ty * TM + i]);
-                av[i] = t4.x; av[i + 1] = t4.y; av[i + 2] = t4.z; av[i + 3] = t4.w;
-            }
-            const float4 b4 = *reinterpret_cast<const float4*>(&Bs[buf][k][tx * TN]);
-            const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        if (kt + 1 < ntiles) {
-            store_tile(buf ^ 1);
-            __syncthreads();
-        }
-    }
-
-    const int nc = n0 + tx * TN;
-    if (nc >= a.Kp) return;
-    const float4 b = load_bias4(bias, nc, a.K, a.has_bias);
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const long m = m0 + ty * TM + i;
-        if (m >= a.M) continue;
-        float4 r = make_float4(acc[i][0] + b.x, acc[i][1] + b.y, acc[i][2] + b.z, acc[i][3] + b.w);
-        r = apply_act4(r, a.act, a.lo, a.hi);
-        if (nc + 0 >= a.K) r.x = 0.f;
-        if (nc + 1 >= a.K) r.y = 0.f;
-        if (nc + 2 >= a.K) r.z = 0.f;
-        if (nc + 3 >= a.K) r.w = 0.f;
-        *reinterpret_cast<float4*>(y + m * a.Ks + a.koff + nc) = r;
-    }
-}
-
 bool conv_smallc_supported(const ConvArgs& a);
 int launch_conv_smallc(const ConvArgs& a, const float* x, const float* w_tap_major, const float* bias, float* y,
                        cudaStream_t s);
@@ -336,14 +192,30 @@ int launch_conv_simt(const ConvArgs& a, int variant, const float* x, const float
         return finish_launch();
     }
     if (variant == CONV_GENERAL && conv_smallc_supported(a)) return launch_conv_smallc(a, x, w, bias, y, s);
-    if (a.Kp <= 32) {
-        dim3 grid(div_up(a.M, 128), div_up(a.Kp, 32));
-        conv_igemm_kernel<128, 32, 4, 4><<<grid, 256, 0, s>>>(x, w, bias, y, a);
-    } else {
-        dim3 grid(div_up(a.M, 128), div_up(a.Kp, 64));
-        conv_igemm_kernel<128, 64, 8, 4><<<grid, 256, 0, s>>>(x, w, bias, y, a);
+    // the kernel numbers input pixels in 32 bits: larger batches go in groups of images
+    const long pixels = (long)a.H * a.W;
+    const long group = pixels * a.N < 0x7fffffffL ? a.N : 0x7fffffffL / pixels;
+    if (group < 1) return OGLE_ERR_UNSUPPORTED;
+    if (group < a.N) {
+        for (int n = 0; n < a.N; n += (int)group) {
+            ConvArgs part = a;
+            part.N = a.N - n < group ? a.N - n : (int)group;
+            part.M = (long)part.N * a.Ho * a.Wo;
+            const int rc = launch_conv_simt(part, variant, x + n * pixels * a.Cs, w, bias, y + (long)n * a.Ho * a.Wo * a.Ks, s);
+            if (rc != OGLE_OK) return rc;
+        }
+        return OGLE_OK;
     }
-    return finish_launch();
+    IgemmArgs g = {};
+    g.x = x; g.w = w; g.bias = bias; g.y = y;
+    g.M = a.M; g.H = a.H; g.W = a.W; g.Ho = a.Ho; g.Wo = a.Wo; g.Cs = a.Cs;
+    g.kernel = a.kernel; g.stride = a.stride; g.pad = a.pad; g.dil = a.dil;
+    g.Cp = a.Cp; g.R = a.kernel * a.kernel * a.Cp;
+    g.ldb = a.Kp; g.n_b = a.Kp; g.N = a.K; g.n_store = a.Kp;
+    g.ldy = a.Ks; g.yoff = a.koff;
+    g.act = a.act; g.lo = a.lo; g.hi = a.hi;
+    g.alpha = 1.f; g.beta = 1.f; g.bias_mode = a.has_bias ? 2 : 0;
+    return launch_igemm(g, false, s);
 }
 
 }  // namespace ogle

@@ -111,3 +111,31 @@ def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
         if spread != 1e-3:         # (scores that differ by less than their rounding may change places)
             assert np.array_equal(anchor[n, :k], ref["anchor"]) and np.array_equal(box[n, :k].astype(np.int32), ref["rect"])
         assert (anchor[n, k:] == -1).all()
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride, pad, dilation: rows, columns and reductions that end inside a tile; launches of
+    # one tile split over a cluster of 8, of a few tiles, and of enough for the large tiles (128 x 32, x 64, x 128)
+    (1, 7, 7, 512, 33, 3, 1, 1, 1), (2, 5, 3, 4, 8, 1, 1, 0, 1), (1, 9, 11, 20, 70, 3, 2, 1, 1), (3, 20, 17, 12, 129, 5, 1, 2, 1),
+    (2, 33, 31, 6, 9, 3, 2, 2, 2), (3, 160, 161, 5, 24, 1, 1, 0, 1), (2, 200, 197, 8, 50, 1, 1, 0, 1), (2, 150, 149, 16, 100, 1, 1, 0, 1)])
+def test_fp32_convolution_edges(oracle_port, shape):
+    from gpu_ops import run_case_cuda
+    N, H, W, C, K, k, s, p, d = shape
+    rng = np.random.default_rng(C + K)
+    x = rng.standard_normal((N, H, W, C), dtype=np.float32)
+    w = (rng.standard_normal((K, C, k, k)) / np.sqrt(C * k * k)).astype(np.float32)
+    b = rng.standard_normal(K, dtype=np.float32)
+    case = dict(op="conv2d", x=x, w=w, bias=b, stride=s, pad=p, dilation=d, group=1, act=1, lo=0.5, hi=2.0)
+    close(run_case_cuda(case), oracle_port.conv2d(x, w, b, s, p, d, 1, 1, 0.5, 2.0))
+
+
+@pytest.mark.parametrize("m,k,n,trans_b", [(1, 5, 3, 0), (1, 5, 3, 1), (65, 129, 63, 0), (63, 131, 66, 1), (8, 512, 1000, 1), (700, 33, 300, 0)])
+def test_fp32_gemm_edges(oracle_port, m, k, n, trans_b):
+    """Rows that end between 16-byte pieces (k and n not multiples of 4), both layouts of B, matrix bias."""
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(m + k + n)
+    A = rng.standard_normal((m, k), dtype=np.float32)
+    B = (rng.standard_normal((n, k) if trans_b else (k, n)) / np.sqrt(k)).astype(np.float32)
+    Cm = rng.standard_normal((m, n), dtype=np.float32)
+    got = run_case_cuda(dict(op="gemm", A=A, B=B, Cm=Cm, transB=trans_b, alpha=0.5, beta=2.0))
+    close(got, oracle_port.gemm(A, B, Cm, trans_b, 0.5, 2.0))
