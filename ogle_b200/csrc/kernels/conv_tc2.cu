@@ -13,9 +13,22 @@
 //               tcgen05.ld -> bias / activation -> shared-memory staging in the
 //               128-byte swizzle -> TMA tensor store (fully coalesced, clipped at the
 //               tensor edge by the hardware);
-//   warps 10-17 two operand-split groups for the split (fp32-grade) mode: they write the
-//               BF16 operand [a_hi | a_lo] of the cross-term pass next to each activation
-//               tile (idle in one-pass mode).
+//   warps 10-17 two operand-split groups for the split (fp32-grade) mode: they build the
+//               BF16 operand [a_hi | a_lo] of the cross-term pass (idle in one-pass mode).
+//               Where the accumulators leave room (tiles of up to 192 columns) both A operands -
+//               TF32 and BF16 - are written into tensor memory, one row per thread, and the
+//               multiplies read them there; else the BF16 one goes next to the activation tile in
+//               shared memory. Same products in the same order either way: the same bits.
+//
+// What a chunk costs (clock stamps of the roles, one block; 3x3 64 -> 64 at 56 x 56 x 128 images, split mode): the
+// ring, the copies and the operand split all wait for the issuing thread, which spent 1230 cycles a chunk: 55 per
+// multiply, because its descriptors went from ordinary to uniform registers each time, and 200-300 per barrier it
+// looks at. Elected by elect.sync it issues in 10 (elect_one), with A in tensor memory it looks at one barrier
+// instead of two, and shared memory carries 16 KB less per chunk: 309 us with both in the old form (217 in the
+// channels-on-M form), 195 us now; 19x19x512->75 3x3, 256 images: 570 (399) -> 318; 512->512 pointwise on SM
+// pairs, 256 images at 19x19: 184 -> 155 (316 of about 400 TFLOP/s that a library reaches with the two passes).
+// The copy producers keep lane 0: elected, they start the copies of bandwidth-bound layers in tighter bursts and
+// those lose 3-4 %.
 // Each group's work item has a latency of about a microsecond (shared-memory round
 // trip plus a proxy fence); two groups per role keep that off the critical path.
 //
@@ -140,13 +153,15 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool split = a.passes == 3;
     const uint32_t b_bytes = (uint32_t)a.BN * 128u;
-    const uint32_t stage_bytes = (split ? 2u : 1u) * (kABytes + b_bytes) + (a.gather ? (uint32_t)a.g_bytes : 0u);
+    const uint32_t a_bytes = (split && !a.ta ? 2u : 1u) * kABytes;      // activation part of a stage
+    const uint32_t stage_bytes = a_bytes + (split ? 2u : 1u) * b_bytes + (a.gather ? (uint32_t)a.g_bytes : 0u);
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    // ring of operand stages (A | A cross (bf16 hi|lo) | B_hi | B cross (bf16 lo|hi)), then the output staging slabs
+    // ring of operand stages (A | A cross (bf16 hi|lo), unless it lives in tensor memory | B_hi | B cross (bf16 lo|hi)),
+    // then the output staging slabs
     auto sA = [&](int s) { return base + (uint32_t)s * stage_bytes; };
-    auto sBhi = [&](int s) { return sA(s) + (split ? 2u : 1u) * kABytes; };
-    auto sWin = [&](int s) { return sA(s) + (split ? 2u : 1u) * (kABytes + b_bytes); };   // gather form: input window
+    auto sBhi = [&](int s) { return sA(s) + a_bytes; };
+    auto sWin = [&](int s) { return sA(s) + a_bytes + (split ? 2u : 1u) * b_bytes; };   // gather form: input window
     const uint32_t staging_off = (uint32_t)a.stages * stage_bytes;
     {
         // the layout must fit what the launch reserved (it does when the base is 1024-aligned as
@@ -177,7 +192,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (threadIdx.x == 0) {
         for (int s = 0; s < a.stages; ++s) {
             mbar_init(&bar_full[s], 2);     // one arrive.expect_tx from each producer
-            mbar_init(&bar_xf[s], (uint32_t)(a.xf_groups * 128));
+            mbar_init(&bar_xf[s], a.ta ? 128u : (uint32_t)(a.xf_groups * 128));
             mbar_init(&bar_empty[s], 1);
         }
         for (int i = 0; i < 4; ++i) {
@@ -211,6 +226,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = tmem_slot;
+    const uint32_t tmem_a = tmem_d + (uint32_t)(a.n_acc * acc_cols);      // A operands in tensor memory: 64 columns per stage
     // barriers, tensor memory and tables are set up; what follows reads and writes global memory
     grid_dependency_wait();
 
@@ -285,7 +301,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
             // kind::f16 with BF16 operands (format code 1), fp32 accumulation
             const uint32_t idesc_bf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
@@ -301,12 +317,21 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem_d + (uint32_t)(as * acc_cols);
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
-                    // gather form: the operand exists only once the split warps have built it
-                    ok = wait_or_abort(a.gather ? &bar_xf[s] : &bar_full[s], ph, abort_flag, a.spin_limit);
+                    // gather form, A in tensor memory: the operand exists only once the split warps have built it (they
+                    // arrive after the stage's copies have landed)
+                    ok = wait_or_abort(a.gather || a.ta ? &bar_xf[s] : &bar_full[s], ph, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 2); s_abort = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = umma_desc(sA(s)), bd = umma_desc(sBhi(s));
                     const uint32_t acc_flag = it > (kSplit ? wi.c_begin : 0) ? 1u : 0u;     // the first chunk overwrites
+                    if (a.ta) {
+                        const uint32_t ta = tmem_a + (uint32_t)s * 64u;
+                        umma_tf32_chunk_ta(d, ta, bd, idesc, acc_flag);
+                        umma_bf16_chunk_ta(d, ta + 32u, bd + (b_bytes >> 4), idesc_bf16);
+                        umma_commit(&bar_empty[s]);
+                        if (++s == a.stages) { s = 0; ph ^= 1u; }
+                        continue;
+                    }
                     umma_tf32_chunk(d, ad, bd, idesc, acc_flag);            // a x b_hi (a is read as its high part)
                     if (split) {
                         // cross terms [a_hi | a_lo] x [b_lo | b_hi] in BF16, once the split role has
@@ -338,7 +363,37 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         // and a_lo = a - a_hi. The fp32 tile itself is left as TMA delivered it. One or two
         // warp groups work on EVERY chunk together.
         const int xg = (warp - 10) >> 2;           // group 0 or 1
-        if ((split || a.gather) && xg < a.xf_groups) {
+        if (a.ta) {
+            // A operands in tensor memory: a thread takes one row, the two groups take alternate chunks
+            const int r = (warp & 3) * 32 + lane;
+            const uint32_t lanes = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+            int s = 0, turn = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
+                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                for (int it = wi.c_begin; it < wi.c_end; ++it) {
+                    // Every stage is waited for in turn, also those of the other group's chunks: copies land out of
+                    // order, and a group that only looked at every second chunk could, in a ring of three or five
+                    // stages, meet a barrier two phases behind and take its parity for the coming one.
+                    // The stage is refilled only after the multiplies that read it - shared and tensor memory - are done.
+                    // (The lanes leave the polling loop one by one; the tensor-memory stores want the whole warp.)
+                    ok = wait_or_abort(&bar_full[s], ph, abort_flag, a.spin_limit);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { record_error(err_flag, 3); s_abort = 1; break; }
+                    if (turn == xg) {
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        split_row_to_tmem(reinterpret_cast<const float4*>(base_ptr + (size_t)s * stage_bytes + (size_t)r * 128), r,
+                                          lanes + (uint32_t)s * 64u);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&bar_xf[s]);
+                    }
+                    turn ^= 1;
+                    if (++s == a.stages) { s = 0; ph ^= 1u; }
+                }
+            }
+        } else if ((split || a.gather) && xg < a.xf_groups) {
             const int nthr = a.xf_groups * 128;
             const int t = threadIdx.x - 320;       // 0 .. nthr-1
             int s = 0;
@@ -638,7 +693,18 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
                  const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
                  cudaStream_t s) {
     if (t.BN % 32 || t.BN > 256) return OGLE_ERR_UNSUPPORTED;
-    const size_t stage = (size_t)(t.passes == 3 ? 2 : 1) * (kABytes + (size_t)t.BN * 128) + (t.gather ? (size_t)t.g_bytes : 0);
+    // accumulators: two, or four when they fit (half of) the 512 columns of tensor memory - the multiplies
+    // of a tile can then start while the epilogues of the two tiles before it still drain theirs
+    const int acc_cols = t.BN;
+    // Split mode: the A operands of both passes go through tensor memory where two stages or more of them fit beside
+    // the accumulators (tiles of up to 192 columns).
+    t.n_acc = 4 * acc_cols <= (t.passes == 3 && !t.gather ? 256 : 512) ? 4 : 2;
+    static const bool ta_off = [] { const char* e = getenv("OGLE_TC_TA"); return e && e[0] == '0'; }();
+    const int ta_stages = (512 - t.n_acc * acc_cols) / 64;
+    t.ta = t.passes == 3 && !t.gather && !ta_off && ta_stages >= 2 ? 1 : 0;
+    if (!t.ta) t.n_acc = 4 * acc_cols <= 512 ? 4 : 2;
+    const size_t stage = (size_t)(t.passes == 3 && !t.ta ? 2 : 1) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * t.BN * 128 +
+                         (t.gather ? (size_t)t.g_bytes : 0);
     // Shared memory is split between the operand ring and the epilogue's staging slabs
     // (128 rows x 32 columns each). Preference: two epilogue groups with two slabs each;
     // give slabs back to the ring while that buys another stage and the ring is shallow.
@@ -667,14 +733,11 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     const size_t budget = kBudget - staging;
     int stages = (int)(budget / stage);
     if (stages > kMaxStages) stages = kMaxStages;
+    if (t.ta && stages > ta_stages) stages = ta_stages;
     if (stages < 2) return OGLE_ERR_UNSUPPORTED;
     t.stages = stages;
-    // accumulators: two, or four when they fit the 512 columns of tensor memory - the multiplies
-    // of a tile can then start while the epilogues of the two tiles before it still drain theirs
-    const int acc_cols = t.BN;
-    t.n_acc = 4 * acc_cols <= 512 ? 4 : 2;
     int cols = 32;
-    while (cols < t.n_acc * acc_cols) cols <<= 1;
+    while (cols < t.n_acc * acc_cols + (t.ta ? t.stages * 64 : 0)) cols <<= 1;
     t.tmem_cols = cols;
     const long total = m_tiles * t.n_tiles;
     if (total <= 0 || total > 0x7fffffffL) return OGLE_ERR_UNSUPPORTED;

@@ -292,7 +292,7 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     } else if (warp == 1 && leader) {
         // -------------------------------------------------------------- MMA issuer (leader block)
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             const uint32_t idesc_bf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             int s = 0;

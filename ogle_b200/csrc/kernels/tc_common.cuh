@@ -1,6 +1,7 @@
 // Device helpers shared by the tcgen05 kernels: mbarrier, TMA, UMMA descriptors.
 #pragma once
 #include <cuda.h>
+#include <cuda_bf16.h>
 
 #include "conv_args.cuh"
 
@@ -31,6 +32,7 @@ struct TcArgs {
     int ldc;
     int passes;               // 1 (TF32) or 3 (split mode: a TF32 pass + a BF16 pass of the cross terms)
     int stages;
+    int ta;                   // split mode with the A operands in tensor memory (64 columns per stage, after the accumulators)
     int tmem_cols;
     int n_acc;                // accumulator buffers in tensor memory (2 or 4)
     int total_tiles;          // m_tiles * n_tiles (persistent kernel)
@@ -163,6 +165,85 @@ __device__ __forceinline__ void umma_bf16_chunk(uint32_t tmem_d, uint64_t ad, ui
         "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, q;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, q;\n\t}"
         ::"r"(tmem_d), "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate_first) : "memory");
+}
+
+// The same two chunks with the A operand in tensor memory: lane = row, one 32-bit column per TF32 value (32 columns a
+// chunk, 8 per K step) or per pair of BF16 values (32 columns, 8 per K step).
+__device__ __forceinline__ void umma_tf32_chunk_ta(uint32_t tmem_d, uint32_t ta, uint64_t bd, uint32_t idesc,
+                                                   uint32_t accumulate_first) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.eq.b32 q, 0, 0;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.s64 b1, %2, 2;\n\t"
+        "add.u32 a2, %1, 16;\n\tadd.s64 b2, %2, 4;\n\t"
+        "add.u32 a3, %1, 24;\n\tadd.s64 b3, %2, 6;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [a1], b1, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [a2], b2, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [a3], b3, %3, q;\n\t}"
+        ::"r"(tmem_d), "r"(ta), "l"(bd), "r"(idesc), "r"(accumulate_first) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_chunk_ta(uint32_t tmem_d, uint32_t ta, uint64_t bd, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "setp.eq.b32 q, 0, 0;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.s64 b1, %2, 2;\n\t"
+        "add.u32 a2, %1, 16;\n\tadd.s64 b2, %2, 4;\n\t"
+        "add.u32 a3, %1, 24;\n\tadd.s64 b3, %2, 6;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, q;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, q;\n\t}"
+        ::"r"(tmem_d), "r"(ta), "l"(bd), "r"(idesc) : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
+// Operand split into tensor memory: one row (32 fp32 values, 128 bytes in the 128-byte swizzle at `row`, which is row
+// r of its tile) becomes the A operands of both passes in this thread's lane: columns 0..31 the TF32 values (low 13
+// mantissa bits cleared), 32..63 the BF16 pairs [bf16(a_hi) x 32 | bf16(a_lo) x 32]. Warp-collective; the caller
+// waits for the stores (tcgen05.wait::st).
+__device__ __forceinline__ void split_row_to_tmem(const float4* row, int r, uint32_t taddr) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        uint32_t hi[16], ph[8], pl[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 v = row[(half * 4 + q) ^ (r & 7)];
+            const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int l = 0; l < 4; ++l) hi[q * 4 + l] = __float_as_uint(f[l]) & 0xffffe000u;
+#pragma unroll
+            for (int l = 0; l < 4; l += 2) {
+                const float h0 = __uint_as_float(hi[q * 4 + l]), h1 = __uint_as_float(hi[q * 4 + l + 1]);
+                const __nv_bfloat162 a = __floats2bfloat162_rn(h0, h1), b = __floats2bfloat162_rn(f[l] - h0, f[l + 1] - h1);
+                ph[q * 2 + l / 2] = *reinterpret_cast<const uint32_t*>(&a);
+                pl[q * 2 + l / 2] = *reinterpret_cast<const uint32_t*>(&b);
+            }
+        }
+        tmem_st16(taddr + half * 16, hi);
+        tmem_st8(taddr + 32 + half * 8, ph);
+        tmem_st8(taddr + 48 + half * 8, pl);
+    }
+}
+
+// One lane of a converged warp, for the roles that a single thread plays. Chosen this way - not as lane 0 - the compiler
+// knows that exactly one thread runs the role and keeps addresses and descriptors in uniform registers, which is where
+// the tensor-core and copy instructions take them from: an MMA costs its issuer 10 cycles instead of 55.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
