@@ -37,6 +37,8 @@ int launch_tc_pair(tc::TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi
                    const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
                    cudaStream_t s);
 
+const int* tc_cluster_capacity();      // [k], 2 <= k <= 8: clusters of k blocks that can be resident at once
+
 __device__ int g_tc_error = 0;   // first error seen by any block (0 = none)
 
 int* error_flag_ptr() {
@@ -101,6 +103,45 @@ int pair_mode_override() {
 bool split_k_enabled() {
     static const bool v = [] { const char* e = getenv("OGLE_TC_SPLIT_K"); return !(e && e[0] == '0'); }();
     return v;
+}
+
+// Tile width and number of ranges of a reduction split inside a cluster, for launches whose tiles leave SMs idle. All
+// clusters have to fit the GPU at once (a block takes a whole SM; the GPU is asked how many clusters of a size fit), and
+// the model has to see a tenth less time than in one piece. Times in clocks: a chunk costs its multiplies, with a
+// floor for narrow tiles; a block its start, fill and drain; the cluster its barriers and the exchange of partial tiles.
+// n_tile, split: the caller's choice (0 = any). otherwise: the ranges that the launch would have in its other forms.
+// Where the caller leaves the number open, a split-mode result must not move by more than 8e-6 of its norm with it: sums
+// in tensor memory are truncated, and results in k and in `otherwise` ranges of a reduction over R elements differ by
+// 6e-9 * R * |1/k - 1/otherwise| (R = 512: 2.4e-6, R = 1500: 6.0e-6; the shorter ranges are the more exact).
+// 1000 x 1500 x 700 gemm: 32.8 -> 28.8 us with its packing pass; MobileNet-SSD, one frame: 374 -> 335 us.
+bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int split, int otherwise) {
+    if (!split_k_enabled() || t->gather || split == 1 || split > 8 || m_tiles > kNumSMs / 2) return false;
+    const int* capacity = tc_cluster_capacity();
+    const int kmax = (Kp + 31) / 32 * 32;
+    auto chunk = [&](int bn) {
+        const double c = t->passes == 3 ? 4.4 * bn : 2.2 * bn + 50.0, least = t->passes == 3 ? 600.0 : 350.0;
+        return c < least ? least : c;
+    };
+    const long tiles0 = m_tiles * t->n_tiles;
+    double best = otherwise > 1 || split ? 1e30 : 0.9 * ((tiles0 + kNumSMs - 1) / kNumSMs * (chunks * chunk(t->BN)) + 4000.0 + 14.0 * t->BN);
+    int best_bn = 0, best_k = 0;
+    for (int bn = n_tile ? n_tile : 32; bn <= (n_tile ? n_tile : 256) && bn <= kmax; bn += 32) {
+        const long tiles = m_tiles * ((Kp + bn - 1) / bn);
+        for (int k = split ? split : 2; k <= (split ? split : 8); ++k) {
+            const int cps = (chunks + k - 1) / k;
+            if ((k - 1) * cps >= chunks || tiles > capacity[k]) continue;
+            if (!split && t->passes == 3 && chunks * kChunk * fabs(1.0 / k - 1.0 / otherwise) > 1330.0) continue;
+            const double cost = cps * chunk(bn) + 5500.0 + 18.0 * bn;
+            if (cost < best) { best = cost; best_bn = bn; best_k = k; }
+        }
+    }
+    if (!best_k) return false;
+    t->BN = best_bn;
+    t->n_tiles = (Kp + best_bn - 1) / best_bn;
+    t->split_k = best_k;
+    t->ws_mode = 0;
+    t->cluster = 1;
+    return true;
 }
 
 // Whether a launch takes the channels-on-M form (conv_tc2_t.cu): at most 128 (stacked) output channels, an
@@ -349,6 +390,66 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     choose_n_tiling_v2(a.Kp, m_tiles, &t, a.n_tile,
                        (plan_only || (ws != nullptr && aligned16(ws))) && !t.gather && split_k_enabled() &&
                            taps * t.chunks_per_tap >= 16);
+    // Split the reduction when whole tiles would leave SMs idle (few tiles) or a last round
+    // mostly empty. Two forms, for reductions that do not fit clusters (below):
+    //  - through scratch memory (the caller lent some): any number of ranges and any activation;
+    //    each range stores its partial tile into its own slice and a small second kernel adds the
+    //    slices in slice order, then bias and activation - bit-reproducible whatever the order in
+    //    which blocks finish;
+    //  - in place, two ranges, no activation: the output (a dense tensor, or this convolution's
+    //    channel slice of a wider one) is zeroed first and the two partial tiles are added to it by
+    //    TMA reduce stores; a sum of two addends onto zero does not depend on their order either.
+    t.split_k = 1;
+    const int chunks = t.kernel * t.kernel * t.chunks_per_tap;
+    const double tiles = (double)m_tiles * t.n_tiles;
+    const int ws_cols = t.n_tiles * t.BN;
+    // rows (flat form) or images between consecutive slices: whole tiles, so that a tile that
+    // hangs over the end of its slice writes padding, not the next slice
+    const long slice_units = t.flat ? m_tiles * kTileM : (long)((a.N + t.tn - 1) / t.tn) * t.tn;
+    const size_t slice_bytes = (size_t)(t.flat ? slice_units : slice_units * a.Ho * a.Wo) * ws_cols * sizeof(float);
+    if (split_k_enabled() && chunks >= 8 && !residual) {      // (a residual operand is added by whole tiles only)
+        // cost of the layer in units of one reduction chunk of one tile: rounds of one work item per SM,
+        // each item paying its chunks plus a fixed fill / drain of about four chunks
+        auto cost_of = [&](int k) {
+            const int cps = (chunks + k - 1) / k;
+            return ceil(tiles * k / kNumSMs) * (cps + 4.0);
+        };
+        double best = cost_of(1);
+        int best_k = 1;
+        bool best_ws = false;
+        if (a.act == OGLE_ACT_NONE && chunks / 2 >= 8 && cost_of(2) + 2.0 < 0.9 * best) { best = cost_of(2) + 2.0; best_k = 2; }
+        const bool ws_usable = plan_only || (ws != nullptr && aligned16(ws));
+        if (ws_usable && !t.gather) {
+            static const int cand[] = {2, 3, 4, 6, 8, 12, 16};
+            for (int k : cand) {
+                if (chunks / k < 4) break;
+                if (!plan_only && slice_bytes * k > ws_bytes) break;
+                if (slice_bytes * k > ((size_t)192 << 20)) break;
+                // + the second kernel: a launch and a pass over k slices
+                const double c = cost_of(k) + 10.0 + 0.5 * k;
+                if (c < 0.85 * best) { best = c; best_k = k; best_ws = true; }
+            }
+        }
+        if (a.split >= 1) {
+            // the caller's choice, as far as it can be served: the in-place form for two ranges without an
+            // activation, else the scratch form when scratch of the right size was lent
+            int k = a.split;
+            while (k > 1 && chunks / k < 1) --k;
+            const bool fits = ws_usable && !t.gather && (plan_only || slice_bytes * k <= ws_bytes) &&
+                              slice_bytes * k <= ((size_t)192 << 20);
+            if (k == 1) { best_k = 1; best_ws = false; }
+            else if (k == 2 && a.act == OGLE_ACT_NONE && !fits) { best_k = 2; best_ws = false; }
+            else if (fits) { best_k = k; best_ws = true; }
+        }
+        t.split_k = best_k;
+        t.ws_mode = best_ws ? 1 : 0;
+        const int cps = (chunks + t.split_k - 1) / t.split_k;
+        while (t.split_k > 1 && (t.split_k - 1) * cps >= chunks) --t.split_k;     // no empty ranges
+        if (t.split_k == 1) t.ws_mode = 0;
+    }
+    // (the scratch a layer asks for does not depend on whether the launch then splits inside clusters instead)
+    if (!plan_only && !(a.on_m == 2 && t.ws_mode) && !want_channels_on_m(t, a.Kp, m_tiles, a.on_m) && !want_pair(t, m_tiles, a.pair))
+        choose_cluster(&t, a.Kp, m_tiles, chunks, a.n_tile, a.split, t.split_k);
     const int Kp128 = (a.K + 127) / 128 * 128;
     const cuuint64_t bcols = t.gather ? (cuuint64_t)t.Cp32 : (cuuint64_t)taps * t.Cp32;
     const cuuint64_t bdims[2] = {bcols, (cuuint64_t)Kp128};
@@ -357,64 +458,14 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     const cuuint32_t bes[2] = {1, 1};
     if (!make_map(&mBhi, w_hi, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
     if (!make_map(&mBlo, w_lo, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
+    if (t.cluster) {
+        t.res = residual;
+        t.res_ld = res_ld;
+        t.y = y + a.koff; t.y_ld = ks_a;
+        t.y2 = y2; t.y2_ld = kp_b;
+        return launch_tc_v2(t, mA, mBhi, mBlo, mY, y2 ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
+    }
     if (v2) {
-        // Split the reduction when whole tiles would leave SMs idle (few tiles) or a last round
-        // mostly empty. Two forms:
-        //  - through scratch memory (the caller lent some): any number of ranges and any activation;
-        //    each range stores its partial tile into its own slice and a small second kernel adds the
-        //    slices in slice order, then bias and activation - bit-reproducible whatever the order in
-        //    which blocks finish;
-        //  - in place, two ranges, no activation: the output (a dense tensor, or this convolution's
-        //    channel slice of a wider one) is zeroed first and the two partial tiles are added to it by
-        //    TMA reduce stores; a sum of two addends onto zero does not depend on their order either.
-        t.split_k = 1;
-        const int chunks = t.kernel * t.kernel * t.chunks_per_tap;
-        const double tiles = (double)m_tiles * t.n_tiles;
-        const int ws_cols = t.n_tiles * t.BN;
-        // rows (flat form) or images between consecutive slices: whole tiles, so that a tile that
-        // hangs over the end of its slice writes padding, not the next slice
-        const long slice_units = t.flat ? m_tiles * kTileM : (long)((a.N + t.tn - 1) / t.tn) * t.tn;
-        const size_t slice_bytes = (size_t)(t.flat ? slice_units : slice_units * a.Ho * a.Wo) * ws_cols * sizeof(float);
-        if (split_k_enabled() && chunks >= 8 && !residual) {      // (a residual operand is added by whole tiles only)
-            // cost of the layer in units of one reduction chunk of one tile: rounds of one work item per SM,
-            // each item paying its chunks plus a fixed fill / drain of about four chunks
-            auto cost_of = [&](int k) {
-                const int cps = (chunks + k - 1) / k;
-                return ceil(tiles * k / kNumSMs) * (cps + 4.0);
-            };
-            double best = cost_of(1);
-            int best_k = 1;
-            bool best_ws = false;
-            if (a.act == OGLE_ACT_NONE && chunks / 2 >= 8 && cost_of(2) + 2.0 < 0.9 * best) { best = cost_of(2) + 2.0; best_k = 2; }
-            const bool ws_usable = plan_only || (ws != nullptr && aligned16(ws));
-            if (ws_usable && !t.gather) {
-                static const int cand[] = {2, 3, 4, 6, 8, 12, 16};
-                for (int k : cand) {
-                    if (chunks / k < 4) break;
-                    if (!plan_only && slice_bytes * k > ws_bytes) break;
-                    if (slice_bytes * k > ((size_t)192 << 20)) break;
-                    // + the second kernel: a launch and a pass over k slices
-                    const double c = cost_of(k) + 10.0 + 0.5 * k;
-                    if (c < 0.85 * best) { best = c; best_k = k; best_ws = true; }
-                }
-            }
-            if (a.split >= 1) {
-                // the caller's choice, as far as it can be served: the in-place form for two ranges without an
-                // activation, else the scratch form when scratch of the right size was lent
-                int k = a.split;
-                while (k > 1 && chunks / k < 1) --k;
-                const bool fits = ws_usable && !t.gather && (plan_only || slice_bytes * k <= ws_bytes) &&
-                                  slice_bytes * k <= ((size_t)192 << 20);
-                if (k == 1) { best_k = 1; best_ws = false; }
-                else if (k == 2 && a.act == OGLE_ACT_NONE && !fits) { best_k = 2; best_ws = false; }
-                else if (fits) { best_k = k; best_ws = true; }
-            }
-            t.split_k = best_k;
-            t.ws_mode = best_ws ? 1 : 0;
-            const int cps = (chunks + t.split_k - 1) / t.split_k;
-            while (t.split_k > 1 && (t.split_k - 1) * cps >= chunks) --t.split_k;     // no empty ranges
-            if (t.split_k == 1) t.ws_mode = 0;
-        }
         if (plan_only) {
             *ws_needed = t.ws_mode ? slice_bytes * t.split_k : 0;
             return OGLE_OK;
@@ -519,6 +570,8 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
     const bool v2 = true;
     const long m_tiles = (p.M + kTileM - 1) / kTileM;
     choose_n_tiling_v2(t.Kp, m_tiles, &t);
+    choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 0, 1);
+    t.y = Y; t.y_ld = p.ldy;
     CUtensorMap mA, mBhi, mBlo, mY;
     const cuuint64_t dims[4] = {(cuuint64_t)p.K, (cuuint64_t)p.M, 1, 1};
     const cuuint64_t str[3] = {(cuuint64_t)p.lda * 4, (cuuint64_t)p.lda * 4 * (cuuint64_t)p.M, (cuuint64_t)p.lda * 4 * (cuuint64_t)p.M};

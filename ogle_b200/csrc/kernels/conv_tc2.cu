@@ -53,6 +53,7 @@ using namespace tc;
 
 constexpr int kThreads2 = 608;
 constexpr int kMaxStages = 8;
+constexpr int kTcSmem = 224 * 1024;           // a block always takes the whole of it: it then has its SM to itself
 constexpr int kStagingBytes = kTileM * 128;   // one 128-row x 32-column fp32 slab
 
 // Bounded wait of a role for its turn; also gives up early when another role of the block has
@@ -112,11 +113,17 @@ __device__ __forceinline__ TileCoord tile_coord(const TcArgs& a, int tile) {
 
 struct WorkItem { int tile, ks, c_begin, c_end; };
 
-// kSplit is a compile-time switch so that the common, unsplit kernel carries none of this
-template <bool kSplit>
+// Compile-time form of the kernel, so that the common, unsplit one carries nothing of the others.
+enum TcForm {
+    kWhole = 0,       // a work item is a tile
+    kRanges = 1,      // a range of a tile's reduction, combined through scratch or by reduce-add stores
+    kCluster = 2      // a range of a tile's reduction; the blocks of a cluster hold one tile's ranges and add them up
+};
+
+template <TcForm kForm>
 __device__ __forceinline__ WorkItem work_item(const TcArgs& a, int w, int chunks) {
     WorkItem it;
-    if (!kSplit) {
+    if (kForm == kWhole) {
         it.tile = w; it.ks = 0; it.c_begin = 0; it.c_end = chunks;
     } else {
         it.tile = w / a.split_k;
@@ -132,13 +139,82 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, uint32
                  ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
 
-template <bool kSplit>
+// A float4 of another block's shared memory (addr: the same variable's address in this block).
+__device__ __forceinline__ float4 load_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Cluster form: this block's band of the tile's rows, summed over the partial tiles of the cluster in rank order (the
+// order the slices of the scratch form are added in: the same bits), then bias, residual operand and activation, and
+// plain coalesced stores. The band's columns are dealt out as float4s, a row's neighbours to neighbouring threads.
+__device__ __forceinline__ void cluster_reduce(const TcArgs& a, uint32_t partial, const float* __restrict__ bias) {
+    const int ranks = a.split_k, tile = (int)blockIdx.x / ranks, rank = (int)blockIdx.x - tile * ranks;
+    const TileCoord tc_ = tile_coord(a, tile);
+    const int nbase = tc_.n_tile * a.BN;
+    const int rows = a.flat ? kTileM : a.tn * a.th * a.tw;
+    const int r0 = rows * rank / ranks, r1 = rows * (rank + 1) / ranks;
+    const int quads = (a.Kp - nbase < a.BN ? a.Kp - nbase : a.BN) >> 2;
+    for (int i = threadIdx.x; i < (r1 - r0) * quads; i += kThreads2) {
+        const int row = r0 + i / quads, q = i % quads;
+        long pixel;
+        if (a.flat) {
+            pixel = (long)tc_.w0 + row;
+            if (pixel >= a.Wo) continue;
+        } else {
+            const int rw = row % a.tw, t2 = row / a.tw;
+            const int n = tc_.n0 + t2 / a.th, h = tc_.h0 + t2 % a.th, w = tc_.w0 + rw;
+            if (n >= a.N || h >= a.Ho || w >= a.Wo) continue;
+            pixel = ((long)n * a.Ho + h) * a.Wo + w;
+        }
+        const int col = nbase + q * 4;                     // stacked column
+        const bool second = a.split_col > 0 && col >= a.split_col;
+        const int lcol = second ? col - a.split_col : col;
+        const int real = second ? a.K - a.split_col : (a.split_col > 0 ? a.K1 : a.K);
+        if (lcol >= real) continue;                        // between the two outputs
+        const uint32_t at = partial + (uint32_t)((q >> 3) * kStagingBytes + row * 128 + (((q & 7) ^ (row & 7)) << 4));
+        float4 part[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+            if (p < ranks) part[p] = load_cluster(at, (uint32_t)p);
+        float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+        for (int p = 1; p < 8; ++p)
+            if (p < ranks) { v[0] += part[p].x; v[1] += part[p].y; v[2] += part[p].z; v[3] += part[p].w; }
+        float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.res) res = __ldg(reinterpret_cast<const float4*>(a.res + pixel * a.res_ld + lcol));
+        const float rr[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (lcol + l < real) {
+                if (a.bias_mode == 1) v[l] = fmaf(a.beta, __ldg(bias + pixel * a.ldc + lcol + l), a.alpha * v[l]);
+                else v[l] = fmaf(a.alpha, v[l], a.bias_mode == 2 ? a.beta * __ldg(bias + col + l) : 0.f);
+                if (a.res) v[l] += rr[l];
+                v[l] = apply_act(v[l], a.act, a.lo, a.hi);
+            } else {
+                v[l] = 0.f;                                // padded lanes stay zero
+            }
+        }
+        float* y = second ? a.y2 + pixel * a.y2_ld : a.y + pixel * a.y_ld;
+        *reinterpret_cast<float4*>(y + lcol) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+template <TcForm kForm>
 __global__ void __launch_bounds__(kThreads2, 1)
 conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBhi,
                 const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmY,
                 const __grid_constant__ CUtensorMap tmY2, const float* __restrict__ bias, const TcArgs a, int* err_flag) {
     // 1024-byte alignment (the 128-byte swizzle atom) comes from the declaration, so that
     // every byte of the 224 KB request is usable
+    constexpr bool kSplit = kForm != kWhole;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_xf[kMaxStages], bar_empty[kMaxStages];
     __shared__ __align__(8) uint64_t bar_acc_full[4], bar_acc_empty[4];
@@ -241,7 +317,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int issued = 0;            // chunks in flight bookkeeping for the abort path
             bool ok = true;
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord(a, wi.tile);
                 const int ax = a.flat ? tc_.w0 : tc_.w0 * a.stride - a.pad;
                 const int ay = a.flat ? 0 : tc_.h0 * a.stride - a.pad;
@@ -282,7 +358,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int issued = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const int bcol = (wi.tile % a.n_tiles) * a.BN;
                 int brow = wi.c_begin * kChunk;
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
@@ -310,7 +386,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             bool ok = true;
             int ti = 0;
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
                 if (use > 0) ok = wait_or_abort(&bar_acc_empty[as], (uint32_t)((use - 1) & 1), abort_flag, a.spin_limit);
                 if (!ok) { record_error(err_flag, 5); s_abort = 1; break; }
@@ -371,7 +447,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             uint32_t ph = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     // Every stage is waited for in turn, also those of the other group's chunks: copies land out of
                     // order, and a group that only looked at every second chunk could, in a ring of three or five
@@ -411,7 +487,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     ok = wait_or_abort(&bar_full[s], ph, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 3); s_abort = 1; break; }
@@ -479,6 +555,25 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
         }
+    } else if constexpr (kForm == kCluster) {
+        // ------------------------------------------------------------ partial tile
+        // One work item per block: its raw sums go to the operand ring, which the last multiply has left, slab by slab
+        // in the swizzle of the staging slabs; both groups take part.
+        const int row = (warp & 3) * 32 + lane;
+        bool ok = wait_or_abort(&bar_acc_full[0], 0u, abort_flag, a.spin_limit);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) { record_error(err_flag, 4); s_abort = 1; }
+        else {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int g = (warp - 2) >> 2; g < a.BN / 32; g += 2) {
+                uint32_t r[32];
+                tmem_ld32(r, tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 32));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                uint4* dst = reinterpret_cast<uint4*>(base_ptr + (size_t)g * kStagingBytes + (size_t)row * 128);
+#pragma unroll
+                for (int c4 = 0; c4 < 8; ++c4) dst[c4 ^ (row & 7)] = make_uint4(r[c4 * 4], r[c4 * 4 + 1], r[c4 * 4 + 2], r[c4 * 4 + 3]);
+            }
+        }
     } else {
         // ------------------------------------------------------------------ epilogue
         const int eg = (warp - 2) >> 2;               // group 0 or 1
@@ -497,7 +592,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int round_no = 0;          // rounds of this group so far (selects the staging slab)
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
                 if (ti % a.epi_groups != eg) continue;
-                const WorkItem wi = work_item<kSplit>(a, w, chunks);
+                const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord(a, wi.tile);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
                 const int nbase = tc_.n_tile * a.BN;
@@ -672,6 +767,15 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)a.tmem_cols));
     }
+    if constexpr (kForm == kCluster) {
+        // Every block of the cluster gets here, also one that gave up (its sums are then meaningless, and the status
+        // word says so); none leaves while another may still read its partial tile.
+        __syncwarp();
+        cluster_sync();
+        cluster_reduce(a, base, bias);
+        __syncwarp();
+        cluster_sync();
+    }
 }
 
 int num_sms() {
@@ -688,6 +792,38 @@ int num_sms() {
 }
 
 }  // namespace
+
+// [k]: how many clusters of k blocks can be resident at once (a block has its SM to itself): the GPU's own answer,
+// asked once per thread and device. 0 = such clusters cannot run.
+const int* tc_cluster_capacity() {
+    static thread_local int device = -1, known[9];
+    static const int none[9] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return none;
+    if (device != dev) {
+        if (cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return none;
+        }
+        for (int b = 2; b <= 8; ++b) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)b);
+            cfg.blockDim = dim3(kThreads2);
+            cfg.dynamicSmemBytes = kTcSmem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)b; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&known[b], conv_tc2_kernel<kCluster>, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                known[b] = 0;
+            }
+        }
+        device = dev;
+    }
+    return known;
+}
 
 int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, const CUtensorMap& mBlo,
                  const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
@@ -708,7 +844,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     // Shared memory is split between the operand ring and the epilogue's staging slabs
     // (128 rows x 32 columns each). Preference: two epilogue groups with two slabs each;
     // give slabs back to the ring while that buys another stage and the ring is shallow.
-    const size_t kBudget = 224 * 1024;
+    const size_t kBudget = kTcSmem;
     const int chunks = t.kernel * t.kernel * t.chunks_per_tap;
     t.xf_groups = (t.passes == 3 || t.gather) ? 2 : 1;   // both operand-split groups work on each chunk
     t.epi_groups = 2;
@@ -729,6 +865,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     if (t.gather) t.xf_groups = 2;        // the gather code is laid out for 256 threads
     if (const char* e = getenv("OGLE_TC_EPI_GROUPS")) t.epi_groups = e[0] == '1' ? 1 : 2;
     if (const char* e = getenv("OGLE_TC_EPI_SLABS")) t.epi_slabs = e[0] == '1' ? 1 : 2;
+    if (t.cluster) t.epi_slabs = 0;       // partial tiles go where the operand ring was
     const size_t staging = (size_t)t.epi_groups * t.epi_slabs * kStagingBytes;
     const size_t budget = kBudget - staging;
     int stages = (int)(budget / stage);
@@ -747,6 +884,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     if (total * t.split_k > 0x7fffffffL) return OGLE_ERR_UNSUPPORTED;
     t.total_work = (int)(total * t.split_k);
     t.chunks_per_split = (chunks + t.split_k - 1) / t.split_k;
+    if (t.cluster && (t.split_k < 2 || t.split_k > 8 || (size_t)t.BN * 512 > kBudget)) return OGLE_ERR_UNSUPPORTED;
     // Always the whole budget, also when the layout needs less: a block then has its SM to
     // itself whatever else is running, so its tensor-memory allocation can never wait for
     // another resident block's columns.
@@ -756,17 +894,36 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kRanges>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
     }
     const int sms = num_sms();
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
+    if (t.cluster) {
+        // every block one work item; the blocks of a tile are consecutive, and a cluster
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)t.total_work);
+        cfg.blockDim = dim3(kThreads2);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = overlapped_launches_enabled() ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)t.split_k; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc2_kernel<kCluster>, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+        if (e != cudaSuccess) { set_last_error(e); (void)cudaGetLastError(); return OGLE_ERR_CUDA; }
+        return finish_launch();
+    }
     if (t.split_k > 1)
-        launch_overlapped(conv_tc2_kernel<true>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+        launch_overlapped(conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else
-        launch_overlapped(conv_tc2_kernel<false>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+        launch_overlapped(conv_tc2_kernel<kWhole>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     return finish_launch();
 }
 

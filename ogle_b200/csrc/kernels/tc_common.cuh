@@ -54,6 +54,13 @@ struct TcArgs {
     // a second, small kernel adds the slices in a fixed order, then bias and activation. Results do not
     // depend on which block finishes first.
     int ws_mode, ws_cols, ws_slice;
+    // Split reduction inside a cluster (cluster = 1): the split_k <= 8 blocks of a cluster hold one tile's ranges, leave
+    // their partial tiles in shared memory and each adds up and stores a band of the tile's rows: one launch, no
+    // scratch, any activation, a residual operand. Stores go straight to y (first channel; y_ld floats a pixel) and,
+    // with two outputs, y2.
+    int cluster;
+    float *y, *y2;
+    int y_ld, y2_ld;
     // Gather form (k x k convolution over at most four input channels, e.g. an RGB stem): the
     // activation "tile" that TMA delivers is the tile's input window of 16-byte pixels
     // (g_iw x g_ih of them, halo included), once per reduction chunk; the operand-split warps
@@ -62,7 +69,7 @@ struct TcArgs {
     // (chunks_per_tap chunks; kernel = 1 in this form). g_C = input channels, g_k = filter
     // size, g_bytes = window bytes rounded up to 1 KB (its slot at the end of every stage).
     int gather, g_iw, g_ih, g_C, g_bytes, g_k;
-    // Residual operand (one-SM form, unsplit reduction): res[pixel * res_ld + channel] is added to the
+    // Residual operand (one-SM form, reduction unsplit or split inside a cluster): res[pixel * res_ld + channel] is added to the
     // convolution's value (after the bias, before the activation) - a residual block's Add and activation in
     // the convolution's own pass. Null = none.
     const float* res;

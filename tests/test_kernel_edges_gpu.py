@@ -139,3 +139,63 @@ def test_fp32_gemm_edges(oracle_port, m, k, n, trans_b):
     Cm = rng.standard_normal((m, n), dtype=np.float32)
     got = run_case_cuda(dict(op="gemm", A=A, B=B, Cm=Cm, transB=trans_b, alpha=0.5, beta=2.0))
     close(got, oracle_port.gemm(A, B, Cm, trans_b, 0.5, 2.0))
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride, pad, act, split: one tile over 2-8 blocks, ranges of unequal length, rows and columns
+    # that end inside a tile, several tiles, three tile widths
+    (1, 7, 7, 512, 30, 3, 1, 1, 0, 8), (1, 9, 11, 100, 129, 3, 2, 1, 2, 3), (2, 19, 19, 256, 75, 3, 1, 1, 1, 5), (1, 1, 1, 96, 4, 1, 1, 0, 2, 3),
+    (3, 20, 17, 64, 510, 1, 1, 0, 2, 2), (1, 40, 150, 48, 33, 5, 1, 2, 0, 7), (5, 3, 3, 160, 257, 1, 1, 0, 0, 4)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_reduction_split_inside_a_cluster(oracle_port, shape, math):
+    """Into a channel slice of a wider tensor, alone and with a residual operand; the same sums on every call."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K, k, s, pd, act, split = shape
+    rng = np.random.default_rng(C + K)
+    x = rng.standard_normal((N, H, W, C), dtype=np.float32)
+    w = (rng.standard_normal((K, C, k, k)) / np.sqrt(C * k * k)).astype(np.float32)
+    b = rng.standard_normal(K, dtype=np.float32)
+    p = ops.conv_params(N, H, W, C, K, k, s, pd, 1, 1, True, act, -0.5, 1.5, getattr(ops, math))
+    p.split = split
+    packed = ops.conv2d_prepack(p, ops.dense_to_device(w))
+    x4, b4 = ops.upload(x), ops.dense_to_device(b)
+    if act != 1:
+        res = rng.standard_normal((N,) + tuple(p.out_hwc), dtype=np.float32)
+        fused = ops.conv2d_residual(p, x4, packed, b4, ops.upload(res))
+    p.out_channel_stride, p.out_channel_offset = ops.up4(K) + 8, 4
+    outs = [torch.full((N, p.out_hwc[0], p.out_hwc[1], ops.up4(K) + 8), -7.0, device="cuda") for _ in range(2)]
+    for out in outs:
+        ops.conv2d(p, x4, packed, b4, out, workspace=None)
+    assert torch.equal(outs[0], outs[1])
+    got = outs[0].cpu().numpy()
+    assert (got[..., :4] == -7).all() and (got[..., 4 + ops.up4(K):] == -7).all() and (got[..., 4 + K:4 + ops.up4(K)] == 0).all()
+    # fp32-grade products and sums, or operands of ten mantissa bits (2^-11 relative each) over the reduction
+    tol = 3e-5 if math == "MATH_TF32X3" else 6e-3
+    ref = oracle_port.conv2d(x, w, b, s, pd, 1, 1, act, -0.5, 1.5)
+    assert np.abs(got[..., 4:4 + K] - ref).max() <= tol * max(1.0, np.abs(ref).max())
+    if act != 1:
+        plain = oracle_port.conv2d(x, w, b, s, pd, 1, 1, 0, 0.0, 0.0) + res
+        want = np.maximum(plain, 0) if act == 2 else plain
+        assert np.abs(ops.download(fused, K) - want).max() <= tol * np.abs(plain).max()
+
+
+@pytest.mark.parametrize("m,k,n,bias_mode", [(1, 512, 1000, 2), (1, 130, 10, 0), (129, 1500, 700, 1), (300, 4096, 33, 2), (1000, 1500, 700, 2)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_gemm_over_clusters(m, k, n, bias_mode, math):
+    """Launches of few tiles, whose reductions split over clusters: vector and matrix bias, odd sizes, against 64 bits."""
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator().manual_seed(m + k)
+    a, b = torch.randn((m, k), generator=g), torch.randn((n, k), generator=g)
+    c = torch.randn((n,) if bias_mode == 2 else (m, n), generator=g)
+    c4 = None if bias_mode == 0 else torch.nn.functional.pad(c, (0, ops.up4(n) - n)).cuda()
+    pad = lambda t: torch.nn.functional.pad(t, (0, ops.up4(k) - k)).cuda()
+    mode = getattr(ops, math)
+    got = ops.gemm_ws(pad(a), pad(b), c4, m, k, n, 1, 0.5, 2.0 if bias_mode else 0.0, bias_mode, mode)
+    want = 0.5 * (a.double() @ b.double().t()) + (2.0 * c.double() if bias_mode else 0.0)
+    err = (got[:, :n].cpu().double() - want).norm() / want.norm()
+    # k/8 + k/16 truncated additions to a sum, each off by at most 2^-23 of it, 2^-24 on average: k * 1.1e-8 in an
+    # unsplit reduction, less in a split one; in one-pass mode 2^-11 per operand
+    assert err <= (1.2e-8 * k + 2e-6 if mode == ops.MATH_TF32X3 else 2e-3)
+    assert (got[:, n:] == 0).all()
