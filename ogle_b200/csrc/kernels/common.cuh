@@ -56,8 +56,8 @@ bool overlapped_launches_enabled();
 void set_overlapped_launches(int on);
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                     Args&&... args) {
+inline cudaError_t launch_overlapped_if(bool overlapped, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -65,10 +65,16 @@ inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 b
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = overlapped_launches_enabled() ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = overlapped ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                     Args&&... args) {
+    return launch_overlapped_if(overlapped_launches_enabled(), kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 
 __device__ __forceinline__ float apply_act(float v, int act, float lo, float hi) {

@@ -113,7 +113,7 @@ bool split_k_enabled() {
 // Where the caller leaves the number open, a split-mode result must not move by more than 8e-6 of its norm with it: sums
 // in tensor memory are truncated, and results in k and in `otherwise` ranges of a reduction over R elements differ by
 // 6e-9 * R * |1/k - 1/otherwise| (R = 512: 2.4e-6, R = 1500: 6.0e-6; the shorter ranges are the more exact).
-// 1000 x 1500 x 700 gemm: 32.8 -> 28.8 us with its packing pass; MobileNet-SSD, one frame: 374 -> 335 us.
+// 1000 x 1500 x 700 gemm: 32.8 -> 28.8 us with its packing pass (24.6 with that pass as it is now); MobileNet-SSD, one frame: 374 -> 335 us.
 bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int split, int otherwise) {
     if (!split_k_enabled() || t->gather || split == 1 || split > 8 || m_tiles > kNumSMs / 2) return false;
     const int* capacity = tc_cluster_capacity();
@@ -557,8 +557,10 @@ bool gemm_tc_supported(const OgleGemmParams& p, const float* A, const float* B) 
 }
 
 static int launch_gemm_common(const OgleGemmParams& p, const float* A, const float* Bhi, const float* Blo,
-                              long b_row_stride, long b_rows, const float* C, float* Y, cudaStream_t s, int passes) {
+                              long b_row_stride, long b_rows, const float* C, float* Y, cudaStream_t s, int passes,
+                              bool overlapped = false) {
     TcArgs t = {};
+    t.overlapped = overlapped;
     t.flat = 1; t.N = 1; t.Ho = 1; t.Wo = p.M; t.tn = 1; t.th = 1; t.tw = kTileM;
     t.kernel = 1; t.stride = 1; t.pad = 0; t.dil = 1;
     t.Cp32 = (p.K + 31) / 32 * 32;
@@ -598,10 +600,10 @@ int launch_gemm_tc(const OgleGemmParams& p, const float* A, const float* B, cons
 }
 
 int launch_gemm_tc_packed(const OgleGemmParams& p, const float* A, const float* Bhi, const float* Blo,
-                          const float* C, float* Y, cudaStream_t s) {
+                          const float* C, float* Y, cudaStream_t s, bool overlapped) {
     const long Cp32 = (p.K + 31) / 32 * 32;
     const long rows = (p.N + 127) / 128 * 128;
-    return launch_gemm_common(p, A, Bhi, Blo, Cp32, rows, C, Y, s, p.math_mode == OGLE_MATH_TF32X3 ? 3 : 1);
+    return launch_gemm_common(p, A, Bhi, Blo, Cp32, rows, C, Y, s, p.math_mode == OGLE_MATH_TF32X3 ? 3 : 1, overlapped);
 }
 
 namespace {

@@ -902,6 +902,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     }
     const int sms = num_sms();
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
+    const bool overlapped = t.overlapped || overlapped_launches_enabled();
     if (t.cluster) {
         // every block one work item; the blocks of a tile are consecutive, and a cluster
         cudaLaunchConfig_t cfg = {};
@@ -911,7 +912,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         cfg.stream = s;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = overlapped_launches_enabled() ? 1 : 0;
+        attr[0].val.programmaticStreamSerializationAllowed = overlapped ? 1 : 0;
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = (unsigned)t.split_k; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
@@ -921,9 +922,9 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         return finish_launch();
     }
     if (t.split_k > 1)
-        launch_overlapped(conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else
-        launch_overlapped(conv_tc2_kernel<kWhole>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kWhole>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     return finish_launch();
 }
 

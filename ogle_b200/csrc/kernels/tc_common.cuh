@@ -74,6 +74,7 @@ struct TcArgs {
     // the convolution's own pass. Null = none.
     const float* res;
     int res_ld;
+    int overlapped;           // this launch may start its set-up while the launch before it - the library's own - still runs
     uint32_t spin_limit;      // polls a role waits for its turn before it gives up (kSpinLimit by default)
 };
 
