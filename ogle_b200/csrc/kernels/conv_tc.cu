@@ -85,8 +85,8 @@ void choose_n_tiling_v2(int Kp, long m_tiles, TcArgs* t, int requested = 0, bool
         // narrower one when everything fits in one round (more SMs busy, shorter epilogues)
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && (rounds > 1 || wide_ties))) { best_cost = cost; best_bn = bn; }
     }
-    if (const char* e = getenv("OGLE_TC_BN")) {      // experiments: force the tile width
-        const int v = atoi(e);
+    static const int forced = [] { const char* e = getenv("OGLE_TC_BN"); return e ? atoi(e) : 0; }();      // experiments
+    if (const int v = forced) {
         if (v >= 32 && v <= 256 && v % 32 == 0 && v <= kmax) best_bn = v;
     }
     if (requested >= 32 && requested <= 256 && requested % 32 == 0 && requested <= kmax) best_bn = requested;
@@ -105,10 +105,78 @@ bool split_k_enabled() {
     return v;
 }
 
+// Time of one reduction chunk (us) of an unsplit split-mode tile of 32, 64, ... columns on operands that come from L2:
+// up to 160 columns the activation operands go through tensor memory, wider tiles build them in shared memory.
+// On SM pairs: a chunk of both blocks' tiles. (148 tiles of one kind, 3x3, 18 and 36 chunks.)
+constexpr double kChunkUs[8] = {0.355, 0.355, 0.355, 0.386, 0.48, 0.725, 0.81, 0.84};
+constexpr double kPairChunkUs[4] = {0.65, 0.675, 0.70, 0.71};
+// ... and of an epilogue, per column: in the shadow of the next tile's multiplies (two groups), and at the end.
+constexpr double kEpilogueUs = 0.018, kTailUs = 0.035;
+
+// Width and form of an unsplit split-mode launch (the sums of an output value are the same in all of them): rounds of
+// tiles times the measured time of a tile; pointwise layers, whose tiles are read once, wait more for L2. true: on SM
+// pairs. 250 columns, 1350 elements, 14335 pixels: one tile of 256 columns 53.9 us, pairs 44.1, two tiles of 128 45.5;
+// 512 -> 1024 pointwise, 25600 pixels: 118, 88, 95.
+bool refine_width(TcArgs* t, int Kp, long m_tiles, int chunks, bool may_pair) {
+    if (t->passes != 3 || t->gather || chunks < 8) return false;      // (short reductions are bound by HBM and the epilogue)
+    const int kmax = (Kp + 31) / 32 * 32;
+    auto one = [&](int bn) {
+        const long tiles = m_tiles * ((Kp + bn - 1) / bn);
+        const double mul = chunks * kChunkUs[bn / 32 - 1] * (t->flat ? 1.25 : 1.0), epi = kEpilogueUs * bn;
+        return (double)((tiles + kNumSMs - 1) / kNumSMs) * (mul > epi ? mul : epi) + 4.5 + kTailUs * bn;
+    };
+    auto pair = [&](int bn) {
+        const long work = (m_tiles + 1) / 2 * ((Kp + bn - 1) / bn);
+        const double mul = chunks * kPairChunkUs[bn / 64 - 1] * (t->flat ? 1.1 : 1.0), epi = kEpilogueUs * bn;
+        return (double)((work + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (mul > epi ? mul : epi) + 5.5 + kTailUs * bn;
+    };
+    double best = 0.97 * one(t->BN);
+    int best_bn = t->BN;
+    bool best_pair = false;
+    for (int bn = 32; bn <= 256 && bn <= kmax; bn += 32) {
+        if (one(bn) < best) { best = one(bn); best_bn = bn; best_pair = false; }
+        if (may_pair && m_tiles >= 2 && bn % 64 == 0 && pair(bn) < best) { best = pair(bn); best_bn = bn; best_pair = true; }
+    }
+    t->BN = best_bn;
+    t->n_tiles = (Kp + best_bn - 1) / best_bn;
+    return best_pair;
+}
+
+// Tiles of a k x k layer cut along the width too: a map 75 pixels wide fills 75 of a tile's 128 rows in whole rows, and
+// 114 in pieces of 38 x 3. Replaces the tile in t where that saves rounds (or, below one round, tiles); the sums of an
+// output value do not change. 4 x 75 x 75 x 128 -> 256, 3x3: 103 -> 74 us (51 with tiles of 128 columns). cols: tiles
+// along the output channels.
+void cut_tiles(const ConvArgs& a, long cols, TcArgs* t, long* m_tiles) {
+    auto cost = [&](long tiles) {
+        tiles *= cols;
+        return tiles > kNumSMs ? (double)((tiles + kNumSMs - 1) / kNumSMs) : 0.6 + 0.4 * tiles / kNumSMs;
+    };
+    double best = 0.92 * cost(*m_tiles);
+    int best_parts = 0;
+    for (int parts = (a.Wo + kTileM - 1) / kTileM; parts <= 16; ++parts) {
+        const int tw = (a.Wo + parts - 1) / parts;
+        if (tw < 8) break;
+        if ((tw - 1) * a.stride + 1 > 256) continue;               // TMA box limit
+        for (int th = 1; th <= a.Ho && th * tw <= kTileM && (th - 1) * a.stride + 1 <= 256; ++th) {
+            int tn = kTileM / (th * tw);
+            if (tn > a.N) tn = a.N;
+            const long tiles_w = (a.Wo + tw - 1) / tw, tiles_h = (a.Ho + th - 1) / th;
+            const long tiles = tiles_w * tiles_h * ((a.N + tn - 1) / tn);
+            const double c = cost(tiles);
+            if (c < (best_parts && parts != best_parts ? 0.97 * best : best) || (parts == best_parts && c == best)) {
+                best = c; best_parts = parts;                     // (among equals of a width the tallest)
+                t->tw = tw; t->th = th; t->tn = tn;
+                t->tiles_w = (int)tiles_w; t->tiles_h = (int)tiles_h;
+                *m_tiles = tiles;
+            }
+        }
+    }
+}
+
 // Tile width and number of ranges of a reduction split inside a cluster, for launches whose tiles leave SMs idle. All
 // clusters have to fit the GPU at once (a block takes a whole SM; the GPU is asked how many clusters of a size fit), and
-// the model has to see a tenth less time than in one piece. Times in clocks: a chunk costs its multiplies, with a
-// floor for narrow tiles; a block its start, fill and drain; the cluster its barriers and the exchange of partial tiles.
+// the model has to see a tenth less time than in one piece: rounds of chunks, a block's start, fill and drain, and the
+// cluster's barriers and exchange of partial tiles.
 // n_tile, split: the caller's choice (0 = any). otherwise: the ranges that the launch would have in its other forms.
 // Where the caller leaves the number open, a split-mode result must not move by more than 8e-6 of its norm with it: sums
 // in tensor memory are truncated, and results in k and in `otherwise` ranges of a reduction over R elements differ by
@@ -118,12 +186,9 @@ bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int
     if (!split_k_enabled() || t->gather || split == 1 || split > 8 || m_tiles > kNumSMs / 2) return false;
     const int* capacity = tc_cluster_capacity();
     const int kmax = (Kp + 31) / 32 * 32;
-    auto chunk = [&](int bn) {
-        const double c = t->passes == 3 ? 4.4 * bn : 2.2 * bn + 50.0, least = t->passes == 3 ? 600.0 : 350.0;
-        return c < least ? least : c;
-    };
+    auto chunk = [&](int bn) { return t->passes == 3 ? kChunkUs[bn / 32 - 1] : 0.26 + 0.0002 * bn; };
     const long tiles0 = m_tiles * t->n_tiles;
-    double best = otherwise > 1 || split ? 1e30 : 0.9 * ((tiles0 + kNumSMs - 1) / kNumSMs * (chunks * chunk(t->BN)) + 4000.0 + 14.0 * t->BN);
+    double best = otherwise > 1 || split ? 1e30 : 0.9 * ((tiles0 + kNumSMs - 1) / kNumSMs * (chunks * chunk(t->BN)) + 4.5 + kTailUs * t->BN);
     int best_bn = 0, best_k = 0;
     for (int bn = n_tile ? n_tile : 32; bn <= (n_tile ? n_tile : 256) && bn <= kmax; bn += 32) {
         const long tiles = m_tiles * ((Kp + bn - 1) / bn);
@@ -131,7 +196,7 @@ bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int
             const int cps = (chunks + k - 1) / k;
             if ((k - 1) * cps >= chunks || tiles > capacity[k]) continue;
             if (!split && t->passes == 3 && chunks * kChunk * fabs(1.0 / k - 1.0 / otherwise) > 1330.0) continue;
-            const double cost = cps * chunk(bn) + 5500.0 + 18.0 * bn;
+            const double cost = cps * chunk(bn) + 5.7 + (kTailUs + 0.004) * bn;
             if (cost < best) { best = cost; best_bn = bn; best_k = k; }
         }
     }
@@ -367,25 +432,6 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.tiles_w = (a.Wo + t.tw - 1) / t.tw;
         t.tiles_h = (a.Ho + t.th - 1) / t.th;
         m_tiles = (long)t.tiles_w * t.tiles_h * ((a.N + t.tn - 1) / t.tn);
-        const cuuint64_t dims[4] = {(cuuint64_t)a.Cp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
-        const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
-        // the box spans the traversed input extent; one element in `stride` is taken
-        const cuuint32_t box[4] = {kChunk, (cuuint32_t)((t.tw - 1) * a.stride + 1), (cuuint32_t)((t.th - 1) * a.stride + 1),
-                                   (cuuint32_t)t.tn};
-        const cuuint32_t es[4] = {1, (cuuint32_t)a.stride, (cuuint32_t)a.stride, 1};
-        if (!make_map(&mA, x, 4, dims, str, box, es)) return OGLE_ERR_CUDA;
-        if (v2) {
-            const cuuint64_t yd[4] = {(cuuint64_t)kp_a, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
-            const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * a.Wo, (cuuint64_t)ks_a * 4 * a.Wo * a.Ho};
-            const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, (cuuint32_t)t.tn};
-            const cuuint32_t ye[4] = {1, 1, 1, 1};
-            if (!make_map(&mY, y + a.koff, 4, yd, ys, yb, ye)) return OGLE_ERR_CUDA;
-            if (y2) {
-                const cuuint64_t yd2[4] = {(cuuint64_t)kp_b, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
-                const cuuint64_t ys2[3] = {(cuuint64_t)kp_b * 4, (cuuint64_t)kp_b * 4 * a.Wo, (cuuint64_t)kp_b * 4 * a.Wo * a.Ho};
-                if (!make_map(&mY2, y2, 4, yd2, ys2, yb, ye)) return OGLE_ERR_CUDA;
-            }
-        }
     }
     choose_n_tiling_v2(a.Kp, m_tiles, &t, a.n_tile,
                        (plan_only || (ws != nullptr && aligned16(ws))) && !t.gather && split_k_enabled() &&
@@ -447,9 +493,45 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         while (t.split_k > 1 && (t.split_k - 1) * cps >= chunks) --t.split_k;     // no empty ranges
         if (t.split_k == 1) t.ws_mode = 0;
     }
+    bool on_pairs = want_pair(t, m_tiles, a.pair);
+    const bool on_m = want_channels_on_m(t, a.Kp, m_tiles, a.on_m);
+    const bool tiled = variant != CONV_POINTWISE && !t.gather;       // tiles of image pieces
     // (the scratch a layer asks for does not depend on whether the launch then splits inside clusters instead)
-    if (!plan_only && !(a.on_m == 2 && t.ws_mode) && !want_channels_on_m(t, a.Kp, m_tiles, a.on_m) && !want_pair(t, m_tiles, a.pair))
-        choose_cluster(&t, a.Kp, m_tiles, chunks, a.n_tile, a.split, t.split_k);
+    // How many ranges a reduction has, and so its bits, is settled on whole-row tiles; an unsplit launch is then free to cut
+    // its tiles and choose their width and form, and so is one that splits inside clusters.
+    if (!plan_only) {
+        TcArgs c = t;
+        long cut = m_tiles;
+        if (tiled) cut_tiles(a, (a.Kp + 127) / 128, &c, &cut);
+        const bool cluster = !(a.on_m == 2 && t.ws_mode) && !on_m && !on_pairs &&
+                             choose_cluster(&c, a.Kp, cut, chunks, a.n_tile, a.split, t.split_k);
+        if (cluster || t.split_k <= 1) { t = c; m_tiles = cut; }
+        if (!cluster && t.split_k <= 1 && !a.n_tile && !a.pair && !on_m)
+            on_pairs = refine_width(&t, a.Kp, m_tiles, chunks, !residual && pair_mode_override() != 1);
+    }
+    auto make_tile_maps = [&] {
+        const cuuint64_t dims[4] = {(cuuint64_t)a.Cp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
+        const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
+        // the box spans the traversed input extent; one element in `stride` is taken
+        const cuuint32_t box[4] = {kChunk, (cuuint32_t)((t.tw - 1) * a.stride + 1), (cuuint32_t)((t.th - 1) * a.stride + 1),
+                                   (cuuint32_t)t.tn};
+        const cuuint32_t es[4] = {1, (cuuint32_t)a.stride, (cuuint32_t)a.stride, 1};
+        if (!make_map(&mA, x, 4, dims, str, box, es)) return false;
+        if (v2) {
+            const cuuint64_t yd[4] = {(cuuint64_t)kp_a, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
+            const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * a.Wo, (cuuint64_t)ks_a * 4 * a.Wo * a.Ho};
+            const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, (cuuint32_t)t.tn};
+            const cuuint32_t ye[4] = {1, 1, 1, 1};
+            if (!make_map(&mY, y + a.koff, 4, yd, ys, yb, ye)) return false;
+            if (y2) {
+                const cuuint64_t yd2[4] = {(cuuint64_t)kp_b, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
+                const cuuint64_t ys2[3] = {(cuuint64_t)kp_b * 4, (cuuint64_t)kp_b * 4 * a.Wo, (cuuint64_t)kp_b * 4 * a.Wo * a.Ho};
+                if (!make_map(&mY2, y2, 4, yd2, ys2, yb, ye)) return false;
+            }
+        }
+        return true;
+    };
+    if (tiled && !plan_only && !make_tile_maps()) return OGLE_ERR_CUDA;
     const int Kp128 = (a.K + 127) / 128 * 128;
     const cuuint64_t bcols = t.gather ? (cuuint64_t)t.Cp32 : (cuuint64_t)taps * t.Cp32;
     const cuuint64_t bdims[2] = {bcols, (cuuint64_t)Kp128};
@@ -527,7 +609,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         }
         t.res = residual;
         t.res_ld = res_ld;
-        if (want_channels_on_m(t, a.Kp, m_tiles, a.on_m)) {
+        if (on_m) {
             // the filter tile is the M-side operand: all (stacked) channels in one tile of FR rows
             t.BN = (a.Kp + 31) / 32 * 32;
             t.n_tiles = 1;
@@ -536,7 +618,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             if (!ogle::make_map(&mBlo, w_lo, 2, bdims, bstr, fbox, bes)) return OGLE_ERR_CUDA;
             return launch_tc_t(t, mA, mBhi, mBlo, mY, y2 ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
         }
-        if (!residual && want_pair(t, m_tiles, a.pair)) {
+        if (!residual && on_pairs) {
             // each block of a pair loads half of the filter tile's rows
             const cuuint32_t hbox[2] = {kChunk, (cuuint32_t)(t.BN / 2)};
             if (!ogle::make_map(&mBhi, w_hi, 2, bdims, bstr, hbox, bes)) return OGLE_ERR_CUDA;
@@ -572,7 +654,8 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
     const bool v2 = true;
     const long m_tiles = (p.M + kTileM - 1) / kTileM;
     choose_n_tiling_v2(t.Kp, m_tiles, &t);
-    choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 0, 1);
+    const bool on_pairs = !choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 0, 1) &&
+                          refine_width(&t, t.Kp, m_tiles, t.chunks_per_tap, pair_mode_override() != 1);
     t.y = Y; t.y_ld = p.ldy;
     CUtensorMap mA, mBhi, mBlo, mY;
     const cuuint64_t dims[4] = {(cuuint64_t)p.K, (cuuint64_t)p.M, 1, 1};
@@ -582,7 +665,7 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
     if (!make_map(&mA, A, 4, dims, str, box, es)) return OGLE_ERR_CUDA;
     const cuuint64_t bdims[2] = {(cuuint64_t)(Blo ? t.Cp32 : p.K), (cuuint64_t)b_rows};
     const cuuint64_t bstr[1] = {(cuuint64_t)b_row_stride * 4};
-    const cuuint32_t bbox[2] = {kChunk, (cuuint32_t)t.BN};
+    const cuuint32_t bbox[2] = {kChunk, (cuuint32_t)(on_pairs ? t.BN / 2 : t.BN)};      // each block of a pair loads half
     const cuuint32_t bes[2] = {1, 1};
     if (!make_map(&mBhi, Bhi, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
     if (!make_map(&mBlo, Blo ? Blo : Bhi, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
@@ -590,6 +673,7 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
         const cuuint64_t yd[4] = {(cuuint64_t)t.Kp, (cuuint64_t)p.M, 1, 1};
         const cuuint64_t ys[3] = {(cuuint64_t)p.ldy * 4, (cuuint64_t)p.ldy * 4 * (cuuint64_t)p.M, (cuuint64_t)p.ldy * 4 * (cuuint64_t)p.M};
         if (!make_map(&mY, Y, 4, yd, ys, box, es)) return OGLE_ERR_CUDA;
+        if (on_pairs) return launch_tc_pair(t, mA, mBhi, mBlo, mY, mY, m_tiles, C, error_flag_ptr(), s);
         return launch_tc_v2(t, mA, mBhi, mBlo, mY, mY, m_tiles, C, error_flag_ptr(), s);
     }
     return OGLE_ERR_UNSUPPORTED;

@@ -850,9 +850,17 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     t.epi_groups = 2;
     t.epi_slabs = 2;
     if (t.passes == 3 && chunks >= 8) {
-        // long reductions: the epilogue is rare, the ring needs the room
+        // long reductions: the epilogue is rare, the ring needs the room. What it leaves over (where tensor memory bounds
+        // it, or the last stage does not fit) goes to the epilogue: a tile of 128 columns and eight chunks takes as
+        // long to store by one group as to multiply
         t.epi_groups = 1;
         t.epi_slabs = 1;
+        int ring = (int)((kBudget - kStagingBytes) / stage);
+        if (ring > kMaxStages) ring = kMaxStages;
+        if (t.ta && ring > ta_stages) ring = ta_stages;
+        const size_t over = kBudget - (size_t)ring * stage;
+        if (over >= 2 * (size_t)kStagingBytes) t.epi_groups = 2;
+        if (over >= 4 * (size_t)kStagingBytes) t.epi_slabs = 2;
     } else {
         auto stages_with = [&](int groups, int slabs) { return (int)((kBudget - (size_t)groups * slabs * kStagingBytes) / stage); };
         // (measured: the bandwidth-bound pointwise layers want the second slab more than a
@@ -861,10 +869,13 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         if (stages_with(2, 2) < shallow && stages_with(2, 1) > stages_with(2, 2)) t.epi_slabs = 1;
         if (stages_with(t.epi_groups, t.epi_slabs) < 2) { t.epi_groups = 1; t.epi_slabs = 1; }
     }
-    if (const char* e = getenv("OGLE_TC_XF_GROUPS")) t.xf_groups = ((t.passes == 3 || t.gather) && e[0] == '2') ? 2 : 1;
+    static const char* env_xf = getenv("OGLE_TC_XF_GROUPS");
+    static const char* env_groups = getenv("OGLE_TC_EPI_GROUPS");
+    static const char* env_slabs = getenv("OGLE_TC_EPI_SLABS");
+    if (const char* e = env_xf) t.xf_groups = ((t.passes == 3 || t.gather) && e[0] == '2') ? 2 : 1;
     if (t.gather) t.xf_groups = 2;        // the gather code is laid out for 256 threads
-    if (const char* e = getenv("OGLE_TC_EPI_GROUPS")) t.epi_groups = e[0] == '1' ? 1 : 2;
-    if (const char* e = getenv("OGLE_TC_EPI_SLABS")) t.epi_slabs = e[0] == '1' ? 1 : 2;
+    if (const char* e = env_groups) t.epi_groups = e[0] == '1' ? 1 : 2;
+    if (const char* e = env_slabs) t.epi_slabs = e[0] == '1' ? 1 : 2;
     if (t.cluster) t.epi_slabs = 0;       // partial tiles go where the operand ring was
     const size_t staging = (size_t)t.epi_groups * t.epi_slabs * kStagingBytes;
     const size_t budget = kBudget - staging;

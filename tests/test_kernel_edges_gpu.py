@@ -199,3 +199,33 @@ def test_gemm_over_clusters(m, k, n, bias_mode, math):
     # unsplit reduction, less in a split one; in one-pass mode 2^-11 per operand
     assert err <= (1.2e-8 * k + 2e-6 if mode == ops.MATH_TF32X3 else 2e-3)
     assert (got[:, n:] == 0).all()
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride, pad: maps cut along the width (75, 70, 150, 129 pixels), reductions of eight chunks
+    # and more whose tile width and form the launch chooses (pairs of SMs among them)
+    (2, 75, 75, 20, 40, 3, 1, 1), (3, 141, 139, 17, 30, 3, 2, 1), (1, 150, 150, 32, 96, 3, 1, 1), (2, 9, 129, 16, 8, 3, 1, 1),
+    (3, 66, 90, 32, 160, 5, 1, 2), (6, 60, 64, 40, 256, 3, 1, 1), (1, 120, 120, 288, 250, 1, 1, 0)])
+def test_tile_choice_keeps_the_sums(oracle_port, shape):
+    """Whatever tiles an unsplit launch chooses, an output value sums its reduction in the same order: the bits of the
+    launch with a fixed width on single SMs, with and without a residual operand."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K, k, s, pd = shape
+    rng = np.random.default_rng(W + K)
+    x = rng.standard_normal((N, H, W, C), dtype=np.float32)
+    w = (rng.standard_normal((K, C, k, k)) / np.sqrt(C * k * k)).astype(np.float32)
+    b = rng.standard_normal(K, dtype=np.float32)
+    x4, b4, w4 = ops.upload(x), ops.dense_to_device(b), ops.dense_to_device(w)
+    ref = oracle_port.conv2d(x[:1], w, b, s, pd, 1, 1, 2, 0.0, 0.0)
+    for math, tol in ((ops.MATH_TF32X3, 3e-5), (ops.MATH_TF32, 6e-3)):
+        outs, fused = [], []
+        for n_tile, pair in ((0, 0), (32, 1)):
+            p = ops.conv_params(N, H, W, C, K, k, s, pd, 1, 1, True, 2, 0.0, 0.0, math)
+            p.split, p.n_tile, p.sm_pair = 1, n_tile, pair
+            packed = ops.conv2d_prepack(p, w4)
+            res = ops.upload(np.random.default_rng(1).standard_normal((N,) + tuple(p.out_hwc), dtype=np.float32))
+            outs.append(ops.conv2d(p, x4, packed, b4, workspace=None))
+            fused.append(ops.conv2d_residual(p, x4, packed, b4, res))
+        assert torch.equal(outs[0], outs[1]) and torch.equal(fused[0], fused[1])
+        assert np.abs(ops.download(outs[0], K)[:1] - ref).max() <= tol * max(1.0, np.abs(ref).max())
