@@ -229,7 +229,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool split = a.passes == 3;
     const uint32_t b_bytes = (uint32_t)a.BN * 128u;
-    const uint32_t a_bytes = (split && !a.ta ? 2u : 1u) * kABytes;      // activation part of a stage
+    // activation part of a stage (none where the gather form builds its operand in tensor memory)
+    const uint32_t a_bytes = a.gather && a.ta ? 0u : (split && !a.ta ? 2u : 1u) * kABytes;
     const uint32_t stage_bytes = a_bytes + (split ? 2u : 1u) * b_bytes + (a.gather ? (uint32_t)a.g_bytes : 0u);
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -443,6 +444,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // A operands in tensor memory: a thread takes one row, the two groups take alternate chunks
             const int r = (warp & 3) * 32 + lane;
             const uint32_t lanes = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+            // gather form: this row's first tap in the input window
+            const int g_row = a.gather ? ((r / a.tw * a.stride) * a.g_iw + r % a.tw * a.stride) * 4 : 0;
             int s = 0, turn = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -459,8 +462,16 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (!ok) { record_error(err_flag, 3); s_abort = 1; break; }
                     if (turn == xg) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        split_row_to_tmem(reinterpret_cast<const float4*>(base_ptr + (size_t)s * stage_bytes + (size_t)r * 128), r,
-                                          lanes + (uint32_t)s * 64u);
+                        const unsigned char* stage = base_ptr + (size_t)s * stage_bytes;
+                        const uint32_t to = lanes + (uint32_t)s * 64u;
+                        if (!a.gather) {
+                            split_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
+                        } else {
+                            const float* win = reinterpret_cast<const float*>(stage + 2u * b_bytes) + g_row;
+                            if (a.g_k == 7) gather_row_to_tmem<7>(win, a.g_iw * 4, it, to);
+                            else if (a.g_k == 5) gather_row_to_tmem<5>(win, a.g_iw * 4, it, to);
+                            else gather_row_to_tmem<3>(win, a.g_iw * 4, it, to);
+                        }
                         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         mbar_arrive(&bar_xf[s]);
@@ -834,12 +845,14 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     const int acc_cols = t.BN;
     // Split mode: the A operands of both passes go through tensor memory where two stages or more of them fit beside
     // the accumulators (tiles of up to 192 columns).
-    t.n_acc = 4 * acc_cols <= (t.passes == 3 && !t.gather ? 256 : 512) ? 4 : 2;
+    // (In the gather form too, for three input channels.)
+    const bool ta_form = t.passes == 3 && (!t.gather || t.g_C == 3);
+    t.n_acc = 4 * acc_cols <= (ta_form ? 256 : 512) ? 4 : 2;
     static const bool ta_off = [] { const char* e = getenv("OGLE_TC_TA"); return e && e[0] == '0'; }();
     const int ta_stages = (512 - t.n_acc * acc_cols) / 64;
-    t.ta = t.passes == 3 && !t.gather && !ta_off && ta_stages >= 2 ? 1 : 0;
+    t.ta = ta_form && !ta_off && ta_stages >= 2 ? 1 : 0;
     if (!t.ta) t.n_acc = 4 * acc_cols <= 512 ? 4 : 2;
-    const size_t stage = (size_t)(t.passes == 3 && !t.ta ? 2 : 1) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * t.BN * 128 +
+    const size_t stage = (size_t)(t.ta && t.gather ? 0 : (t.passes == 3 && !t.ta ? 2 : 1)) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * t.BN * 128 +
                          (t.gather ? (size_t)t.g_bytes : 0);
     // Shared memory is split between the operand ring and the epilogue's staging slabs
     // (128 rows x 32 columns each). Preference: two epilogue groups with two slabs each;
