@@ -9,7 +9,8 @@
 //               costs its issuer over a hundred cycles;
 //   warp 1      MMA issuer: accumulates tile i into one of 2-4 tensor-memory buffers while
 //               the epilogues drain earlier tiles from the others;
-//   warps 2-9   two epilogue groups of four warps, taking alternate tiles:
+//   warps 2-9   two epilogue groups of four warps, taking alternate 32-column slabs of a tile (so that the last
+//               tile, or the only one, is stored by both; 128 x 256 by one group: 8 us):
 //               tcgen05.ld -> bias / activation -> shared-memory staging in the
 //               128-byte swizzle -> TMA tensor store (fully coalesced, clipped at the
 //               tensor edge by the hardware);
@@ -274,7 +275,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(&bar_acc_full[i], 1);
-            mbar_init(&bar_acc_empty[i], 128);
+            mbar_init(&bar_acc_empty[i], (uint32_t)(128 * a.epi_groups));
         }
         mbar_init(&bar_drain, 1);
         s_abort = 0;
@@ -602,13 +603,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int staged_nbase = -1;
             int round_no = 0;          // rounds of this group so far (selects the staging slab)
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
-                if (ti % a.epi_groups != eg) continue;
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord(a, wi.tile);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
                 const int nbase = tc_.n_tile * a.BN;
                 int groups = (a.Kp - nbase + 31) / 32;
                 if (groups > a.BN / 32) groups = a.BN / 32;
+                const int first = a.epi_groups == 2 ? (eg + ti) & 1 : 0;      // this group's slabs: first, first + epi_groups, ...
                 long pix = 0;
                 if (a.bias_mode == 1) {
                     pix = (long)tc_.w0 + row;
@@ -641,10 +642,14 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
                 if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (first >= groups) {                  // none of them this time
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(&bar_acc_empty[as]);
+                }
                 // one 32-column slab per round through a ring of one or two staging slabs: a slab
                 // is reused once the store issued from it (one or two rounds ago) has read it, so
                 // with two slabs a round never waits for the store of the round just before
-                for (int g0 = 0; g0 < groups; ++g0) {
+                for (int g0 = first; g0 < groups; g0 += a.epi_groups) {
                     const int sb = round_no % a.epi_slabs;
                     ++round_no;
                     if (t == 0) {
@@ -653,13 +658,12 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                     group_sync(bar_id);
                     {
-                        const int b = 0;
                         const int col = g0 * 32;
                         uint32_t r[32];
                         const uint32_t taddr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * acc_cols + col);
                         tmem_ld32(r, taddr);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (g0 + b == groups - 1) {
+                        if (g0 + a.epi_groups >= groups) {
                             // this thread's part of the accumulator is in registers: hand the buffer back
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                             mbar_arrive(&bar_acc_empty[as]);

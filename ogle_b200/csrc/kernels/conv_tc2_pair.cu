@@ -219,7 +219,7 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_acc_full[i], 1);
-            mbar_init(&bar_acc_empty[i], 256);        // the epilogue groups of both blocks
+            mbar_init(&bar_acc_empty[i], (uint32_t)(256 * a.epi_groups));        // the epilogue groups of both blocks
         }
         mbar_init(&bar_drain, 1);
         s_abort = 0;
@@ -417,13 +417,13 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             int staged_nbase = -1;
             int round_no = 0;
             for (int w = my_pair; w < a.total_work && ok; w += n_pairs, ++ti) {
-                if (ti % a.epi_groups != eg) continue;
                 const PairCoord pc = pair_coord(a, w, rank);
                 const bool live = pc.m_tile < m_tiles;
                 const int as = ti & 1, use = ti >> 1;
                 const int nbase = pc.n_tile * a.BN;
                 int groups = (a.Kp - nbase + 31) / 32;
                 if (groups > a.BN / 32) groups = a.BN / 32;
+                const int first = a.epi_groups == 2 ? (eg + ti) & 1 : 0;      // the groups take alternate slabs of a tile
                 long pix = 0;
                 if (a.bias_mode == 1) {
                     pix = (long)pc.w0 + row;
@@ -437,7 +437,11 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 ok = wait_pair(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
                 if (!ok) { record_error(err_flag, 18); raise_abort(); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int g0 = 0; g0 < groups; ++g0) {
+                if (first >= groups) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive_cluster(l_acc_empty + (uint32_t)as * 8u);
+                }
+                for (int g0 = first; g0 < groups; g0 += a.epi_groups) {
                     const int sb = round_no % a.epi_slabs;
                     ++round_no;
                     if (t == 0) {
@@ -450,7 +454,7 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     const uint32_t taddr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * acc_cols + col);
                     tmem_ld32_p(r, taddr);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (g0 == groups - 1) {
+                    if (g0 + a.epi_groups >= groups) {
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         mbar_arrive_cluster(l_acc_empty + (uint32_t)as * 8u);
                     }
