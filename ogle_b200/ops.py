@@ -18,11 +18,14 @@ from ._lib import (ACT_CLIP, ACT_NONE, ACT_RELU, MATH_FP32, MATH_TF32, MATH_TF32
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle. (torch.cuda.current_stream() builds an object around it: 3.3 us of a call that takes
+    15, against 0.3.)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    """Address for a `void *` argument."""
+    return t.data_ptr() if t is not None else None
 
 
 def up4(v):
@@ -251,9 +254,8 @@ def gemm_ws(A4, B4, C4, M, K, N, transB=0, alpha=1.0, beta=1.0, bias_mode=0, mat
     _require_cuda(A4, B4, C4)
     p = _gemm_params(A4, B4, C4, M, K, N, transB, alpha, beta, bias_mode, math_mode)
     lib = _lib.cuda_lib()
-    need = lib.ogle_cuda_gemm_packed_b_bytes(C.byref(p))
     if workspace is None:
-        workspace = torch.empty(need // 4, dtype=torch.float32, device="cuda")
+        workspace = torch.empty(lib.ogle_cuda_gemm_packed_b_bytes(C.byref(p)) // 4, dtype=torch.float32, device="cuda")
     out = torch.empty((M, up4(N)), dtype=torch.float32, device="cuda")
     check(lib.ogle_cuda_gemm_ws(C.byref(p), _p(A4), _p(B4), _p(C4), _p(out), _p(workspace), workspace.numel() * 4,
                                 _stream()), "gemm_ws")

@@ -237,7 +237,7 @@ class FBOSession:
             buf = np.empty(max((n + 3) // 4 * 4, 4), np.float32)
             _check(self._lib.ogle_session_get_output(self._h, name.encode(), f.encode(), buf.ctypes.data_as(_vp), buf.size),
                    "GetOutputs")
-            outs.append(buf[:n].reshape(hshape).copy())
+            outs.append(buf[:n].reshape(hshape))          # (a view of the array made for it, which nothing else holds)
         return outs
 
     def num_active_kernels(self):
