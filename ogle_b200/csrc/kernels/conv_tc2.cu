@@ -9,8 +9,8 @@
 //               costs its issuer over a hundred cycles;
 //   warp 1      MMA issuer: accumulates tile i into one of 2-4 tensor-memory buffers while
 //               the epilogues drain earlier tiles from the others;
-//   warps 2-9   two epilogue groups of four warps, taking alternate 32-column slabs of a tile (so that the last
-//               tile, or the only one, is stored by both; 128 x 256 by one group: 8 us):
+//   warps 2-9   two epilogue groups of four warps, taking alternate 32-column slabs of every tile (so that the last
+//               tile, or the only one, is stored by both), or alternate tiles where that is the faster rhythm:
 //               tcgen05.ld -> bias / activation -> shared-memory staging in the
 //               128-byte swizzle -> TMA tensor store (fully coalesced, clipped at the
 //               tensor edge by the hardware);
@@ -609,7 +609,9 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int nbase = tc_.n_tile * a.BN;
                 int groups = (a.Kp - nbase + 31) / 32;
                 if (groups > a.BN / 32) groups = a.BN / 32;
-                const int first = a.epi_groups == 2 ? (eg + ti) & 1 : 0;      // this group's slabs: first, first + epi_groups, ...
+                // this group's slabs: first, first + step, ...
+                const int step = a.epi_share ? a.epi_groups : 1;
+                const int first = a.epi_groups == 1 || ((eg + ti) & 1) == 0 ? 0 : (a.epi_share ? 1 : groups);
                 long pix = 0;
                 if (a.bias_mode == 1) {
                     pix = (long)tc_.w0 + row;
@@ -649,7 +651,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 // one 32-column slab per round through a ring of one or two staging slabs: a slab
                 // is reused once the store issued from it (one or two rounds ago) has read it, so
                 // with two slabs a round never waits for the store of the round just before
-                for (int g0 = first; g0 < groups; g0 += a.epi_groups) {
+                for (int g0 = first; g0 < groups; g0 += step) {
                     const int sb = round_no % a.epi_slabs;
                     ++round_no;
                     if (t == 0) {
@@ -663,7 +665,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         const uint32_t taddr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * acc_cols + col);
                         tmem_ld32(r, taddr);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (g0 + a.epi_groups >= groups) {
+                        if (g0 + step >= groups) {
                             // this thread's part of the accumulator is in registers: hand the buffer back
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                             mbar_arrive(&bar_acc_empty[as]);
@@ -929,6 +931,11 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         attr_device = dev;
     }
     const int sms = num_sms();
+    // A tile of 128 x 256 takes one group 8 us after the last multiply, which launches of a round or two feel; and a wide
+    // tile's buffer is handed back sooner by two. Many rounds of one or two chunks are bound by HBM and keep a better
+    // rhythm with whole tiles per group: 5.76 M pixels 32 -> 64, split mode 443 against 454 us, one pass 414 against 436;
+    // 1.44 M 64 -> 128: 195 against 201, 184 against 188. At four chunks 128 -> 256 (0.37 M) it is 182-189 against 166.
+    t.epi_share = t.total_work <= 4 * sms || chunks > 2 ? 1 : 0;
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
     const bool overlapped = t.overlapped || overlapped_launches_enabled();
     if (t.cluster) {

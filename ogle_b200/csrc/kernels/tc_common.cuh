@@ -37,6 +37,7 @@ struct TcArgs {
     int n_acc;                // accumulator buffers in tensor memory (2 or 4)
     int total_tiles;          // m_tiles * n_tiles (persistent kernel)
     int epi_groups, xf_groups; // persistent kernel: warp groups per role (1 or 2)
+    int epi_share;            // one-SM form: the epilogue groups take alternate slabs of every tile (else alternate tiles)
     int epi_slabs;            // staging slabs (128 rows x 32 columns) per epilogue group (1 or 2)
     // Two outputs from one pass (sibling convolutions over the same input, filters stacked):
     // columns [0, K1) go to the first tensor, columns [split_col, K) to the second.
