@@ -251,7 +251,8 @@ void Detector::PostProcess(Slot& slot, int N, int H, int W, const OgleImageDesc*
     Tensor* anchors = session_->FindTensorByName(options_.output_names[2]);
     OGLE_CHECK(cls_logits && box_preds && anchors);
     OGLE_CHECK_EQ(cls_logits->shape()[0], N);
-    // detector.cc:242-258 (box decode) and 150-228 (selection) in one pass on the device
+    // detector.cc:242-258 (box decode) and 150-228 (selection) in one pass on the device, which reads [N][A][4] deltas
+    OGLE_CHECK(box_preds->shape() == (IntList{N, num_anchors_, 4})) << "box deltas must be [images, anchors, 4]";
     OGLE_CHECK_EQ(anchors->num_elements(), size_t(num_anchors_) * 4);
     OGLE_CHECK_EQ(options_.variances.size(), 4u);
     OgleDetectParams p;

@@ -312,6 +312,26 @@ def test_detector_end_to_end_matches_oracle_post_process(oracle_port):
         det.close()
 
 
+def test_detector_refuses_box_deltas_of_another_shape():
+    """The selection decodes deltas of four values per anchor: a model whose box output has five is an error, not
+    detections with boxes taken from the wrong places."""
+    from ogle_b200 import models, session
+    model, _ = models.mobilenet_v1_ssd(batch=1, num_classes=5, seed=3, weight_std="he")
+    lib = session.rt_lib()
+    x = np.zeros((1, 300, 300, 3), np.float32)
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "ssd.dlx")
+        model.save(path)
+        for boxes, fine in ((b"cls_logits", False), (b"box_preds", True)):
+            h = lib.ogle_detector_create(-1, None, path.encode(), 0, 0.3, 100, 0.45, -1, None, b"cls_logits", boxes, b"anchors")
+            assert h
+            rc = lib.ogle_detector_detect_async(h, x.ctypes.data, 1, 300, 300)
+            message = lib.ogle_rt_last_error()
+            lib.ogle_detector_destroy(h)
+            assert (rc == 0) == fine
+            assert fine or b"box deltas" in message
+
+
 def test_concat_in_place_is_transparent(oracle_port):
     """Convolutions whose results only a channel Concat reads write straight into their slices of its tensor
     (widths 8, 12, 16 and a ragged last one of 6) and the Concat leaves the sequence; the tensors downstream are
