@@ -270,7 +270,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (threadIdx.x == 0) {
         for (int s = 0; s < a.stages; ++s) {
             mbar_init(&bar_full[s], 2);     // one arrive.expect_tx from each producer
-            mbar_init(&bar_xf[s], a.ta ? 128u : (uint32_t)(a.xf_groups * 128));
+            mbar_init(&bar_xf[s], a.ta ? kXfBuilders + kXfPassers : (uint32_t)(a.xf_groups * 128));
             mbar_init(&bar_empty[s], 1);
         }
         for (int i = 0; i < 4; ++i) {
@@ -455,7 +455,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     // Every stage is waited for in turn, also those of the other group's chunks: copies land out of
                     // order, and a group that only looked at every second chunk could, in a ring of three or five
-                    // stages, meet a barrier two phases behind and take its parity for the coming one.
+                    // stages, meet a barrier two phases behind and take its parity for the coming one. And the multiply
+                    // waits for both groups, so that the ring cannot pass the one that has nothing to build.
                     // The stage is refilled only after the multiplies that read it - shared and tensor memory - are done.
                     // (The lanes leave the polling loop one by one; the tensor-memory stores want the whole warp.)
                     ok = wait_or_abort(&bar_full[s], ph, abort_flag, a.spin_limit);
@@ -475,6 +476,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         }
                         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&bar_xf[s]);
+                    } else if (lane == 0) {
                         mbar_arrive(&bar_xf[s]);
                     }
                     turn ^= 1;

@@ -286,6 +286,12 @@ __device__ __forceinline__ void gather_row_to_tmem(const float* win, int iw4, in
     if (kK >= 7 && chunk == 4) gather_chunk_to_tmem<kK, 4>(win, iw4, taddr);
 }
 
+// Arrivals that complete a stage's operand in tensor memory: the threads of the split group that built it, and one per
+// warp of the other group, which has seen the stage's copies land. Without the second the ring could refill the stage
+// twice before a warp that was not scheduled looked at it; waits name a phase by its parity, and that warp would sleep on.
+constexpr uint32_t kXfBuilders = 128;
+constexpr uint32_t kXfPassers = 4;
+
 // One lane of a converged warp, for the roles that a single thread plays. Chosen this way - not as lane 0 - the compiler
 // knows that exactly one thread runs the role and keeps addresses and descriptors in uniform registers, which is where
 // the tensor-core and copy instructions take them from: an MMA costs its issuer 10 cycles instead of 55.

@@ -1,0 +1,57 @@
+"""The operand ring of the tensor-core kernel, its waits and arrivals played through on the CPU.
+
+A wait on an mbarrier names the parity of the phase it waits for, so a waiter that is passed by two phases sleeps for
+good. Every interleaving of the roles over one ring is walked here; the counts come from the kernels' header.
+"""
+import os
+import re
+
+import pytest
+
+KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ogle_b200", "csrc", "kernels")
+
+
+def _passers():
+    """How many of the arrivals that complete a stage's operand come from the group that does not build it."""
+    text = open(os.path.join(KERNELS, "tc_common.cuh")).read()
+    m = re.search(r"constexpr uint32_t kXfPassers = (\d+);", text)
+    return int(m.group(1)) if m else 0
+
+
+def _overtaken(stages, chunks, passers_arrive):
+    """Whether some order of events lets a split group wait for a phase of bar_full that lies two or more back.
+    State: copies landed, chunks multiplied, and per split group the chunk it waits for. Copies of a stage are issued
+    once its last multiply is done; the multiply of chunk i waits for group i % 2 to have built its operand - and, where
+    both groups arrive, for the other one to have seen the copy - and multiplies run in order."""
+    start = (0, 0, 0, 0)
+    seen, todo = {start}, [start]
+    while todo:
+        landed, done, g0, g1 = todo.pop()
+        for g in (g0, g1):
+            # bar_full of stage g % stages has completed a phase for each landed chunk of that stage
+            if g < chunks and (landed - 1 - g) // stages >= 1 and landed > g:
+                return True
+        nxt = []
+        if landed < chunks and landed < done + stages:
+            nxt.append((landed + 1, done, g0, g1))
+        if g0 < landed:
+            nxt.append((landed, done, g0 + 1, g1))
+        if g1 < landed:
+            nxt.append((landed, done, g0, g1 + 1))
+        builder, other = (g0, g1) if done % 2 == 0 else (g1, g0)
+        if done < landed and builder > done and (not passers_arrive or other > done):
+            nxt.append((landed, done + 1, g0, g1))
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("stages", [2, 3, 4, 5, 8])
+def test_no_split_group_is_passed_by_the_ring(stages):
+    assert not _overtaken(stages, 3 * stages + 1, _passers() > 0)
+
+
+def test_the_model_sees_a_group_that_nobody_waits_for():
+    assert _overtaken(3, 10, False)
