@@ -468,6 +468,7 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
     while (range_bits < 32 && (a.ks.max_key >> range_bits) != 0) ++range_bits;
     a.ks.shift = range_bits > 9 ? range_bits - 9 : 0;
     static const size_t kSmemBudget = 224 * 1024;
+    static const size_t kSmemRule = 226 * 1024;                      // mode 0: up to 27936 anchors
     int threads;
     size_t smem;
     a.parts = 1;
@@ -488,7 +489,8 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         int warps = classes < 20 ? classes : 20;
         if (p->N * a.parts <= kNumSMs) warps = 20;
         threads = warps * 32;
-        const size_t warp_bytes = per_warp * (size_t)warps;
+        // (only warps that have a class to select from need a list, however many take part in the softmax)
+        const size_t warp_bytes = per_warp * (size_t)(warps < classes ? warps : classes);
         const size_t budget = a.parts == 2 && p->N * a.parts > kNumSMs ? 112 * 1024 : kSmemBudget;
         if (per_class + warp_bytes > budget) return OGLE_ERR_UNSUPPORTED;
         size_t cpp = (budget - warp_bytes) / per_class;
@@ -498,7 +500,7 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
     } else {
         threads = 512;
         smem = (size_t)a.Ap * 8 + kHistWords * 4 + kMaxTopK * 6 * sizeof(int) + kListMax * sizeof(unsigned short);
-        if (smem > kSmemBudget) return OGLE_ERR_UNSUPPORTED;
+        if (smem > kSmemRule) return OGLE_ERR_UNSUPPORTED;
     }
     static thread_local int attr_set_for_device = -1;
     int dev = 0;
@@ -506,7 +508,7 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
     if (attr_set_for_device != dev) {
         cudaError_t e = cudaFuncSetAttribute(ssd_detect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(ssd_detect_rule_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+            e = cudaFuncSetAttribute(ssd_detect_rule_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemRule);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_set_for_device = dev;
     }

@@ -113,6 +113,31 @@ def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
         assert (anchor[n, k:] == -1).all()
 
 
+@pytest.mark.parametrize("batch,anchors,classes,mode", [
+    (1, 56444, 2, 1), (149, 56444, 2, 1), (1, 55548, 3, 1), (148, 53756, 5, 1), (1, 39420, 21, 1), (1, 27774, 2, 0), (200, 27774, 3, 0)])
+def test_detect_takes_the_largest_anchor_counts(oracle_port, batch, anchors, classes, mode):
+    """Scores of one class (mode 1) or one image (mode 0) have to fit a block's shared memory; how many do does not
+    depend on the batch."""
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(anchors)
+    logits = torch.zeros((batch, anchors, ops.up4(classes)), device="cuda")
+    logits[..., :classes] = torch.randn((batch, anchors, classes), generator=g, device="cuda") * 3.0
+    xy = torch.rand((batch, anchors, 2), generator=g, device="cuda")
+    boxes = torch.cat([xy, xy + 0.05], 2)
+    score, anchor, cls, box, count = ops.ssd_detect(logits, boxes, classes, mode, 0.5, 50, 0.0, 300, 300)
+    e = torch.softmax(logits[..., :classes].double(), 2)
+    for c in range(1, classes) if mode else (0,):
+        # (distinct scores: the best fifty of each image, whatever the class in mode 0)
+        want = (e[..., c] if mode else e[..., 1:].max(2).values).topk(50, 1)
+        rows = slice((c - 1) * 50, c * 50) if mode else slice(0, 50)
+        assert (count[:, c - 1] if mode else count).flatten().eq(50).all()
+        assert (score.reshape(batch, -1)[:, rows].double() - want.values).abs().max() <= 2e-6
+        got = anchor.reshape(batch, -1)[:, rows].long()
+        mine = (e[..., c] if mode else e[..., 1:].max(2).values).gather(1, got)
+        assert (mine - want.values).abs().max() <= 2e-6
+
+
 @pytest.mark.parametrize("shape", [
     # N, H, W, C, K, kernel, stride, pad, dilation: rows, columns and reductions that end inside a tile; launches of
     # one tile split over a cluster of 8, of a few tiles, and of enough for the large tiles (128 x 32, x 64, x 128)
