@@ -192,10 +192,11 @@ int launch_conv_simt(const ConvArgs& a, int variant, const float* x, const float
         return finish_launch();
     }
     if (variant == CONV_GENERAL && conv_smallc_supported(a)) return launch_conv_smallc(a, x, w, bias, y, s);
-    // the kernel numbers input pixels in 32 bits: larger batches go in groups of images
+    // the kernel numbers input pixels in 32 bits: larger batches go in groups of images (a single image that is
+    // larger goes alone, numbered in 64)
     const long pixels = (long)a.H * a.W;
-    const long group = pixels * a.N < 0x7fffffffL ? a.N : 0x7fffffffL / pixels;
-    if (group < 1) return OGLE_ERR_UNSUPPORTED;
+    long group = pixels * a.N < 0x7fffffffL ? a.N : 0x7fffffffL / pixels;
+    if (group < 1) group = 1;
     if (group < a.N) {
         for (int n = 0; n < a.N; n += (int)group) {
             ConvArgs part = a;

@@ -73,7 +73,8 @@ __device__ __forceinline__ void store4(const IgemmArgs& a, long m, int n, float4
     *reinterpret_cast<float4*>(a.y + m * a.ldy + a.yoff + n) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <int BM, int BN, bool TRANSB>
+// Pixel: the type that numbers input pixels.
+template <int BM, int BN, bool TRANSB, typename Pixel>
 __global__ void __launch_bounds__(BM * BN / 64, BM * BN / 64 >= 256 ? 2 : (BM * BN / 64 >= 128 ? 3 : 6))
 conv_igemm_kernel(const IgemmArgs a) {
     constexpr int NT = BM * BN / 64, TX = BN / 8, TY = BM / 8;
@@ -91,7 +92,8 @@ conv_igemm_kernel(const IgemmArgs a) {
 
     // Copies of A: this thread always moves the same 4 reduction elements (kq) of the same rows.
     const int kq = (tid & 3) * 4;
-    int iy0[A_COPIES], ix0[A_COPIES], pix[A_COPIES];
+    int iy0[A_COPIES], ix0[A_COPIES];
+    Pixel pix[A_COPIES];
 #pragma unroll
     for (int j = 0; j < A_COPIES; ++j) {
         const long m = m0 + (tid >> 2) + j * (NT / 4);
@@ -101,7 +103,7 @@ conv_igemm_kernel(const IgemmArgs a) {
         const int oy = int(t % a.Ho);
         iy0[j] = m < a.M ? oy * a.stride - a.pad : -0x40000000;       // a row past the end lies outside every image
         ix0[j] = ox * a.stride - a.pad;
-        pix[j] = (int)(t / a.Ho) * a.H * a.W + (oy * a.stride - a.pad) * a.W + ix0[j];
+        pix[j] = (Pixel)(t / a.Ho) * a.H * a.W + (Pixel)(oy * a.stride - a.pad) * a.W + ix0[j];
     }
     int c, ky, kx;                   // the elements' channel and filter tap, carried from step to step
     {
@@ -119,7 +121,7 @@ conv_igemm_kernel(const IgemmArgs a) {
         for (int j = 0; j < A_COPIES; ++j) {
             const int iy = iy0[j] + ky * a.dil, ix = ix0[j] + kx * a.dil;
             const bool ok = r_next + kq < a.R && (unsigned)iy < (unsigned)a.H && (unsigned)ix < (unsigned)a.W;
-            const float* src = ok ? a.x + (long)(pix[j] + (ky * a.W + kx) * a.dil) * a.Cs + c : a.x;
+            const float* src = ok ? a.x + (long)(pix[j] + ((Pixel)ky * a.W + kx) * a.dil) * a.Cs + c : a.x;
             copy16(da + (((tid >> 2) + j * (NT / 4)) * kALd + kq) * 4, src, ok ? tail_a : 0);
         }
 #pragma unroll
@@ -232,7 +234,7 @@ conv_igemm_kernel(const IgemmArgs a) {
     cluster_sync();                              // no block leaves while another still reads its partial tile
 }
 
-template <int BM, int BN, bool TRANSB>
+template <int BM, int BN, bool TRANSB, typename Pixel = int>
 int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
     constexpr size_t ring = (size_t)kStages * (BM * kALd + (TRANSB ? BN * kALd : kBK * BN)) * sizeof(float);
     constexpr size_t tile = (size_t)BM * BN * sizeof(float);
@@ -241,7 +243,7 @@ int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<BM, BN, TRANSB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<BM, BN, TRANSB, Pixel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(tile > ring ? tile : ring));
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
@@ -256,7 +258,7 @@ int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = splits;
     cfg.attrs = attr;
     cfg.numAttrs = splits > 1 ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, conv_igemm_kernel<BM, BN, TRANSB>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, conv_igemm_kernel<BM, BN, TRANSB, Pixel>, a);
     if (e != cudaSuccess) { set_last_error(e); (void)cudaGetLastError(); return OGLE_ERR_CUDA; }
     return finish_launch();
 }
@@ -270,8 +272,9 @@ int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
 // for its start, its partial tile and the cluster's barriers).
 int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s) {
     const long m128 = (a.M + 127) / 128, m64 = (a.M + 63) / 64;
-    if (m64 > 0x7fffffffL || (a.n_store + 31) / 32 > 65535) return OGLE_ERR_UNSUPPORTED;
-    if (!trans_b) {
+    if (m64 > 0x7fffffffL || (a.n_store + 63) / 64 > 65535) return OGLE_ERR_UNSUPPORTED;
+    const bool large = a.M / ((long)a.Ho * a.Wo) * a.H * a.W > 0x7fffffffL;       // (one image of 2^31 pixels or more)
+    if (!trans_b && !large) {
         if (a.n_store > 64 && m128 * ((a.n_store + 127) / 128) >= 2 * kNumSMs && (a.n_store % 128 == 0 || a.n_store % 128 > 64))
             return launch<128, 128, false>(a, 1, s);
         if (a.n_store > 32 && m128 * ((a.n_store + 63) / 64) >= 4 * kNumSMs) return launch<128, 64, false>(a, 1, s);
@@ -286,6 +289,7 @@ int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s) {
         const double cost = (blocks < 4 ? 4.0 : blocks) * ((steps + k - 1) / k + 6.0);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = k; }
     }
+    if (large) return launch<64, 64, false, long>(a, best, s);
     return trans_b ? launch<64, 64, true>(a, best, s) : launch<64, 64, false>(a, best, s);
 }
 

@@ -12,7 +12,7 @@ struct IgemmArgs {
     const float* bias;
     float* y;
     long M;                  // output pixels (rows)
-    int H, W, Ho, Wo, Cs;    // input extent and pixel stride; fewer than 2^31 input pixels
+    int H, W, Ho, Wo, Cs;    // input extent and pixel stride; fewer than 2^31 input pixels, or one image
     int kernel, stride, pad, dil;
     int Cp;                  // reduction elements per filter tap
     int R;                   // kernel * kernel * Cp

@@ -166,6 +166,36 @@ def test_fp32_gemm_edges(oracle_port, m, k, n, trans_b):
     close(got, oracle_port.gemm(A, B, Cm, trans_b, 0.5, 2.0))
 
 
+def test_fp32_gemm_of_many_columns():
+    """Up to 65535 column tiles of 64."""
+    import torch
+    from ogle_b200 import ops
+    k, n = 4, 65535 * 64
+    a, b = torch.randn((1, k), device="cuda"), torch.randn((k, n), device="cuda")
+    got = ops.gemm(a, b, None, 1, k, n, 0, 1.0, 0.0, 0, ops.MATH_FP32)
+    want = a.double() @ b.double()
+    # four products, each sum rounded: 2^-23 of the terms' magnitudes at most
+    assert ((got.double() - want).abs() <= 2.0 ** -22 * (a.abs().double() @ b.abs().double())).all()
+
+
+def test_fp32_convolution_of_an_image_of_2_to_the_31_pixels():
+    """One image that 32-bit pixel numbers do not reach (34 GB of them), every 64th pixel of it taken."""
+    import torch
+    from ogle_b200 import ops
+    if torch.cuda.mem_get_info()[0] < 45 << 30:
+        pytest.skip("needs 45 GB of device memory")
+    h, w, s = 65536, 32768, 64
+    x = torch.zeros((1, h, w, 4), device="cuda")
+    picked = torch.randn((h // s, w // s), device="cuda")
+    x[0, ::s, ::s, 0] = picked
+    p = ops.conv_params(1, h, w, 1, 8, 1, s, 0, 1, 1, True, 0, 0.0, 0.0, ops.MATH_FP32)
+    f, b = torch.randn((8, 1, 1, 1), device="cuda"), torch.randn(8, device="cuda")
+    y = ops.conv2d(p, x, ops.conv2d_prepack(p, f), b)
+    assert torch.equal(y[0], picked[..., None] * f.flatten() + b)       # one product, rounded, and one sum
+    del x
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("shape", [
     # N, H, W, C, K, kernel, stride, pad, act, split: one tile over 2-8 blocks, ranges of unequal length, rows and columns
     # that end inside a tile, several tiles, three tile widths
