@@ -476,8 +476,9 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         // Two blocks per image, each with half of the foreground classes, when that lets two
         // blocks share an SM and the batch is a few rounds of SMs at most (more, smaller blocks
         // fill the last round better; for large batches the softmax done twice costs more than
-        // that gains); one warp per class, ~100 registers each. A batch that leaves SMs idle anyway takes
-        // all 640 threads per block for the softmax.
+        // that gains); one warp per class selects, ~100 registers a thread. An SM has registers for twenty warps: blocks of
+        // fewer classes than its share of them take the rest for the softmax (N = 630, 2 classes, 1917 anchors: 105 us
+        // with one warp a block, 45 with four).
         const size_t per_warp = kListMax * sizeof(unsigned short);
         const size_t per_class = (size_t)a.Ap * sizeof(float) + kHistWords * sizeof(unsigned);
         const int fg = p->C - 1;
@@ -486,11 +487,13 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
             if ((size_t)half * (per_class + per_warp) <= 112 * 1024) a.parts = 2;
         }
         const int classes = (fg + a.parts - 1) / a.parts;
-        int warps = classes < 20 ? classes : 20;
-        if (p->N * a.parts <= kNumSMs) warps = 20;
-        threads = warps * 32;
-        // (only warps that have a class to select from need a list, however many take part in the softmax)
-        const size_t warp_bytes = per_warp * (size_t)(warps < classes ? warps : classes);
+        const int pickers = classes < 20 ? classes : 20;             // (only they need a list)
+        const size_t warp_bytes = per_warp * (size_t)pickers;
+        const size_t block_bytes = classes * per_class + warp_bytes + 1024;
+        const long waiting = ((long)p->N * a.parts + kNumSMs - 1) / kNumSMs;       // blocks to an SM, and how many fit
+        const long fitting = block_bytes < kSmemBudget ? (long)(kSmemBudget / block_bytes) : 1;
+        const int share = (int)(20 / (waiting < fitting ? waiting : fitting));
+        threads = 32 * (pickers > share ? pickers : share);
         const size_t budget = a.parts == 2 && p->N * a.parts > kNumSMs ? 112 * 1024 : kSmemBudget;
         if (per_class + warp_bytes > budget) return OGLE_ERR_UNSUPPORTED;
         size_t cpp = (budget - warp_bytes) / per_class;
