@@ -23,7 +23,10 @@ __device__ __forceinline__ float4 elementwise_op(float4 v, float4 w, float lo, f
     return v;
 }
 
-template <int OP>
+// WIDE: four independent loads (eight with two operands) before the first store, for tensors that give a thread more than
+// three elements. Smaller ones are the launch and one trip to memory, and the loop that is never entered costs them its
+// instruction fetch: 1.6-2.0 us, 1.8-2.2 with it.
+template <int OP, bool WIDE>
 __global__ void elementwise_kernel(const float4* __restrict__ a, const float4* __restrict__ b,
                                    float4* __restrict__ y, long n4, float lo, float hi) {
     constexpr bool kBinary = OP >= EW_ADD;
@@ -32,8 +35,7 @@ __global__ void elementwise_kernel(const float4* __restrict__ a, const float4* _
     const long step = (long)gridDim.x * blockDim.x;
     long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    // four independent loads (eight with two operands) before the first store
-    for (; i + 3 * step < n4; i += 4 * step) {
+    for (; WIDE && i + 3 * step < n4; i += 4 * step) {
         float4 v[4], w[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) { v[u] = a[i + u * step]; w[u] = kBinary ? b[i + u * step] : zero; }
@@ -74,30 +76,51 @@ __device__ __forceinline__ float4 bn_apply(float4 v, const BnChannels& p) {
     return make_float4(out[0], out[1], out[2], out[3]);
 }
 
-// FIXED: the grid's stride is a multiple of the channel quads of a pixel, so a thread meets the same four
-// channels in every step: their parameters (and the square roots) are taken once and the loop holds no index
-// arithmetic. Any other grid looks them up per step. 32 x 38 x 38 x 384 channels: 59 us with the parameters
-// taken per element, 24 us with them hoisted (HBM floor 22 us).
-template <bool FIXED>
+// The grid's stride is a multiple of the channel quads of a pixel, so a thread meets the same four channels in every
+// step: their parameters (and the square roots) are taken once and the loop holds no index arithmetic. 32 x 38 x 38 x
+// 384 channels: 59 us with the parameters taken per element, 24 us with them hoisted (HBM floor 22 us).
 __global__ void __launch_bounds__(256)
 batchnorm_kernel(const float4* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                  const float* __restrict__ mean, const float* __restrict__ var, float4* __restrict__ y,
                  long total, int C, int q, float eps) {
     const long step = (long)gridDim.x * blockDim.x;
     long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (FIXED) {
-        if (i >= total) return;
-        const BnChannels p = bn_channels(gamma, beta, mean, var, int(i % q) * 4, C, eps);
-        for (; i + 3 * step < total; i += 4 * step) {
-            float4 v[4];
+    if (i >= total) return;
+    const BnChannels p = bn_channels(gamma, beta, mean, var, int(i % q) * 4, C, eps);
+    for (; i + 3 * step < total; i += 4 * step) {
+        float4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = x[i + u * step];
+        for (int u = 0; u < 4; ++u) v[u] = x[i + u * step];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) y[i + u * step] = bn_apply(v[u], p);
+        for (int u = 0; u < 4; ++u) y[i + u * step] = bn_apply(v[u], p);
+    }
+    for (; i < total; i += step) y[i] = bn_apply(x[i], p);
+}
+
+// Tensors of one element a thread, whose time is the launch, one trip to memory and the fetch of the kernel's
+// instructions (9 x 28 x 32 x 6: 2.6 us, 3.3 by the kernel above; at two elements a thread 7.9 against 6.8), and pixels of
+// so many channels that no grid keeps a thread on its own.
+__global__ void batchnorm_each_kernel(const float4* __restrict__ x, const float* __restrict__ gamma,
+                                      const float* __restrict__ beta, const float* __restrict__ mean,
+                                      const float* __restrict__ var, float4* __restrict__ y,
+                                      long total, int C, int q, float eps) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
+         i += (long)gridDim.x * blockDim.x) {
+        const int c = int(i % q) * 4;
+        const float4 v = x[i];
+        float in[4] = {v.x, v.y, v.z, v.w};
+        float out[4];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            if (c + l < C) {
+                const float d = __fsqrt_rn(__fadd_rn(var[c + l], eps));
+                const float t = __fdiv_rn(__fsub_rn(in[l], mean[c + l]), d);
+                out[l] = __fadd_rn(__fmul_rn(t, gamma[c + l]), beta[c + l]);
+            } else {
+                out[l] = 0.f;
+            }
         }
-        for (; i < total; i += step) y[i] = bn_apply(x[i], p);
-    } else {
-        for (; i < total; i += step) y[i] = bn_apply(x[i], bn_channels(gamma, beta, mean, var, int(i % q) * 4, C, eps));
+        y[i] = make_float4(out[0], out[1], out[2], out[3]);
     }
 }
 
@@ -112,9 +135,10 @@ static int launch_elementwise(const float* a, const float* b, float* y, long n, 
     if (n == 0) return OGLE_OK;
     if (!a || !y || (OP >= EW_ADD && !b)) return OGLE_ERR_INVALID;
     if (!aligned16(a) || !aligned16(y) || (b && !aligned16(b))) return OGLE_ERR_ALIGNMENT;
-    launch_overlapped(elementwise_kernel<OP>, dim3(grid_for(n / 4, 256)), dim3(256), 0, (cudaStream_t)stream,
-                      reinterpret_cast<const float4*>(a), reinterpret_cast<const float4*>(b), reinterpret_cast<float4*>(y), n / 4,
-                      lo, hi);
+    const int grid = grid_for(n / 4, 256);
+    launch_overlapped(n / 4 > 3L * 256 * grid ? elementwise_kernel<OP, true> : elementwise_kernel<OP, false>, dim3(grid), dim3(256), 0,
+                      (cudaStream_t)stream, reinterpret_cast<const float4*>(a), reinterpret_cast<const float4*>(b),
+                      reinterpret_cast<float4*>(y), n / 4, lo, hi);
     return finish_launch();
 }
 
@@ -155,13 +179,13 @@ int ogle_cuda_batchnorm(const float* x, const float* gamma, const float* beta, c
     int m = q, r = 256;
     while (r) { const int t = m % r; m = r; r = t; }          // greatest common divisor of q and 256
     m = q / m;
-    const bool fixed = m <= kNumSMs * 8;
+    const bool fixed = m <= kNumSMs * 8 && total > 256L * grid;
     if (fixed) grid = grid < m ? m : grid / m * m;
     if (fixed)
-        batchnorm_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        batchnorm_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
             reinterpret_cast<const float4*>(x), gamma, beta, mean, var, reinterpret_cast<float4*>(y), total, C, q, eps);
     else
-        batchnorm_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        batchnorm_each_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
             reinterpret_cast<const float4*>(x), gamma, beta, mean, var, reinterpret_cast<float4*>(y), total, C, q, eps);
     return finish_launch();
 }
