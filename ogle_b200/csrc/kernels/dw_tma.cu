@@ -39,8 +39,9 @@ struct DwTiles {
 
 // KS: window size. CB: float4s of a channel slab (8 = 32 channels, 4 = 16). A 5x5 window keeps its 25 taps
 // in registers too (100 of them), which leaves one block per SM: eight warps with 4-row accumulators are
-// enough to keep the copies ahead of the multiplies.
-template <int KS, int S, int RPG, int CB>
+// enough to keep the copies ahead of the multiplies. RAGGED: the last slab reaches past the channels; widths that
+// fill their slabs carry none of its checks (stride 1: 17.6 us, 19.2 with them, at 6 x 64 x 70 x 384).
+template <int KS, int S, int RPG, int CB, bool RAGGED>
 __global__ void __launch_bounds__(256, KS == 3 ? 2 : 1)
 dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict__ w, const float* __restrict__ bias,
                  float4* __restrict__ y, const ConvArgs a, const DwTiles tl, int* err_flag) {
@@ -110,9 +111,11 @@ dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict_
         // count every tile of a block has the same slab, and they are loaded once
         if (cb != loaded_cb) {
 #pragma unroll
-            for (int k = 0; k < KS * KS; ++k) wk[k] = cq < (a.Kp >> 2) ? w[k * (a.Kp >> 2) + cq] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < KS * KS; ++k) wk[k] = !RAGGED || cq < (a.Kp >> 2) ? w[k * (a.Kp >> 2) + cq] : make_float4(0.f, 0.f, 0.f, 0.f);
             bv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (a.has_bias) {                          // bias holds exactly K floats
+            if (!RAGGED) {
+                if (a.has_bias) bv = make_float4(bias[cq * 4], bias[cq * 4 + 1], bias[cq * 4 + 2], bias[cq * 4 + 3]);
+            } else if (a.has_bias) {                   // bias holds exactly K floats
                 if (cq * 4 + 0 < a.K) bv.x = bias[cq * 4 + 0];
                 if (cq * 4 + 1 < a.K) bv.y = bias[cq * 4 + 1];
                 if (cq * 4 + 2 < a.K) bv.z = bias[cq * 4 + 2];
@@ -155,13 +158,13 @@ dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict_
             }
         }
         const int ox = tx * TW + col;
-        if (ox < a.Wo && cq < (a.Kp >> 2)) {
+        if (ox < a.Wo && (!RAGGED || cq < (a.Kp >> 2))) {
 #pragma unroll
             for (int o = 0; o < RPG; ++o) {
                 const int oy = ty * TH + rg * RPG + o;
                 if (oy >= a.Ho) continue;
                 float4 r = apply_act4(acc[o], a.act, a.lo, a.hi);
-                if (cq * 4 + 4 > a.K) {                // lanes past K stay zero
+                if (RAGGED && cq * 4 + 4 > a.K) {                // lanes past K stay zero
                     if (cq * 4 + 1 >= a.K) r.y = 0.f;
                     if (cq * 4 + 2 >= a.K) r.z = 0.f;
                     r.w = 0.f;
@@ -175,8 +178,8 @@ dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict_
     }
 }
 
-template <int KS, int S, int RPG, int CB>
-int launch(const ConvArgs& a, const DwTiles& shape, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
+template <int KS, int S, int RPG, int CB, bool RAGGED>
+int launch_kernel(const ConvArgs& a, const DwTiles& shape, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
     CUtensorMap mX;
     const cuuint64_t dims[4] = {(cuuint64_t)a.Kp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
     const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
@@ -193,7 +196,7 @@ int launch(const ConvArgs& a, const DwTiles& shape, const float* x, const float*
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(dw_tma_kernel<KS, S, RPG, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmemMax);
+        cudaError_t e = cudaFuncSetAttribute(dw_tma_kernel<KS, S, RPG, CB, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmemMax);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
     }
@@ -202,14 +205,23 @@ int launch(const ConvArgs& a, const DwTiles& shape, const float* x, const float*
     // a multiple of the channel-slab count: block b then always works on slab b % cblocks
     if (tl.cblocks <= blocks) blocks -= blocks % tl.cblocks;
     if (blocks > tl.total) blocks = tl.total;
-    launch_overlapped(dw_tma_kernel<KS, S, RPG, CB>, dim3((unsigned)blocks), dim3(256), smem, s, mX, reinterpret_cast<const float4*>(w),
+    launch_overlapped(dw_tma_kernel<KS, S, RPG, CB, RAGGED>, dim3((unsigned)blocks), dim3(256), smem, s, mX, reinterpret_cast<const float4*>(w),
                       bias, reinterpret_cast<float4*>(y), a, tl, error_flag_ptr());
     return finish_launch();
 }
 
+template <int KS, int S, int RPG, int CB>
+int launch(const ConvArgs& a, const DwTiles& shape, const float* x, const float* w, const float* bias, float* y, cudaStream_t s) {
+    return a.K % (CB * 4) ? launch_kernel<KS, S, RPG, CB, true>(a, shape, x, w, bias, y, s)
+                          : launch_kernel<KS, S, RPG, CB, false>(a, shape, x, w, bias, y, s);
+}
+
 // Float4s of a channel slab: 32 channels, or 16 where slabs of 32 would compute over a sixth more channels than
-// slabs of 16 do (a slab's empty lanes cost shared memory and issue slots, not traffic).
+// slabs of 16 do (a slab's empty lanes cost shared memory and issue slots, not traffic). At stride 2 it is the copies that
+// set the pace, by the pixel and not by the byte, and only layers of one slab are better off with a narrow one
+// (52 x 132 x 116 x 72: 61 us, 50 with slabs of 32).
 int slab_quads(const ConvArgs& a) {
+    if (a.stride == 2) return a.Kp <= 16 ? 4 : 8;
     const int full = (a.Kp + 31) / 32 * 32, half = (a.Kp + 15) / 16 * 16;
     return 6 * full <= 7 * half ? 8 : 4;
 }
@@ -265,7 +277,17 @@ bool dw_tma_supported(const ConvArgs& a) {
           a.C == a.K && a.Wo >= 8 && a.Ho >= 4 && encode_fn() != nullptr))
         return false;
     DwTiles t;
-    return choose_shape(a, &t) != 0;
+    if (!choose_shape(a, &t)) return false;
+    // Widths of whole slabs always. Others at stride 2, where a tile's copies bring two to four times the pixels that it
+    // stores: 60 k pixels of halo, padding and slab per us against the register kernel's 1 us and 7 GB/ms of input and
+    // output, while those stay in L2 (45 x 71 x 119 x 12: 11.6 us by copies, 6.5; 59 x 20 x 41 x 230 13.6 against 11.5;
+    // 44 x 29 x 105 x 228 29.6 against 36).
+    const double bytes = 4.0 * a.N * a.Kp * ((double)a.H * a.W + (double)a.Ho * a.Wo);
+    if (a.kernel == 5 || a.stride == 1 || a.K % 32 == 0 || bytes > 100e6) return true;
+    const int slab = slab_quads(a) * 4;
+    const double tiles = (double)((a.Wo + t.tw - 1) / t.tw) * ((a.Ho + t.th - 1) / t.th) * ((a.Kp + slab - 1) / slab) * a.N;
+    const double copies_us = tiles * t.iw * t.ih / 60e3, registers_us = 1.0 + bytes / 7e6;
+    return copies_us <= (registers_us > 2.7 ? registers_us : 2.7);
 }
 
 template <int CB>
