@@ -1,15 +1,19 @@
 // fp32 contraction on the CUDA cores (OGLE_MATH_FP32, and convolutions with too few input channels for the tensor
 // cores): convolution as implicit GEMM and gemm, one kernel.
 //
-//  * A block computes a BM x BN tile, a thread 8 x 8 of it. The multiply-adds are packed (fma.rn.f32x2 over two
+//  * A block computes a BM x BN tile, a thread TM x 8 of it: 8 x 8 where the reduction is long, 2 x 8 - four times the
+//    threads, each with a quarter of the instructions - where a launch is over before a warp has worked off 64 outputs
+//    (455 pixels, 16 -> 9 channels: 6.4 us by two warps a block, 3.3 by four; 7020 x 84 x 216: 18.3, 16.4). The multiply-adds are packed (fma.rn.f32x2 over two
 //    adjacent output columns): the same IEEE fma per lane in the same order as scalar code, in half the issue slots,
 //    which leaves room for the shared-memory loads and operand moves between them.
 //  * Both operands come through a ring of three stages filled by 16-byte asynchronous copies (zero-filled outside the
-//    image and past the ends). A keeps its channels contiguous - no transposition on the way - in rows of 20 floats,
+//    image and past the ends), but for a transposed B, which is turned over through registers (read as it lies, its rows
+//    put four lanes on a bank: 2001 x 1613 x 3423 984 us, now 532). A keeps its channels contiguous - no transposition on the way - in rows of 20 floats,
 //    so that the rows a warp reads together start in different banks.
 //  * A launch with few tiles splits the reduction over the blocks of a cluster (2, 4 or 8): every block leaves its
 //    partial tile in its own shared memory, and each adds up a band of rows over the cluster, in rank order, through
 //    distributed shared memory: no scratch memory, no second launch, the same bits every time.
+//  * Bias and activation are applied on the way out of a tile in shared memory, row by row, not to 64 registers.
 //
 // Large layers run at 46-47 TFLOP/s (3x3 256 -> 256 at 38 x 38 x 32 images: 1658 -> 1183 us); packed and scalar
 // multiply-adds measure within 5 % of each other there, so it is the FP32 pipe and its operand reads, not issue slots
@@ -58,27 +62,39 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Four output columns of row m from column n on: bias, activation, zeros past N.
-__device__ __forceinline__ void store4(const IgemmArgs& a, long m, int n, float4 acc) {
-    if (m >= a.M || n >= a.n_store) return;
-    float v[4] = {acc.x, acc.y, acc.z, acc.w};
+// Bias of four output columns (row bias).
+__device__ __forceinline__ float4 row_bias(const IgemmArgs& a, int n) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (a.bias_mode == 2) {
 #pragma unroll
-    for (int l = 0; l < 4; ++l) {
-        if (n + l >= a.N) { v[l] = 0.f; continue; }
-        v[l] *= a.alpha;
-        if (a.bias_mode == 2) v[l] = fmaf(a.beta, a.bias[n + l], v[l]);
-        else if (a.bias_mode == 1) v[l] = fmaf(a.beta, a.bias[m * a.ldc + n + l], v[l]);
-        v[l] = apply_act(v[l], a.act, a.lo, a.hi);
+        for (int l = 0; l < 4; ++l)
+            if (n + l < a.N) v[l] = __ldg(a.bias + n + l);
     }
-    *reinterpret_cast<float4*>(a.y + m * a.ldy + a.yoff + n) = make_float4(v[0], v[1], v[2], v[3]);
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 
-// Pixel: the type that numbers input pixels.
-template <int BM, int BN, bool TRANSB, typename Pixel>
-__global__ void __launch_bounds__(BM * BN / 64, BM * BN / 64 >= 256 ? 2 : (BM * BN / 64 >= 128 ? 3 : 6))
+// One value of row m, column n: bias, activation, zero past N.
+__device__ __forceinline__ float finish(const IgemmArgs& a, long m, int n, float v, float bias) {
+    if (n >= a.N) return 0.f;
+    v *= a.alpha;
+    if (a.bias_mode == 2) v = fmaf(a.beta, bias, v);
+    else if (a.bias_mode == 1) v = fmaf(a.beta, __ldg(a.bias + m * a.ldc + n), v);
+    return apply_act(v, a.act, a.lo, a.hi);
+}
+// Four output columns of row m from column n on.
+__device__ __forceinline__ void store4(const IgemmArgs& a, long m, int n, float4 acc, float4 bias) {
+    if (m >= a.M || n >= a.n_store) return;
+    *reinterpret_cast<float4*>(a.y + m * a.ldy + a.yoff + n) =
+        make_float4(finish(a, m, n, acc.x, bias.x), finish(a, m, n + 1, acc.y, bias.y), finish(a, m, n + 2, acc.z, bias.z),
+                    finish(a, m, n + 3, acc.w, bias.w));
+}
+
+// TM: rows of a thread's outputs. Pixel: the type that numbers pixels (unsigned, or long where those are not enough).
+template <int BM, int BN, int TM, bool TRANSB, typename Pixel>
+__global__ void __launch_bounds__(BM * BN / (8 * TM), TM == 8 ? (BM * BN >= 16384 ? 2 : (BM * BN >= 8192 ? 3 : 6)) : (TM == 4 ? 8 : 1024 / (BM * BN / (8 * TM))))
 conv_igemm_kernel(const IgemmArgs a) {
-    constexpr int NT = BM * BN / 64, TX = BN / 8, TY = BM / 8;
-    constexpr int A_FLOATS = BM * kALd, B_FLOATS = TRANSB ? BN * kALd : kBK * BN;
+    constexpr int NT = BM * BN / (8 * TM), TX = BN / 8, TY = BM / TM;
+    constexpr int A_FLOATS = BM * kALd, B_FLOATS = kBK * BN;
     constexpr int A_COPIES = BM * (kBK / 4) / NT, B_COPIES = BN * (kBK / 4) / NT;
     static_assert(A_COPIES * NT == BM * (kBK / 4) && B_COPIES * NT == BN * (kBK / 4), "copies divide over the threads");
     extern __shared__ __align__(16) float smem[];
@@ -96,14 +112,14 @@ conv_igemm_kernel(const IgemmArgs a) {
     Pixel pix[A_COPIES];
 #pragma unroll
     for (int j = 0; j < A_COPIES; ++j) {
-        const long m = m0 + (tid >> 2) + j * (NT / 4);
-        const long mm = m < a.M ? m : 0;
-        const int ox = int(mm % a.Wo);
-        const long t = mm / a.Wo;
-        const int oy = int(t % a.Ho);
-        iy0[j] = m < a.M ? oy * a.stride - a.pad : -0x40000000;       // a row past the end lies outside every image
+        const Pixel m = (Pixel)m0 + (tid >> 2) + j * (NT / 4);
+        const Pixel mm = m < (Pixel)a.M ? m : 0;
+        const Pixel t = mm / (Pixel)a.Wo;
+        const int ox = int(mm - t * (Pixel)a.Wo);
+        const int oy = int(t % (Pixel)a.Ho);
+        iy0[j] = m < (Pixel)a.M ? oy * a.stride - a.pad : -0x40000000;       // a row past the end lies outside every image
         ix0[j] = ox * a.stride - a.pad;
-        pix[j] = (Pixel)(t / a.Ho) * a.H * a.W + (Pixel)(oy * a.stride - a.pad) * a.W + ix0[j];
+        pix[j] = t / (Pixel)a.Ho * a.H * a.W + (Pixel)(oy * a.stride - a.pad) * a.W + ix0[j];
     }
     int c, ky, kx;                   // the elements' channel and filter tap, carried from step to step
     {
@@ -125,69 +141,90 @@ conv_igemm_kernel(const IgemmArgs a) {
             copy16(da + (((tid >> 2) + j * (NT / 4)) * kALd + kq) * 4, src, ok ? tail_a : 0);
         }
 #pragma unroll
-        for (int j = 0; j < B_COPIES; ++j) {
-            if (TRANSB) {
-                const int n = n0 + (tid >> 2) + j * (NT / 4), r = r_next + kq;
-                const bool ok = n < a.n_b && r < a.R;
-                copy16(db + (((tid >> 2) + j * (NT / 4)) * kALd + kq) * 4, ok ? a.w + (long)n * a.ldb + r : a.w,
-                       ok ? min(4, a.R - r) * 4 : 0);
-            } else {
-                const int idx = tid + j * NT, kr = idx / (BN / 4), nc = idx % (BN / 4) * 4;
-                const int n = n0 + nc, r = r_next + kr;
-                const bool ok = n < a.n_b && r < a.R;
-                copy16(db + (kr * BN + nc) * 4, ok ? a.w + (long)r * a.ldb + n : a.w, ok ? min(4, a.n_b - n) * 4 : 0);
-            }
+        for (int j = 0; j < (TRANSB ? 0 : B_COPIES); ++j) {
+            const int idx = tid + j * NT, kr = idx / (BN / 4), nc = idx % (BN / 4) * 4;
+            const int n = n0 + nc, r = r_next + kr;
+            const bool ok = n < a.n_b && r < a.R;
+            copy16(db + (kr * BN + nc) * 4, ok ? a.w + (long)r * a.ldb + n : a.w, ok ? min(4, a.n_b - n) * 4 : 0);
         }
         r_next += kBK;
         c += kBK;
         while (c >= a.Cp) { c -= a.Cp; if (++kx == a.kernel) { kx = 0; ++ky; } }
     };
 
-    const int tx = tid % TX, ty = tid / TX;      // rows ty + i * TY; columns tx * 4 and BN / 2 + tx * 4
-    unsigned long long acc[8][4];
+    // A transposed B is turned over on its way into the ring: this thread's 16-byte pieces (four reduction elements of a
+    // column) wait in registers for a step and are then stored down their columns; columns trade places in groups of
+    // eight with the reduction index, so that a warp stores to different banks.
+    float4 held[TRANSB ? B_COPIES : 1];
+    auto fetch_b = [&](int step) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int j = 0; j < (TRANSB ? B_COPIES : 0); ++j) {
+            const int n = n0 + ((tid + j * NT) >> 2), r = (first + step) * kBK + kq;
+            held[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* src = a.w + (long)n * a.ldb + r;
+            if (n < a.n_b && r + 3 < a.R) {
+                held[j] = __ldg(reinterpret_cast<const float4*>(src));
+            } else if (n < a.n_b) {                              // what lies past the end of a row is not ours to read
+                if (r < a.R) held[j].x = __ldg(src);
+                if (r + 1 < a.R) held[j].y = __ldg(src + 1);
+                if (r + 2 < a.R) held[j].z = __ldg(src + 2);
+            }
+        }
+    };
+    auto put_b = [&](int stage) {
+        float* sb = smem + stage * (A_FLOATS + B_FLOATS) + A_FLOATS + kq * BN;
+#pragma unroll
+        for (int j = 0; j < (TRANSB ? B_COPIES : 0); ++j) {
+            const int col = ((tid + j * NT) >> 2) ^ (2 * kq);
+            sb[col] = held[j].x; sb[BN + col] = held[j].y; sb[2 * BN + col] = held[j].z; sb[3 * BN + col] = held[j].w;
+        }
+    };
+
+    // rows ty + i * TY; columns tx * 4 and BN / 2 + tx * 4, four each
+    const int tx = tid % TX, ty = tid / TX;
+    unsigned long long acc[TM][4];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 
 #pragma unroll
     for (int p = 0; p < kStages - 1; ++p) {
-        if (p < count) load_step(p);
+        if (p < count) {
+            load_step(p);
+            if (TRANSB) { fetch_b(p); put_b(p); }
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    if (TRANSB && kStages - 1 < count) fetch_b(kStages - 1);
     int stage = 0;
     for (int t = 0; t < count; ++t) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         __syncthreads();             // this step's tiles are complete, and everyone is done with the stage refilled next
-        if (t + kStages - 1 < count) load_step(stage == 0 ? kStages - 1 : stage - 1);
+        if (t + kStages - 1 < count) {
+            const int free = stage == 0 ? kStages - 1 : stage - 1;
+            load_step(free);
+            if (TRANSB) {
+                put_b(free);
+                if (t + kStages < count) fetch_b(t + kStages);
+            }
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* sa = smem + stage * (A_FLOATS + B_FLOATS);
         const float* sb = sa + A_FLOATS;
 #pragma unroll
         for (int k2 = 0; k2 < kBK; k2 += 2) {
-            float2 av[8];
+            float2 av[TM];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float2*>(sa + (ty + i * TY) * kALd + k2);
-            float2 bt[8];
-            if (TRANSB) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    bt[j] = *reinterpret_cast<const float2*>(sb + ((j >> 2) * (BN / 2) + tx * 4 + (j & 3)) * kALd + k2);
-            }
+            for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const float2*>(sa + (ty + i * TY) * kALd + k2);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                unsigned long long b[4];
-                if (TRANSB) {
+                const int swap = TRANSB ? (k2 + k) / 4 * 8 : 0;
+                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(sb + (k2 + k) * BN + ((tx * 4) ^ swap));
+                const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(sb + (k2 + k) * BN + ((BN / 2 + tx * 4) ^ swap));
+                const unsigned long long b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        b[j] = k ? pack2(bt[2 * j].y, bt[2 * j + 1].y) : pack2(bt[2 * j].x, bt[2 * j + 1].x);
-                } else {
-                    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(sb + (k2 + k) * BN + tx * 4);
-                    const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(sb + (k2 + k) * BN + BN / 2 + tx * 4);
-                    b[0] = b0.x; b[1] = b0.y; b[2] = b1.x; b[3] = b1.y;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < TM; ++i) {
                     const float u = k ? av[i].y : av[i].x;
                     const unsigned long long uu = pack2(u, u);
 #pragma unroll
@@ -198,59 +235,73 @@ conv_igemm_kernel(const IgemmArgs a) {
         if (++stage == kStages) stage = 0;
     }
 
-    if (splits == 1) {
+    // Few rows a thread: finished and stored from registers.
+    if (TM == 2 && splits == 1) {
+        const float4 bias[2] = {row_bias(a, n0 + tx * 4), row_bias(a, n0 + BN / 2 + tx * 4)};
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float2 p = unpack2(acc[i][h * 2]), q = unpack2(acc[i][h * 2 + 1]);
-                store4(a, m0 + ty + i * TY, n0 + h * (BN / 2) + tx * 4, make_float4(p.x, p.y, q.x, q.y));
+                store4(a, m0 + ty + i * TY, n0 + h * (BN / 2) + tx * 4, make_float4(p.x, p.y, q.x, q.y), bias[h]);
             }
         return;
     }
-    // split reduction: the ring is idle now and takes the partial tile
+    // Else the ring, idle now, takes the partial tile, from which bands of rows - the whole tile, or of a split reduction
+    // this block's share of it, summed over the cluster - are finished and stored row by row: from registers, the 64 copies
+    // of bias and activation were more instructions than a short reduction.
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     float4* part = reinterpret_cast<float4*>(smem);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const float2 p = unpack2(acc[i][h * 2]), q = unpack2(acc[i][h * 2 + 1]);
             part[(ty + i * TY) * (BN / 4) + h * (BN / 8) + tx] = make_float4(p.x, p.y, q.x, q.y);
         }
-    cluster_sync();
-    const int band = BM / splits * (BN / 4);     // float4s of this block's rows
-    for (int i = tid; i < band; i += NT) {
-        const int at = rank * band + i;
-        const uint32_t addr = smem_addr(part + at);
-        float4 sum = load_cluster(addr, 0);
-        for (int p = 1; p < splits; ++p) {
-            const float4 v = load_cluster(addr, (uint32_t)p);
-            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    static_assert(NT % (BN / 4) == 0, "a thread stays on its columns");
+    const int n = n0 + tid % (BN / 4) * 4, band = BM / splits;
+    const float4 bias = row_bias(a, n);
+    if (splits == 1) __syncthreads();
+    else cluster_sync();
+#pragma unroll 2
+    for (int i = tid / (BN / 4); i < band; i += NT / (BN / 4)) {
+        const int row = rank * band + i;
+        const float4* at = part + row * (BN / 4) + tid % (BN / 4);
+        float4 sum;
+        if (splits == 1) {
+            sum = *at;
+        } else {
+            const uint32_t addr = smem_addr(at);
+            sum = load_cluster(addr, 0);
+            for (int p = 1; p < splits; ++p) {
+                const float4 v = load_cluster(addr, (uint32_t)p);
+                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            }
         }
-        store4(a, m0 + at / (BN / 4), n0 + at % (BN / 4) * 4, sum);
+        store4(a, m0 + row, n, sum, bias);
     }
-    cluster_sync();                              // no block leaves while another still reads its partial tile
+    if (splits > 1) cluster_sync();                              // no block leaves while another still reads its partial tile
 }
 
-template <int BM, int BN, bool TRANSB, typename Pixel = int>
+template <int BM, int BN, int TM, bool TRANSB, typename Pixel = unsigned>
 int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
-    constexpr size_t ring = (size_t)kStages * (BM * kALd + (TRANSB ? BN * kALd : kBK * BN)) * sizeof(float);
+    constexpr size_t ring = (size_t)kStages * (BM * kALd + kBK * BN) * sizeof(float);
     constexpr size_t tile = (size_t)BM * BN * sizeof(float);
-    const size_t smem = splits > 1 && tile > ring ? tile : ring;
+    constexpr size_t smem = tile > ring ? tile : ring;
     static thread_local int attr_device = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<BM, BN, TRANSB, Pixel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(tile > ring ? tile : ring));
+        cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<BM, BN, TM, TRANSB, Pixel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(div_up(a.M, BM), div_up(a.n_store, BN), splits);
-    cfg.blockDim = dim3(BM * BN / 64);
+    cfg.blockDim = dim3(BM * BN / (8 * TM));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -258,29 +309,43 @@ int launch(const IgemmArgs& a, int splits, cudaStream_t s) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = splits;
     cfg.attrs = attr;
     cfg.numAttrs = splits > 1 ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, conv_igemm_kernel<BM, BN, TRANSB, Pixel>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, conv_igemm_kernel<BM, BN, TM, TRANSB, Pixel>, a);
     if (e != cudaSuccess) { set_last_error(e); (void)cudaGetLastError(); return OGLE_ERR_CUDA; }
     return finish_launch();
 }
 
 }  // namespace
 
-// Tile and split. The large tiles read the least through L2 per multiply-add and are taken where they alone give
-// every SM its two (128 x 128) or four (128 x 64) resident blocks; 128 x 32 serves narrow outputs over many rows.
-// Everything else runs on 64 x 64 tiles with the reduction split so that the SMs fill: the cost of a split is
-// (blocks on the busiest SM, at least the four that keep its FP32 pipes busy) x (steps of a block, plus about six
-// for its start, its partial tile and the cluster's barriers).
+// Tile and split. Reductions of up to 64 elements are bound by their instructions before and after the multiplies and take
+// the 2 x 8 form; up to 128 it pays where it gives an SM one to three tiles (fewer are better split, 126 x 116 x 24 4.5 us
+// against 9.0; more make better large tiles, 52288 x 108 x 508 177 against 214). The large tiles read the least through L2
+// per multiply-add and are taken where they alone give every SM its two (128 x 128) or four (128 x 64) resident blocks,
+// the larger only where the SM with the most of them ends no later (1419 x 557 x 3436: 324 of them, two on most SMs and
+// three on some, 190 us, 153 in halves); 128 x 32 serves narrow outputs over many rows. Everything else runs on 64 x 64
+// tiles, 64 x 32 for narrow outputs, with the reduction split so that the SMs fill: the cost of a split is (blocks on the
+// busiest SM, at least the four that keep its FP32 pipes busy) x (steps of a block, plus about six for its start, its
+// partial tile and the cluster's barriers).
 int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s) {
     const long m128 = (a.M + 127) / 128, m64 = (a.M + 63) / 64;
     if (m64 > 0x7fffffffL || (a.n_store + 63) / 64 > 65535) return OGLE_ERR_UNSUPPORTED;
-    const bool large = a.M / ((long)a.Ho * a.Wo) * a.H * a.W > 0x7fffffffL;       // (one image of 2^31 pixels or more)
-    if (!trans_b && !large) {
-        if (a.n_store > 64 && m128 * ((a.n_store + 127) / 128) >= 2 * kNumSMs && (a.n_store % 128 == 0 || a.n_store % 128 > 64))
-            return launch<128, 128, false>(a, 1, s);
-        if (a.n_store > 32 && m128 * ((a.n_store + 63) / 64) >= 4 * kNumSMs) return launch<128, 64, false>(a, 1, s);
-        if (a.n_store <= 32 && m128 >= 4 * kNumSMs) return launch<128, 32, false>(a, 1, s);
+    const bool large = a.M > 0x7fffffffL || a.M / ((long)a.Ho * a.Wo) * a.H * a.W > 0x7fffffffL;
+    const long tiles64 = m64 * ((a.n_store + 63) / 64);
+    if (!large && (a.R <= 64 || (a.R <= 128 && tiles64 >= kNumSMs && tiles64 <= 3 * kNumSMs))) {
+        if (trans_b) return launch<64, 64, 2, true>(a, 1, s);
+        return a.n_store <= 32 ? launch<64, 32, 2, false>(a, 1, s) : launch<64, 64, 2, false>(a, 1, s);
     }
-    const long tiles = m64 * ((a.n_store + 63) / 64);
+    if (!large) {
+        const long wide = m128 * ((a.n_store + 127) / 128), half = m128 * ((a.n_store + 63) / 64);
+        // (the SM with the most tiles sets the time)
+        const bool wide_ends_first = 2 * ((wide + kNumSMs - 1) / kNumSMs) <= (half + kNumSMs - 1) / kNumSMs;
+        if (a.n_store > 64 && wide >= 2 * kNumSMs && wide_ends_first)
+            return trans_b ? launch<128, 128, 8, true>(a, 1, s) : launch<128, 128, 8, false>(a, 1, s);
+        if (a.n_store > 32 && half >= 4 * kNumSMs)
+            return trans_b ? launch<128, 64, 8, true>(a, 1, s) : launch<128, 64, 8, false>(a, 1, s);
+        if (a.n_store <= 32 && m128 >= 4 * kNumSMs && !trans_b) return launch<128, 32, 8, false>(a, 1, s);
+    }
+    const bool narrow = a.n_store <= 32 && !trans_b && !large;
+    const long tiles = narrow ? m64 : tiles64;
     const int steps = (a.R + kBK - 1) / kBK;
     int best = 1;
     double best_cost = -1.0;
@@ -289,8 +354,9 @@ int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s) {
         const double cost = (blocks < 4 ? 4.0 : blocks) * ((steps + k - 1) / k + 6.0);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = k; }
     }
-    if (large) return launch<64, 64, false, long>(a, best, s);
-    return trans_b ? launch<64, 64, true>(a, best, s) : launch<64, 64, false>(a, best, s);
+    if (large) return launch<64, 64, 8, false, long>(a, best, s);
+    if (narrow) return launch<64, 32, 4, false>(a, best, s);
+    return trans_b ? launch<64, 64, 8, true>(a, best, s) : launch<64, 64, 8, false>(a, best, s);
 }
 
 }  // namespace ogle

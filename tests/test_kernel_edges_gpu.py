@@ -166,6 +166,31 @@ def test_fp32_gemm_edges(oracle_port, m, k, n, trans_b):
     close(got, oracle_port.gemm(A, B, Cm, trans_b, 0.5, 2.0))
 
 
+@pytest.mark.parametrize("m,k,n,trans_b", [
+    # two rows a thread: tiles of 64 x 64 and 64 x 32, up to 64 elements and, with one to three tiles an SM, up to 128
+    (300, 64, 77, 0), (300, 63, 31, 0), (5000, 117, 100, 0), (77, 62, 90, 1), (5000, 101, 90, 1),
+    # narrow outputs, alone and split over clusters
+    (2000, 300, 31, 0), (130, 1030, 30, 0),
+    # a transposed B: 64 x 64 alone and split, 128 x 128, 128 x 64, a reduction shorter than the ring
+    (700, 90, 700, 1), (60, 2050, 130, 1), (4700, 70, 1000, 1), (9600, 70, 520, 1), (9600, 65, 520, 1),
+    # 128 x 64 where 128 x 128 would leave one tile too many on some SMs
+    (1419, 131, 3435, 0)])
+def test_fp32_contraction_forms(m, k, n, trans_b):
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    pad = lambda t: torch.nn.functional.pad(t, (0, ops.up4(t.shape[-1]) - t.shape[-1]), value=float("nan"))     # never to be read
+    a, b = torch.randn((m, k), generator=g, device="cuda"), torch.randn((n, k) if trans_b else (k, n), generator=g, device="cuda")
+    c = torch.randn(n, generator=g, device="cuda")
+    got = ops.gemm(pad(a), pad(b), torch.nn.functional.pad(c, (0, ops.up4(n) - n)), m, k, n, trans_b, 0.5, 2.0, 2, ops.MATH_FP32)
+    b64 = b.double().t() if trans_b else b.double()
+    want = 0.5 * (a.double() @ b64) + 2.0 * c.double()
+    # every partial sum rounded once: at most k * 2^-24 of the sum of the terms' magnitudes
+    bound = (k + 4) * 2.0 ** -24 * (0.5 * (a.abs().double() @ b64.abs()) + 2.0 * c.abs().double())
+    assert ((got[:, :n].double() - want).abs() <= bound).all()
+    assert (got[:, n:] == 0).all()
+
+
 def test_fp32_gemm_of_many_columns():
     """Up to 65535 column tiles of 64."""
     import torch
