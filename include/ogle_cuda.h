@@ -77,6 +77,17 @@ int ogle_cuda_device_status_detail(void);
  * Captured CUDA graphs keep what was in force when they were captured. */
 int ogle_cuda_set_overlapped_launches(int on);
 
+/* How the calling thread's latest tensor-core contraction (a convolution or gemm) was laid out, for tests and reports;
+ * zeros before the first. */
+typedef struct {
+    int form;        /* 1 whole tiles; 2 ranges of the reduction combined through memory; 3 ranges added up inside a
+                        cluster; 4 tiles on pairs of SMs; 5 channels on M */
+    int ranges;      /* ranges of the reduction (1 = not split) */
+    int n_tile;      /* output channels of a tile */
+    int overlapped;  /* 1: allowed to start its set-up while the launch before it drains */
+} OgleContraction;
+int ogle_cuda_last_contraction(OgleContraction* out);
+
 /* How many times a role of the tensor-core kernels polls for its turn before it gives up, for
  * the launches that follow on any stream (process-wide). polls < 0 restores the default (2^22,
  * tens of milliseconds); 0 makes every such wait give up at once. It exists to exercise the

@@ -46,6 +46,10 @@ class ConcatParams(C.Structure):
     _fields_ = [("n_inputs", C.c_int), ("axis", C.c_int), ("in_shapes", (C.c_int * 4) * OGLE_MAX_CONCAT_INPUTS)]
 
 
+class Contraction(C.Structure):
+    _fields_ = [("form", C.c_int), ("ranges", C.c_int), ("n_tile", C.c_int), ("overlapped", C.c_int)]
+
+
 class DetectParams(C.Structure):
     _fields_ = [
         ("N", C.c_int), ("A", C.c_int), ("C", C.c_int), ("logit_stride", C.c_int), ("mode", C.c_int),
@@ -59,6 +63,7 @@ _vp = C.c_void_p
 CUDA_SYMBOLS = {
     "ogle_cuda_status_string": (C.c_char_p, [C.c_int]),
     "ogle_cuda_set_wait_limit": (C.c_int, [C.c_long]),
+    "ogle_cuda_last_contraction": (C.c_int, [C.POINTER(Contraction)]),
     "ogle_cuda_build_info": (C.c_char_p, []),
     "ogle_cuda_launch_count": (C.c_uint64, []),
     "ogle_cuda_last_error": (C.c_char_p, []),

@@ -33,9 +33,17 @@ void set_last_error(const char* s) {
     for (; s[i] && i < 255; ++i) g_last_error[i] = s[i];
     g_last_error[i] = 0;
 }
+namespace { thread_local OgleContraction g_contraction = {}; }
+void note_contraction(int form, int ranges, int n_tile, bool overlapped) { g_contraction = {form, ranges, n_tile, overlapped ? 1 : 0}; }
 }  // namespace ogle
 
 extern "C" {
+
+int ogle_cuda_last_contraction(OgleContraction* out) {
+    if (!out) return OGLE_ERR_INVALID;
+    *out = ogle::g_contraction;
+    return OGLE_OK;
+}
 
 const char* ogle_cuda_status_string(int status) {
     switch (status) {

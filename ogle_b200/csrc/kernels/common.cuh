@@ -53,6 +53,7 @@ __device__ __forceinline__ void grid_dependency_trigger() { asm volatile("gridde
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 bool overlapped_launches_enabled();
+void note_contraction(int form, int ranges, int n_tile, bool overlapped);     // for ogle_cuda_last_contraction
 void set_overlapped_launches(int on);
 
 template <typename... KArgs, typename... Args>

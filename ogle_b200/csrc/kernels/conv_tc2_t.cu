@@ -522,6 +522,7 @@ int launch_tc_t(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, const
         sms = cudaGetDeviceProperties(&prop, dev) == cudaSuccess ? prop.multiProcessorCount : kNumSMs;
     }
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
+    note_contraction(5, t.split_k < 1 ? 1 : t.split_k, t.BN, overlapped_launches_enabled());
     if (t.res)
         launch_overlapped(conv_tc2_t_kernel<true>, dim3(grid), dim3(kThreadsT), kBudget, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else

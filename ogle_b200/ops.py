@@ -28,6 +28,13 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
+def last_contraction():
+    """Form, ranges, tile width and overlap of this thread's latest tensor-core convolution or gemm."""
+    out = _lib.Contraction()
+    check(_lib.cuda_lib().ogle_cuda_last_contraction(C.byref(out)), "last_contraction")
+    return out
+
+
 def up4(v):
     return (v + 3) // 4 * 4
 

@@ -225,7 +225,9 @@ def test_fp32_convolution_of_an_image_of_2_to_the_31_pixels():
     # N, H, W, C, K, kernel, stride, pad, act, split: one tile over 2-8 blocks, ranges of unequal length, rows and columns
     # that end inside a tile, several tiles, three tile widths
     (1, 7, 7, 512, 30, 3, 1, 1, 0, 8), (1, 9, 11, 100, 129, 3, 2, 1, 2, 3), (2, 19, 19, 256, 75, 3, 1, 1, 1, 5), (1, 1, 1, 96, 4, 1, 1, 0, 2, 3),
-    (3, 20, 17, 64, 510, 1, 1, 0, 2, 2), (1, 40, 150, 48, 33, 5, 1, 2, 0, 7), (5, 3, 3, 160, 257, 1, 1, 0, 0, 4)])
+    (3, 20, 17, 64, 510, 1, 1, 0, 2, 2), (1, 40, 150, 48, 33, 5, 1, 2, 0, 7), (5, 3, 3, 160, 257, 1, 1, 0, 0, 4),
+    # ranges of two, two and one chunk; a map cut along the width
+    (5, 3, 3, 160, 257, 1, 1, 0, 0, 3), (1, 12, 75, 48, 33, 5, 1, 2, 0, 4)])
 @pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
 def test_reduction_split_inside_a_cluster(oracle_port, shape, math):
     """Into a channel slice of a wider tensor, alone and with a residual operand; the same sums on every call."""
@@ -238,15 +240,20 @@ def test_reduction_split_inside_a_cluster(oracle_port, shape, math):
     b = rng.standard_normal(K, dtype=np.float32)
     p = ops.conv_params(N, H, W, C, K, k, s, pd, 1, 1, True, act, -0.5, 1.5, getattr(ops, math))
     p.split = split
+    # (60 tiles of the map that is 150 wide are more clusters of seven blocks than fit, and no scratch is lent; five
+    # chunks do not make four ranges)
+    form = (1, 1) if W == 150 or (C == 160 and split == 4) else (3, split)
     packed = ops.conv2d_prepack(p, ops.dense_to_device(w))
     x4, b4 = ops.upload(x), ops.dense_to_device(b)
     if act != 1:
         res = rng.standard_normal((N,) + tuple(p.out_hwc), dtype=np.float32)
         fused = ops.conv2d_residual(p, x4, packed, b4, ops.upload(res))
+        assert (ops.last_contraction().form, ops.last_contraction().ranges) == form
     p.out_channel_stride, p.out_channel_offset = ops.up4(K) + 8, 4
     outs = [torch.full((N, p.out_hwc[0], p.out_hwc[1], ops.up4(K) + 8), -7.0, device="cuda") for _ in range(2)]
     for out in outs:
         ops.conv2d(p, x4, packed, b4, out, workspace=None)
+        assert (ops.last_contraction().form, ops.last_contraction().ranges) == form
     assert torch.equal(outs[0], outs[1])
     got = outs[0].cpu().numpy()
     assert (got[..., :4] == -7).all() and (got[..., 4 + ops.up4(K):] == -7).all() and (got[..., 4 + K:4 + ops.up4(K)] == 0).all()
@@ -273,6 +280,8 @@ def test_gemm_over_clusters(m, k, n, bias_mode, math):
     pad = lambda t: torch.nn.functional.pad(t, (0, ops.up4(k) - k)).cuda()
     mode = getattr(ops, math)
     got = ops.gemm_ws(pad(a), pad(b), c4, m, k, n, 1, 0.5, 2.0 if bias_mode else 0.0, bias_mode, mode)
+    # (five chunks gain nothing, and a split-mode result may not move as far as it would with a cut of 4096 elements)
+    assert ops.last_contraction().form == (1 if k == 130 or (k == 4096 and mode == ops.MATH_TF32X3) else 3)
     want = 0.5 * (a.double() @ b.double().t()) + (2.0 * c.double() if bias_mode else 0.0)
     err = (got[:, :n].cpu().double() - want).norm() / want.norm()
     # k/8 + k/16 truncated additions to a sum, each off by at most 2^-23 of it, 2^-24 on average: k * 1.1e-8 in an
@@ -309,3 +318,76 @@ def test_tile_choice_keeps_the_sums(oracle_port, shape):
             fused.append(ops.conv2d_residual(p, x4, packed, b4, res))
         assert torch.equal(outs[0], outs[1]) and torch.equal(fused[0], fused[1])
         assert np.abs(ops.download(outs[0], K)[:1] - ref).max() <= tol * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("m,k,n", [(256, 1024, 300), (2560, 512, 1024), (64, 4096, 512), (3000, 96, 200)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_products_queued_on_one_workspace(m, k, n, math):
+    """Each call's packing pass overwrites what the product before it reads, and each product starts its set-up while the
+    packing pass before it still runs: six of them queued without a wait between, each against its own packed B."""
+    import torch
+    from ogle_b200 import ops
+    mode = getattr(ops, math)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a = torch.randn((m, k), generator=g, device="cuda")
+    bs = [torch.randn((k, n), generator=g, device="cuda") for _ in range(6)]
+    packs = [ops.gemm_pack_b(b, m, k, n, 0, mode) for b in bs]
+    wants = [ops.gemm_packed(a, p, None, m, k, n, 0, 1.0, 0.0, 0, mode) for p in packs]
+    workspace = torch.empty_like(packs[0])
+    torch.cuda.synchronize()
+    gots = [ops.gemm_ws(a, b, None, m, k, n, 0, 1.0, 0.0, 0, mode, workspace=workspace) for b in bs]
+    for got, want in zip(gots, wants):
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("width", [75, 90, 150])
+def test_cut_tiles_with_channels_on_m(oracle_port, width):
+    """Maps cut along the width in the channels-on-M form, whose residual operand is then found pixel by pixel, and with
+    two outputs: the bits of the plain form."""
+    import torch
+    from ogle_b200 import ops
+    N, H, C, K = 3, 41, 64, 70
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, w, b, res = rand(N, H, width, C), rand(K, C, 3, 3) / 24.0, rand(K), rand(N, H, width, ops.up4(K))
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        outs = []
+        for on_m in (1, 2):
+            p = ops.conv_params(N, H, width, C, K, 3, 1, 1, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, math)
+            p.split, p.channels_on_m, p.sm_pair = 1, on_m, 1
+            packed = ops.conv2d_prepack(p, w)
+            outs += [ops.conv2d(p, x, packed, b, workspace=None), ops.conv2d_residual(p, x, packed, b, res)]
+            assert ops.last_contraction().form == (5 if on_m == 2 else 1)
+        assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3])
+        one, two = ops.conv2d_pair(x, w[:24], b[:24], w[24:64], b[24:64], N, H, width, C, 3, 1, 1, 1, ops.ACT_RELU, 0.0, 0.0, math,
+                                   use_workspace=False)
+        assert torch.equal(one, outs[0][..., :24]) and torch.equal(two, outs[0][..., 24:64])
+
+
+def test_bounded_waits_of_the_cluster_form(oracle_port):
+    """Zero polls allowed: every block of a cluster gives up, all meet at the cluster's barriers, the launch returns with
+    the status word set, and with the limit restored the same call gives what it gave before."""
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, w, b = rand(1, 9, 9, 256), rand(80, 256, 3, 3) / 48.0, rand(80)
+    assert lib.ogle_cuda_device_status() == 0
+    try:
+        for math in (ops.MATH_TF32, ops.MATH_TF32X3):
+            p = ops.conv_params(1, 9, 9, 256, 80, 3, 1, 1, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, math)
+            p.split = 6
+            packed = ops.conv2d_prepack(p, w)
+            want = ops.conv2d(p, x, packed, b, workspace=None)
+            lib.ogle_cuda_set_wait_limit(0)
+            ops.conv2d(p, x, packed, b, workspace=None)
+            assert ops.last_contraction().form == 3
+            assert lib.ogle_cuda_device_status() == -6 and 1 <= lib.ogle_cuda_device_status_detail() <= 7
+            assert lib.ogle_cuda_clear_device_status() == 0
+            lib.ogle_cuda_set_wait_limit(-1)
+            assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), want)
+            assert lib.ogle_cuda_device_status() == 0
+    finally:
+        lib.ogle_cuda_set_wait_limit(-1)
+        lib.ogle_cuda_clear_device_status()
