@@ -116,18 +116,22 @@ typedef struct {
     int n_tile;              /* tensor-core path: output channels per tile (a multiple of 32, at most
                                 256 and round_up(K,32)); 0 = chosen by the library. Results do not
                                 depend on it bit for bit (each output value sums its reduction in the
-                                same order); a caller may time the candidates and keep the fastest. */
+                                same order: the ranges of `split` are settled without a look at it, or at
+                                sm_pair); a caller may time the candidates and keep the fastest. */
     int split;               /* tensor-core path: ranges the reduction is split into (1 = not split, up to
-                                16; more than 2, or any with an activation, needs the scratch of
-                                ogle_cuda_conv2d_ws); 0 = chosen by the library. Unlike n_tile this changes the
-                                order in which a value's partial sums are added. */
+                                16); 0 = chosen by the library. Two to eight ranges of a launch of few tiles
+                                are added up inside a cluster of SMs; any other number, and launches of more
+                                tiles than such clusters fit, need the scratch of ogle_cuda_conv2d_ws, except
+                                for two ranges without an activation. A number that cannot be served is
+                                replaced by the library's own. Unlike n_tile this changes the order in which a
+                                value's partial sums are added. */
     int channels_on_m;       /* tensor-core path, at most 128 output channels, unsplit reduction: 2 = keep the
                                 accumulator transposed (filters on the 128-row side of the multiply, 256 pixels per
                                 instruction), which halves the tensor-core instructions of layers with 64-128 output
                                 channels; 1 = no, 0 = chosen by the library. Ignored where it cannot run. */
     int sm_pair;             /* tensor-core path: 2 = compute tiles of 256 pixels on pairs of SMs (each SM of a
                                 pair loads half of the filter tile; needs n_tile a multiple of 64 and an unsplit
-                                reduction, else ignored), 1 = one SM per tile, 0 = chosen by the library.
+                                reduction - chosen or asked for by split = 1 - else ignored), 1 = one SM per tile, 0 = chosen by the library.
                                 Results do not depend on it bit for bit. */
 } OgleConvParams;
 
@@ -168,8 +172,9 @@ int ogle_cuda_conv2d_residual(const OgleConvParams* p, const float* x, const voi
  * and few output tiles - 3x3 heads on small feature maps, the whole network at batch 1 - then split
  * their reduction over up to 16 blocks per tile: each block stores its partial tile into its own
  * slice of the scratch and a second small kernel adds the slices in a fixed order, then bias and
- * activation (bit-reproducible; any activation). Without scratch such layers split in two at
- * most, and only without an activation. The scratch may be reused as soon as the stream has
+ * activation (bit-reproducible; any activation); or, up to eight ranges of a few tiles, the blocks of a
+ * tile form a cluster and add up their partial tiles in that order by themselves, without the scratch.
+ * Without scratch launches that do not fit such clusters split in two at most, and only without an activation. The scratch may be reused as soon as the stream has
  * passed this call. */
 size_t ogle_cuda_conv2d_workspace_bytes(const OgleConvParams* p);
 int ogle_cuda_conv2d_ws(const OgleConvParams* p, const float* x, const void* packed_filter, const float* bias,

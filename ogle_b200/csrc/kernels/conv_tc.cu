@@ -177,12 +177,12 @@ void cut_tiles(const ConvArgs& a, long cols, TcArgs* t, long* m_tiles) {
 // clusters have to fit the GPU at once (a block takes a whole SM; the GPU is asked how many clusters of a size fit), and
 // the model has to see a tenth less time than in one piece: rounds of chunks, a block's start, fill and drain, and the
 // cluster's barriers and exchange of partial tiles.
-// n_tile, split: the caller's choice (0 = any). otherwise: the ranges that the launch would have in its other forms.
+// split: the caller's choice (0 = any). otherwise: the ranges that the launch would have in its other forms.
 // Where the caller leaves the number open, a split-mode result must not move by more than 8e-6 of its norm with it: sums
 // in tensor memory are truncated, and results in k and in `otherwise` ranges of a reduction over R elements differ by
 // 6e-9 * R * |1/k - 1/otherwise| (R = 512: 2.4e-6, R = 1500: 6.0e-6; the shorter ranges are the more exact).
 // 1000 x 1500 x 700 gemm: 32.8 -> 28.8 us with its packing pass (24.6 with that pass as it is now); MobileNet-SSD, one frame: 374 -> 335 us.
-bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int split, int otherwise) {
+bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int split, int otherwise) {
     if (!split_k_enabled() || t->gather || split == 1 || split > 8 || m_tiles > kNumSMs / 2) return false;
     const int* capacity = tc_cluster_capacity();
     const int kmax = (Kp + 31) / 32 * 32;
@@ -190,7 +190,7 @@ bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int n_tile, int
     const long tiles0 = m_tiles * t->n_tiles;
     double best = otherwise > 1 || split ? 1e30 : 0.9 * ((tiles0 + kNumSMs - 1) / kNumSMs * (chunks * chunk(t->BN)) + 4.5 + kTailUs * t->BN);
     int best_bn = 0, best_k = 0;
-    for (int bn = n_tile ? n_tile : 32; bn <= (n_tile ? n_tile : 256) && bn <= kmax; bn += 32) {
+    for (int bn = 32; bn <= 256 && bn <= kmax; bn += 32) {
         const long tiles = m_tiles * ((Kp + bn - 1) / bn);
         for (int k = split ? split : 2; k <= (split ? split : 8); ++k) {
             const int cps = (chunks + k - 1) / k;
@@ -433,9 +433,11 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.tiles_h = (a.Ho + t.th - 1) / t.th;
         m_tiles = (long)t.tiles_w * t.tiles_h * ((a.N + t.tn - 1) / t.tn);
     }
-    choose_n_tiling_v2(a.Kp, m_tiles, &t, a.n_tile,
-                       (plan_only || (ws != nullptr && aligned16(ws))) && !t.gather && split_k_enabled() &&
-                           taps * t.chunks_per_tap >= 16);
+    // How many ranges the reduction has is settled at the library's own tile width, whatever width or form the caller
+    // asks for: those change how a launch is laid out, not the order in which a value's products are added.
+    const bool wide_ties = (plan_only || (ws != nullptr && aligned16(ws))) && !t.gather && split_k_enabled() &&
+                           taps * t.chunks_per_tap >= 16;
+    choose_n_tiling_v2(a.Kp, m_tiles, &t, 0, wide_ties);
     // Split the reduction when whole tiles would leave SMs idle (few tiles) or a last round
     // mostly empty. Two forms, for reductions that do not fit clusters (below):
     //  - through scratch memory (the caller lent some): any number of ranges and any activation;
@@ -448,11 +450,11 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     t.split_k = 1;
     const int chunks = t.kernel * t.kernel * t.chunks_per_tap;
     const double tiles = (double)m_tiles * t.n_tiles;
-    const int ws_cols = t.n_tiles * t.BN;
     // rows (flat form) or images between consecutive slices: whole tiles, so that a tile that
     // hangs over the end of its slice writes padding, not the next slice
     const long slice_units = t.flat ? m_tiles * kTileM : (long)((a.N + t.tn - 1) / t.tn) * t.tn;
-    const size_t slice_bytes = (size_t)(t.flat ? slice_units : slice_units * a.Ho * a.Wo) * ws_cols * sizeof(float);
+    const size_t slice_rows = (size_t)(t.flat ? slice_units : slice_units * a.Ho * a.Wo);
+    size_t slice_bytes = slice_rows * (t.n_tiles * t.BN) * sizeof(float);
     if (split_k_enabled() && chunks >= 8 && !residual) {      // (a residual operand is added by whole tiles only)
         // cost of the layer in units of one reduction chunk of one tile: rounds of one work item per SM,
         // each item paying its chunks plus a fixed fill / drain of about four chunks
@@ -493,21 +495,41 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         while (t.split_k > 1 && (t.split_k - 1) * cps >= chunks) --t.split_k;     // no empty ranges
         if (t.split_k == 1) t.ws_mode = 0;
     }
-    bool on_pairs = want_pair(t, m_tiles, a.pair);
+    const TcArgs own = t;
+    const bool wish = a.n_tile >= 32 && a.n_tile <= (a.Kp + 31) / 32 * 32;      // (a wider tile than the layer is no wish)
+    if (wish) {
+        choose_n_tiling_v2(a.Kp, m_tiles, &t, a.n_tile, wide_ties);
+        const size_t wished = slice_rows * (t.n_tiles * t.BN) * sizeof(float), most = (size_t)192 << 20;
+        if (t.ws_mode && wished * t.split_k > (plan_only || ws_bytes > most ? most : ws_bytes)) t = own;
+        else slice_bytes = wished;
+    }
+    const int ws_cols = t.n_tiles * t.BN;
     const bool on_m = want_channels_on_m(t, a.Kp, m_tiles, a.on_m);
     const bool tiled = variant != CONV_POINTWISE && !t.gather;       // tiles of image pieces
+    bool on_pairs = false;
     // (the scratch a layer asks for does not depend on whether the launch then splits inside clusters instead)
-    // How many ranges a reduction has, and so its bits, is settled on whole-row tiles; an unsplit launch is then free to cut
-    // its tiles and choose their width and form, and so is one that splits inside clusters.
+    // The ranges are settled on whole-row tiles; an unsplit launch is then free to cut its tiles and choose their width
+    // and form, and so is one that splits inside clusters.
     if (!plan_only) {
-        TcArgs c = t;
+        TcArgs c = own;
         long cut = m_tiles;
         if (tiled) cut_tiles(a, (a.Kp + 127) / 128, &c, &cut);
-        const bool cluster = !(a.on_m == 2 && t.ws_mode) && !on_m && !on_pairs &&
-                             choose_cluster(&c, a.Kp, cut, chunks, a.n_tile, a.split, t.split_k);
+        bool cluster = !(a.on_m == 2 && t.ws_mode) && !on_m && choose_cluster(&c, a.Kp, cut, chunks, a.split, own.split_k);
+        if (cluster && wish) {
+            c.BN = t.BN;
+            c.n_tiles = t.n_tiles;
+            // as many ranges, in more clusters than fit at once: through scratch where that is lent (the same bits)
+            if (t.ws_mode && t.split_k == c.split_k && cut * c.n_tiles > tc_cluster_capacity()[c.split_k]) cluster = false;
+        } else if (!cluster) {
+            c.BN = t.BN;
+            c.n_tiles = t.n_tiles;
+        }
         if (cluster || t.split_k <= 1) { t = c; m_tiles = cut; }
-        if (!cluster && t.split_k <= 1 && !a.n_tile && !a.pair && !on_m)
-            on_pairs = refine_width(&t, a.Kp, m_tiles, chunks, !residual && pair_mode_override() != 1);
+        if (!cluster) {
+            on_pairs = want_pair(t, m_tiles, a.pair);
+            if (t.split_k <= 1 && !wish && !a.pair && !on_m)
+                on_pairs = refine_width(&t, a.Kp, m_tiles, chunks, !residual && pair_mode_override() != 1);
+        }
     }
     auto make_tile_maps = [&] {
         const cuuint64_t dims[4] = {(cuuint64_t)a.Cp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
@@ -654,7 +676,7 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
     const bool v2 = true;
     const long m_tiles = (p.M + kTileM - 1) / kTileM;
     choose_n_tiling_v2(t.Kp, m_tiles, &t);
-    const bool on_pairs = !choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 0, 1) &&
+    const bool on_pairs = !choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 1) &&
                           refine_width(&t, t.Kp, m_tiles, t.chunks_per_tap, pair_mode_override() != 1);
     t.y = Y; t.y_ld = p.ldy;
     CUtensorMap mA, mBhi, mBlo, mY;

@@ -259,8 +259,8 @@ public:
 
     // The tensor-core path's tile width (output channels per tile) decides how many tiles a layer has, how
     // deep its operand ring is and how long a tile's epilogue takes; which width wins depends on the batch
-    // (rounds of tiles over the SMs) in ways a cost model only approximates. Every width gives the same bits,
-    // so the layer simply times the candidates on its own tensors and keeps the fastest; then, at that width, the
+    // (rounds of tiles over the SMs) in ways a cost model only approximates. Every width gives the same bits
+    // (the library settles the ranges of the reduction before it looks at the width), so the layer simply times the candidates on its own tensors and keeps the fastest; then, at that width, the
     // number of ranges its reduction is split into (which does change the order of the partial sums); last, for
     // an unsplit reduction, whether pairs of SMs should share the filter tiles (same bits again).
     void Tune() override {

@@ -391,3 +391,30 @@ def test_bounded_waits_of_the_cluster_form(oracle_port):
     finally:
         lib.ogle_cuda_set_wait_limit(-1)
         lib.ogle_cuda_clear_device_status()
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel: few tiles, whose reductions the library splits by itself inside clusters or through scratch
+    (1, 19, 19, 512, 512, 1), (1, 10, 10, 1024, 150, 3), (2, 7, 7, 512, 512, 3), (1, 19, 19, 128, 300, 3), (4, 14, 14, 256, 256, 3),
+    (1, 38, 38, 256, 90, 1)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_width_and_form_do_not_touch_the_sums(shape, math):
+    """n_tile and sm_pair change how a launch is laid out, not its results, also where the library chooses the number of
+    ranges of the reduction: with an activation and no scratch, with scratch, with a residual operand, two outputs."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K, k = shape
+    g = torch.Generator(device="cuda").manual_seed(C + K)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, w, b, res = rand(N, H, W, C), rand(K, C, k, k) / (C * k * k) ** 0.5, rand(K), rand(N, H, W, ops.up4(K))
+    lent = torch.empty(48 << 18, device="cuda")
+    first = None
+    for n_tile, pair in ((0, 0), (32, 0), (64, 0), (96, 1), (128, 0), (256, 0), (64, 2), (256, 2), (0, 2)):
+        p = ops.conv_params(N, H, W, C, K, k, 1, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, getattr(ops, math))
+        p.n_tile, p.sm_pair = n_tile, pair
+        packed = ops.conv2d_prepack(p, w)
+        outs = [ops.conv2d(p, x, packed, b, workspace=None), ops.conv2d(p, x, packed, b, workspace=lent),
+                ops.conv2d_residual(p, x, packed, b, res)]
+        first = first or outs
+        for a, c in zip(first, outs):
+            assert torch.equal(a, c), (n_tile, pair)
