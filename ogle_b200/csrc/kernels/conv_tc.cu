@@ -178,9 +178,10 @@ void cut_tiles(const ConvArgs& a, long cols, TcArgs* t, long* m_tiles) {
 // the model has to see a tenth less time than in one piece: rounds of chunks, a block's start, fill and drain, and the
 // cluster's barriers and exchange of partial tiles.
 // split: the caller's choice (0 = any). otherwise: the ranges that the launch would have in its other forms.
-// Where the caller leaves the number open, a split-mode result must not move by more than 8e-6 of its norm with it: sums
-// in tensor memory are truncated, and results in k and in `otherwise` ranges of a reduction over R elements differ by
-// 6e-9 * R * |1/k - 1/otherwise| (R = 512: 2.4e-6, R = 1500: 6.0e-6; the shorter ranges are the more exact).
+// Where the caller leaves the number open, there are never fewer ranges than otherwise: sums in tensor memory are truncated,
+// so that a range's error grows with its length (6e-9 of the result's norm per element in split mode), and results are to
+// be as exact as in the launch's other forms. Nor do they move by more than 8e-6 of their norm against those: k and
+// `otherwise` ranges of a reduction over R elements differ by 6e-9 * R * |1/k - 1/otherwise| (R = 512: 2.4e-6, R = 1500: 6.0e-6).
 // 1000 x 1500 x 700 gemm: 32.8 -> 28.8 us with its packing pass (24.6 with that pass as it is now); MobileNet-SSD, one frame: 374 -> 335 us.
 bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int split, int otherwise) {
     if (!split_k_enabled() || t->gather || split == 1 || split > 8 || m_tiles > kNumSMs / 2) return false;
@@ -195,6 +196,7 @@ bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int split, int 
         for (int k = split ? split : 2; k <= (split ? split : 8); ++k) {
             const int cps = (chunks + k - 1) / k;
             if ((k - 1) * cps >= chunks || tiles > capacity[k]) continue;
+            if (!split && k < otherwise) continue;
             if (!split && t->passes == 3 && chunks * kChunk * fabs(1.0 / k - 1.0 / otherwise) > 1330.0) continue;
             const double cost = cps * chunk(bn) + 5.7 + (kTailUs + 0.004) * bn;
             if (cost < best) { best = cost; best_bn = bn; best_k = k; }

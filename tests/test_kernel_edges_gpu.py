@@ -418,3 +418,35 @@ def test_width_and_form_do_not_touch_the_sums(shape, math):
         first = first or outs
         for a, c in zip(first, outs):
             assert torch.equal(a, c), (n_tile, pair)
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, C, K, kernel: heads and late layers whose reductions go through scratch in 2 to 16 ranges
+    (1, 10, 1024, 150, 3), (8, 10, 1024, 150, 3), (1, 19, 512, 75, 3), (4, 5, 512, 150, 3), (4, 7, 512, 512, 3), (8, 10, 512, 1024, 1),
+    (1, 5, 820, 100, 5), (2, 3, 256, 126, 3), (8, 10, 1024, 256, 1)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_clusters_do_not_take_longer_ranges(shape, math):
+    """With scratch lent, a reduction that is added up inside clusters instead has at least as many ranges as the scratch
+    was planned for (sums in tensor memory lose with their length), and is no further from 64 bits."""
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    N, H, ch, K, k = shape
+    g = torch.Generator(device="cuda").manual_seed(ch + K)
+    x = torch.rand((N, H, H, ch), generator=g, device="cuda")
+    w = torch.randn((K, ch, k, k), generator=g, device="cuda") / (ch * k * k) ** 0.5 + 0.02
+    want = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), w.double(), padding=k // 2).permute(0, 2, 3, 1)
+    need = _lib.cuda_lib().ogle_cuda_conv2d_workspace_bytes
+
+    def run(split):
+        p = ops.conv_params(N, H, H, ch, K, k, 1, k // 2, 1, 1, False, ops.ACT_RELU, 0.0, 0.0, getattr(ops, math))
+        p.split = split
+        y = ops.conv2d(p, x, ops.conv2d_prepack(p, w))
+        want_act = want.clamp(min=0)
+        return ops.last_contraction().ranges, float((y[..., :K].double() - want_act).norm() / want_act.norm()), need(C.byref(p))
+
+    ranges, err, planned = run(0)
+    planned = round(planned * 4 / max(run(4)[2], 1)) if planned else 1
+    assert ranges >= planned, (ranges, planned)
+    # (two numbers of ranges that round alike differ by their remainders only)
+    assert err <= 1.05 * run(planned)[1] + 1e-8
