@@ -85,13 +85,15 @@ void choose_n_tiling_v2(int Kp, long m_tiles, TcArgs* t, int requested = 0, bool
         // narrower one when everything fits in one round (more SMs busy, shorter epilogues)
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && (rounds > 1 || wide_ties))) { best_cost = cost; best_bn = bn; }
     }
-    static const int forced = [] { const char* e = getenv("OGLE_TC_BN"); return e ? atoi(e) : 0; }();      // experiments
-    if (const int v = forced) {
-        if (v >= 32 && v <= 256 && v % 32 == 0 && v <= kmax) best_bn = v;
-    }
     if (requested >= 32 && requested <= 256 && requested % 32 == 0 && requested <= kmax) best_bn = requested;
     t->BN = best_bn;
     t->n_tiles = (Kp + best_bn - 1) / best_bn;
+}
+
+// Tile width that the environment forces on layers it fits, 0 = none (experiments).
+int forced_width(int Kp) {
+    static const int v = [] { const char* e = getenv("OGLE_TC_BN"); return e ? atoi(e) : 0; }();
+    return v >= 32 && v <= 256 && v % 32 == 0 && v <= (Kp + 31) / 32 * 32 ? v : 0;
 }
 
 // Two-SM form (conv_tc2_pair.cu): 0 = the built-in rule, 1 = never, 2 = wherever it can run.
@@ -223,10 +225,9 @@ bool want_channels_on_m(const TcArgs& t, int Kp_total, long m_tiles, int request
     return mode == 2 || requested == 2;
 }
 
-// Whether a launch takes the two-SM form: it can (no gather, no split reduction, a tile width that
-// halves into multiples of 32 columns, at least one pair of tiles) and either the caller asked for it
-// or the rule holds: wide tiles, a reduction long enough that operand traffic dominates, and enough
-// pairs of tiles for two rounds of the GPU's SM pairs.
+// Whether a launch takes the two-SM form because the caller or the environment asked for it: it can (no gather, no split
+// reduction, a tile width that halves into multiples of 32 columns, at least one pair of tiles). Where neither asks,
+// refine_width decides.
 bool want_pair(const TcArgs& t, long m_tiles, int requested) {
     if (t.gather || t.split_k > 1 || t.ws_mode || t.BN % 64 || m_tiles < 2) return false;
     const int mode = pair_mode_override();
@@ -498,9 +499,10 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         if (t.split_k == 1) t.ws_mode = 0;
     }
     const TcArgs own = t;
-    const bool wish = a.n_tile >= 32 && a.n_tile <= (a.Kp + 31) / 32 * 32;      // (a wider tile than the layer is no wish)
+    // (a wider tile than the layer is no wish)
+    const int wish = a.n_tile >= 32 && a.n_tile <= (a.Kp + 31) / 32 * 32 ? a.n_tile : forced_width(a.Kp);
     if (wish) {
-        choose_n_tiling_v2(a.Kp, m_tiles, &t, a.n_tile, wide_ties);
+        choose_n_tiling_v2(a.Kp, m_tiles, &t, wish, wide_ties);
         const size_t wished = slice_rows * (t.n_tiles * t.BN) * sizeof(float), most = (size_t)192 << 20;
         if (t.ws_mode && wished * t.split_k > (plan_only || ws_bytes > most ? most : ws_bytes)) t = own;
         else slice_bytes = wished;
@@ -516,7 +518,9 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         TcArgs c = own;
         long cut = m_tiles;
         if (tiled) cut_tiles(a, (a.Kp + 127) / 128, &c, &cut);
-        bool cluster = !(a.on_m == 2 && t.ws_mode) && !on_m && choose_cluster(&c, a.Kp, cut, chunks, a.split, own.split_k);
+        // (the environment's SM pairs, "wherever they can run", come before the cluster form)
+        const bool forced_pairs = !residual && pair_mode_override() == 2 && want_pair(t, m_tiles, a.pair);
+        bool cluster = !(a.on_m == 2 && t.ws_mode) && !on_m && !forced_pairs && choose_cluster(&c, a.Kp, cut, chunks, a.split, own.split_k);
         if (cluster && wish) {
             c.BN = t.BN;
             c.n_tiles = t.n_tiles;
@@ -529,7 +533,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         if (cluster || t.split_k <= 1) { t = c; m_tiles = cut; }
         if (!cluster) {
             on_pairs = want_pair(t, m_tiles, a.pair);
-            if (t.split_k <= 1 && !wish && !a.pair && !on_m)
+            if (t.split_k <= 1 && !wish && !a.pair && !on_m && !forced_pairs)
                 on_pairs = refine_width(&t, a.Kp, m_tiles, chunks, !residual && pair_mode_override() != 1);
         }
     }
@@ -678,8 +682,18 @@ static int launch_gemm_common(const OgleGemmParams& p, const float* A, const flo
     const bool v2 = true;
     const long m_tiles = (p.M + kTileM - 1) / kTileM;
     choose_n_tiling_v2(t.Kp, m_tiles, &t);
-    const bool on_pairs = !choose_cluster(&t, t.Kp, m_tiles, t.chunks_per_tap, 0, 1) &&
-                          refine_width(&t, t.Kp, m_tiles, t.chunks_per_tap, pair_mode_override() != 1);
+    const int forced = forced_width(t.Kp);
+    if (forced) choose_n_tiling_v2(t.Kp, m_tiles, &t, forced);
+    bool on_pairs = pair_mode_override() == 2 && want_pair(t, m_tiles, 0);
+    if (!on_pairs) {
+        TcArgs c = t;
+        if (choose_cluster(&c, t.Kp, m_tiles, t.chunks_per_tap, 0, 1)) {
+            if (forced) { c.BN = t.BN; c.n_tiles = t.n_tiles; }
+            t = c;
+        } else if (!forced) {
+            on_pairs = refine_width(&t, t.Kp, m_tiles, t.chunks_per_tap, pair_mode_override() != 1);
+        }
+    }
     t.y = Y; t.y_ld = p.ldy;
     CUtensorMap mA, mBhi, mBlo, mY;
     const cuuint64_t dims[4] = {(cuuint64_t)p.K, (cuuint64_t)p.M, 1, 1};

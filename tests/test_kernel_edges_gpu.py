@@ -450,3 +450,40 @@ def test_clusters_do_not_take_longer_ranges(shape, math):
     assert ranges >= planned, (ranges, planned)
     # (two numbers of ranges that round alike differ by their remainders only)
     assert err <= 1.05 * run(planned)[1] + 1e-8
+
+
+@pytest.mark.parametrize("name,value", [("OGLE_TC_PAIR", "1"), ("OGLE_TC_PAIR", "0"), ("OGLE_TC_BN", "64"), ("OGLE_TC_BN", "192")])
+def test_forced_forms_are_the_ones_that_run(name, value):
+    """The switches for measurements are read once per process: convolutions, with and without a residual operand, and
+    gemms of launches that would otherwise take clusters, pairs or another width."""
+    import subprocess
+    code = """
+import os, torch
+from ogle_b200 import ops
+name, value = %r, %r
+for N, H, C, K, k in ((1, 19, 512, 512, 1), (16, 38, 256, 512, 1), (4, 20, 64, 256, 3), (2, 30, 40, 192, 3)):
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        p = ops.conv_params(N, H, H, C, K, k, 1, k // 2, 1, 1, True, 2, 0.0, 0.0, math)
+        p.n_tile = 64 if name == "OGLE_TC_PAIR" else 0        # (pairs need a width that halves)
+        packed = ops.conv2d_prepack(p, torch.randn((K, C, k, k), device="cuda"))
+        x, b = torch.randn((N, H, H, C), device="cuda"), torch.randn(K, device="cuda")
+        ops.conv2d(p, x, packed, b, workspace=None)
+        seen = [ops.last_contraction()]
+        if name == "OGLE_TC_BN":
+            ops.conv2d_residual(p, x, packed, b, torch.randn((N, H, H, K), device="cuda"))
+            seen.append(ops.last_contraction())
+        if k == 1 and value != "1":
+            a, w = x.reshape(-1, C), torch.randn((K, C), device="cuda")
+            ops.gemm_packed(a, ops.gemm_pack_b(w, a.shape[0], C, K, 1, math), None, a.shape[0], C, K, 1, 1.0, 0.0, 0, math)
+            seen.append(ops.last_contraction())
+        for s in seen:
+            if name == "OGLE_TC_BN":
+                assert s.n_tile == int(value), (N, H, K, s.form, s.n_tile)
+            elif value == "0":
+                assert s.form != 4
+            else:
+                assert s.form == 4, (N, H, K, s.form, s.n_tile)
+""" % (name, value)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, **{name: value}), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
