@@ -208,6 +208,14 @@ __device__ __forceinline__ float4 result_box(const DetectArgs& a, const float4* 
     return a.anchors ? decode_box(b, a.anchors[anchor], a.var) : b;
 }
 
+// The smaller of a score and one. NaN stays NaN and is no candidate: rows with a NaN logit, or with an exponential that
+// overflows (inf / inf), have no scores, by either rule. (fminf would give them one in every class.)
+__device__ __forceinline__ float at_most_one(float s) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(s), "f"(1.0f));
+    return r;
+}
+
 // A row of at most 32 logits in registers by 128-bit loads, its exponentials taken once.
 __device__ __forceinline__ void load_row(const DetectArgs& a, const float* row, float (&e)[32]) {
     const float4* row4 = reinterpret_cast<const float4*>(row);
@@ -267,7 +275,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
                 const float inv = 1.0f / total;
 #pragma unroll
                 for (int j = 1; j < 32; ++j)
-                    if (j >= c0 && j < c0 + nc) put(j - c0, i, fminf(e[j] * inv, 1.0f));
+                    if (j >= c0 && j < c0 + nc) put(j - c0, i, at_most_one(e[j] * inv));
             }
         } else {
             for (int i = tid; i < a.A; i += blockDim.x) {
@@ -275,7 +283,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
                 float total = 0.f;
                 for (int j = 0; j < a.C; ++j) total += expf(row[j]);
                 const float inv = 1.0f / total;
-                for (int j = 0; j < nc; ++j) put(j, i, fminf(expf(row[c0 + j]) * inv, 1.0f));
+                for (int j = 0; j < nc; ++j) put(j, i, at_most_one(expf(row[c0 + j]) * inv));
             }
         }
         __syncthreads();

@@ -113,6 +113,38 @@ def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
         assert (anchor[n, k:] == -1).all()
 
 
+@pytest.mark.parametrize("anchors,classes", [(200, 5), (200, 40)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_detect_drops_rows_without_scores(mode, anchors, classes):
+    """NaN logits, and logits whose exponentials overflow (their quotients are inf / inf): no class of such an anchor is a
+    candidate, in rows held in registers and in longer ones."""
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator().manual_seed(classes)
+    z = torch.randn((1, anchors, classes), generator=g)
+    z[0, 7, 2] = float("nan")
+    z[0, 31, 0] = float("nan")
+    z[0, 50, 1] = 95.0
+    z[0, 51, :] = 89.0
+    z[0, 77, 3] = float("inf")
+    z[0, 78, 1] = float("-inf")           # a class that cannot be, the others have scores
+    e = torch.exp(z[0])
+    s = e / e.sum(1, keepdim=True)
+    bad = {7, 31, 50, 51, 77}
+    logits = torch.nn.functional.pad(z, (0, ops.up4(classes) - classes)).cuda()
+    boxes = torch.zeros((1, anchors, 4), device="cuda")
+    thr = 1e-4
+    score, anchor, cls, box, count = [t.cpu() for t in ops.ssd_detect(logits, boxes, classes, mode, thr, 256, 0.0, 300, 300)]
+    for c in range(1, classes) if mode else (0,):
+        rows = slice((c - 1) * 256, c * 256) if mode else slice(0, 256)
+        n = int(count.flatten()[c - 1 if mode else 0])
+        got = anchor.flatten()[rows][:n].tolist()
+        v = s[:, c] if mode else s[:, 1:].max(1).values
+        want = {i for i in range(anchors) if i not in bad and v[i] > thr}
+        edge = {i for i in range(anchors) if i not in bad and abs(v[i] - thr) < 1e-6}
+        assert set(got) ^ want <= edge and not set(got) & bad
+
+
 @pytest.mark.parametrize("batch,anchors,classes,mode", [
     (1, 56444, 2, 1), (149, 56444, 2, 1), (1, 55548, 3, 1), (148, 53756, 5, 1), (1, 39420, 21, 1), (1, 27774, 2, 0), (200, 27774, 3, 0)])
 def test_detect_takes_the_largest_anchor_counts(oracle_port, batch, anchors, classes, mode):
