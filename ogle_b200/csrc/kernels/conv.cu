@@ -249,7 +249,7 @@ const char* ogle_cuda_conv2d_kernel_name(const OgleConvParams* p) {
     if (fill_args(p, &a, &variant) != OGLE_OK) return "";
     if (served_by_tc(p, a, variant)) return "conv_tc2_kernel";
     if (variant == CONV_DEPTHWISE) {
-        if (dw_tma_supported(a)) return a.kernel == 3 ? "dw3x3_tma_kernel" : "dw5x5_tma_kernel";
+        if (dw_tma_supported(a)) return "dw_tma_kernel";
         return (a.kernel == 3 && a.dil == 1 && (a.stride == 1 || a.stride == 2)) ? "dw3x3_kernel" : "dw_generic_kernel";
     }
     if (variant == CONV_GROUPED) return "grouped_kernel";

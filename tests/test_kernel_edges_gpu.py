@@ -519,3 +519,23 @@ for N, H, C, K, k in ((1, 19, 512, 512, 1), (16, 38, 256, 512, 1), (4, 20, 64, 2
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, **{name: value}), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("case", [
+    # C, K, kernel, stride, group, math, size
+    (64, 64, 3, 1, 64, 2, 40), (50, 50, 5, 2, 50, 2, 40), (64, 64, 3, 1, 64, 2, 3), (64, 64, 7, 1, 64, 2, 40), (64, 32, 3, 1, 4, 2, 40),
+    (3, 32, 3, 2, 1, 2, 40), (64, 64, 1, 1, 1, 0, 40), (64, 64, 1, 1, 1, 2, 40)])
+def test_kernel_names_are_those_of_the_sources(case):
+    """What a profile is filtered by is the name of a kernel that exists."""
+    import ctypes as C
+    import glob
+    import re
+    from ogle_b200 import _lib, ops
+    ci, k, f, s, g, math, size = case
+    p = ops.conv_params(1, size, size, ci, k, f, s, f // 2, 1, g, True, 0, 0.0, 0.0, math)
+    name = _lib.cuda_lib().ogle_cuda_conv2d_kernel_name(C.byref(p)).decode()
+    root = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ogle_b200", "csrc", "kernels")
+    kernels = set()
+    for path in glob.glob(os.path.join(root, "*.cu")):
+        kernels |= set(re.findall(r"__global__[^;{]*?\b(\w+)\s*\(\s*(?:const|CUtensorMap|float)", open(path).read()))
+    assert name in kernels
