@@ -20,12 +20,12 @@ namespace {
 // -1: not set by the caller. The environment, when it names a value, wins over the caller.
 std::atomic<int> g_overlapped{-1};
 }
-bool overlapped_launches_enabled() {
+bool overlapped_launches_enabled(bool asked_for) {
     // measured 5 % faster at one image per step, nothing at 32, 1-2 % slower at 256: off unless the
     // environment or the caller (a session whose tensors are small) turns it on
     static const int env = [] { const char* e = getenv("OGLE_PDL"); return e ? (e[0] == '1' ? 1 : 0) : -1; }();
     if (env >= 0) return env == 1;
-    return g_overlapped.load(std::memory_order_relaxed) == 1;
+    return asked_for || g_overlapped.load(std::memory_order_relaxed) == 1;
 }
 void set_overlapped_launches(int on) { g_overlapped.store(on ? 1 : 0, std::memory_order_relaxed); }
 void set_last_error(const char* s) {

@@ -52,7 +52,8 @@ inline int grid_for(long items, int threads, int max_per_sm = 8) {
 __device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-bool overlapped_launches_enabled();
+// asked_for: the launch wants it whatever the caller has set for launches in general (the environment still wins).
+bool overlapped_launches_enabled(bool asked_for = false);
 void note_contraction(int form, int ranges, int n_tile, bool overlapped);     // for ogle_cuda_last_contraction
 void set_overlapped_launches(int on);
 

@@ -940,7 +940,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     // 1.44 M 64 -> 128: 195 against 201, 184 against 188. At four chunks 128 -> 256 (0.37 M) it is 182-189 against 166.
     t.epi_share = t.total_work <= 4 * sms || chunks > 2 ? 1 : 0;
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
-    const bool overlapped = t.overlapped || overlapped_launches_enabled();
+    const bool overlapped = overlapped_launches_enabled(t.overlapped);
     note_contraction(t.cluster ? 3 : (t.split_k > 1 ? 2 : 1), t.split_k, t.BN, overlapped);
     if (t.cluster) {
         // every block one work item; the blocks of a tile are consecutive, and a cluster

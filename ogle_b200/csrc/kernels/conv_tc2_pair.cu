@@ -597,8 +597,9 @@ int launch_tc_pair(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, co
     if (!sms) sms = num_sms_for_pairs();
     int pairs = sms / 2;
     if (t.total_work < pairs) pairs = t.total_work;
-    note_contraction(4, 1, t.BN, overlapped_launches_enabled());
-    launch_overlapped(conv_tc2_pair_kernel, dim3((unsigned)(2 * pairs)), dim3(kThreadsP), kBudget, s, mA, mBhi, mBlo, mY, mY2, bias, t,
+    const bool overlapped = overlapped_launches_enabled(t.overlapped);
+    note_contraction(4, 1, t.BN, overlapped);
+    launch_overlapped_if(overlapped, conv_tc2_pair_kernel, dim3((unsigned)(2 * pairs)), dim3(kThreadsP), kBudget, s, mA, mBhi, mBlo, mY, mY2, bias, t,
                       err_flag);
     return finish_launch();
 }

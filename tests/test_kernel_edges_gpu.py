@@ -539,3 +539,26 @@ def test_kernel_names_are_those_of_the_sources(case):
     for path in glob.glob(os.path.join(root, "*.cu")):
         kernels |= set(re.findall(r"__global__[^;{]*?\b(\w+)\s*\(\s*(?:const|CUtensorMap|float)", open(path).read()))
     assert name in kernels
+
+
+@pytest.mark.parametrize("env,overlapped", [(None, 1), ("0", 0), ("1", 1)])
+def test_products_overlap_their_packing_pass_unless_told_otherwise(env, overlapped):
+    """gemm_ws in all its forms - clusters, pairs of SMs, whole tiles - asks for it; OGLE_PDL, read once per process, wins."""
+    import subprocess
+    code = """
+import torch
+from ogle_b200 import ops
+forms = set()
+for m, k, n in ((64, 512, 300), (25600, 512, 1024), (20000, 64, 100)):
+    a, b = torch.randn((m, k), device="cuda"), torch.randn((k, n), device="cuda")
+    ops.gemm_ws(a, b, None, m, k, n, 0, 1.0, 0.0, 0, ops.MATH_TF32X3)
+    last = ops.last_contraction()
+    forms.add(last.form)
+    assert last.overlapped == %d, (m, last.form, last.overlapped)
+assert forms == {1, 3, 4}, forms
+""" % overlapped
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    clean = {k: v for k, v in os.environ.items() if k != "OGLE_PDL"}
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(clean, **({"OGLE_PDL": env} if env else {})), capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
