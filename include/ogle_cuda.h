@@ -160,7 +160,8 @@ int ogle_cuda_conv2d(const OgleConvParams* p, const float* x, const void* packed
 /* y = act(conv(x, w) + bias + residual): the convolution, the Add of a residual block and the activation that
  * follows it in one pass (replaces the binary.glsl pass of nn/kernels/binary.cc and, with act != none, the relu.glsl /
  * clip.glsl pass after it; same fp32 operations in the same order as the separate passes, so the result is bit-identical
- * to them). residual: a tensor with the output's pixels, residual_stride floats per pixel (0 = round_up(K,4)), channel c of
+ * to them where both sum the reduction in the same ranges: always with split = 1; by itself, a convolution without an
+ * activation or with scratch may split where this one does not). residual: a tensor with the output's pixels, residual_stride floats per pixel (0 = round_up(K,4)), channel c of
  * the convolution at residual[pixel * residual_stride + c]. Served by the tensor-core path only
  * (ogle_cuda_conv2d_residual_supported: math_mode TF32 or TF32X3, >= 16 input channels); OGLE_ERR_UNSUPPORTED otherwise -
  * the caller then runs ogle_cuda_conv2d and ogle_cuda_add_act. */

@@ -3,17 +3,17 @@
 //
 // One block per SM slot walks a list of tiles. A tile is th x tw output pixels of
 // one image for a slab of 32 channels (16 where 32 would leave much of the last slab
-// empty; channels past the tensor arrive as zeros and are not stored); tw is the map's width when that is at most 32
-// (so 19- and 10-wide maps are covered without ragged column tiles), else 32 or 16. Its input window, halo included, is ONE TMA
-// box [IH rows][IW cols][32 channels]; pixels outside the image arrive as zeros,
+// empty; channels past the tensor arrive as zeros and are not stored); tw is the map's width up to 16, half of it up to
+// 32 (19 is 10 + 9), a third up to 48, else 32 or, at stride 2, 16. Its input window, halo included, is ONE TMA box
+// [IH rows][IW cols][channels of the slab]; pixels outside the image arrive as zeros,
 // which is the convolution's padding. A ring of two to four shared-memory stages: while
 // the block computes tile i from one stage, the TMA engine fills the others with the next tiles, so
 // the only HBM traffic is the input read once (halo rows come from L2) and the
 // output written once, both as 128-byte runs.
-// A thread owns 4 channels (one float4) of one output column and slides a 3-row
-// window down RPG output rows of it; 8 lanes cover one pixel's 128 bytes, so
-// shared-memory reads are conflict-free. The 32 pixel slots of a block are split into
-// 32 / tw row groups.
+// A thread owns 4 channels (one float4) of one output column and slides the window
+// down RPG output rows of it; 8 lanes cover one pixel's 128 bytes, so
+// shared-memory reads are conflict-free (slabs of 16 at stride 2 are not: two wavefronts).
+// The 32 pixel slots of a block (64 with slabs of 16) are split into row groups of tw.
 // Widths that are no multiple of 32 channels, and 5x5 windows, ran on kernels that fetch every
 // tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 25 us here (16 us floor).
 #include <cstdlib>
