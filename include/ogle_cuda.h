@@ -82,7 +82,7 @@ int ogle_cuda_set_overlapped_launches(int on);
  * zeros before the first. */
 typedef struct {
     int form;        /* 1 whole tiles; 2 ranges of the reduction combined through memory; 3 ranges added up inside a
-                        cluster; 4 tiles on pairs of SMs; 5 channels on M */
+                        cluster; 4 tiles on pairs of SMs; 5 channels on M; 6 taps of a filter row side by side */
     int ranges;      /* ranges of the reduction (1 = not split) */
     int n_tile;      /* output channels of a tile */
     int overlapped;  /* 1: allowed to start its set-up while the launch before it drains */
@@ -118,7 +118,9 @@ typedef struct {
                                 256 and round_up(K,32)); 0 = chosen by the library. Results do not
                                 depend on it bit for bit (each output value sums its reduction in the
                                 same order: the ranges of `split` are settled without a look at it, or at
-                                sm_pair); a caller may time the candidates and keep the fastest. */
+                                sm_pair); a caller may time the candidates and keep the fastest. Many-tile 3x3
+                                layers of stride 1 have tiles of 32 or 64 channels whatever is asked for, the
+                                taps of a filter row side by side. */
     int split;               /* tensor-core path: ranges the reduction is split into (1 = not split, up to
                                 16); 0 = chosen by the library. Two to eight ranges of a launch of few tiles
                                 are added up inside a cluster of SMs; any other number, and launches of more

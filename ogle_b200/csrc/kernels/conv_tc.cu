@@ -115,6 +115,63 @@ constexpr double kPairChunkUs[4] = {0.65, 0.675, 0.70, 0.71};
 // ... and of an epilogue, per column: in the shadow of the next tile's multiplies (two groups), and at the end.
 constexpr double kEpilogueUs = 0.018, kTailUs = 0.035;
 
+// Modelled time (us) of an unsplit launch in tiles of bn columns, and on SM pairs (split mode): rounds of tiles times the
+// measured time of a tile; pointwise layers, whose tiles are read once, wait more for L2.
+double whole_tiles_us(const TcArgs& t, int bn, int Kp, long m_tiles, int chunks) {
+    const long tiles = m_tiles * ((Kp + bn - 1) / bn);
+    // (one pass: 0.28 us up to 160 columns, bound by the copies, then by the multiplies)
+    const double chunk = t.passes == 3 ? kChunkUs[bn / 32 - 1] : (0.0016 * bn + 0.01 > 0.28 ? 0.0016 * bn + 0.01 : 0.28);
+    const double mul = chunks * chunk * (t.flat ? 1.25 : 1.0), epi = kEpilogueUs * bn;
+    return (double)((tiles + kNumSMs - 1) / kNumSMs) * (mul > epi ? mul : epi) + 4.5 + (t.passes == 3 ? kTailUs : 0.02) * bn;
+}
+double pair_tiles_us(const TcArgs& t, int bn, int Kp, long m_tiles, int chunks) {
+    const long work = (m_tiles + 1) / 2 * ((Kp + bn - 1) / bn);
+    const double mul = chunks * kPairChunkUs[bn / 64 - 1] * (t.flat ? 1.1 : 1.0), epi = kEpilogueUs * bn;
+    return (double)((work + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (mul > epi ? mul : epi) + 5.5 + kTailUs * bn;
+}
+
+// Channels of a tile whose taps lie side by side (kTaps form), 0 = the launch does not take it: 3x3, stride 1, padding 1,
+// where rounds of its tiles - 32 or 64 channels, a chunk and filter row at the measured time, and a longer epilogue - are
+// modelled to take less than whole tiles in their better form. OGLE_TC_TAPS: 0 never, 1 wherever it can run.
+int taps_width(const ConvArgs& a, const TcArgs& t, long m_tiles, int chunks) {
+    static const int mode = [] { const char* e = getenv("OGLE_TC_TAPS"); return e ? (e[0] == '0' ? 1 : (e[0] == '1' ? 2 : 0)) : 0; }();
+    if (mode == 1 || a.kernel != 3 || a.stride != 1 || a.pad != 1 || a.dil != 1 || a.M > 0x7fffff00L || !encode_im2col_fn()) return 0;
+    if (mode == 0 && (forced_width(a.Kp) || pair_mode_override() == 2)) return 0;        // (those switches come first)
+    double other = 1e30, best = 1e30;
+    for (int bn = 32; bn <= 256 && bn <= (a.Kp + 31) / 32 * 32; bn += 32) {
+        if (t.passes != 3 && bn != t.BN) continue;
+        const double one = whole_tiles_us(t, bn, a.Kp, m_tiles, chunks);
+        const double two = t.passes == 3 && m_tiles >= 2 && bn % 64 == 0 ? pair_tiles_us(t, bn, a.Kp, m_tiles, chunks) : one;
+        other = one < other ? one : other;
+        other = two < other ? two : other;
+    }
+    int width = 0;
+    for (int bn = 32; bn <= 64; bn += 32) {
+        const long tiles = (a.M + kTapsPixels - 1) / kTapsPixels * ((a.Kp + bn - 1) / bn);
+        // (a single round is mostly start, fill and drain; stacked siblings are padded to 32 channels each and seldom fill
+        // tiles of 64: in few rounds the model cannot tell which form is the better one)
+        if (mode == 0 && tiles <= (t.split_col ? 4 : 1) * kNumSMs) continue;
+        const double chunk = t.passes == 3 ? (bn == 64 ? 0.57 : 0.45) : (bn == 64 ? 0.33 : 0.28);
+        const double least = t.passes == 3 ? (bn == 64 ? 3.7 : 2.5) : (bn == 64 ? 3.1 : 2.2), tile = chunks / 3 * chunk + 1.0;
+        const double us = (double)((tiles + kNumSMs - 1) / kNumSMs) * (tile > least ? tile : least) + 7.0;
+        if (us < best) { best = us; width = bn; }
+    }
+    // (split mode, tensors that come from HBM: whole tiles take 1.08 of the model and 3 us more, 20-170 us measured)
+    if (t.passes == 3) other = 1.08 * other + 3.0;
+    return mode == 2 || best < 0.97 * other ? width : 0;
+}
+
+// Tiles of a launch whose taps lie side by side, bn channels each.
+long tile_taps(const ConvArgs& a, int bn, TcArgs* t) {
+    t->taps = 1;
+    t->oH = a.Ho; t->oW = a.Wo;
+    t->flat = 1; t->N = 1; t->Ho = 1; t->Wo = (int)a.M;
+    t->tn = 1; t->th = 1; t->tw = kTapsPixels;
+    t->BN = bn;
+    t->n_tiles = (a.Kp + bn - 1) / bn;
+    return (a.M + kTapsPixels - 1) / kTapsPixels;
+}
+
 // Width and form of an unsplit split-mode launch (the sums of an output value are the same in all of them): rounds of
 // tiles times the measured time of a tile; pointwise layers, whose tiles are read once, wait more for L2. true: on SM
 // pairs. 250 columns, 1350 elements, 14335 pixels: one tile of 256 columns 53.9 us, pairs 44.1, two tiles of 128 45.5;
@@ -122,16 +179,8 @@ constexpr double kEpilogueUs = 0.018, kTailUs = 0.035;
 bool refine_width(TcArgs* t, int Kp, long m_tiles, int chunks, bool may_pair) {
     if (t->passes != 3 || t->gather || chunks < 8) return false;      // (short reductions are bound by HBM and the epilogue)
     const int kmax = (Kp + 31) / 32 * 32;
-    auto one = [&](int bn) {
-        const long tiles = m_tiles * ((Kp + bn - 1) / bn);
-        const double mul = chunks * kChunkUs[bn / 32 - 1] * (t->flat ? 1.25 : 1.0), epi = kEpilogueUs * bn;
-        return (double)((tiles + kNumSMs - 1) / kNumSMs) * (mul > epi ? mul : epi) + 4.5 + kTailUs * bn;
-    };
-    auto pair = [&](int bn) {
-        const long work = (m_tiles + 1) / 2 * ((Kp + bn - 1) / bn);
-        const double mul = chunks * kPairChunkUs[bn / 64 - 1] * (t->flat ? 1.1 : 1.0), epi = kEpilogueUs * bn;
-        return (double)((work + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (mul > epi ? mul : epi) + 5.5 + kTailUs * bn;
-    };
+    auto one = [&](int bn) { return whole_tiles_us(*t, bn, Kp, m_tiles, chunks); };
+    auto pair = [&](int bn) { return pair_tiles_us(*t, bn, Kp, m_tiles, chunks); };
     double best = 0.97 * one(t->BN);
     int best_bn = t->BN;
     bool best_pair = false;
@@ -533,13 +582,30 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         if (cluster || t.split_k <= 1) { t = c; m_tiles = cut; }
         if (!cluster) {
             on_pairs = want_pair(t, m_tiles, a.pair);
-            if (t.split_k <= 1 && !wish && !a.pair && !on_m && !forced_pairs)
+            // (whether taps lie side by side is settled without a look at n_tile and sm_pair: it does touch the bits)
+            const int beside = t.split_k <= 1 && !a.on_m && tiled ? taps_width(a, own, m_tiles, chunks) : 0;
+            if (beside) {
+                m_tiles = tile_taps(a, beside, &t);
+                on_pairs = false;
+            } else if (t.split_k <= 1 && !wish && !a.pair && !on_m && !forced_pairs)
                 on_pairs = refine_width(&t, a.Kp, m_tiles, chunks, !residual && pair_mode_override() != 1);
         }
     }
     auto make_tile_maps = [&] {
         const cuuint64_t dims[4] = {(cuuint64_t)a.Cp, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
         const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
+        if (t.taps) {
+            // rows from the one above the image on; of its columns every one, whose neighbours meet in the accumulator
+            const int lower[2] = {0, -1}, upper[2] = {0, -1};
+            const cuuint32_t yb[4] = {kChunk, kTapsPixels, 1, 1}, ye[4] = {1, 1, 1, 1};
+            auto rows = [&](CUtensorMap* m, const float* p, int columns, int stride) {
+                const cuuint64_t d[4] = {(cuuint64_t)columns, (cuuint64_t)a.M, 1, 1};
+                const cuuint64_t st[3] = {(cuuint64_t)stride * 4, (cuuint64_t)stride * 4 * (cuuint64_t)a.M, (cuuint64_t)stride * 4 * (cuuint64_t)a.M};
+                return make_map(m, p, 4, d, st, yb, ye);
+            };
+            return make_map_im2col(&mA, x, dims, str, lower, upper, kChunk, kTileM) && rows(&mY, y + a.koff, kp_a, ks_a) &&
+                   (!y2 || rows(&mY2, y2, kp_b, kp_b));
+        }
         // the box spans the traversed input extent; one element in `stride` is taken
         const cuuint32_t box[4] = {kChunk, (cuuint32_t)((t.tw - 1) * a.stride + 1), (cuuint32_t)((t.th - 1) * a.stride + 1),
                                    (cuuint32_t)t.tn};
@@ -566,8 +632,16 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     const cuuint64_t bstr[1] = {bcols * 4};
     const cuuint32_t bbox[2] = {kChunk, (cuuint32_t)t.BN};
     const cuuint32_t bes[2] = {1, 1};
-    if (!make_map(&mBhi, w_hi, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
-    if (!make_map(&mBlo, w_lo, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
+    if (t.taps) {
+        // [channel][filter][tap]: a box takes the taps of a filter row one after the other
+        const cuuint64_t d[3] = {(cuuint64_t)t.Cp32, (cuuint64_t)Kp128, (cuuint64_t)taps};
+        const cuuint64_t st[2] = {bcols * 4, (cuuint64_t)t.Cp32 * 4};
+        const cuuint32_t b[3] = {kChunk, (cuuint32_t)t.BN, 3}, e[3] = {1, 1, 1};
+        if (!make_map(&mBhi, w_hi, 3, d, st, b, e) || !make_map(&mBlo, w_lo, 3, d, st, b, e)) return OGLE_ERR_CUDA;
+    } else {
+        if (!make_map(&mBhi, w_hi, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
+        if (!make_map(&mBlo, w_lo, 2, bdims, bstr, bbox, bes)) return OGLE_ERR_CUDA;
+    }
     if (t.cluster) {
         t.res = residual;
         t.res_ld = res_ld;

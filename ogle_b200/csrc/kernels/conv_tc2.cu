@@ -93,6 +93,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
         : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t taddr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+
 struct TileCoord { int n_tile, n0, h0, w0; };
 
 __device__ __forceinline__ TileCoord tile_coord(const TcArgs& a, int tile) {
@@ -101,7 +110,7 @@ __device__ __forceinline__ TileCoord tile_coord(const TcArgs& a, int tile) {
     const int m_tile = tile / a.n_tiles;
     c.n0 = 0; c.h0 = 0;
     if (a.flat) {
-        c.w0 = m_tile * kTileM;
+        c.w0 = m_tile * (a.taps ? kTapsPixels : kTileM);
     } else {
         const int tw_i = m_tile % a.tiles_w;
         const int t = m_tile / a.tiles_w;
@@ -118,13 +127,22 @@ struct WorkItem { int tile, ks, c_begin, c_end; };
 enum TcForm {
     kWhole = 0,       // a work item is a tile
     kRanges = 1,      // a range of a tile's reduction, combined through scratch or by reduce-add stores
-    kCluster = 2      // a range of a tile's reduction; the blocks of a cluster hold one tile's ranges and add them up
+    kCluster = 2,     // a range of a tile's reduction; the blocks of a cluster hold one tile's ranges and add them up
+    // A tile of a 3x3 convolution whose filter rows lie side by side: per filter row (ky) and 32 channels one multiply of
+    // 128 input pixels by [kx = 0 | 1 | 2] x BN channels; output pixel p is the sum of the first set's row p - 1, the
+    // second's row p and the third's row p + 1, which the epilogue brings together. A third of the activation copies and
+    // operand splits, and 3 BN columns a multiply: 64 channels alone leave the tensor cores half idle. With 64 channels a
+    // tile a split-mode chunk moves 144 KB through shared memory (copies 64, operand split 16, multiplies 64), at the
+    // 117 bytes a clock seen here 0.6 us, which is what it takes; a tile's epilogue adds about 1 us to that.
+    // Split mode, before and after: 128 x 56 x 56 x 64 -> 64 172 -> 114 us, 128 x 28 x 28 x 128 -> 128 107 -> 99,
+    // 128 x 14 x 14 x 256 -> 256 102 -> 96, 128 x 7 x 7 x 512 -> 512 114 -> 94; one pass, the first: 131 -> 82.
+    kTaps = 3
 };
 
 template <TcForm kForm>
 __device__ __forceinline__ WorkItem work_item(const TcArgs& a, int w, int chunks) {
     WorkItem it;
-    if (kForm == kWhole) {
+    if (kForm == kWhole || kForm == kTaps) {
         it.tile = w; it.ks = 0; it.c_begin = 0; it.c_end = chunks;
     } else {
         it.tile = w / a.split_k;
@@ -215,7 +233,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmY2, const float* __restrict__ bias, const TcArgs a, int* err_flag) {
     // 1024-byte alignment (the 128-byte swizzle atom) comes from the declaration, so that
     // every byte of the 224 KB request is usable
-    constexpr bool kSplit = kForm != kWhole;
+    constexpr bool kSplit = kForm == kRanges || kForm == kCluster;
+    constexpr int kSets = kForm == kTaps ? 3 : 1;       // of BN accumulator columns
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_xf[kMaxStages], bar_empty[kMaxStages];
     __shared__ __align__(8) uint64_t bar_acc_full[4], bar_acc_empty[4];
@@ -223,13 +242,15 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ int s_issued[2];                     // operand copies issued by the two producers (abort path)
-    __shared__ __align__(16) float s_bias[2][256];
-    __shared__ __align__(8) short s_goff[kMaxGatherK];   // gather form: window offset of each reduction index
+    __shared__ __align__(16) float s_bias[2][kForm == kTaps ? 64 : 256];
+    __shared__ __align__(8) short s_goff[kForm == kTaps ? 4 : kMaxGatherK];   // gather form: window offset of each reduction index
+    // taps side by side: the rows that the neighbouring warps of a group need, [group][warp][last or first row][column]
+    __shared__ __align__(16) float s_edge[kForm == kTaps ? 2 * 4 * 2 * 32 : 4];
 
     grid_dependency_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool split = a.passes == 3;
-    const uint32_t b_bytes = (uint32_t)a.BN * 128u;
+    const uint32_t b_bytes = (uint32_t)(a.BN * kSets) * 128u;
     // activation part of a stage (none where the gather form builds its operand in tensor memory)
     const uint32_t a_bytes = a.gather && a.ta ? 0u : (split && !a.ta ? 2u : 1u) * kABytes;
     const uint32_t stage_bytes = a_bytes + (split ? 2u : 1u) * b_bytes + (a.gather ? (uint32_t)a.g_bytes : 0u);
@@ -254,8 +275,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
 
-    const int chunks = a.kernel * a.kernel * a.chunks_per_tap;
-    const int acc_cols = a.BN;     // tensor-memory columns of one accumulator
+    const int chunks = (kForm == kTaps ? 1 : a.kernel) * a.kernel * a.chunks_per_tap;
+    const int acc_cols = a.BN * kSets;     // tensor-memory columns of one accumulator
     const int rows_in_tile = a.flat ? kTileM : a.tn * a.th * a.tw;
     volatile int* abort_flag = &s_abort;
 
@@ -282,7 +303,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         s_issued[0] = 0; s_issued[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (a.gather) {
+    if (kForm != kTaps && a.gather) {
         // reduction index k = (ky * kernel + kx) * C + c -> float offset of that value in the
         // [g_ih][g_iw][4] input window relative to the output pixel's first tap; -1 = padding column
         const int kred = a.g_k * a.g_k * a.g_C;
@@ -304,7 +325,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = tmem_slot;
-    const uint32_t tmem_a = tmem_d + (uint32_t)(a.n_acc * acc_cols);      // A operands in tensor memory: 64 columns per stage
+    const uint32_t tmem_a = tmem_d + (uint32_t)(a.n_acc * acc_cols);      // A operands in tensor memory: 64 (32) columns per stage
     // barriers, tensor memory and tables are set up; what follows reads and writes global memory
     grid_dependency_wait();
 
@@ -321,8 +342,18 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord(a, wi.tile);
-                const int ax = a.flat ? tc_.w0 : tc_.w0 * a.stride - a.pad;
-                const int ay = a.flat ? 0 : tc_.h0 * a.stride - a.pad;
+                int ax, ay, an;
+                if constexpr (kForm == kTaps) {
+                    // from the pixel before the first output pixel on
+                    const int p = tc_.w0 > 0 ? tc_.w0 - 1 : 0, line = p / a.oW;
+                    an = line / a.oH;
+                    ax = p - line * a.oW;
+                    ay = line - an * a.oH - 1;
+                } else {
+                    ax = a.flat ? tc_.w0 : tc_.w0 * a.stride - a.pad;
+                    ay = a.flat ? 0 : tc_.h0 * a.stride - a.pad;
+                    an = tc_.n0;
+                }
                 // position of the first chunk: filter row, filter column, channel offset
                 int ky = 0, kx = 0, c0 = 0;
                 if (kSplit && wi.c_begin != 0) {      // only the later ranges of a split reduction pay the divisions
@@ -336,16 +367,17 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (!ok) { record_error(err_flag, 1); break; }
                     if (a.gather) {
                         mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
-                        tma_load_4d(sWin(s), &tmA, &bar_full[s], 0, ax, ay, tc_.n0);
+                        tma_load_4d(sWin(s), &tmA, &bar_full[s], 0, ax, ay, an);
                     } else {
                         mbar_expect_tx(&bar_full[s], tx);
-                        tma_load_4d(sA(s), &tmA, &bar_full[s], c0, ax + kx * a.dil, ay + ky * a.dil, tc_.n0);
+                        if constexpr (kForm == kTaps) tma_load_im2col(sA(s), &tmA, &bar_full[s], c0, ax, ay, an, 0, ky);
+                        else tma_load_4d(sA(s), &tmA, &bar_full[s], c0, ax + kx * a.dil, ay + ky * a.dil, an);
                     }
                     ++issued;
                     if (++s == a.stages) { s = 0; ++wrap; }
                     // next chunk: channels fastest, then filter column, then filter row
                     c0 += kChunk;
-                    if (c0 == a.Cp32) { c0 = 0; if (++kx == a.kernel) { kx = 0; ++ky; } }
+                    if (c0 == a.Cp32) { c0 = 0; if (kForm == kTaps || ++kx == a.kernel) { kx = 0; ++ky; } }
                 }
             }
             if (!ok) s_abort = 1;
@@ -362,16 +394,24 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const int bcol = (wi.tile % a.n_tiles) * a.BN;
-                int brow = wi.c_begin * kChunk;
+                int brow = wi.c_begin * kChunk, ky = 0;      // (taps side by side: channel and filter row)
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     if (wrap > 0) ok = wait_or_abort(&bar_empty[s], (wrap - 1) & 1u, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 7); break; }
                     mbar_expect_tx(&bar_full[s], tx);
-                    tma_load_2d(sBhi(s), &tmBhi, &bar_full[s], brow, bcol);
-                    if (split) tma_load_2d(sBhi(s) + b_bytes, &tmBlo, &bar_full[s], brow, bcol);   // the BF16 cross operand
+                    if constexpr (kForm == kTaps) {
+                        // the filter row's three taps, one below the other in shared memory (with a copy for each its
+                        // issuer falls behind: one pass, 7 x 7 x 512, 128 images, 67.6 us, 61.3 with one for all)
+                        tma_load_3d(sBhi(s), &tmBhi, &bar_full[s], brow, bcol, ky * 3);
+                        if (split) tma_load_3d(sBhi(s) + b_bytes, &tmBlo, &bar_full[s], brow, bcol, ky * 3);
+                    } else {
+                        tma_load_2d(sBhi(s), &tmBhi, &bar_full[s], brow, bcol);
+                        if (split) tma_load_2d(sBhi(s) + b_bytes, &tmBlo, &bar_full[s], brow, bcol);   // the BF16 cross operand
+                    }
                     ++issued;
                     if (++s == a.stages) { s = 0; ++wrap; }
                     brow += kChunk;       // packed filter rows follow the chunk order
+                    if (kForm == kTaps && brow == a.Cp32) { brow = 0; ++ky; }
                 }
             }
             if (!ok) s_abort = 1;
@@ -380,9 +420,9 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     } else if (warp == 1) {
         // -------------------------------------------------------------- MMA issuer
         if (elect_one()) {
-            const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+            const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(acc_cols >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
             // kind::f16 with BF16 operands (format code 1), fp32 accumulation
-            const uint32_t idesc_bf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.BN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+            const uint32_t idesc_bf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(acc_cols >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
             int s = 0;
             uint32_t ph = 0;           // parity of the ring pass
             bool ok = true;
@@ -397,12 +437,12 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     // gather form, A in tensor memory: the operand exists only once the split warps have built it (they
                     // arrive after the stage's copies have landed)
-                    ok = wait_or_abort(a.gather || a.ta ? &bar_xf[s] : &bar_full[s], ph, abort_flag, a.spin_limit);
+                    ok = wait_or_abort(a.gather || a.ta == 1 ? &bar_xf[s] : &bar_full[s], ph, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 2); s_abort = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = umma_desc(sA(s)), bd = umma_desc(sBhi(s));
                     const uint32_t acc_flag = it > (kSplit ? wi.c_begin : 0) ? 1u : 0u;     // the first chunk overwrites
-                    if (a.ta) {
+                    if (a.ta == 1) {
                         const uint32_t ta = tmem_a + (uint32_t)s * 64u;
                         umma_tf32_chunk_ta(d, ta, bd, idesc, acc_flag);
                         umma_bf16_chunk_ta(d, ta + 32u, bd + (b_bytes >> 4), idesc_bf16);
@@ -419,7 +459,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                             if (!ok) { record_error(err_flag, 2); s_abort = 1; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         }
-                        umma_bf16_chunk(d, ad + (kABytes >> 4), bd + (b_bytes >> 4), idesc_bf16, 1u);
+                        if (kForm == kTaps && a.ta == 2) umma_bf16_chunk_ta(d, tmem_a + (uint32_t)s * 32u, bd + (b_bytes >> 4), idesc_bf16);
+                        else umma_bf16_chunk(d, ad + (kABytes >> 4), bd + (b_bytes >> 4), idesc_bf16, 1u);
                     }
                     umma_commit(&bar_empty[s]);
                     if (++s == a.stages) { s = 0; ph ^= 1u; }
@@ -465,8 +506,10 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (turn == xg) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const unsigned char* stage = base_ptr + (size_t)s * stage_bytes;
-                        const uint32_t to = lanes + (uint32_t)s * 64u;
-                        if (!a.gather) {
+                        const uint32_t to = lanes + (uint32_t)s * (kForm == kTaps && a.ta == 2 ? 32u : 64u);
+                        if (kForm == kTaps && a.ta == 2) {
+                            cross_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
+                        } else if (kForm == kTaps || !a.gather) {
                             split_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
                         } else {
                             const float* win = reinterpret_cast<const float*>(stage + 2u * b_bytes) + g_row;
@@ -569,6 +612,120 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (++s == a.stages) { s = 0; ph ^= 1u; }
                 }
             }
+        }
+    } else if constexpr (kForm == kTaps) {
+        // -------------------------------------------- epilogue, taps side by side
+        // The groups take alternate 32-channel slabs. A thread's value is the sum of its own row of the second set, the
+        // row before it of the first and the row behind it of the third - a neighbouring lane's, or, at a warp's ends,
+        // left in shared memory by the neighbouring warp - where those pixels lie in the same row of the image.
+        const int eg = (warp - 2) >> 2, t = (threadIdx.x - 64) & 127, q = warp & 3, row = q * 32 + lane, bar_id = 1 + eg;
+        if (eg < a.epi_groups) {
+            const uint32_t my_staging = staging_off + (uint32_t)(eg * a.epi_slabs) * (uint32_t)kStagingBytes;
+            unsigned char* staging = base_ptr + my_staging;
+            float* edge = s_edge + eg * 256;
+            float* my_bias = s_bias[eg];
+            bool ok = true;
+            int ti = 0, staged_nbase = -1, round_no = 0;
+            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
+                const TileCoord tc_ = tile_coord(a, w);
+                const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
+                const int nbase = tc_.n_tile * a.BN;
+                int groups = (a.Kp - nbase + 31) / 32;
+                if (groups > a.BN / 32) groups = a.BN / 32;
+                const int step = a.epi_groups;
+                const int first = a.epi_groups == 1 || ((eg + ti) & 1) == 0 ? 0 : 1;
+                if (nbase != staged_nbase) {
+                    for (int i = t; i < a.BN; i += 128) my_bias[i] = a.bias_mode == 2 && nbase + i < a.K ? a.beta * bias[nbase + i] : 0.f;
+                    staged_nbase = nbase;
+                }
+                // this thread's pixel, its place in the image row and in the staging slab
+                const int shift = tc_.w0 > 0 ? 1 : 0, out_row = row - shift, pixel = tc_.w0 + out_row;
+                const int x = (pixel < 0 ? 0 : pixel) % a.oW;
+                const bool left = x > 0, right = x + 1 < a.oW, mine = out_row >= 0 && out_row < kTapsPixels;
+                const float* res_row = a.res && mine && pixel < a.Wo ? a.res + (long)pixel * a.res_ld : nullptr;
+                ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (first >= groups) {                  // none of them this time
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(&bar_acc_empty[as]);
+                }
+                for (int g0 = first; g0 < groups; g0 += step) {
+                    const int sb = round_no % a.epi_slabs;
+                    ++round_no;
+                    const int col = g0 * 32;
+                    const uint32_t taddr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * acc_cols + col);
+#pragma unroll
+                    for (int side = 0; side < 2; ++side) {
+                        uint32_t r[32];
+                        tmem_ld32(r, taddr + (uint32_t)(side * 2 * a.BN));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (lane == (side ? 0 : 31)) {
+                            uint4* e = reinterpret_cast<uint4*>(edge + (q * 2 + side) * 32);
+#pragma unroll
+                            for (int c4 = 0; c4 < 8; ++c4) e[c4] = make_uint4(r[c4 * 4], r[c4 * 4 + 1], r[c4 * 4 + 2], r[c4 * 4 + 3]);
+                        }
+                    }
+                    if (t == 0) {
+                        if (a.epi_slabs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    }
+                    group_sync(bar_id);
+                    float4* dst = reinterpret_cast<float4*>(staging + (size_t)sb * kStagingBytes + (size_t)(mine ? out_row : 0) * 128);
+                    // which output this slab belongs to, and its first column there
+                    const bool second = a.split_col > 0 && nbase + col >= a.split_col;
+                    const int lcol = second ? nbase + col - a.split_col : nbase + col;
+                    const int kout = second ? a.K - a.split_col : (a.split_col > 0 ? a.K1 : a.K);
+                    const bool fast = lcol + 32 <= kout;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        uint32_t r0[16], r1[16], r2[16];
+                        tmem_ld16(r0, taddr + (uint32_t)(half * 16));
+                        tmem_ld16(r1, taddr + (uint32_t)(a.BN + half * 16));
+                        tmem_ld16(r2, taddr + (uint32_t)(2 * a.BN + half * 16));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (half == 1 && g0 + step >= groups) {
+                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                            mbar_arrive(&bar_acc_empty[as]);
+                        }
+#pragma unroll
+                        for (int c4 = 0; c4 < 4; ++c4) {
+                            float4 before = make_float4(0.f, 0.f, 0.f, 0.f), behind = before;
+                            if (lane == 0 && q > 0) before = *reinterpret_cast<const float4*>(edge + (q - 1) * 64 + half * 16 + c4 * 4);
+                            if (lane == 31 && q < 3) behind = *reinterpret_cast<const float4*>(edge + (q + 1) * 64 + 32 + half * 16 + c4 * 4);
+                            const float eb[4] = {before.x, before.y, before.z, before.w}, ea[4] = {behind.x, behind.y, behind.z, behind.w};
+                            const float4 bb = *reinterpret_cast<const float4*>(my_bias + col + half * 16 + c4 * 4);
+                            const float bv[4] = {bb.x, bb.y, bb.z, bb.w};
+                            float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (res_row && lcol + half * 16 + c4 * 4 < a.Kp) res = __ldg(reinterpret_cast<const float4*>(res_row + lcol + half * 16) + c4);
+                            const float rv[4] = {res.x, res.y, res.z, res.w};
+                            float v[4];
+#pragma unroll
+                            for (int l = 0; l < 4; ++l) {
+                                float l0 = __uint_as_float(__shfl_up_sync(0xffffffffu, r0[c4 * 4 + l], 1));
+                                float l2 = __uint_as_float(__shfl_down_sync(0xffffffffu, r2[c4 * 4 + l], 1));
+                                if (lane == 0) l0 = eb[l];
+                                if (lane == 31) l2 = ea[l];
+                                float sum = (left ? l0 : 0.f) + __uint_as_float(r1[c4 * 4 + l]);
+                                if (right) sum += l2;
+                                v[l] = fmaf(a.alpha, sum, bv[l]);
+                                if (res_row) v[l] += rv[l];
+                                v[l] = apply_act(v[l], a.act, a.lo, a.hi);
+                                if (!fast && lcol + half * 16 + c4 * 4 + l >= kout) v[l] = 0.f;         // padded lanes stay zero
+                            }
+                            if (mine) dst[(half * 4 + c4) ^ (out_row & 7)] = make_float4(v[0], v[1], v[2], v[3]);
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    group_sync(bar_id);
+                    if (t == 0) {
+                        tma_store_4d(second ? &tmY2 : &tmY, base + my_staging + (uint32_t)sb * (uint32_t)kStagingBytes, lcol, tc_.w0, 0, 0);
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                }
+            }
+            if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         }
     } else if constexpr (kForm == kCluster) {
         // ------------------------------------------------------------ partial tile
@@ -851,23 +1008,26 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     if (t.BN % 32 || t.BN > 256) return OGLE_ERR_UNSUPPORTED;
     // accumulators: two, or four when they fit (half of) the 512 columns of tensor memory - the multiplies
     // of a tile can then start while the epilogues of the two tiles before it still drain theirs
-    const int acc_cols = t.BN;
+    const int b_rows = t.BN * (t.taps ? 3 : 1), acc_cols = b_rows;
     // Split mode: the A operands of both passes go through tensor memory where two stages or more of them fit beside
     // the accumulators (tiles of up to 192 columns).
     // (In the gather form too, for three input channels.)
     const bool ta_form = t.passes == 3 && (!t.gather || t.g_C == 3);
     t.n_acc = 4 * acc_cols <= (ta_form ? 256 : 512) ? 4 : 2;
     static const bool ta_off = [] { const char* e = getenv("OGLE_TC_TA"); return e && e[0] == '0'; }();
-    const int ta_stages = (512 - t.n_acc * acc_cols) / 64;
-    t.ta = ta_form && !ta_off && ta_stages >= 2 ? 1 : 0;
+    // Taps side by side, 64 channels a tile: with both in tensor memory the ring would have two stages; the BF16 one alone
+    // leaves room for four, and shared memory for three.
+    const int ta_cols = t.taps && t.n_acc * acc_cols > 256 ? 32 : 64;
+    const int ta_stages = (512 - t.n_acc * acc_cols) / ta_cols;
+    t.ta = ta_form && !ta_off && ta_stages >= 2 ? (ta_cols == 32 ? 2 : 1) : 0;
     if (!t.ta) t.n_acc = 4 * acc_cols <= 512 ? 4 : 2;
-    const size_t stage = (size_t)(t.ta && t.gather ? 0 : (t.passes == 3 && !t.ta ? 2 : 1)) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * t.BN * 128 +
+    const size_t stage = (size_t)(t.ta && t.gather ? 0 : (t.passes == 3 && !t.ta ? 2 : 1)) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * b_rows * 128 +
                          (t.gather ? (size_t)t.g_bytes : 0);
     // Shared memory is split between the operand ring and the epilogue's staging slabs
     // (128 rows x 32 columns each). Preference: two epilogue groups with two slabs each;
     // give slabs back to the ring while that buys another stage and the ring is shallow.
     const size_t kBudget = kTcSmem;
-    const int chunks = t.kernel * t.kernel * t.chunks_per_tap;
+    const int chunks = (t.taps ? 1 : t.kernel) * t.kernel * t.chunks_per_tap;
     t.xf_groups = (t.passes == 3 || t.gather) ? 2 : 1;   // both operand-split groups work on each chunk
     t.epi_groups = 2;
     t.epi_slabs = 2;
@@ -907,7 +1067,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     if (stages < 2) return OGLE_ERR_UNSUPPORTED;
     t.stages = stages;
     int cols = 32;
-    while (cols < t.n_acc * acc_cols + (t.ta ? t.stages * 64 : 0)) cols <<= 1;
+    while (cols < t.n_acc * acc_cols + (t.ta ? t.stages * ta_cols : 0)) cols <<= 1;
     t.tmem_cols = cols;
     const long total = m_tiles * t.n_tiles;
     if (total <= 0 || total > 0x7fffffffL) return OGLE_ERR_UNSUPPORTED;
@@ -930,6 +1090,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kRanges>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
     }
@@ -941,7 +1102,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     t.epi_share = t.total_work <= 4 * sms || chunks > 2 ? 1 : 0;
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
     const bool overlapped = overlapped_launches_enabled(t.overlapped);
-    note_contraction(t.cluster ? 3 : (t.split_k > 1 ? 2 : 1), t.split_k, t.BN, overlapped);
+    note_contraction(t.cluster ? 3 : (t.split_k > 1 ? 2 : (t.taps ? 6 : 1)), t.split_k, t.BN, overlapped);
     if (t.cluster) {
         // every block one work item; the blocks of a tile are consecutive, and a cluster
         cudaLaunchConfig_t cfg = {};
@@ -962,6 +1123,8 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     }
     if (t.split_k > 1)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+    else if (t.taps)
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kTaps>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else
         launch_overlapped_if(overlapped, conv_tc2_kernel<kWhole>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     return finish_launch();

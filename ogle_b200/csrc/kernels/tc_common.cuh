@@ -12,6 +12,7 @@ namespace tc {
 constexpr int kTileM = 128;
 constexpr int kChunk = 32;              // reduction elements per pipeline stage (128 bytes)
 constexpr int kABytes = kTileM * 128;   // one A tile
+constexpr int kTapsPixels = kTileM - 2; // output pixels of a tile whose taps lie side by side: their neighbours are rows of it too
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 constexpr int kMaxGatherK = 224;     // reduction indices of the gather form (k * k * C rounded up to 32); offsets fit 16 bits
@@ -22,6 +23,10 @@ struct TcArgs {
     int tiles_w, tiles_h;     // tile grid along w and h (n follows)
     int N, Ho, Wo;            // output extent (flat: rows = Wo)
     int stride, pad, dil, kernel;
+    // 1 (3x3 windows of stride 1 and padding 1; flat): the taps of a filter row side by side along the multiply's column side
+    // (kTaps form of conv_tc2.cu). A tile is kTapsPixels consecutive output pixels, which run on over rows and images of
+    // oH x oW - an im2col map fetches them -, and BN counts its output channels, of which the accumulator has three sets.
+    int taps, oH, oW;
     int chunks_per_tap, Cp32;
     int K, Kp, Ks, koff;      // output channels, padded to 4, row stride, first channel
     int BN, n_tiles;          // N tile and how many cover Kp
@@ -32,7 +37,7 @@ struct TcArgs {
     int ldc;
     int passes;               // 1 (TF32) or 3 (split mode: a TF32 pass + a BF16 pass of the cross terms)
     int stages;
-    int ta;                   // split mode with the A operands in tensor memory (64 columns per stage, after the accumulators)
+    int ta;                   // split mode: 1 = A operands in tensor memory (64 columns per stage, after the accumulators), 2 = the BF16 one (32)
     int tmem_cols;
     int n_acc;                // accumulator buffers in tensor memory (2 or 4)
     int total_tiles;          // m_tiles * n_tiles (persistent kernel)
@@ -113,6 +118,19 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+// 128 pixels of an im2col map from input pixel (c1, c2, c3) on, each moved by the filter tap (ox, oy).
+__device__ __forceinline__ void tma_load_im2col(uint32_t dst, const CUtensorMap* map, uint64_t* bar,
+                                                int c0, int c1, int c2, int c3, int ox, int oy) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+        ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "h"((unsigned short)ox), "h"((unsigned short)oy)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile(
@@ -235,6 +253,27 @@ __device__ __forceinline__ void split_half_to_tmem(const float (&f)[16], int hal
     tmem_st16(taddr + half * 16, hi);
     tmem_st8(taddr + 32 + half * 8, ph);
     tmem_st8(taddr + 48 + half * 8, pl);
+}
+// The BF16 part of it alone, in the 32 columns at taddr (the TF32 pass then reads the tile as it landed in shared memory).
+__device__ __forceinline__ void cross_row_to_tmem(const float4* row, int r, uint32_t taddr) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        uint32_t ph[8], pl[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 v = row[(half * 4 + q) ^ (r & 7)];
+            const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int l = 0; l < 4; l += 2) {
+                const float h0 = __uint_as_float(__float_as_uint(f[l]) & 0xffffe000u), h1 = __uint_as_float(__float_as_uint(f[l + 1]) & 0xffffe000u);
+                const __nv_bfloat162 a = __floats2bfloat162_rn(h0, h1), b = __floats2bfloat162_rn(f[l] - h0, f[l + 1] - h1);
+                ph[q * 2 + l / 2] = *reinterpret_cast<const uint32_t*>(&a);
+                pl[q * 2 + l / 2] = *reinterpret_cast<const uint32_t*>(&b);
+            }
+        }
+        tmem_st8(taddr + half * 8, ph);
+        tmem_st8(taddr + 16 + half * 8, pl);
+    }
 }
 // One row of an activation tile (128 bytes in the 128-byte swizzle at `row`, which is row r of its tile).
 __device__ __forceinline__ void split_row_to_tmem(const float4* row, int r, uint32_t taddr) {

@@ -12,15 +12,22 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const int*, const int*, cuuint32_t, cuuint32_t, const cuuint32_t*,
+                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+inline void* driver_entry(const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+    return p;
+}
 inline EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
+    static EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(driver_entry("cuTensorMapEncodeTiled"));
+    return fn;
+}
+inline EncodeIm2colFn encode_im2col_fn() {
+    static EncodeIm2colFn fn = reinterpret_cast<EncodeIm2colFn>(driver_entry("cuTensorMapEncodeIm2col"));
     return fn;
 }
 
@@ -39,6 +46,19 @@ inline bool make_map_sw(CUtensorMapSwizzle swizzle, CUtensorMap* m, const void* 
 inline bool make_map(CUtensorMap* m, const void* ptr, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
                      const cuuint32_t* box, const cuuint32_t* estr) {
     return make_map_sw(CU_TENSOR_MAP_SWIZZLE_128B, m, ptr, rank, dims, strides_bytes, box, estr);
+}
+
+// im2col map of an activation tensor [n][h][w][c] (dims and strides channel first, as above): a copy takes `channels` of
+// `pixels` consecutive positions of the window's first tap, which walk the image from `lower` to its far edge plus `upper`
+// ({w, h} each), row after row and image after image; positions outside the image read zero.
+inline bool make_map_im2col(CUtensorMap* m, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
+                            const int* lower, const int* upper, int channels, int pixels) {
+    EncodeIm2colFn fn = encode_im2col_fn();
+    if (!fn) return false;
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides_bytes, lower, upper, (cuuint32_t)channels,
+              (cuuint32_t)pixels, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace ogle

@@ -396,6 +396,84 @@ def test_cut_tiles_with_channels_on_m(oracle_port, width):
         assert torch.equal(one, outs[0][..., :24]) and torch.equal(two, outs[0][..., 24:64])
 
 
+TAPS_CODE = """
+import sys, torch
+from ogle_b200 import ops
+g = torch.Generator(device="cuda").manual_seed(3)
+rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+# N, H, W, C, K: one pixel a row and one row an image, tiles that end at, before and behind a row, an image and the tensor
+# (126 pixels each), channels and filters that fill no chunk, slab or tile
+for N, H, W, C, K in [(126, 1, 1, 32, 32), (127, 1, 1, 16, 4), (1, 1, 125, 32, 64), (1, 1, 127, 32, 64), (64, 2, 1, 40, 64), (3, 6, 7, 64, 65), (2, 7, 9, 70, 33),
+                      (1, 126, 2, 32, 96), (2, 3, 126, 64, 64), (5, 16, 128, 36, 100), (4, 56, 56, 64, 64), (150, 28, 28, 32, 130), (3, 90, 129, 100, 62)]:
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        for act in (ops.ACT_NONE, ops.ACT_RELU, ops.ACT_CLIP):
+            p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, True, act, -0.5, 1.5, math)
+            p.split = 1
+            x = torch.zeros((N, H, W, ops.up4(C)), device="cuda")
+            x[..., :C] = rand(N, H, W, C)
+            w, b, res = rand(K, C, 3, 3) / (9 * C) ** 0.5, rand(K), rand(N, H, W, ops.up4(K))
+            packed = ops.conv2d_prepack(p, w)
+            sums = torch.nn.functional.conv2d(x[..., :C].permute(0, 3, 1, 2).double(), w.double(), b.double(), padding=1).permute(0, 2, 3, 1)
+            finish = lambda v: v if act == ops.ACT_NONE else (v.clamp(min=0) if act == ops.ACT_RELU else v.clamp(-0.5, 1.5))
+            # split mode: sums in tensor memory lose 6e-9 of their norm per element, products and operands 1e-6; one pass:
+            # operands of ten mantissa bits, the activation's cut off (2^-10 at most, half of it on average)
+            bound = (2e-6 + 6e-9 * 9 * C if math == ops.MATH_TF32X3 else 1e-3) * float(sums.norm())
+            def check(got, want, form=6):
+                assert ops.last_contraction().form == form, (N, H, W, C, K, ops.last_contraction().form)
+                assert float((got.double() - want).norm()) <= bound, (N, H, W, C, K, math, act, float((got.double() - want).norm()) / bound)
+            wide = torch.full((N, H, W, ops.up4(K) + 8), -7.0, device="cuda")
+            p.out_channel_stride, p.out_channel_offset = ops.up4(K) + 8, 4
+            ops.conv2d(p, x, packed, b, wide)
+            check(wide[..., 4:4 + K], finish(sums))
+            assert (wide[..., :4] == -7).all() and (wide[..., 4 + ops.up4(K):] == -7).all() and (wide[..., 4 + K:4 + ops.up4(K)] == 0).all()
+            p.out_channel_stride = p.out_channel_offset = 0
+            plain = ops.conv2d(p, x, packed, b)
+            assert torch.equal(plain[..., :K], wide[..., 4:4 + K])
+            if act != ops.ACT_CLIP:
+                check(ops.conv2d_residual(p, x, packed, b, res)[..., :K], finish(sums + res[..., :K]))
+            for tile, pair in ((32, 0), (0, 2)):                      # neither touches the bits
+                p.n_tile, p.sm_pair = tile, pair
+                assert torch.equal(ops.conv2d(p, x, packed, b), plain)
+"""
+
+
+def test_taps_side_by_side_at_the_edges_of_their_tiles():
+    """Forced (the switch is read once per process), so that the smallest launches take the form too."""
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", TAPS_CODE], cwd=root, env=dict(os.environ, OGLE_TC_TAPS="1"), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_taps_side_by_side_two_outputs_and_bounded_waits():
+    """By the library's own choice: the two outputs of sibling layers, and roles that give up at once."""
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    N, H, C, K = 64, 38, 64, 52
+    x, w, b = rand(N, H, H, C), rand(K, C, 3, 3) / 24.0, rand(K)
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        p = ops.conv_params(N, H, H, C, K, 3, 1, 1, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, math)
+        packed = ops.conv2d_prepack(p, w)
+        want = ops.conv2d(p, x, packed, b, workspace=None)
+        assert ops.last_contraction().form == 6
+        one, two = ops.conv2d_pair(x, w[:20], b[:20], w[20:], b[20:], N, H, H, C, 3, 1, 1, 1, ops.ACT_RELU, 0.0, 0.0, math, use_workspace=False)
+        assert ops.last_contraction().form == 6
+        assert torch.equal(one, want[..., :20]) and torch.equal(two, want[..., 20:])
+        try:
+            assert lib.ogle_cuda_device_status() == 0
+            lib.ogle_cuda_set_wait_limit(0)
+            ops.conv2d(p, x, packed, b, workspace=None)
+            assert lib.ogle_cuda_device_status() == -6 and 1 <= lib.ogle_cuda_device_status_detail() <= 7
+        finally:
+            lib.ogle_cuda_set_wait_limit(-1)
+            lib.ogle_cuda_clear_device_status()
+        assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), want)
+        assert lib.ogle_cuda_device_status() == 0
+
+
 def test_bounded_waits_of_the_cluster_form(oracle_port):
     """Zero polls allowed: every block of a cluster gives up, all meet at the cluster's barriers, the launch returns with
     the status word set, and with the limit restored the same call gives what it gave before."""
