@@ -306,13 +306,13 @@ bool conv_tc_supported(const ConvArgs& a, int variant) {
 // (the RGB stem), whole reduction (9 x C <= 27 values) in one chunk.
 // Tile of the gather form: tw x th output pixels of one image, tw * th = 128; the shape that
 // wastes the fewest rows among those whose input window (halo included) is at most 1024
-// pixels = 16 KB of shared memory per stage and at most 256 pixels wide (a TMA box limit).
+// pixels = 16 KB of shared memory per stage and at most 128 pixels wide (a limit of its map).
 static bool gather_tile(const ConvArgs& a, int* tw_out, int* th_out) {
     long best = -1;
     for (int tw = 128; tw >= 16; tw >>= 1) {
         const int th = kTileM / tw;
         const int iw = (tw - 1) * a.stride + a.kernel, ih = (th - 1) * a.stride + a.kernel;
-        if (iw > 256 || iw * ih > 1024) continue;
+        if (iw > 128 || iw * ih > 1024) continue;
         const long covered = (long)((a.Wo + tw - 1) / tw) * tw * ((a.Ho + th - 1) / th) * th;
         if (best < 0 || covered < best) { best = covered; *tw_out = tw; *th_out = th; }
     }
@@ -410,10 +410,6 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     // planning needs the tile geometry only
     auto make_map = [&](CUtensorMap* m, const void* p, int rank, const cuuint64_t* d, const cuuint64_t* st, const cuuint32_t* b,
                         const cuuint32_t* e) { return plan_only ? true : ogle::make_map(m, p, rank, d, st, b, e); };
-    auto make_map_sw = [&](CUtensorMapSwizzle sw, CUtensorMap* m, const void* p, int rank, const cuuint64_t* d,
-                           const cuuint64_t* st, const cuuint32_t* b, const cuuint32_t* e) {
-        return plan_only ? true : ogle::make_map_sw(sw, m, p, rank, d, st, b, e);
-    };
     if (variant == CONV_POINTWISE) {
         t.flat = 1;
         t.N = 1; t.Ho = 1; t.Wo = (int)a.M;
@@ -448,11 +444,8 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.g_iw = (t.tw - 1) * a.stride + a.kernel;
         t.g_ih = (t.th - 1) * a.stride + a.kernel;
         t.g_bytes = (t.g_iw * t.g_ih * 16 + 1023) / 1024 * 1024;
-        const cuuint64_t dims[4] = {4, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
-        const cuuint64_t str[3] = {(cuuint64_t)a.Cs * 4, (cuuint64_t)a.Cs * 4 * a.W, (cuuint64_t)a.Cs * 4 * a.W * a.H};
-        const cuuint32_t box[4] = {4, (cuuint32_t)t.g_iw, (cuuint32_t)t.g_ih, 1};
+        if (!plan_only && !make_map_pixels(&mA, x, a.W, a.H, a.N, t.g_iw, t.g_ih)) return OGLE_ERR_CUDA;
         const cuuint32_t es[4] = {1, 1, 1, 1};
-        if (!make_map_sw(CU_TENSOR_MAP_SWIZZLE_NONE, &mA, x, 4, dims, str, box, es)) return OGLE_ERR_CUDA;
         const cuuint64_t yd[4] = {(cuuint64_t)kp_a, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
         const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * a.Wo, (cuuint64_t)ks_a * 4 * a.Wo * a.Ho};
         const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, 1};

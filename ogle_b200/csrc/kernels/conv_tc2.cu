@@ -367,7 +367,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (!ok) { record_error(err_flag, 1); break; }
                     if (a.gather) {
                         mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
-                        tma_load_4d(sWin(s), &tmA, &bar_full[s], 0, ax, ay, an);
+                        tma_load_4d(sWin(s), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
                     } else {
                         mbar_expect_tx(&bar_full[s], tx);
                         if constexpr (kForm == kTaps) tma_load_im2col(sA(s), &tmA, &bar_full[s], c0, ax, ay, an, 0, ky);

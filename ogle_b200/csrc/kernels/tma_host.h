@@ -48,6 +48,19 @@ inline bool make_map(CUtensorMap* m, const void* ptr, int rank, const cuuint64_t
     return make_map_sw(CU_TENSOR_MAP_SWIZZLE_128B, m, ptr, rank, dims, strides_bytes, box, estr);
 }
 
+// Map of an image tensor of 16-byte pixels [n][h][w] whose boxes take `cols` pixels of `rows` rows. A pixel is two 8-byte
+// elements of one row-long extent, not an extent of its own: the copy engine takes a row of a box as a whole instead of
+// pixel by pixel. At most 128 columns; coordinates (2 * column, row, image, 0).
+inline bool make_map_pixels(CUtensorMap* m, const void* ptr, int W, int H, int N, int cols, int rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)W * 2, (cuuint64_t)H, (cuuint64_t)N, 1};
+    const cuuint64_t str[3] = {(cuuint64_t)W * 16, (cuuint64_t)W * 16 * H, (cuuint64_t)W * 16 * H * N};
+    const cuuint32_t box[4] = {(cuuint32_t)cols * 2, (cuuint32_t)rows, 1, 1}, es[4] = {1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(ptr), dims, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // im2col map of an activation tensor [n][h][w][c] (dims and strides channel first, as above): a copy takes `channels` of
 // `pixels` consecutive positions of the window's first tap, which walk the image from `lower` to its far edge plus `upper`
 // ({w, h} each), row after row and image after image; positions outside the image read zero.
