@@ -597,7 +597,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
                 return make_map(m, p, 4, d, st, yb, ye);
             };
             return make_map_im2col(&mA, x, dims, str, lower, upper, kChunk, kTileM) && rows(&mY, y + a.koff, kp_a, ks_a) &&
-                   (!y2 || rows(&mY2, y2, kp_b, kp_b));
+                   (!y2 || rows(&mY2, y2, kp_b, kp_b)) && (!residual || rows(&mY2, residual, a.Kp, res_ld));
         }
         // the box spans the traversed input extent; one element in `stride` is taken
         const cuuint32_t box[4] = {kChunk, (cuuint32_t)((t.tw - 1) * a.stride + 1), (cuuint32_t)((t.th - 1) * a.stride + 1),
@@ -720,7 +720,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             if (!ogle::make_map(&mBlo, w_lo, 2, bdims, bstr, hbox, bes)) return OGLE_ERR_CUDA;
             return launch_tc_pair(t, mA, mBhi, mBlo, mY, y2 ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
         }
-        return launch_tc_v2(t, mA, mBhi, mBlo, mY, y2 ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
+        return launch_tc_v2(t, mA, mBhi, mBlo, mY, y2 || (t.taps && residual) ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
     }
     return OGLE_ERR_UNSUPPORTED;
 }

@@ -76,6 +76,14 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
+// The same, and whether all 128 threads say so.
+__device__ __forceinline__ bool group_and(int id, bool mine) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbar.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"(id), "r"((uint32_t)mine) : "memory");
+    return all != 0;
+}
+
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                  ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
@@ -136,13 +144,14 @@ enum TcForm {
     // 117 bytes a clock seen here 0.6 us, which is what it takes; a tile's epilogue adds about 1 us to that.
     // Split mode, before and after: 128 x 56 x 56 x 64 -> 64 172 -> 114 us, 128 x 28 x 28 x 128 -> 128 107 -> 99,
     // 128 x 14 x 14 x 256 -> 256 102 -> 96, 128 x 7 x 7 x 512 -> 512 114 -> 94; one pass, the first: 131 -> 82.
-    kTaps = 3
+    kTaps = 3,
+    kTapsRes = 4      // ... with a residual operand (checked for at run time it costs 7 us of 110 where there is none)
 };
 
 template <TcForm kForm>
 __device__ __forceinline__ WorkItem work_item(const TcArgs& a, int w, int chunks) {
     WorkItem it;
-    if (kForm == kWhole || kForm == kTaps) {
+    if (kForm != kRanges && kForm != kCluster) {
         it.tile = w; it.ks = 0; it.c_begin = 0; it.c_end = chunks;
     } else {
         it.tile = w / a.split_k;
@@ -234,18 +243,20 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // 1024-byte alignment (the 128-byte swizzle atom) comes from the declaration, so that
     // every byte of the 224 KB request is usable
     constexpr bool kSplit = kForm == kRanges || kForm == kCluster;
-    constexpr int kSets = kForm == kTaps ? 3 : 1;       // of BN accumulator columns
+    constexpr bool kBeside = kForm == kTaps || kForm == kTapsRes;
+    constexpr int kSets = kBeside ? 3 : 1;       // of BN accumulator columns
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_xf[kMaxStages], bar_empty[kMaxStages];
     __shared__ __align__(8) uint64_t bar_acc_full[4], bar_acc_empty[4];
     __shared__ __align__(8) uint64_t bar_drain;     // abort path: the MMAs issued so far have finished
+    __shared__ __align__(8) uint64_t bar_res[kBeside ? 2 : 1];    // taps side by side: a group's slab of the residual operand has landed
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ int s_issued[2];                     // operand copies issued by the two producers (abort path)
-    __shared__ __align__(16) float s_bias[2][kForm == kTaps ? 64 : 256];
-    __shared__ __align__(8) short s_goff[kForm == kTaps ? 4 : kMaxGatherK];   // gather form: window offset of each reduction index
+    __shared__ __align__(16) float s_bias[2][kBeside ? 64 : 256];
+    __shared__ __align__(8) short s_goff[kBeside ? 4 : kMaxGatherK];   // gather form: window offset of each reduction index
     // taps side by side: the rows that the neighbouring warps of a group need, [group][warp][last or first row][column]
-    __shared__ __align__(16) float s_edge[kForm == kTaps ? 2 * 4 * 2 * 32 : 4];
+    __shared__ __align__(16) float s_edge[kBeside ? 2 * 4 * 2 * 32 : 4];
 
     grid_dependency_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -275,7 +286,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
 
-    const int chunks = (kForm == kTaps ? 1 : a.kernel) * a.kernel * a.chunks_per_tap;
+    const int chunks = (kBeside ? 1 : a.kernel) * a.kernel * a.chunks_per_tap;
     const int acc_cols = a.BN * kSets;     // tensor-memory columns of one accumulator
     const int rows_in_tile = a.flat ? kTileM : a.tn * a.th * a.tw;
     volatile int* abort_flag = &s_abort;
@@ -299,11 +310,12 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             mbar_init(&bar_acc_empty[i], (uint32_t)(128 * a.epi_groups));
         }
         mbar_init(&bar_drain, 1);
+        if (kBeside) { mbar_init(&bar_res[0], 1); mbar_init(&bar_res[1], 1); }
         s_abort = 0;
         s_issued[0] = 0; s_issued[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (kForm != kTaps && a.gather) {
+    if (!kBeside && a.gather) {
         // reduction index k = (ky * kernel + kx) * C + c -> float offset of that value in the
         // [g_ih][g_iw][4] input window relative to the output pixel's first tap; -1 = padding column
         const int kred = a.g_k * a.g_k * a.g_C;
@@ -343,7 +355,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord(a, wi.tile);
                 int ax, ay, an;
-                if constexpr (kForm == kTaps) {
+                if constexpr (kBeside) {
                     // from the pixel before the first output pixel on
                     const int p = tc_.w0 > 0 ? tc_.w0 - 1 : 0, line = p / a.oW;
                     an = line / a.oH;
@@ -370,14 +382,14 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         tma_load_4d(sWin(s), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
                     } else {
                         mbar_expect_tx(&bar_full[s], tx);
-                        if constexpr (kForm == kTaps) tma_load_im2col(sA(s), &tmA, &bar_full[s], c0, ax, ay, an, 0, ky);
+                        if constexpr (kBeside) tma_load_im2col(sA(s), &tmA, &bar_full[s], c0, ax, ay, an, 0, ky);
                         else tma_load_4d(sA(s), &tmA, &bar_full[s], c0, ax + kx * a.dil, ay + ky * a.dil, an);
                     }
                     ++issued;
                     if (++s == a.stages) { s = 0; ++wrap; }
                     // next chunk: channels fastest, then filter column, then filter row
                     c0 += kChunk;
-                    if (c0 == a.Cp32) { c0 = 0; if (kForm == kTaps || ++kx == a.kernel) { kx = 0; ++ky; } }
+                    if (c0 == a.Cp32) { c0 = 0; if (kBeside || ++kx == a.kernel) { kx = 0; ++ky; } }
                 }
             }
             if (!ok) s_abort = 1;
@@ -399,7 +411,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (wrap > 0) ok = wait_or_abort(&bar_empty[s], (wrap - 1) & 1u, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 7); break; }
                     mbar_expect_tx(&bar_full[s], tx);
-                    if constexpr (kForm == kTaps) {
+                    if constexpr (kBeside) {
                         // the filter row's three taps, one below the other in shared memory (with a copy for each its
                         // issuer falls behind: one pass, 7 x 7 x 512, 128 images, 67.6 us, 61.3 with one for all)
                         tma_load_3d(sBhi(s), &tmBhi, &bar_full[s], brow, bcol, ky * 3);
@@ -411,7 +423,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     ++issued;
                     if (++s == a.stages) { s = 0; ++wrap; }
                     brow += kChunk;       // packed filter rows follow the chunk order
-                    if (kForm == kTaps && brow == a.Cp32) { brow = 0; ++ky; }
+                    if (kBeside && brow == a.Cp32) { brow = 0; ++ky; }
                 }
             }
             if (!ok) s_abort = 1;
@@ -459,7 +471,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                             if (!ok) { record_error(err_flag, 2); s_abort = 1; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         }
-                        if (kForm == kTaps && a.ta == 2) umma_bf16_chunk_ta(d, tmem_a + (uint32_t)s * 32u, bd + (b_bytes >> 4), idesc_bf16);
+                        if (kBeside && a.ta == 2) umma_bf16_chunk_ta(d, tmem_a + (uint32_t)s * 32u, bd + (b_bytes >> 4), idesc_bf16);
                         else umma_bf16_chunk(d, ad + (kABytes >> 4), bd + (b_bytes >> 4), idesc_bf16, 1u);
                     }
                     umma_commit(&bar_empty[s]);
@@ -506,10 +518,10 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (turn == xg) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const unsigned char* stage = base_ptr + (size_t)s * stage_bytes;
-                        const uint32_t to = lanes + (uint32_t)s * (kForm == kTaps && a.ta == 2 ? 32u : 64u);
-                        if (kForm == kTaps && a.ta == 2) {
+                        const uint32_t to = lanes + (uint32_t)s * (kBeside && a.ta == 2 ? 32u : 64u);
+                        if (kBeside && a.ta == 2) {
                             cross_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
-                        } else if (kForm == kTaps || !a.gather) {
+                        } else if (kBeside || !a.gather) {
                             split_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
                         } else {
                             const float* win = reinterpret_cast<const float*>(stage + 2u * b_bytes) + g_row;
@@ -613,7 +625,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
         }
-    } else if constexpr (kForm == kTaps) {
+    } else if constexpr (kBeside) {
         // -------------------------------------------- epilogue, taps side by side
         // The groups take alternate 32-channel slabs. A thread's value is the sum of its own row of the second set, the
         // row before it of the first and the row behind it of the third - a neighbouring lane's, or, at a warp's ends,
@@ -623,9 +635,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const uint32_t my_staging = staging_off + (uint32_t)(eg * a.epi_slabs) * (uint32_t)kStagingBytes;
             unsigned char* staging = base_ptr + my_staging;
             float* edge = s_edge + eg * 256;
+            // (the tile's first and last rows have none: nothing of them is kept, or they are an image row's ends)
+            const bool at_end = (lane == 0 && q > 0) || (lane == 31 && q < 3);
+            const float* my_edge = lane == 0 ? edge + (q - 1) * 64 : edge + (q + 1) * 64 + 32;
             float* my_bias = s_bias[eg];
             bool ok = true;
             int ti = 0, staged_nbase = -1, round_no = 0;
+            int res_copies = 0;        // of the residual operand, asked for by this thread
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
                 const TileCoord tc_ = tile_coord(a, w);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
@@ -642,7 +658,19 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int shift = tc_.w0 > 0 ? 1 : 0, out_row = row - shift, pixel = tc_.w0 + out_row;
                 const int x = (pixel < 0 ? 0 : pixel) % a.oW;
                 const bool left = x > 0, right = x + 1 < a.oW, mine = out_row >= 0 && out_row < kTapsPixels;
-                const float* res_row = a.res && mine && pixel < a.Wo ? a.res + (long)pixel * a.res_ld : nullptr;
+                // A slab is free once the store from it has been read; the residual operand's values are then copied to it
+                // - a thread that loads its own row of them holds up the tile: 56 x 56 x 64, 128 images, 145 us -,
+                // and each thread adds its row and leaves the sum in their place.
+                auto free_slab = [&](int slab, int lcol) {
+                    if (a.epi_slabs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    if constexpr (kForm == kTapsRes) {
+                        ++res_copies;
+                        mbar_expect_tx(&bar_res[eg], (uint32_t)kTapsPixels * 128u);
+                        tma_load_4d(base + my_staging + (uint32_t)slab * (uint32_t)kStagingBytes, &tmY2, &bar_res[eg], lcol, tc_.w0, 0, 0);
+                    }
+                };
+                if (t == 0 && first < groups) free_slab(round_no % a.epi_slabs, nbase + first * 32);
                 ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
@@ -656,6 +684,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     ++round_no;
                     const int col = g0 * 32;
                     const uint32_t taddr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * acc_cols + col);
+                    if (t == 0 && g0 != first) free_slab(sb, nbase + col);
 #pragma unroll
                     for (int side = 0; side < 2; ++side) {
                         uint32_t r[32];
@@ -667,11 +696,12 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                             for (int c4 = 0; c4 < 8; ++c4) e[c4] = make_uint4(r[c4 * 4], r[c4 * 4 + 1], r[c4 * 4 + 2], r[c4 * 4 + 3]);
                         }
                     }
-                    if (t == 0) {
-                        if (a.epi_slabs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    if constexpr (kForm == kTapsRes) {
+                        ok = group_and(bar_id, wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
+                        if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
+                    } else {
+                        group_sync(bar_id);
                     }
-                    group_sync(bar_id);
                     float4* dst = reinterpret_cast<float4*>(staging + (size_t)sb * kStagingBytes + (size_t)(mine ? out_row : 0) * 128);
                     // which output this slab belongs to, and its first column there
                     const bool second = a.split_col > 0 && nbase + col >= a.split_col;
@@ -691,28 +721,37 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         }
 #pragma unroll
                         for (int c4 = 0; c4 < 4; ++c4) {
-                            float4 before = make_float4(0.f, 0.f, 0.f, 0.f), behind = before;
-                            if (lane == 0 && q > 0) before = *reinterpret_cast<const float4*>(edge + (q - 1) * 64 + half * 16 + c4 * 4);
-                            if (lane == 31 && q < 3) behind = *reinterpret_cast<const float4*>(edge + (q + 1) * 64 + 32 + half * 16 + c4 * 4);
-                            const float eb[4] = {before.x, before.y, before.z, before.w}, ea[4] = {behind.x, behind.y, behind.z, behind.w};
+                            float4 over = make_float4(0.f, 0.f, 0.f, 0.f);          // the neighbouring warp's row
+                            if (at_end) over = *reinterpret_cast<const float4*>(my_edge + half * 16 + c4 * 4);
+                            const float ov[4] = {over.x, over.y, over.z, over.w};
                             const float4 bb = *reinterpret_cast<const float4*>(my_bias + col + half * 16 + c4 * 4);
                             const float bv[4] = {bb.x, bb.y, bb.z, bb.w};
                             float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (res_row && lcol + half * 16 + c4 * 4 < a.Kp) res = __ldg(reinterpret_cast<const float4*>(res_row + lcol + half * 16) + c4);
+                            if (kForm == kTapsRes && mine) res = dst[(half * 4 + c4) ^ (out_row & 7)];
                             const float rv[4] = {res.x, res.y, res.z, res.w};
                             float v[4];
 #pragma unroll
                             for (int l = 0; l < 4; ++l) {
                                 float l0 = __uint_as_float(__shfl_up_sync(0xffffffffu, r0[c4 * 4 + l], 1));
                                 float l2 = __uint_as_float(__shfl_down_sync(0xffffffffu, r2[c4 * 4 + l], 1));
-                                if (lane == 0) l0 = eb[l];
-                                if (lane == 31) l2 = ea[l];
+                                if (lane == 0) l0 = ov[l];
+                                if (lane == 31) l2 = ov[l];
                                 float sum = (left ? l0 : 0.f) + __uint_as_float(r1[c4 * 4 + l]);
                                 if (right) sum += l2;
                                 v[l] = fmaf(a.alpha, sum, bv[l]);
-                                if (res_row) v[l] += rv[l];
-                                v[l] = apply_act(v[l], a.act, a.lo, a.hi);
-                                if (!fast && lcol + half * 16 + c4 * 4 + l >= kout) v[l] = 0.f;         // padded lanes stay zero
+                                if (kForm == kTapsRes) v[l] += rv[l];
+                            }
+                            if (a.act == OGLE_ACT_RELU) {
+#pragma unroll
+                                for (int l = 0; l < 4; ++l) v[l] = fmaxf(v[l], 0.f);
+                            } else if (a.act == OGLE_ACT_CLIP) {
+#pragma unroll
+                                for (int l = 0; l < 4; ++l) v[l] = fminf(fmaxf(v[l], a.lo), a.hi);
+                            }
+                            if (!fast) {
+#pragma unroll
+                                for (int l = 0; l < 4; ++l)
+                                    if (lcol + half * 16 + c4 * 4 + l >= kout) v[l] = 0.f;             // padded lanes stay zero
                             }
                             if (mine) dst[(half * 4 + c4) ^ (out_row & 7)] = make_float4(v[0], v[1], v[2], v[3]);
                         }
@@ -725,6 +764,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 }
             }
+            // (an aborting block waits for the copy it has asked for)
+            if (!ok && res_copies > 0) mbar_wait(&bar_res[eg], (uint32_t)((res_copies - 1) & 1));
             if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         }
     } else if constexpr (kForm == kCluster) {
@@ -1090,6 +1131,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kRanges>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTapsRes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
         attr_device = dev;
@@ -1123,6 +1165,8 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     }
     if (t.split_k > 1)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+    else if (t.taps && t.res)
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kTapsRes>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else if (t.taps)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kTaps>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else
