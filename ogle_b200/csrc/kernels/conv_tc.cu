@@ -424,6 +424,10 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             const cuuint64_t yd[4] = {(cuuint64_t)kp_a, (cuuint64_t)a.M, 1, 1};
             const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * (cuuint64_t)a.M, (cuuint64_t)ks_a * 4 * (cuuint64_t)a.M};
             if (!make_map(&mY, y + a.koff, 4, yd, ys, box, es)) return OGLE_ERR_CUDA;
+            if (residual) {
+                const cuuint64_t rs[3] = {(cuuint64_t)res_ld * 4, (cuuint64_t)res_ld * 4 * (cuuint64_t)a.M, (cuuint64_t)res_ld * 4 * (cuuint64_t)a.M};
+                if (!make_map(&mY2, residual, 4, yd, rs, box, es)) return OGLE_ERR_CUDA;
+            }
             if (y2) {
                 const cuuint64_t yd2[4] = {(cuuint64_t)kp_b, (cuuint64_t)a.M, 1, 1};
                 const cuuint64_t ys2[3] = {(cuuint64_t)kp_b * 4, (cuuint64_t)kp_b * 4 * (cuuint64_t)a.M, (cuuint64_t)kp_b * 4 * (cuuint64_t)a.M};
@@ -450,6 +454,10 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * a.Wo, (cuuint64_t)ks_a * 4 * a.Wo * a.Ho};
         const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, 1};
         if (!make_map(&mY, y + a.koff, 4, yd, ys, yb, es)) return OGLE_ERR_CUDA;
+        if (residual) {
+            const cuuint64_t rs[3] = {(cuuint64_t)res_ld * 4, (cuuint64_t)res_ld * 4 * a.Wo, (cuuint64_t)res_ld * 4 * a.Wo * a.Ho};
+            if (!make_map(&mY2, residual, 4, yd, rs, yb, es)) return OGLE_ERR_CUDA;
+        }
     } else {
         t.flat = 0;
         t.N = a.N; t.Ho = a.Ho; t.Wo = a.Wo;
@@ -610,6 +618,10 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, (cuuint32_t)t.tn};
             const cuuint32_t ye[4] = {1, 1, 1, 1};
             if (!make_map(&mY, y + a.koff, 4, yd, ys, yb, ye)) return false;
+            if (residual) {
+                const cuuint64_t rs[3] = {(cuuint64_t)res_ld * 4, (cuuint64_t)res_ld * 4 * a.Wo, (cuuint64_t)res_ld * 4 * a.Wo * a.Ho};
+                if (!make_map(&mY2, residual, 4, yd, rs, yb, ye)) return false;
+            }
             if (y2) {
                 const cuuint64_t yd2[4] = {(cuuint64_t)kp_b, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
                 const cuuint64_t ys2[3] = {(cuuint64_t)kp_b * 4, (cuuint64_t)kp_b * 4 * a.Wo, (cuuint64_t)kp_b * 4 * a.Wo * a.Ho};
@@ -720,7 +732,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             if (!ogle::make_map(&mBlo, w_lo, 2, bdims, bstr, hbox, bes)) return OGLE_ERR_CUDA;
             return launch_tc_pair(t, mA, mBhi, mBlo, mY, y2 ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
         }
-        return launch_tc_v2(t, mA, mBhi, mBlo, mY, y2 || (t.taps && residual) ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
+        return launch_tc_v2(t, mA, mBhi, mBlo, mY, y2 || residual ? mY2 : mY, m_tiles, bias, error_flag_ptr(), s);
     }
     return OGLE_ERR_UNSUPPORTED;
 }

@@ -112,13 +112,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t taddr) {
 
 struct TileCoord { int n_tile, n0, h0, w0; };
 
+template <bool kBeside = false>
 __device__ __forceinline__ TileCoord tile_coord(const TcArgs& a, int tile) {
     TileCoord c;
     c.n_tile = tile % a.n_tiles;
     const int m_tile = tile / a.n_tiles;
     c.n0 = 0; c.h0 = 0;
     if (a.flat) {
-        c.w0 = m_tile * (a.taps ? kTapsPixels : kTileM);
+        c.w0 = m_tile * (kBeside ? kTapsPixels : kTileM);
     } else {
         const int tw_i = m_tile % a.tiles_w;
         const int t = m_tile / a.tiles_w;
@@ -145,7 +146,8 @@ enum TcForm {
     // Split mode, before and after: 128 x 56 x 56 x 64 -> 64 172 -> 114 us, 128 x 28 x 28 x 128 -> 128 107 -> 99,
     // 128 x 14 x 14 x 256 -> 256 102 -> 96, 128 x 7 x 7 x 512 -> 512 114 -> 94; one pass, the first: 131 -> 82.
     kTaps = 3,
-    kTapsRes = 4      // ... with a residual operand (checked for at run time it costs 7 us of 110 where there is none)
+    kTapsRes = 4,     // ... with a residual operand (checked for at run time it costs 7 us of 110 where there is none)
+    kWholeRes = 5     // a work item is a tile, with a residual operand
 };
 
 template <TcForm kForm>
@@ -249,7 +251,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_xf[kMaxStages], bar_empty[kMaxStages];
     __shared__ __align__(8) uint64_t bar_acc_full[4], bar_acc_empty[4];
     __shared__ __align__(8) uint64_t bar_drain;     // abort path: the MMAs issued so far have finished
-    __shared__ __align__(8) uint64_t bar_res[kBeside ? 2 : 1];    // taps side by side: a group's slab of the residual operand has landed
+    __shared__ __align__(8) uint64_t bar_res[2];    // a group's slab of the residual operand has landed
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ int s_issued[2];                     // operand copies issued by the two producers (abort path)
@@ -310,7 +312,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             mbar_init(&bar_acc_empty[i], (uint32_t)(128 * a.epi_groups));
         }
         mbar_init(&bar_drain, 1);
-        if (kBeside) { mbar_init(&bar_res[0], 1); mbar_init(&bar_res[1], 1); }
+        mbar_init(&bar_res[0], 1);
+        mbar_init(&bar_res[1], 1);
         s_abort = 0;
         s_issued[0] = 0; s_issued[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -353,7 +356,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             bool ok = true;
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
-                const TileCoord tc_ = tile_coord(a, wi.tile);
+                const TileCoord tc_ = tile_coord<kBeside>(a, wi.tile);
                 int ax, ay, an;
                 if constexpr (kBeside) {
                     // from the pixel before the first output pixel on
@@ -643,7 +646,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int ti = 0, staged_nbase = -1, round_no = 0;
             int res_copies = 0;        // of the residual operand, asked for by this thread
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
-                const TileCoord tc_ = tile_coord(a, w);
+                const TileCoord tc_ = tile_coord<kBeside>(a, w);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
                 const int nbase = tc_.n_tile * a.BN;
                 int groups = (a.Kp - nbase + 31) / 32;
@@ -803,9 +806,10 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int ti = 0;
             int staged_nbase = -1;
             int round_no = 0;          // rounds of this group so far (selects the staging slab)
+            int res_copies = 0;        // of the residual operand, asked for by this thread
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
-                const TileCoord tc_ = tile_coord(a, wi.tile);
+                const TileCoord tc_ = tile_coord<kBeside>(a, wi.tile);
                 const int as = a.n_acc == 4 ? (ti & 3) : (ti & 1), use = a.n_acc == 4 ? (ti >> 2) : (ti >> 1);
                 const int nbase = tc_.n_tile * a.BN;
                 int groups = (a.Kp - nbase + 31) / 32;
@@ -829,19 +833,18 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         my_bias[i] = (a.bias_mode == 2 && (!kSplit || (wi.ks == 0 && !a.ws_mode)) && nbase + i < a.K) ? a.beta * bias[nbase + i] : 0.f;
                     staged_nbase = bias_key;
                 }
-                // residual operand: this thread's pixel (its accumulator row) in the residual tensor
-                const float* res_row = nullptr;
-                if (!kSplit && a.res) {
-                    if (a.flat) {
-                        const long pixel = (long)tc_.w0 + row;
-                        if (pixel < a.Wo) res_row = a.res + pixel * a.res_ld;
-                    } else if (row < rows_in_tile) {
-                        const int rw = row % a.tw, t2 = row / a.tw;
-                        const int rh = t2 % a.th, rn = t2 / a.th;
-                        const int n = tc_.n0 + rn, h = tc_.h0 + rh, w_ = tc_.w0 + rw;
-                        if (n < a.N && h < a.Ho && w_ < a.Wo) res_row = a.res + (((long)n * a.Ho + h) * a.Wo + w_) * a.res_ld;
+                // A slab is free once the store from it has been read. A residual operand's values are then copied to it, and
+                // each thread adds its row and leaves the sum in their place.
+                auto free_slab = [&](int slab, int lcol) {
+                    if (a.epi_slabs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    if constexpr (kForm == kWholeRes) {
+                        ++res_copies;
+                        mbar_expect_tx(&bar_res[eg], (uint32_t)rows_in_tile * 128u);
+                        tma_load_4d(base + my_staging + (uint32_t)slab * (uint32_t)kStagingBytes, &tmY2, &bar_res[eg], lcol, tc_.w0, tc_.h0, tc_.n0);
                     }
-                }
+                };
+                if (kForm == kWholeRes && t == 0 && first < groups) free_slab(round_no % a.epi_slabs, nbase + first * 32);
                 ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
                 if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -855,11 +858,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int g0 = first; g0 < groups; g0 += step) {
                     const int sb = round_no % a.epi_slabs;
                     ++round_no;
-                    if (t == 0) {
-                        if (a.epi_slabs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    if (t == 0 && (kForm != kWholeRes || g0 != first)) free_slab(sb, nbase + g0 * 32);
+                    if constexpr (kForm == kWholeRes) {
+                        ok = group_and(bar_id, wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
+                        if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
+                    } else {
+                        group_sync(bar_id);
                     }
-                    group_sync(bar_id);
                     {
                         const int col = g0 * 32;
                         uint32_t r[32];
@@ -894,8 +899,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                 v.y = fmaf(a.alpha, __uint_as_float(r[c4 * 4 + 1]), bb.y);
                                 v.z = fmaf(a.alpha, __uint_as_float(r[c4 * 4 + 2]), bb.z);
                                 v.w = fmaf(a.alpha, __uint_as_float(r[c4 * 4 + 3]), bb.w);
-                                if (!kSplit && res_row) {
-                                    const float4 rr = __ldg(reinterpret_cast<const float4*>(res_row + lcol) + c4);
+                                if constexpr (kForm == kWholeRes) {
+                                    const float4 rr = dst[c4 ^ (row & 7)];
                                     v.x += rr.x; v.y += rr.y; v.z += rr.z; v.w += rr.w;
                                 }
                                 if (a.act == OGLE_ACT_RELU) {
@@ -913,6 +918,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                             for (int c4 = 0; c4 < 8; ++c4) {
                                 float v[4];
+                                float rr[4] = {0.f, 0.f, 0.f, 0.f};
+                                if constexpr (kForm == kWholeRes) {
+                                    const float4 q4 = dst[c4 ^ (row & 7)];
+                                    rr[0] = q4.x; rr[1] = q4.y; rr[2] = q4.z; rr[3] = q4.w;
+                                }
 #pragma unroll
                                 for (int l = 0; l < 4; ++l) {
                                     const int n = lcol + c4 * 4 + l;
@@ -920,7 +930,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                     if (n < kout) {
                                         if (a.bias_mode == 2) acc += my_bias[col + c4 * 4 + l];
                                         else if (a.bias_mode == 1) acc = fmaf(a.beta, bias[pix * a.ldc + n], acc);
-                                        if (!kSplit && res_row) acc += __ldg(res_row + n);
+                                        if (kForm == kWholeRes) acc += rr[l];
                                         acc = apply_act(acc, a.act, a.lo, a.hi);
                                     } else {
                                         acc = 0.f;         // padded lanes stay zero
@@ -957,6 +967,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 }
             }
+            // (an aborting block waits for the copy it has asked for)
+            if (!ok && res_copies > 0) mbar_wait(&bar_res[eg], (uint32_t)((res_copies - 1) & 1));
             // the staging slabs must outlive the stores that read them (their writes to global memory are
             // complete, like every write of the grid, when the grid is)
             if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -1131,6 +1143,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kRanges>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kWholeRes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTapsRes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
@@ -1169,6 +1182,8 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         launch_overlapped_if(overlapped, conv_tc2_kernel<kTapsRes>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else if (t.taps)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kTaps>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+    else if (t.res)
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kWholeRes>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else
         launch_overlapped_if(overlapped, conv_tc2_kernel<kWhole>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     return finish_launch();

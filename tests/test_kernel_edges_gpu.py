@@ -474,6 +474,44 @@ def test_taps_side_by_side_two_outputs_and_bounded_waits():
         assert lib.ogle_cuda_device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride: one tile and many, rows and columns that end inside a tile or slab, several slabs a
+    # group, pieces of images, the gather form
+    (1, 3, 5, 64, 4, 1, 1), (3, 41, 67, 32, 70, 1, 1), (2, 61, 50, 48, 256, 1, 1), (7, 15, 13, 96, 130, 1, 2), (4, 27, 40, 40, 100, 3, 2),
+    (3, 33, 150, 16, 33, 5, 1), (2, 64, 50, 3, 64, 7, 2), (150, 56, 56, 32, 64, 1, 1)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_residual_operand_by_the_copy_engine(shape, math):
+    """The values of the convolution, the residual added and the activation, in those single-precision steps; roles that
+    give up with a copy of the operand in flight."""
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    N, H, W, C, K, k, s = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *d: torch.randn(d, generator=g, device="cuda")
+    x, w, b = torch.zeros((N, H, W, ops.up4(C)), device="cuda"), rand(K, C, k, k) / (C * k * k) ** 0.5, rand(K)
+    x[..., :C] = rand(N, H, W, C)
+    p = ops.conv_params(N, H, W, C, K, k, s, k // 2, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    p.split = 1
+    packed = ops.conv2d_prepack(p, w)
+    plain = ops.conv2d(p, x, packed, b, workspace=None)
+    res = rand(*plain.shape)
+    res[..., K:] = 0.0
+    for act in (ops.ACT_NONE, ops.ACT_RELU):
+        p.act = act
+        got = ops.conv2d_residual(p, x, packed, b, res)
+        assert ops.last_contraction().form in (1, 6)
+        assert torch.equal(got, plain + res if act == ops.ACT_NONE else (plain + res).clamp(min=0))
+    try:
+        lib.ogle_cuda_set_wait_limit(0)
+        ops.conv2d_residual(p, x, packed, b, res)
+        assert lib.ogle_cuda_device_status() == -6
+    finally:
+        lib.ogle_cuda_set_wait_limit(-1)
+        lib.ogle_cuda_clear_device_status()
+    assert torch.equal(ops.conv2d_residual(p, x, packed, b, res), got)
+
+
 def test_bounded_waits_of_the_cluster_form(oracle_port):
     """Zero polls allowed: every block of a cluster gives up, all meet at the cluster's barriers, the launch returns with
     the status word set, and with the limit restored the same call gives what it gave before."""
