@@ -197,6 +197,7 @@ struct DetectArgs {
     KeySpace ks;
     float nms_thr;
     int classes_per_pass;   // mode 1: foreground classes whose scores fit in shared memory at once
+    int ahead;              // mode 1: a block has the image this many further on fetched while it selects (0 = none)
     int parts;              // mode 1: blocks per image, each taking a contiguous range of the foreground classes
     const OgleImageDesc* frames;   // mode 0: per-image frame sizes, or null
     const float4* anchors;         // not null: `boxes` holds deltas, decoded against these as they are written
@@ -230,6 +231,12 @@ __device__ __forceinline__ void load_row(const DetectArgs& a, const float* row, 
         if (j < a.C) e[j] = expf(e[j]);
 }
 
+// Bytes [0, bytes) at p on their way into L2, a line a thread.
+__device__ __forceinline__ void prefetch_l2(const void* p, long bytes) {
+    for (long o = (long)threadIdx.x * 128; o < bytes; o += (long)blockDim.x * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + o));
+}
+
 // Mode 1: per class. Dynamic shared memory: float scores[classes_per_pass][Ap], histograms of as many classes
 // (kHistWords words each), one list of survivors per warp (kListMax 16-bit indices).
 __global__ void __launch_bounds__(640)
@@ -247,6 +254,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
     unsigned* hists = reinterpret_cast<unsigned*>(scores + (size_t)a.classes_per_pass * a.Ap);
     unsigned short* list = reinterpret_cast<unsigned short*>(hists + (size_t)a.classes_per_pass * kHistWords) + warp * kListMax;
     const int rows = (a.C - 1) * a.top_k;
+    if (a.ahead > 0) prefetch_l2(bx, (long)a.A * sizeof(float4));
     const int per_part = (a.C - 1 + a.parts - 1) / a.parts;
     const int c_lo = 1 + part * per_part, c_hi = min(a.C, c_lo + per_part);     // this block's classes
     for (int c0 = c_lo; c0 < c_hi; c0 += a.classes_per_pass) {
@@ -287,6 +295,8 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
             }
         }
         __syncthreads();
+        if (a.ahead > 0 && c0 == c_lo && n + a.ahead < a.N)
+            prefetch_l2(lg + (long)a.ahead * a.A * a.logit_stride, (long)a.A * a.logit_stride * sizeof(float));
         for (int j = warp; j < nc; j += nwarps) {
             const int cls = c0 + j;
             const float* vals = scores + j * a.Ap;
@@ -507,6 +517,7 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         size_t cpp = (budget - warp_bytes) / per_class;
         if (cpp > (size_t)classes) cpp = classes;
         a.classes_per_pass = (int)cpp;
+        a.ahead = p->N > kNumSMs ? kNumSMs : 0;
         smem = cpp * per_class + warp_bytes;
     } else {
         threads = 512;
