@@ -147,7 +147,11 @@ enum TcForm {
     // 128 x 14 x 14 x 256 -> 256 102 -> 96, 128 x 7 x 7 x 512 -> 512 114 -> 94; one pass, the first: 131 -> 82.
     kTaps = 3,
     kTapsRes = 4,     // ... with a residual operand (checked for at run time it costs 7 us of 110 where there is none)
-    kWholeRes = 5     // a work item is a tile, with a residual operand
+    kWholeRes = 5,    // a work item is a tile, with a residual operand
+    // Gather form whose filters all fit beside two input windows: filters copied once a block, a tile's window once, and the
+    // ring's stages are places in tensor memory alone. Copied per chunk they were 140 KB a tile of the shared-memory
+    // traffic that bounds the form.
+    kKept = 6
 };
 
 template <TcForm kForm>
@@ -266,7 +270,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const uint32_t b_bytes = (uint32_t)(a.BN * kSets) * 128u;
     // activation part of a stage (none where the gather form builds its operand in tensor memory)
     const uint32_t a_bytes = a.gather && a.ta ? 0u : (split && !a.ta ? 2u : 1u) * kABytes;
-    const uint32_t stage_bytes = a_bytes + (split ? 2u : 1u) * b_bytes + (a.gather ? (uint32_t)a.g_bytes : 0u);
+    const int chunks = (kBeside ? 1 : a.kernel) * a.kernel * a.chunks_per_tap;
+    const uint32_t stage_bytes = kForm == kKept ? 0u : a_bytes + (split ? 2u : 1u) * b_bytes + (a.gather ? (uint32_t)a.g_bytes : 0u);
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
     // ring of operand stages (A | A cross (bf16 hi|lo), unless it lives in tensor memory | B_hi | B cross (bf16 lo|hi)),
@@ -274,7 +279,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     auto sA = [&](int s) { return base + (uint32_t)s * stage_bytes; };
     auto sBhi = [&](int s) { return sA(s) + a_bytes; };
     auto sWin = [&](int s) { return sA(s) + a_bytes + (split ? 2u : 1u) * b_bytes; };   // gather form: input window
-    const uint32_t staging_off = (uint32_t)a.stages * stage_bytes;
+    const uint32_t kept_filters = (uint32_t)chunks * 2u * b_bytes;           // (kKept) then the two windows
+    const uint32_t staging_off = kForm == kKept ? kept_filters + 2u * (uint32_t)a.g_bytes : (uint32_t)a.stages * stage_bytes;
     {
         // the layout must fit what the launch reserved (it does when the base is 1024-aligned as
         // declared); checked, not assumed, because an overrun would write past the block's window
@@ -288,7 +294,6 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
 
-    const int chunks = (kBeside ? 1 : a.kernel) * a.kernel * a.chunks_per_tap;
     const int acc_cols = a.BN * kSets;     // tensor-memory columns of one accumulator
     const int rows_in_tile = a.flat ? kTileM : a.tn * a.th * a.tw;
     volatile int* abort_flag = &s_abort;
@@ -312,8 +317,10 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             mbar_init(&bar_acc_empty[i], (uint32_t)(128 * a.epi_groups));
         }
         mbar_init(&bar_drain, 1);
-        mbar_init(&bar_res[0], 1);
-        mbar_init(&bar_res[1], 1);
+        if (kForm == kTapsRes || kForm == kWholeRes) {
+            mbar_init(&bar_res[0], 1);
+            mbar_init(&bar_res[1], 1);
+        }
         s_abort = 0;
         s_issued[0] = 0; s_issued[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -354,7 +361,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             uint32_t wrap = 0;         // how many times the ring has wrapped
             int issued = 0;            // chunks in flight bookkeeping for the abort path
             bool ok = true;
-            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
+            int window = 0;
+            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, window ^= 1) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 const TileCoord tc_ = tile_coord<kBeside>(a, wi.tile);
                 int ax, ay, an;
@@ -380,7 +388,15 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     if (wrap > 0) ok = wait_or_abort(&bar_empty[s], (wrap - 1) & 1u, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 1); break; }
-                    if (a.gather) {
+                    if (kForm == kKept) {
+                        // (the ring is at most a stage longer than a tile's reduction: the window before the last has been read)
+                        if (it == 0) {
+                            mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
+                            tma_load_4d(base + kept_filters + (uint32_t)(window * a.g_bytes), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
+                        } else {
+                            mbar_arrive(&bar_full[s]);
+                        }
+                    } else if (a.gather) {
                         mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
                         tma_load_4d(sWin(s), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
                     } else {
@@ -413,6 +429,20 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     if (wrap > 0) ok = wait_or_abort(&bar_empty[s], (wrap - 1) & 1u, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 7); break; }
+                    if (kForm == kKept) {
+                        if (w == (int)blockIdx.x) {
+                            const uint32_t to = base + (uint32_t)it * 2u * b_bytes;
+                            mbar_expect_tx(&bar_full[s], tx);
+                            tma_load_2d(to, &tmBhi, &bar_full[s], brow, bcol);
+                            tma_load_2d(to + b_bytes, &tmBlo, &bar_full[s], brow, bcol);
+                        } else {
+                            mbar_arrive(&bar_full[s]);
+                        }
+                        ++issued;
+                        if (++s == a.stages) { s = 0; ++wrap; }
+                        brow += kChunk;
+                        continue;
+                    }
                     mbar_expect_tx(&bar_full[s], tx);
                     if constexpr (kBeside) {
                         // the filter row's three taps, one below the other in shared memory (with a copy for each its
@@ -455,7 +485,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     ok = wait_or_abort(a.gather || a.ta == 1 ? &bar_xf[s] : &bar_full[s], ph, abort_flag, a.spin_limit);
                     if (!ok) { record_error(err_flag, 2); s_abort = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = umma_desc(sA(s)), bd = umma_desc(sBhi(s));
+                    const uint64_t ad = umma_desc(sA(s)), bd = umma_desc(kForm == kKept ? base + (uint32_t)it * 2u * b_bytes : sBhi(s));
                     const uint32_t acc_flag = it > (kSplit ? wi.c_begin : 0) ? 1u : 0u;     // the first chunk overwrites
                     if (a.ta == 1) {
                         const uint32_t ta = tmem_a + (uint32_t)s * 64u;
@@ -506,7 +536,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int s = 0, turn = 0;
             uint32_t ph = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x) {
+            int window = 0;
+            for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, window ^= 1) {
                 const WorkItem wi = work_item<kForm>(a, w, chunks);
                 for (int it = wi.c_begin; it < wi.c_end; ++it) {
                     // Every stage is waited for in turn, also those of the other group's chunks: copies land out of
@@ -527,7 +558,8 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         } else if (kBeside || !a.gather) {
                             split_row_to_tmem(reinterpret_cast<const float4*>(stage + (size_t)r * 128), r, to);
                         } else {
-                            const float* win = reinterpret_cast<const float*>(stage + 2u * b_bytes) + g_row;
+                            const float* win = reinterpret_cast<const float*>(kForm == kKept ? base_ptr + kept_filters + (size_t)(window * a.g_bytes)
+                                                                                             : stage + 2u * b_bytes) + g_row;
                             if (a.g_k == 7) gather_row_to_tmem<7>(win, a.g_iw * 4, it, to);
                             else if (a.g_k == 5) gather_row_to_tmem<5>(win, a.g_iw * 4, it, to);
                             else gather_row_to_tmem<3>(win, a.g_iw * 4, it, to);
@@ -1074,7 +1106,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     const int ta_stages = (512 - t.n_acc * acc_cols) / ta_cols;
     t.ta = ta_form && !ta_off && ta_stages >= 2 ? (ta_cols == 32 ? 2 : 1) : 0;
     if (!t.ta) t.n_acc = 4 * acc_cols <= 512 ? 4 : 2;
-    const size_t stage = (size_t)(t.ta && t.gather ? 0 : (t.passes == 3 && !t.ta ? 2 : 1)) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * b_rows * 128 +
+    size_t stage = (size_t)(t.ta && t.gather ? 0 : (t.passes == 3 && !t.ta ? 2 : 1)) * kABytes + (size_t)(t.passes == 3 ? 2 : 1) * b_rows * 128 +
                          (t.gather ? (size_t)t.g_bytes : 0);
     // Shared memory is split between the operand ring and the epilogue's staging slabs
     // (128 rows x 32 columns each). Preference: two epilogue groups with two slabs each;
@@ -1112,11 +1144,24 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     if (const char* e = env_groups) t.epi_groups = e[0] == '1' ? 1 : 2;
     if (const char* e = env_slabs) t.epi_slabs = e[0] == '1' ? 1 : 2;
     if (t.cluster) t.epi_slabs = 0;       // partial tiles go where the operand ring was
-    const size_t staging = (size_t)t.epi_groups * t.epi_slabs * kStagingBytes;
+    size_t staging = (size_t)t.epi_groups * t.epi_slabs * kStagingBytes;
     const size_t budget = kBudget - staging;
     int stages = (int)(budget / stage);
     if (stages > kMaxStages) stages = kMaxStages;
     if (t.ta && stages > ta_stages) stages = ta_stages;
+    // Filters and windows kept where they fit; two windows are enough while the ring is at most a stage longer than a tile's
+    // reduction, and one filter tile serves all.
+    const size_t kept = (size_t)chunks * 2 * b_rows * 128 + 2 * (size_t)t.g_bytes;
+    const int kept_stages = ta_stages < chunks + 1 ? ta_stages : chunks + 1;
+    const bool keep = t.gather && t.ta && !t.res && t.n_tiles == 1 && t.split_k <= 1 && chunks >= 2 && kept_stages >= 2 &&
+                      kept + 4 * (size_t)kStagingBytes <= kBudget;
+    if (keep) {
+        t.epi_groups = 2;
+        t.epi_slabs = 2;
+        staging = 4 * (size_t)kStagingBytes + kept;
+        stage = 0;
+        stages = kept_stages < kMaxStages ? kept_stages : kMaxStages;
+    }
     if (stages < 2) return OGLE_ERR_UNSUPPORTED;
     t.stages = stages;
     int cols = 32;
@@ -1143,6 +1188,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
         cudaError_t e = cudaFuncSetAttribute(conv_tc2_kernel<kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kRanges>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kKept>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kWholeRes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTapsRes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(conv_tc2_kernel<kTaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
@@ -1178,6 +1224,8 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     }
     if (t.split_k > 1)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kRanges>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
+    else if (keep)
+        launch_overlapped_if(overlapped, conv_tc2_kernel<kKept>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else if (t.taps && t.res)
         launch_overlapped_if(overlapped, conv_tc2_kernel<kTapsRes>, dim3(grid), dim3(kThreads2), smem, s, mA, mBhi, mBlo, mY, mY2, bias, t, err_flag);
     else if (t.taps)

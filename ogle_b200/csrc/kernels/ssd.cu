@@ -296,7 +296,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
         }
         __syncthreads();
         if (a.ahead > 0 && c0 == c_lo && n + a.ahead < a.N)
-            prefetch_l2(lg + (long)a.ahead * a.A * a.logit_stride, (long)a.A * a.logit_stride * sizeof(float));
+            prefetch_l2(lg + (long)a.ahead * a.A * a.logit_stride, ((long)(a.A - 1) * a.logit_stride + a.C) * sizeof(float));
         for (int j = warp; j < nc; j += nwarps) {
             const int cls = c0 + j;
             const float* vals = scores + j * a.Ap;

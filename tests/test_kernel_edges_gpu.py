@@ -512,6 +512,39 @@ def test_residual_operand_by_the_copy_engine(shape, math):
     assert torch.equal(ops.conv2d_residual(p, x, packed, b, res), got)
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, K, kernel, stride: one tile, several a block, tiles that hang over every edge; filters that fit beside the windows and not
+    (1, 32, 32, 16, 7, 2), (9, 113, 75, 64, 7, 2), (40, 70, 70, 40, 5, 1), (3, 130, 130, 128, 7, 1), (5, 64, 64, 200, 5, 2), (30, 64, 64, 8, 3, 2)])
+def test_kept_filters_and_windows_of_rgb_stems(shape):
+    """Filters copied once a block and a window once a tile, against copies per chunk - the form with a residual operand, here
+    zeros - bit for bit, and with roles that give up."""
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    N, H, W, K, k, s = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = torch.zeros((N, H, W, 4), device="cuda")
+    x[..., :3] = torch.randn((N, H, W, 3), generator=g, device="cuda")
+    w, b = torch.randn((K, 3, k, k), generator=g, device="cuda") / (3 * k * k) ** 0.5, torch.randn(K, generator=g, device="cuda")
+    p = ops.conv_params(N, H, W, 3, K, k, s, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_TF32X3)
+    packed = ops.conv2d_prepack(p, w)
+    want = torch.nn.functional.conv2d(x[..., :3].permute(0, 3, 1, 2).double(), w.double(), b.double(), s, k // 2).permute(0, 2, 3, 1).clamp(min=0)
+    got = ops.conv2d(p, x, packed, b, workspace=None)
+    # 147 products and sums of fp32 grade
+    assert float((got[..., :K].double() - want).norm()) <= 3e-6 * float(want.norm())
+    if k == 3:
+        return                                                        # (the direct kernel's)
+    assert torch.equal(ops.conv2d_residual(p, x, packed, b, torch.zeros_like(got)), got)
+    try:
+        lib.ogle_cuda_set_wait_limit(0)
+        ops.conv2d(p, x, packed, b, workspace=None)
+        assert lib.ogle_cuda_device_status() == -6
+    finally:
+        lib.ogle_cuda_set_wait_limit(-1)
+        lib.ogle_cuda_clear_device_status()
+    assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), got)
+
+
 def test_bounded_waits_of_the_cluster_form(oracle_port):
     """Zero polls allowed: every block of a cluster gives up, all meet at the cluster's barriers, the launch returns with
     the status word set, and with the limit restored the same call gives what it gave before."""
