@@ -70,11 +70,9 @@ dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict_
     __syncthreads();
 
     // tile id -> (channel slab fastest, then x, y, image): neighbouring blocks share halo rows in L2
-    // (tile counts fit 32 bits: the launch refuses more). The list is walked from the tensor's end: what the kernel before
-    // wrote last is still in L2 then, and where this one ends the next one, which walks the other way, begins.
-    const unsigned last_tile = (unsigned)tl.total - 1u;
+    // (tile counts fit 32 bits: the launch refuses more)
     auto issue = [&](long tile, int stage) {
-        unsigned t = last_tile - (unsigned)tile;
+        unsigned t = (unsigned)tile;
         const int cb = (int)(t % (unsigned)tl.cblocks); t /= (unsigned)tl.cblocks;
         const int tx = (int)(t % (unsigned)tl.tiles_x); t /= (unsigned)tl.tiles_x;
         const int ty = (int)(t % (unsigned)tl.tiles_y); t /= (unsigned)tl.tiles_y;
@@ -103,7 +101,7 @@ dw_tma_kernel(const __grid_constant__ CUtensorMap tmX, const float4* __restrict_
             const long ahead = tile + (long)(nst - 1) * gridDim.x;
             if (ahead < tl.total) { issue(ahead, stage == 0 ? nst - 1 : stage - 1); ++issued; }
         }
-        unsigned t = last_tile - (unsigned)tile;
+        unsigned t = (unsigned)tile;
         const int cb = (int)(t % (unsigned)tl.cblocks); t /= (unsigned)tl.cblocks;
         const int tx = (int)(t % (unsigned)tl.tiles_x); t /= (unsigned)tl.tiles_x;
         const int ty = (int)(t % (unsigned)tl.tiles_y); t /= (unsigned)tl.tiles_y;
