@@ -87,17 +87,14 @@ batchnorm_kernel(const float4* __restrict__ x, const float* __restrict__ gamma, 
     long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= total) return;
     const BnChannels p = bn_channels(gamma, beta, mean, var, int(i % q) * 4, C, eps);
-    // from the tensor's end: what the kernel before wrote last is still in L2
-    long left = (total - i + step - 1) / step;
-    i += (left - 1) * step;
-    for (; left >= 4; left -= 4, i -= 4 * step) {
+    for (; i + 3 * step < total; i += 4 * step) {
         float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = x[i - u * step];
+        for (int u = 0; u < 4; ++u) v[u] = x[i + u * step];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) y[i - u * step] = bn_apply(v[u], p);
+        for (int u = 0; u < 4; ++u) y[i + u * step] = bn_apply(v[u], p);
     }
-    for (; left > 0; --left, i -= step) y[i] = bn_apply(x[i], p);
+    for (; i < total; i += step) y[i] = bn_apply(x[i], p);
 }
 
 // Tensors of one element a thread, whose time is the launch, one trip to memory and the fetch of the kernel's

@@ -58,9 +58,7 @@ __global__ void __launch_bounds__(128) pool_patch_kernel(const float4* __restric
     const float init = MAX ? -FLT_MAX : 0.f;
     const Index step = (Index)gridDim.x * blockDim.x;
     for (Index i = blockIdx.x * (Index)blockDim.x + threadIdx.x; i < total; i += step) {
-        // (maxima from the tensor's end: what the kernel before wrote last is still in L2, and an average of the same
-        // tensor then begins where this ends)
-        Index t = MAX ? total - 1 - i : i;
+        Index t = i;
         const int c4 = int(t % a.C4); t /= a.C4;
         const int px = int(t % gx); t /= gx;
         const int py = int(t % gy); t /= gy;
