@@ -143,8 +143,8 @@ enum TcForm {
     // operand splits, and 3 BN columns a multiply: 64 channels alone leave the tensor cores half idle. With 64 channels a
     // tile a split-mode chunk moves 144 KB through shared memory (copies 64, operand split 16, multiplies 64), at the
     // 117 bytes a clock seen here 0.6 us, which is what it takes; a tile's epilogue adds about 1 us to that.
-    // Split mode, before and after: 128 x 56 x 56 x 64 -> 64 172 -> 114 us, 128 x 28 x 28 x 128 -> 128 107 -> 99,
-    // 128 x 14 x 14 x 256 -> 256 102 -> 96, 128 x 7 x 7 x 512 -> 512 114 -> 94; one pass, the first: 131 -> 82.
+    // Split mode, before and after: 128 x 56 x 56 x 64 -> 64 172 -> 110 us, 128 x 28 x 28 x 128 -> 128 107 -> 94,
+    // 128 x 14 x 14 x 256 -> 256 101 -> 95, 128 x 7 x 7 x 512 -> 512 115 -> 92; one pass, the first: 131 -> 74.
     kTaps = 3,
     kTapsRes = 4,     // ... with a residual operand (checked for at run time it costs 7 us of 110 where there is none)
     kWholeRes = 5,    // a work item is a tile, with a residual operand
