@@ -131,7 +131,8 @@ typedef struct {
     int channels_on_m;       /* tensor-core path, at most 128 output channels, unsplit reduction: 2 = keep the
                                 accumulator transposed (filters on the 128-row side of the multiply, 256 pixels per
                                 instruction), which halves the tensor-core instructions of layers with 64-128 output
-                                channels; 1 = no, 0 = chosen by the library. Ignored where it cannot run. */
+                                channels; 1 = no, 0 = chosen by the library. Ignored where it cannot run. 1 and 2 give the
+                                same bits: where it could run, neither lets the taps of a 3x3 layer lie side by side. */
     int sm_pair;             /* tensor-core path: 2 = compute tiles of 256 pixels on pairs of SMs (each SM of a
                                 pair loads half of the filter tile; needs n_tile a multiple of 64 and an unsplit
                                 reduction - chosen or asked for by split = 1 - else ignored), 1 = one SM per tile, 0 = chosen by the library.

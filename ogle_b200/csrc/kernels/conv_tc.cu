@@ -264,12 +264,16 @@ bool choose_cluster(TcArgs* t, int Kp, long m_tiles, int chunks, int split, int 
     return true;
 }
 
-// Whether a launch takes the channels-on-M form (conv_tc2_t.cu): at most 128 (stacked) output channels, an
-// unsplit reduction, no gather, at least two 128-pixel tiles, and the caller asked for it (2) or the
-// environment forces it for experiments.
+// Whether an unsplit launch can take the channels-on-M form (conv_tc2_t.cu): at most 128 (stacked) output channels, no
+// gather, at least two 128-pixel tiles.
+bool fits_channels_on_m(const TcArgs& t, int Kp_total, long m_tiles) {
+    return !t.gather && t.bias_mode != 1 && Kp_total <= 128 && m_tiles >= 2;
+}
+// Whether a launch takes it: it can, its reduction is unsplit, and the caller asked for it (2) or the environment forces it
+// for experiments.
 bool want_channels_on_m(const TcArgs& t, int Kp_total, long m_tiles, int requested, bool through_scratch = false) {
     static const int mode = [] { const char* e = getenv("OGLE_TC_T"); return e ? (e[0] == '0' ? 1 : (e[0] == '1' ? 2 : 0)) : 0; }();
-    if (t.gather || t.bias_mode == 1 || Kp_total > 128 || m_tiles < 2) return false;
+    if (!fits_channels_on_m(t, Kp_total, m_tiles)) return false;
     // a split reduction only in the form that goes through scratch
     if (through_scratch ? !(t.ws_mode && t.split_k > 1) : (t.split_k > 1 || t.ws_mode)) return false;
     if (mode == 1 || requested == 1) return false;
@@ -585,8 +589,11 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         if (cluster || t.split_k <= 1) { t = c; m_tiles = cut; }
         if (!cluster) {
             on_pairs = want_pair(t, m_tiles, a.pair);
-            // (whether taps lie side by side is settled without a look at n_tile and sm_pair: it does touch the bits)
-            const int beside = t.split_k <= 1 && !a.on_m && tiled ? taps_width(a, own, m_tiles, chunks) : 0;
+            // (whether taps lie side by side is settled without a look at n_tile and sm_pair: it does touch the bits. Not
+            // where channels lie on M, by the caller's wish or the environment's; and a caller who says 1 or 2 to that, of a
+            // layer it fits, gets the same bits for both)
+            const bool on_m_form = on_m || (a.on_m && fits_channels_on_m(t, a.Kp, m_tiles));
+            const int beside = t.split_k <= 1 && !on_m_form && tiled ? taps_width(a, own, m_tiles, chunks) : 0;
             if (beside) {
                 m_tiles = tile_taps(a, beside, &t);
                 on_pairs = false;

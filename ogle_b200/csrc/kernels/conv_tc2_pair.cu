@@ -560,7 +560,7 @@ int num_sms_for_pairs() {
 int launch_tc_pair(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, const CUtensorMap& mBlo,
                    const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
                    cudaStream_t s) {
-    if (t.BN % 64 || t.BN > 256 || t.BN < 64 || t.gather || t.split_k > 1 || t.ws_mode) return OGLE_ERR_UNSUPPORTED;
+    if (t.BN % 64 || t.BN > 256 || t.BN < 64 || t.gather || t.taps || t.split_k > 1 || t.ws_mode) return OGLE_ERR_UNSUPPORTED;
     const size_t stage = (size_t)(t.passes == 3 ? 2 : 1) * (kABytes + (size_t)(t.BN / 2) * 128);
     const size_t kBudget = 224 * 1024;
     t.xf_groups = t.passes == 3 ? 2 : 1;

@@ -478,7 +478,7 @@ int launch_tc_t(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, const
                 const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
                 cudaStream_t s) {
     const int FR = t.BN;
-    if (FR % 32 || FR < 32 || FR > 128 || t.n_tiles != 1 || t.gather || t.bias_mode == 1 || (t.res && t.split_col > 0))
+    if (FR % 32 || FR < 32 || FR > 128 || t.n_tiles != 1 || t.gather || t.taps || t.bias_mode == 1 || (t.res && t.split_col > 0))
         return OGLE_ERR_UNSUPPORTED;
     if (t.split_k < 1) t.split_k = 1;
     if ((t.split_k > 1) != (t.ws_mode != 0) || (t.ws_mode && t.res)) return OGLE_ERR_UNSUPPORTED;   // splits go through scratch only

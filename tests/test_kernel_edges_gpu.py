@@ -474,6 +474,65 @@ def test_taps_side_by_side_two_outputs_and_bounded_waits():
         assert lib.ogle_cuda_device_status() == 0
 
 
+ON_M_CODE = """
+import torch
+from ogle_b200 import _lib, ops
+g = torch.Generator(device="cuda").manual_seed(7)
+rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+# many-tile 3x3 layers, which would lie with their taps side by side; the last has too many channels to lie on M
+for N, H, W, C, K in [(128, 28, 28, 64, 64), (6, 75, 75, 40, 96), (9, 50, 61, 32, 128), (16, 28, 28, 128, 160)]:
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        x, w, b = rand(N, H, W, C), rand(K, C, 3, 3) / (9 * C) ** 0.5, rand(K)
+        res = rand(N, H, W, ops.up4(K))
+        p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, math)
+        p.split = 1
+        packed = ops.conv2d_prepack(p, w)
+        want = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), w.double(), b.double(), padding=1).permute(0, 2, 3, 1)
+        # (as for the taps: sums in tensor memory lose 6e-9 of their norm per element, products and operands 1e-6; one pass: 2^-10)
+        bound = (2e-6 + 6e-9 * 9 * C if math == ops.MATH_TF32X3 else 1e-3) * float(want.norm())
+        form = 5 if K <= 128 else 6
+        for got, ref in ((ops.conv2d(p, x, packed, b, workspace=None), want), (ops.conv2d_residual(p, x, packed, b, res), want + res[..., :K])):
+            assert ops.last_contraction().form == form, (N, H, W, C, K, math, ops.last_contraction().form)
+            assert float((got[..., :K].double() - ref).norm()) <= bound, (N, H, W, C, K, math)
+        if K == 64:
+            one, two = ops.conv2d_pair(x, w[:20], b[:20], w[20:], b[20:], N, H, W, C, 3, 1, 1, 1, ops.ACT_NONE, 0.0, 0.0, math, use_workspace=False)
+            assert ops.last_contraction().form == 5
+            assert float((torch.cat([one[..., :20], two[..., :44]], -1).double() - want).norm()) <= bound
+assert _lib.cuda_lib().ogle_cuda_device_status() == 0
+"""
+
+
+def test_channels_on_m_forced_on_layers_of_taps_side_by_side():
+    """The switch that puts channels on M wherever they fit (switches are read once per process) comes before the taps' own."""
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", ON_M_CODE], cwd=root, env=dict(os.environ, OGLE_TC_T="1", OGLE_TC_TAPS="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("K", [64, 128, 160])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_channels_on_m_only_where_it_runs(K, math):
+    """Where channels on M cannot run, channels_on_m = 1 and 2 leave a layer as it is; where it can, the two give the same
+    bits."""
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    N, H = (64, 28) if K <= 128 else (8, 56)
+    x, w, b = rand(N, H, H, 64), rand(K, 64, 3, 3) / 24.0, rand(K)
+    p = ops.conv_params(N, H, H, 64, K, 3, 1, 1, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, getattr(ops, math))
+    p.split = 1
+    packed = ops.conv2d_prepack(p, w)
+    outs, forms = [], []
+    for p.channels_on_m in (0, 1, 2):
+        outs.append(ops.conv2d(p, x, packed, b, workspace=None))
+        forms.append(ops.last_contraction().form)
+    assert forms[0] == 6 or math == "MATH_TF32"                        # (one pass, many channels: whole tiles)
+    assert forms[1] in (1, 4) and forms[2] == 5 if K <= 128 else forms == forms[:1] * 3
+    assert torch.equal(outs[1], outs[2]) and (K <= 128 or torch.equal(outs[0], outs[1]))
+
+
 @pytest.mark.parametrize("shape", [
     # N, H, W, C, K, kernel, stride: one tile and many, rows and columns that end inside a tile or slab, several slabs a
     # group, pieces of images, the gather form
