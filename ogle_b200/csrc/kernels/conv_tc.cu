@@ -130,39 +130,6 @@ double pair_tiles_us(const TcArgs& t, int bn, int Kp, long m_tiles, int chunks) 
     return (double)((work + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (mul > epi ? mul : epi) + 5.5 + kTailUs * bn;
 }
 
-// Channels of a tile whose taps lie side by side (kTaps form), 0 = the launch does not take it: 3x3, stride 1, padding 1,
-// where rounds of its tiles - 32 or 64 channels, a chunk and filter row at the measured time, and a longer epilogue - are
-// modelled to take less than whole tiles in their better form. OGLE_TC_TAPS: 0 never, 1 wherever it can run.
-int taps_width(const ConvArgs& a, const TcArgs& t, long m_tiles, int chunks) {
-    static const int mode = [] { const char* e = getenv("OGLE_TC_TAPS"); return e ? (e[0] == '0' ? 1 : (e[0] == '1' ? 2 : 0)) : 0; }();
-    if (mode == 1 || a.kernel != 3 || a.stride != 1 || a.pad != 1 || a.dil != 1 || a.M > 0x7fffff00L || !encode_im2col_fn()) return 0;
-    if (mode == 0 && (forced_width(a.Kp) || pair_mode_override() == 2)) return 0;        // (those switches come first)
-    double other = 1e30, best = 1e30;
-    for (int bn = 32; bn <= 256 && bn <= (a.Kp + 31) / 32 * 32; bn += 32) {
-        if (t.passes != 3 && bn != t.BN) continue;
-        const double one = whole_tiles_us(t, bn, a.Kp, m_tiles, chunks);
-        const double two = t.passes == 3 && m_tiles >= 2 && bn % 64 == 0 ? pair_tiles_us(t, bn, a.Kp, m_tiles, chunks) : one;
-        other = one < other ? one : other;
-        other = two < other ? two : other;
-    }
-    int width = 0;
-    long rounds = 0;
-    for (int bn = 32; bn <= 64; bn += 32) {
-        const long tiles = (a.M + kTapsPixels - 1) / kTapsPixels * ((a.Kp + bn - 1) / bn);
-        // (a single round is mostly start, fill and drain; stacked siblings are padded to 32 channels each and seldom fill
-        // tiles of 64: in few rounds the model cannot tell which form is the better one)
-        if (mode == 0 && tiles <= (t.split_col ? 4 : 1) * kNumSMs) continue;
-        const double chunk = t.passes == 3 ? (bn == 64 ? 0.57 : 0.45) : (bn == 64 ? 0.33 : 0.28);
-        const double least = t.passes == 3 ? (bn == 64 ? 3.7 : 2.5) : (bn == 64 ? 3.1 : 2.2), tile = chunks / 3 * chunk + 1.0;
-        const double us = (double)((tiles + kNumSMs - 1) / kNumSMs) * (tile > least ? tile : least) + 7.0;
-        if (us < best) { best = us; width = bn; rounds = (tiles + kNumSMs - 1) / kNumSMs; }
-    }
-    // (split mode, tensors that come from HBM: whole tiles take 1.08 of the model and 3 us more, 20-170 us measured)
-    if (t.passes == 3) other = 1.08 * other + 3.0;
-    // (in two rounds start and drain are most of the time, and the models further off: 4 x 8 x 64 x 16 -> 577 11.3 us, 11.9)
-    return mode == 2 || best < (rounds <= 2 ? 0.88 : 0.97) * other ? width : 0;
-}
-
 // Tiles of a launch whose taps lie side by side, bn channels each.
 long tile_taps(const ConvArgs& a, int bn, TcArgs* t) {
     t->taps = 1;
@@ -195,6 +162,34 @@ bool refine_width(TcArgs* t, int Kp, long m_tiles, int chunks, bool may_pair) {
     return best_pair;
 }
 
+// Tiles of a k x k layer in whole rows of the map (pieces of one where it is wider than a tile); returns their number.
+// may_split: the reduction may be split in two where that fills the SMs.
+long whole_row_tiles(const ConvArgs& a, bool may_split, TcArgs* t) {
+    if (a.Wo >= kTileM) {
+        const int parts = (a.Wo + kTileM - 1) / kTileM;
+        t->tw = (a.Wo + parts - 1) / parts; t->th = 1; t->tn = 1;
+    } else {
+        // full-width tiles of th rows from tn consecutive images (th * tn * Wo <= 128):
+        // take the shape that needs the fewest rounds of one tile per SM; among equals the
+        // tallest, whose filter taps overlap most in L2
+        t->tw = a.Wo;
+        long best = -1;
+        for (int th = 1; th <= a.Ho && th * a.Wo <= kTileM; ++th) {
+            int tn = kTileM / (th * a.Wo);
+            if (tn > a.N) tn = a.N;
+            if ((th - 1) * a.stride + 1 > 256) continue;          // TMA box limit
+            const long tiles = (long)((a.Ho + th - 1) / th) * ((a.N + tn - 1) / tn);
+            // in half-rounds; a reduction split in two can fill a ragged last round
+            long rounds = 2 * ((tiles + kNumSMs - 1) / kNumSMs);
+            if (may_split && (2 * tiles + kNumSMs - 1) / kNumSMs < rounds) rounds = (2 * tiles + kNumSMs - 1) / kNumSMs;
+            if (best < 0 || rounds <= best) { best = rounds; t->th = th; t->tn = tn; }
+        }
+    }
+    t->tiles_w = (a.Wo + t->tw - 1) / t->tw;
+    t->tiles_h = (a.Ho + t->th - 1) / t->th;
+    return (long)t->tiles_w * t->tiles_h * ((a.N + t->tn - 1) / t->tn);
+}
+
 // Tiles of a k x k layer cut along the width too: a map 75 pixels wide fills 75 of a tile's 128 rows in whole rows, and
 // 114 in pieces of 38 x 3. Replaces the tile in t where that saves rounds (or, below one round, tiles); the sums of an
 // output value do not change. 4 x 75 x 75 x 128 -> 256, 3x3: 103 -> 74 us (51 with tiles of 128 columns). cols: tiles
@@ -224,6 +219,47 @@ void cut_tiles(const ConvArgs& a, long cols, TcArgs* t, long* m_tiles) {
             }
         }
     }
+}
+
+// Channels of a tile whose taps lie side by side (kTaps form), 0 = the launch does not take it: 3x3, stride 1, padding 1,
+// where rounds of its tiles - 32 or 64 channels, a chunk and filter row at the measured time, and a longer epilogue - are
+// modelled to take less than whole tiles in their better form. OGLE_TC_TAPS: 0 never, 1 wherever it can run.
+// The sums are others than those of whole tiles, so that the layer's shape alone decides: the whole tiles compared with are
+// those of a launch with an activation and without scratch, whatever this one has.
+int taps_width(const ConvArgs& a, const TcArgs& own, int chunks) {
+    static const int mode = [] { const char* e = getenv("OGLE_TC_TAPS"); return e ? (e[0] == '0' ? 1 : (e[0] == '1' ? 2 : 0)) : 0; }();
+    if (mode == 1 || a.kernel != 3 || a.stride != 1 || a.pad != 1 || a.dil != 1 || a.M > 0x7fffff00L || !encode_im2col_fn()) return 0;
+    if (mode == 0 && (forced_width(a.Kp) || pair_mode_override() == 2)) return 0;        // (those switches come first)
+    double best = 1e30;
+    int width = 0;
+    long rounds = 0;
+    for (int bn = 32; bn <= 64; bn += 32) {
+        const long tiles = (a.M + kTapsPixels - 1) / kTapsPixels * ((a.Kp + bn - 1) / bn);
+        // (a single round is mostly start, fill and drain; stacked siblings are padded to 32 channels each and seldom fill
+        // tiles of 64: in few rounds the model cannot tell which form is the better one)
+        if (mode == 0 && tiles <= (own.split_col ? 4 : 1) * kNumSMs) continue;
+        const double chunk = own.passes == 3 ? (bn == 64 ? 0.57 : 0.45) : (bn == 64 ? 0.33 : 0.28);
+        const double least = own.passes == 3 ? (bn == 64 ? 3.7 : 2.5) : (bn == 64 ? 3.1 : 2.2), tile = chunks / 3 * chunk + 1.0;
+        const double us = (double)((tiles + kNumSMs - 1) / kNumSMs) * (tile > least ? tile : least) + 7.0;
+        if (us < best) { best = us; width = bn; rounds = (tiles + kNumSMs - 1) / kNumSMs; }
+    }
+    if (!width || mode == 2) return width;
+    TcArgs t = own;
+    long m_tiles = whole_row_tiles(a, false, &t);
+    choose_n_tiling_v2(a.Kp, m_tiles, &t);
+    cut_tiles(a, (a.Kp + 127) / 128, &t, &m_tiles);
+    double other = 1e30;
+    for (int bn = 32; bn <= 256 && bn <= (a.Kp + 31) / 32 * 32; bn += 32) {
+        if (t.passes != 3 && bn != t.BN) continue;
+        const double one = whole_tiles_us(t, bn, a.Kp, m_tiles, chunks);
+        const double two = t.passes == 3 && m_tiles >= 2 && bn % 64 == 0 ? pair_tiles_us(t, bn, a.Kp, m_tiles, chunks) : one;
+        other = one < other ? one : other;
+        other = two < other ? two : other;
+    }
+    // (split mode, tensors that come from HBM: whole tiles take 1.08 of the model and 3 us more, 20-170 us measured)
+    if (t.passes == 3) other = 1.08 * other + 3.0;
+    // (in two rounds start and drain are most of the time, and the models further off: 4 x 8 x 64 x 16 -> 577 11.3 us, 11.9)
+    return best < (rounds <= 2 ? 0.88 : 0.97) * other ? width : 0;
 }
 
 // Tile width and number of ranges of a reduction split inside a cluster, for launches whose tiles leave SMs idle. All
@@ -467,30 +503,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
     } else {
         t.flat = 0;
         t.N = a.N; t.Ho = a.Ho; t.Wo = a.Wo;
-        const bool may_split = v2 && a.act == OGLE_ACT_NONE && split_k_enabled() && taps * t.chunks_per_tap >= 16;
-        if (a.Wo >= kTileM) {
-            const int parts = (a.Wo + kTileM - 1) / kTileM;
-            t.tw = (a.Wo + parts - 1) / parts; t.th = 1; t.tn = 1;
-        } else {
-            // full-width tiles of th rows from tn consecutive images (th * tn * Wo <= 128):
-            // take the shape that needs the fewest rounds of one tile per SM; among equals the
-            // tallest, whose filter taps overlap most in L2
-            t.tw = a.Wo;
-            long best = -1;
-            for (int th = 1; th <= a.Ho && th * a.Wo <= kTileM; ++th) {
-                int tn = kTileM / (th * a.Wo);
-                if (tn > a.N) tn = a.N;
-                if ((th - 1) * a.stride + 1 > 256) continue;          // TMA box limit
-                const long tiles = (long)((a.Ho + th - 1) / th) * ((a.N + tn - 1) / tn);
-                // in half-rounds; a reduction split in two (see below) can fill a ragged last round
-                long rounds = 2 * ((tiles + kNumSMs - 1) / kNumSMs);
-                if (may_split && (2 * tiles + kNumSMs - 1) / kNumSMs < rounds) rounds = (2 * tiles + kNumSMs - 1) / kNumSMs;
-                if (best < 0 || rounds <= best) { best = rounds; t.th = th; t.tn = tn; }
-            }
-        }
-        t.tiles_w = (a.Wo + t.tw - 1) / t.tw;
-        t.tiles_h = (a.Ho + t.th - 1) / t.th;
-        m_tiles = (long)t.tiles_w * t.tiles_h * ((a.N + t.tn - 1) / t.tn);
+        m_tiles = whole_row_tiles(a, v2 && a.act == OGLE_ACT_NONE && split_k_enabled() && taps * t.chunks_per_tap >= 16, &t);
     }
     // How many ranges the reduction has is settled at the library's own tile width, whatever width or form the caller
     // asks for: those change how a launch is laid out, not the order in which a value's products are added.
@@ -593,7 +606,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             // where channels lie on M, by the caller's wish or the environment's; and a caller who says 1 or 2 to that, of a
             // layer it fits, gets the same bits for both)
             const bool on_m_form = on_m || (a.on_m && fits_channels_on_m(t, a.Kp, m_tiles));
-            const int beside = t.split_k <= 1 && !on_m_form && tiled ? taps_width(a, own, m_tiles, chunks) : 0;
+            const int beside = t.split_k <= 1 && !on_m_form && tiled ? taps_width(a, own, chunks) : 0;
             if (beside) {
                 m_tiles = tile_taps(a, beside, &t);
                 on_pairs = false;

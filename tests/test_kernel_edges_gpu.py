@@ -474,6 +474,36 @@ def test_taps_side_by_side_two_outputs_and_bounded_waits():
         assert lib.ogle_cuda_device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, math: near the line between whole tiles and taps side by side, where tiles laid out for a split reduction
+    # (no activation), or widths chosen with scratch at hand, would have it fall to either side
+    (1, 34, 34, 192, 512, "MATH_TF32"), (1, 67, 56, 160, 150, "MATH_TF32"), (21, 10, 36, 191, 294, "MATH_TF32"),
+    (4, 77, 11, 176, 316, "MATH_TF32"), (2, 37, 108, 218, 122, "MATH_TF32"), (128, 47, 61, 512, 512, "MATH_TF32X3")])
+def test_taps_by_shape_alone(shape):
+    """Unsplit, a layer's bits depend neither on scratch nor on where the residual operand and the activation are applied."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K, math = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *d: torch.randn(d, generator=g, device="cuda")
+    x, w, b = torch.zeros((N, H, W, ops.up4(C)), device="cuda"), rand(K, C, 3, 3) / (9 * C) ** 0.5, rand(K)
+    x[..., :C] = rand(N, H, W, C)
+    res = rand(N, H, W, ops.up4(K))
+    res[..., K:] = 0.0
+    lent = torch.empty(48 << 18, device="cuda")
+    p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    p.split = 1
+    packed = ops.conv2d_prepack(p, w)
+    plain = ops.conv2d(p, x, packed, b, workspace=None)
+    form = ops.last_contraction().form
+    assert torch.equal(ops.conv2d(p, x, packed, b, workspace=lent), plain)
+    p.act = ops.ACT_RELU
+    for scratch in (None, lent):
+        assert torch.equal(ops.conv2d(p, x, packed, b, workspace=scratch), plain.clamp(min=0))
+    assert torch.equal(ops.conv2d_residual(p, x, packed, b, res), (plain + res).clamp(min=0))
+    assert (ops.last_contraction().form == 6) == (form == 6)
+
+
 ON_M_CODE = """
 import torch
 from ogle_b200 import _lib, ops
