@@ -197,7 +197,7 @@ struct DetectArgs {
     KeySpace ks;
     float nms_thr;
     int classes_per_pass;   // mode 1: foreground classes whose scores fit in shared memory at once
-    int ahead;              // mode 1: a block has the image this many further on fetched while it selects (0 = none)
+    int ahead;              // mode 1, kAhead: a block has the image this many further on fetched while it selects (0 = none)
     int parts;              // mode 1: blocks per image, each taking a contiguous range of the foreground classes
     const OgleImageDesc* frames;   // mode 0: per-image frame sizes, or null
     const float4* anchors;         // not null: `boxes` holds deltas, decoded against these as they are written
@@ -239,7 +239,10 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long bytes) {
 
 // Mode 1: per class. Dynamic shared memory: float scores[classes_per_pass][Ap], histograms of as many classes
 // (kHistWords words each), one list of survivors per warp (kListMax 16-bit indices).
-__global__ void __launch_bounds__(640)
+// kAhead: what the SM reads next is on its way into L2 while a block selects, at 71 registers a thread (a block an SM is all
+// it is compiled for); else 48, for launches whose shared memory and threads let more blocks onto an SM than that (below).
+template <bool kAhead>
+__global__ void __launch_bounds__(640, kAhead ? 1 : 0)
 ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ boxes,
                   float* __restrict__ out_score, int* __restrict__ out_anchor, int* __restrict__ out_class,
                   float4* __restrict__ out_box, int* __restrict__ out_count, const DetectArgs a) {
@@ -254,7 +257,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
     unsigned* hists = reinterpret_cast<unsigned*>(scores + (size_t)a.classes_per_pass * a.Ap);
     unsigned short* list = reinterpret_cast<unsigned short*>(hists + (size_t)a.classes_per_pass * kHistWords) + warp * kListMax;
     const int rows = (a.C - 1) * a.top_k;
-    if (a.ahead > 0) prefetch_l2(bx, (long)a.A * sizeof(float4));
+    if (kAhead && a.ahead > 0) prefetch_l2(bx, (long)a.A * sizeof(float4));
     const int per_part = (a.C - 1 + a.parts - 1) / a.parts;
     const int c_lo = 1 + part * per_part, c_hi = min(a.C, c_lo + per_part);     // this block's classes
     for (int c0 = c_lo; c0 < c_hi; c0 += a.classes_per_pass) {
@@ -295,7 +298,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
             }
         }
         __syncthreads();
-        if (a.ahead > 0 && c0 == c_lo && n + a.ahead < a.N)
+        if (kAhead && a.ahead > 0 && c0 == c_lo && n + a.ahead < a.N)
             prefetch_l2(lg + (long)a.ahead * a.A * a.logit_stride, ((long)(a.A - 1) * a.logit_stride + a.C) * sizeof(float));
         for (int j = warp; j < nc; j += nwarps) {
             const int cls = c0 + j;
@@ -517,24 +520,47 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         size_t cpp = (budget - warp_bytes) / per_class;
         if (cpp > (size_t)classes) cpp = classes;
         a.classes_per_pass = (int)cpp;
-        a.ahead = p->N > kNumSMs ? kNumSMs : 0;
         smem = cpp * per_class + warp_bytes;
     } else {
         threads = 512;
         smem = (size_t)a.Ap * 8 + kHistWords * 4 + kMaxTopK * 6 * sizeof(int) + kListMax * sizeof(unsigned short);
         if (smem > kSmemRule) return OGLE_ERR_UNSUPPORTED;
     }
-    static thread_local int attr_set_for_device = -1;
+    static thread_local int attr_set_for_device = -1, regs[2];
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_set_for_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(ssd_detect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+        cudaFuncAttributes fa;
+        cudaError_t e = cudaFuncSetAttribute(ssd_detect_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_detect_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(ssd_detect_rule_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemRule);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, ssd_detect_kernel<false>);
+        if (e == cudaSuccess) { regs[0] = fa.numRegs; e = cudaFuncGetAttributes(&fa, ssd_detect_kernel<true>); }
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
+        regs[1] = fa.numRegs;
         attr_set_for_device = dev;
     }
-    launch_overlapped(p->mode == 1 ? ssd_detect_kernel : ssd_detect_rule_kernel, dim3(p->N * a.parts), dim3(threads), smem,
+    bool wide = false;
+    if (p->mode == 1) {
+        // The kernel with more registers where that leaves as many blocks on an SM (of its shared memory, threads, and
+        // registers by warps and quarters of the SM), or all there are: 1024 images, 1917 anchors, 21 classes 171.4 -> 162.6 us,
+        // 12 classes 121.0 -> 109.2, 4000 anchors, 9 classes 229.5 -> 210.3. Where it does not, it loses what the blocks
+        // gave (77 registers in every launch: 300 anchors, 21 classes 50.3 -> 70.9, 1917 anchors, 9 classes 92.8 -> 103.7).
+        const int waiting = (p->N * a.parts + kNumSMs - 1) / kNumSMs;
+        int blocks = (int)(228 * 1024 / (smem + 1024));
+        if (blocks > 2048 / threads) blocks = 2048 / threads;
+        if (blocks > waiting) blocks = waiting;
+        int fit[2];
+        for (int i = 0; i < 2; ++i) {
+            const int warps = 4 * (16384 / ((regs[i] + 7) / 8 * 8 * 32)) / (threads / 32);
+            fit[i] = blocks < warps ? blocks : warps;
+        }
+        wide = fit[1] >= fit[0];
+        a.ahead = p->N > kNumSMs ? kNumSMs * fit[1] / a.parts : 0;
+    }
+    const auto kernel = p->mode != 1 ? ssd_detect_rule_kernel : (wide ? ssd_detect_kernel<true> : ssd_detect_kernel<false>);
+    launch_overlapped(kernel, dim3(p->N * a.parts), dim3(threads), smem,
                       (cudaStream_t)stream, logits, reinterpret_cast<const float4*>(boxes), out_score, out_anchor, out_class,
                       reinterpret_cast<float4*>(out_box), out_count, a);
     return finish_launch();
