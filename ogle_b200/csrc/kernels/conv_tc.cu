@@ -348,14 +348,18 @@ bool conv_tc_supported(const ConvArgs& a, int variant) {
 // (the RGB stem), whole reduction (9 x C <= 27 values) in one chunk.
 // Tile of the gather form: tw x th output pixels of one image, tw * th = 128; the shape that
 // wastes the fewest rows among those whose input window (halo included) is at most 1024
-// pixels = 16 KB of shared memory per stage and at most 128 pixels wide (a limit of its map).
-static bool gather_tile(const ConvArgs& a, int* tw_out, int* th_out) {
-    long best = -1;
+// pixels = 16 KB of shared memory per stage. Windows of up to 128 pixels a row have their map of row-long extents, which
+// is the faster copy; wider ones, up to 256 (a TMA box limit), are taken where they waste a good deal less, on maps one to
+// five rows high mostly: one pass, 512 images of 1 x 1024 5x5 64 us, 111 in the best narrow tile, 5 x 128 44 and 48;
+// at 7 % fewer rows (13 x 128) 97 and 99, split mode 95 and 91. Split-mode tiles of 256 channels leave no room for two
+// stages with wider windows. wide = 0: narrow ones only.
+static bool gather_tile(const ConvArgs& a, bool wide, int* tw_out, int* th_out) {
+    double best = -1;
     for (int tw = 128; tw >= 16; tw >>= 1) {
         const int th = kTileM / tw;
         const int iw = (tw - 1) * a.stride + a.kernel, ih = (th - 1) * a.stride + a.kernel;
-        if (iw > 128 || iw * ih > 1024) continue;
-        const long covered = (long)((a.Wo + tw - 1) / tw) * tw * ((a.Ho + th - 1) / th) * th;
+        if (iw > (wide ? 256 : 128) || iw * ih > 1024) continue;
+        const double covered = (double)((a.Wo + tw - 1) / tw) * tw * ((a.Ho + th - 1) / th) * th * (iw > 128 ? 1.08 : 1.0);
         if (best < 0 || covered < best) { best = covered; *tw_out = tw; *th_out = th; }
     }
     return best >= 0;
@@ -370,7 +374,7 @@ bool conv_tc_gather_supported(const ConvArgs& a, int variant) {
     int tw, th;
     return variant == CONV_GENERAL && filter_compact(a.C / a.group, a.kernel, a.group) && a.dil == 1 &&
            filter_compact_cols(a.C, a.kernel) <= kMaxGatherK &&
-           (a.stride == 1 || a.stride == 2) && a.Cp == 4 && a.Cs == 4 && a.Wo >= 16 && a.K <= 256 && gather_tile(a, &tw, &th) &&
+           (a.stride == 1 || a.stride == 2) && a.Cp == 4 && a.Cs == 4 && a.Wo >= 16 && a.K <= 256 && gather_tile(a, false, &tw, &th) &&
            encode_fn() != nullptr;
 }
 
@@ -482,7 +486,7 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.gather = 1; t.g_C = a.C; t.g_k = a.kernel;
         t.kernel = 1;                                            // the reduction is a run of gathered chunks
         t.Cp32 = filter_compact_cols(a.C, a.kernel); t.chunks_per_tap = t.Cp32 / kChunk;
-        if (!gather_tile(a, &t.tw, &t.th)) return OGLE_ERR_UNSUPPORTED;
+        if (!gather_tile(a, t.passes == 1 || a.Kp <= 224, &t.tw, &t.th)) return OGLE_ERR_UNSUPPORTED;
         t.tn = 1;
         t.tiles_w = (a.Wo + t.tw - 1) / t.tw;
         t.tiles_h = (a.Ho + t.th - 1) / t.th;
@@ -490,8 +494,16 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.g_iw = (t.tw - 1) * a.stride + a.kernel;
         t.g_ih = (t.th - 1) * a.stride + a.kernel;
         t.g_bytes = (t.g_iw * t.g_ih * 16 + 1023) / 1024 * 1024;
-        if (!plan_only && !make_map_pixels(&mA, x, a.W, a.H, a.N, t.g_iw, t.g_ih)) return OGLE_ERR_CUDA;
         const cuuint32_t es[4] = {1, 1, 1, 1};
+        if (t.g_iw > 128) {
+            t.g_pixels = 1;
+            const cuuint64_t dims[4] = {4, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
+            const cuuint64_t str[3] = {16, (cuuint64_t)a.W * 16, (cuuint64_t)a.W * 16 * a.H};
+            const cuuint32_t box[4] = {4, (cuuint32_t)t.g_iw, (cuuint32_t)t.g_ih, 1};
+            if (!plan_only && !make_map_sw(CU_TENSOR_MAP_SWIZZLE_NONE, &mA, x, 4, dims, str, box, es)) return OGLE_ERR_CUDA;
+        } else if (!plan_only && !make_map_pixels(&mA, x, a.W, a.H, a.N, t.g_iw, t.g_ih)) {
+            return OGLE_ERR_CUDA;
+        }
         const cuuint64_t yd[4] = {(cuuint64_t)kp_a, (cuuint64_t)a.Wo, (cuuint64_t)a.Ho, (cuuint64_t)a.N};
         const cuuint64_t ys[3] = {(cuuint64_t)ks_a * 4, (cuuint64_t)ks_a * 4 * a.Wo, (cuuint64_t)ks_a * 4 * a.Wo * a.Ho};
         const cuuint32_t yb[4] = {kChunk, (cuuint32_t)t.tw, (cuuint32_t)t.th, 1};

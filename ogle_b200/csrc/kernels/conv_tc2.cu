@@ -377,6 +377,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     ay = a.flat ? 0 : tc_.h0 * a.stride - a.pad;
                     an = tc_.n0;
                 }
+                // gather form: the tile's input window
+                auto load_window = [&](uint32_t to, uint64_t* bar) {
+                    if (a.g_pixels) tma_load_4d(to, &tmA, bar, 0, ax, ay, an);
+                    else tma_load_4d(to, &tmA, bar, 2 * ax, ay, an, 0);
+                };
                 // position of the first chunk: filter row, filter column, channel offset
                 int ky = 0, kx = 0, c0 = 0;
                 if (kSplit && wi.c_begin != 0) {      // only the later ranges of a split reduction pay the divisions
@@ -392,13 +397,13 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         // (the ring is at most a stage longer than a tile's reduction: the window before the last has been read)
                         if (it == 0) {
                             mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
-                            tma_load_4d(base + kept_filters + (uint32_t)(window * a.g_bytes), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
+                            load_window(base + kept_filters + (uint32_t)(window * a.g_bytes), &bar_full[s]);
                         } else {
                             mbar_arrive(&bar_full[s]);
                         }
                     } else if (a.gather) {
                         mbar_expect_tx(&bar_full[s], (uint32_t)(a.g_iw * a.g_ih * 16));
-                        tma_load_4d(sWin(s), &tmA, &bar_full[s], 2 * ax, ay, an, 0);
+                        load_window(sWin(s), &bar_full[s]);
                     } else {
                         mbar_expect_tx(&bar_full[s], tx);
                         if constexpr (kBeside) tma_load_im2col(sA(s), &tmA, &bar_full[s], c0, ax, ay, an, 0, ky);

@@ -632,6 +632,50 @@ def test_residual_operand_by_the_copy_engine(shape, math):
 
 
 @pytest.mark.parametrize("shape", [
+    # N, H, W, K, kernel, stride: maps of few rows, whose windows are up to 134 pixels wide (of as many rows as fit), and the
+    # widths, strides and channel counts at which they are not
+    (3, 1, 300, 64, 5, 1), (2, 1, 128, 40, 7, 1), (2, 3, 257, 130, 5, 1), (9, 5, 128, 64, 5, 1), (2, 2, 200, 64, 5, 2), (3, 1, 1000, 224, 5, 1),
+    (3, 1, 300, 250, 5, 1), (2, 1, 127, 256, 5, 1), (2, 4, 16, 64, 7, 1)])
+@pytest.mark.parametrize("channels", [3, 2])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_stems_of_flat_maps(shape, channels, math):
+    import torch
+    from ogle_b200 import ops
+    N, H, W, K, k, s = shape
+    g = torch.Generator(device="cuda").manual_seed(W + K)
+    x = torch.zeros((N, H, W, 4), device="cuda")
+    x[..., :channels] = torch.randn((N, H, W, channels), generator=g, device="cuda")
+    w, b = torch.randn((K, channels, k, k), generator=g, device="cuda") / (3 * k * k) ** 0.5, torch.randn(K, generator=g, device="cuda")
+    p = ops.conv_params(N, H, W, channels, K, k, s, k // 2, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    packed = ops.conv2d_prepack(p, w)
+    want = torch.nn.functional.conv2d(x[..., :channels].permute(0, 3, 1, 2).double(), w.double(), b.double(), s, k // 2).permute(0, 2, 3, 1)
+    # 147 products and sums of fp32 grade, or of operands with ten mantissa bits
+    bound = (3e-6 if math == "MATH_TF32X3" else 1e-3) * float(want.norm())
+    got = ops.conv2d(p, x, packed, b, workspace=None)
+    assert float((got[..., :K].double() - want).norm()) <= bound
+    res = torch.randn(got.shape, generator=g, device="cuda")
+    p.split = 1
+    got = ops.conv2d_residual(p, x, packed, b, res)
+    assert float((got[..., :K].double() - want - res[..., :K].double()).norm()) <= bound
+
+
+def test_flat_maps_fill_their_tiles():
+    """A map one row high takes about what a square one of as many pixels does: 1.05 of it with tiles of a row, 1.9 in tiles
+    of two."""
+    import torch
+    from ogle_b200 import ops
+
+    def took(N, H, W):
+        g = torch.Generator(device="cuda").manual_seed(W)
+        p = ops.conv_params(N, H, W, 3, 64, 5, 1, 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_TF32)
+        packed = ops.conv2d_prepack(p, torch.randn((64, 3, 5, 5), generator=g, device="cuda") / 8.0)
+        x, b = torch.randn((N, H, W, 4), generator=g, device="cuda"), torch.randn(64, generator=g, device="cuda")
+        return _median_us(lambda: ops.conv2d(p, x, packed, b, workspace=None))
+
+    assert took(512, 1, 1024) <= 1.4 * took(32, 128, 128)
+
+
+@pytest.mark.parametrize("shape", [
     # N, H, W, K, kernel, stride: one tile, several a block, tiles that hang over every edge; filters that fit beside the windows and not
     (1, 32, 32, 16, 7, 2), (9, 113, 75, 64, 7, 2), (40, 70, 70, 40, 5, 1), (3, 130, 130, 128, 7, 1), (5, 64, 64, 200, 5, 2), (30, 64, 64, 8, 3, 2)])
 def test_kept_filters_and_windows_of_rgb_stems(shape):
