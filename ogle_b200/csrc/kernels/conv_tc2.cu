@@ -37,7 +37,7 @@
 // once, the output tile written once; filters come from L2.
 // All mbarrier waits are bounded and abort the block cleanly: the role records a code in
 // the status word and raises the block's abort flag, the other roles leave at their next
-// wait, the MMA issuer waits for the multiplies it has issued, the teardown waits for the
+// wait, the teardown waits for the multiplies and the
 // operand copies still in flight, and only then is tensor memory freed and the block retired.
 // The number of polls of the role waits can be shortened at run time (ogle_cuda_set_wait_limit,
 // for tests of this path); the waits of the abort path itself always use the full bound.
@@ -516,12 +516,6 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (++s == a.stages) { s = 0; ph ^= 1u; }
                 }
                 if (ok) umma_commit(&bar_acc_full[as]);
-            }
-            if (!ok) {
-                // abort: the multiplies already issued still read shared memory and write tensor
-                // memory; the block may free neither before they are done
-                umma_commit(&bar_drain);
-                mbar_wait(&bar_drain, 0u);
             }
         }
     } else if (warp >= 10) {
@@ -1017,11 +1011,17 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncthreads();
     if (s_abort) {
         // Some role gave up. Every role has left its loop (a role that was not waiting finished
-        // what it had issued), but operand copies may still be in flight towards this block's
-        // shared memory, and the block must not retire before they have landed. A ring stage's
+        // what it had issued), but multiplies and operand copies may still be in flight - also where the
+        // issuer itself came to its end and only an epilogue gave up -, and tensor memory may not be freed
+        // nor the block retire before they are done. The thread that issued the multiplies (the one that is
+        // elected each time) waits for them. A ring stage's
         // barrier completes when BOTH producers have announced their copy and the bytes are in;
         // the producers may have stopped up to a ring apart, so first supply the announcement
         // the other one never made, then wait (full bound) for the last ring of stages.
+        if (warp == 1 && elect_one()) {
+            umma_commit(&bar_drain);
+            mbar_wait(&bar_drain, 0u);
+        }
         if (threadIdx.x == 0) {
             const int na = s_issued[0], nb = s_issued[1];
             const int lo = na < nb ? na : nb, hi = na < nb ? nb : na;

@@ -324,10 +324,6 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
                 if (ok) umma2_commit_both(&bar_acc_full[as]);
             }
-            if (!ok) {
-                umma2_commit_local(&bar_drain);
-                mbar_wait(&bar_drain, 0u);
-            }
         }
     } else if (warp == 1) {
         // ------------------------------------------------- relay (the other block): tell the leader
@@ -524,11 +520,16 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
 
     // ------------------------------------------------------------------ teardown
-    // Every role of both blocks has left its loop; the multiplies have finished (their results
-    // were read, or the leader drained them). After the cluster barrier neither block touches
-    // the other's shared memory again.
+    // Every role of this block has left its loop. Where one gave up, the thread that issued the pair's multiplies waits
+    // for them. (A flag that the other block raises only now makes no difference: the epilogues of this one have then seen
+    // the last accumulator come.) After the cluster barrier neither block touches the other's shared memory again.
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (leader && warp == 1 && __any_sync(0xffffffffu, *abort_flag) && elect_one()) {
+        umma2_commit_local(&bar_drain);
+        mbar_wait(&bar_drain, 0u);
+    }
+    __syncwarp();
     cluster_sync_all();
     if (s_abort) {
         if (threadIdx.x == 0) {

@@ -275,10 +275,6 @@ conv_tc2_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 }
                 if (ok) umma_commit(&bar_acc_full[as]);
             }
-            if (!ok) {
-                umma_commit(&bar_drain);
-                mbar_wait(&bar_drain, 0u);
-            }
         }
     } else if (warp >= 10) {
         // --------------------------------------------------- operand split (fp32-grade mode): 256 rows per chunk
@@ -456,6 +452,10 @@ conv_tc2_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (s_abort) {
+        if (threadIdx.x == 32) {                     // the issuer's thread
+            umma_commit(&bar_drain);
+            mbar_wait(&bar_drain, 0u);
+        }
         if (threadIdx.x == 0) {
             const int na = s_issued[0], nb = s_issued[1];
             const int lo = na < nb ? na : nb, hi = na < nb ? nb : na;

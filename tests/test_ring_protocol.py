@@ -55,3 +55,51 @@ def test_no_split_group_is_passed_by_the_ring(stages):
 
 def test_the_model_sees_a_group_that_nobody_waits_for():
     assert _overtaken(3, 10, False)
+
+
+TENSOR_CORE_KERNELS = ["conv_tc2.cu", "conv_tc2_pair.cu", "conv_tc2_t.cu"]
+
+
+def _teardown_drains(name):
+    """Whether the block as a whole waits for the multiplies in flight when a role has given up, not the issuer alone."""
+    text = open(os.path.join(KERNELS, name)).read()
+    end = text[text.index("-- teardown"):]
+    return re.search(r"commit\w*\(&bar_drain\);\s+mbar_wait\(&bar_drain", end[:end.index("tcgen05.dealloc")]) is not None
+
+
+def _freed_in_flight(chunks, teardown_drains):
+    """Whether tensor memory can be freed with multiplies in flight. The issuer issues them all and leaves, or gives up at
+    some point and waits for its own; an epilogue waits for the last of them, or gives up; the block frees when both left."""
+    start = (0, 0, "runs", "waits")                       # issued, finished, issuer, epilogue
+    seen, todo = {start}, [start]
+    while todo:
+        issued, done, issuer, epilogue = todo.pop()
+        gave_up = "gave up" in (issuer, epilogue)
+        left = issuer in ("left", "gave up") and epilogue in ("left", "gave up")
+        drained = done == issued
+        if left and not drained and not (gave_up and teardown_drains) and not issuer == "gave up":
+            return True
+        nxt = []
+        if done < issued:
+            nxt.append((issued, done + 1, issuer, epilogue))
+        if issuer == "runs":
+            nxt.append((issued + 1, done, issuer, epilogue) if issued < chunks else (issued, done, "left", epilogue))
+            nxt.append((issued, done, "gave up", epilogue))
+        if epilogue == "waits":
+            if done == chunks:
+                nxt.append((issued, done, issuer, "left"))
+            nxt.append((issued, done, issuer, "gave up"))
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("name", TENSOR_CORE_KERNELS)
+def test_tensor_memory_is_freed_after_the_last_multiply(name):
+    assert not _freed_in_flight(4, _teardown_drains(name))
+
+
+def test_the_model_sees_an_epilogue_that_gives_up_alone():
+    assert _freed_in_flight(4, False)
