@@ -130,9 +130,6 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
-__device__ __forceinline__ void umma2_commit_local(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 struct PairCoord { int n_tile, m_tile, n0, h0, w0; };
 
@@ -520,18 +517,16 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
 
     // ------------------------------------------------------------------ teardown
-    // Every role of this block has left its loop. Where one gave up, the thread that issued the pair's multiplies waits
-    // for them. (A flag that the other block raises only now makes no difference: the epilogues of this one have then seen
-    // the last accumulator come.) After the cluster barrier neither block touches the other's shared memory again.
+    // Every role of both blocks has left its loop once both are through the cluster barrier, and both know whether one of
+    // them gave up. Multiplies may then still be in flight, and completions of theirs on their way to the other block's
+    // barriers: the thread that issued them has both blocks told of the last, and neither goes on before that, nor before
+    // the copies of both have landed.
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (leader && warp == 1 && __any_sync(0xffffffffu, *abort_flag) && elect_one()) {
-        umma2_commit_local(&bar_drain);
-        mbar_wait(&bar_drain, 0u);
-    }
-    __syncwarp();
     cluster_sync_all();
     if (s_abort) {
+        if (leader && warp == 1 && elect_one()) umma2_commit_both(&bar_drain);
+        mbar_wait(&bar_drain, 0u);
         if (threadIdx.x == 0) {
             const int na = s_issued[0], nb = s_issued[1];
             const int lo = na < nb ? na : nb, hi = na < nb ? nb : na;
@@ -540,6 +535,7 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 mbar_wait(&bar_full[i % a.stages], (uint32_t)((i / a.stages) & 1));
         }
         __syncthreads();
+        cluster_sync_all();
     }
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)a.tmem_cols));
