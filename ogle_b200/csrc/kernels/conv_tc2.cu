@@ -39,6 +39,11 @@
 // the status word and raises the block's abort flag, the other roles leave at their next
 // wait, the teardown waits for the multiplies and the
 // operand copies still in flight, and only then is tensor memory freed and the block retired.
+// The threads of an epilogue group may disagree about whether an accumulator came in time, and one that left by itself would
+// be missed at the group's barriers: it goes on to the end of the block's tiles with them - with the block's abort flag up no
+// wait lasts -, and what the group stores is then no valid output. With a residual operand, whose copies it would have to
+// wait for, the group votes and leaves as one. (That vote in every form: 256 x 150 x 150 x 32 -> 64 pointwise 389 -> 440 us;
+// a flag in shared memory that all look at, 427; this way 399.)
 // The number of polls of the role waits can be shortened at run time (ogle_cuda_set_wait_limit,
 // for tests of this path); the waits of the abort path itself always use the full bound.
 #include <cuda_bf16.h>
@@ -76,9 +81,10 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
-// The same, and whether all 128 threads say so.
+// The same, and whether all 128 threads say so. (The lanes leave a polling loop one by one; bar.red wants the whole warp.)
 __device__ __forceinline__ bool group_and(int id, bool mine) {
     uint32_t all;
+    mine = __all_sync(0xffffffffu, mine);
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbar.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
                  : "=r"(all) : "r"(id), "r"((uint32_t)mine) : "memory");
     return all != 0;
@@ -673,7 +679,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const bool at_end = (lane == 0 && q > 0) || (lane == 31 && q < 3);
             const float* my_edge = lane == 0 ? edge + (q - 1) * 64 : edge + (q + 1) * 64 + 32;
             float* my_bias = s_bias[eg];
-            bool ok = true;
+            bool ok = true, came = true;        // (came: looked at with a residual operand only)
             int ti = 0, staged_nbase = -1, round_no = 0;
             int res_copies = 0;        // of the residual operand, asked for by this thread
             for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
@@ -705,9 +711,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 };
                 if (t == 0 && first < groups) free_slab(round_no % a.epi_slabs, nbase + first * 32);
-                ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
+                if (!__all_sync(0xffffffffu, wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit))) {
+                    record_error(err_flag, 4);
+                    s_abort = 1;
+                    came = false;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (first >= groups) {                  // none of them this time
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -731,7 +739,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         }
                     }
                     if constexpr (kForm == kTapsRes) {
-                        ok = group_and(bar_id, wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
+                        ok = group_and(bar_id, came && wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
                         if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
                     } else {
                         group_sync(bar_id);
@@ -833,7 +841,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // each group owns one or two staging slabs and fills them in rounds
             const uint32_t my_staging = staging_off + (uint32_t)(eg * a.epi_slabs) * (uint32_t)kStagingBytes;
             unsigned char* staging = base_ptr + my_staging;
-            bool ok = true;
+            bool ok = true, came = true;
             int ti = 0;
             int staged_nbase = -1;
             int round_no = 0;          // rounds of this group so far (selects the staging slab)
@@ -876,8 +884,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 };
                 if (kForm == kWholeRes && t == 0 && first < groups) free_slab(round_no % a.epi_slabs, nbase + first * 32);
-                ok = wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
-                if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
+                if (!wait_or_abort(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit)) {
+                    record_error(err_flag, 4);
+                    s_abort = 1;
+                    came = false;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (first >= groups) {                  // none of them this time
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -891,7 +902,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     ++round_no;
                     if (t == 0 && (kForm != kWholeRes || g0 != first)) free_slab(sb, nbase + g0 * 32);
                     if constexpr (kForm == kWholeRes) {
-                        ok = group_and(bar_id, wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
+                        ok = group_and(bar_id, came && wait_or_abort(&bar_res[eg], (uint32_t)((round_no - 1) & 1), abort_flag, a.spin_limit));
                         if (!ok) { record_error(err_flag, 4); s_abort = 1; break; }
                     } else {
                         group_sync(bar_id);

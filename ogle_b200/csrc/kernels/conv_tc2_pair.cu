@@ -405,11 +405,10 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             unsigned char* staging = base_ptr + my_staging;
             // the leader's barrier counts the arrivals of both blocks' groups
             const uint32_t l_acc_empty = peer_addr(smem_u32(&bar_acc_empty[0]), 0u);
-            bool ok = true;
             int ti = 0;
             int staged_nbase = -1;
             int round_no = 0;
-            for (int w = my_pair; w < a.total_work && ok; w += n_pairs, ++ti) {
+            for (int w = my_pair; w < a.total_work; w += n_pairs, ++ti) {
                 const PairCoord pc = pair_coord(a, w, rank);
                 const bool live = pc.m_tile < m_tiles;
                 const int as = ti & 1, use = ti >> 1;
@@ -427,8 +426,11 @@ conv_tc2_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                         my_bias[i] = (a.bias_mode == 2 && nbase + i < a.K) ? a.beta * bias[nbase + i] : 0.f;
                     staged_nbase = nbase;
                 }
-                ok = wait_pair(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
-                if (!ok) { record_error(err_flag, 18); raise_abort(); break; }
+                // (a thread that gives up stays with its group: see conv_tc2.cu)
+                if (!wait_pair(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit)) {
+                    record_error(err_flag, 18);
+                    raise_abort();
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (first >= groups) {
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -344,13 +344,15 @@ conv_tc2_t_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const float my_b = (!raw && a.bias_mode == 2 && real && ch < a.K) ? a.beta * bias[ch] : 0.f;
         const int act = raw ? OGLE_ACT_NONE : a.act;
         const CUtensorMap* my_map = second ? &tmY2 : &tmY;
-        bool ok = true;
         int ti = 0;
-        for (int w = blockIdx.x; w < a.total_work && ok; w += gridDim.x, ++ti) {
+        for (int w = blockIdx.x; w < a.total_work; w += gridDim.x, ++ti) {
             const int as = ti & 1, use = ti >> 1;
             const TItem wi = t_item(a, w, chunks);
-            ok = wait_t(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit);
-            if (!ok) { record_error(err_flag, 24); s_abort = 1; break; }
+            // (a warp that gives up stays with the others, who may take turns with it: see conv_tc2.cu)
+            if (!__all_sync(0xffffffffu, wait_t(&bar_acc_full[as], (uint32_t)(use & 1), abort_flag, a.spin_limit))) {
+                record_error(err_flag, 24);
+                s_abort = 1;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // the warps take the staging slabs in rounds of epi_slabs warps
             const bool turns = a.epi_slabs < active_warps;

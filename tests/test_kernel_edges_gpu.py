@@ -708,6 +708,49 @@ def test_kept_filters_and_windows_of_rgb_stems(shape):
     assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), got)
 
 
+@pytest.mark.parametrize("form", ["whole", "whole, alternate tiles", "whole, residual", "taps", "taps, residual", "kept", "scratch", "cluster", "pairs",
+                                  "channels on M", "channels on M, turns"])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_waits_that_run_out_for_some(form, math):
+    """Limits at which some roles, warps or blocks give up and others do not: the launch returns, with the status set or with
+    the result, and the next one is right again."""
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    # N, H, C, K, kernel, stride
+    N, H, C, K, k, s = {"whole": (16, 40, 96, 160, 1, 1), "whole, alternate tiles": (64, 40, 32, 64, 1, 1), "whole, residual": (16, 40, 96, 160, 3, 2),
+                        "taps": (64, 28, 64, 64, 3, 1), "taps, residual": (64, 28, 64, 32, 3, 1), "kept": (20, 112, 3, 64, 7, 2),
+                        "scratch": (8, 10, 512, 100, 3, 1), "cluster": (1, 19, 256, 256, 1, 1), "pairs": (16, 40, 96, 256, 1, 1),
+                        "channels on M": (32, 28, 64, 64, 3, 1), "channels on M, turns": (32, 28, 64, 128, 3, 1)}[form]
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *d: torch.randn(d, generator=g, device="cuda")
+    x, w, b = torch.zeros((N, H, H, ops.up4(C)), device="cuda"), rand(K, C, k, k) / (C * k * k) ** 0.5, rand(K)
+    x[..., :C] = rand(N, H, H, C)
+    p = ops.conv_params(N, H, H, C, K, k, s, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, getattr(ops, math))
+    p.split = {"scratch": 12, "cluster": 4}.get(form, 1)
+    p.sm_pair, p.channels_on_m = 2 if form == "pairs" else 0, 2 if "M" in form else 0
+    p.n_tile = 128 if form == "pairs" else 0
+    packed = ops.conv2d_prepack(p, w)
+    res = rand(N, p.out_hwc[0], p.out_hwc[1], ops.up4(K))
+    run = (lambda: ops.conv2d_residual(p, x, packed, b, res)) if "residual" in form else (lambda: ops.conv2d(p, x, packed, b))
+    want = run()
+    assert lib.ogle_cuda_device_status() == 0
+    seen = set()
+    try:
+        for limit in [0, 1, 2, 3, 4, 6, 8, 11, 16, 23, 32, 45, 64, 90, 128, 181, 256, 362, 512, 1024, 2048, 4096] * 2:
+            lib.ogle_cuda_set_wait_limit(limit)
+            got = run()
+            status = lib.ogle_cuda_device_status()
+            assert status == -6 or (status == 0 and torch.equal(got, want)), (limit, status)
+            seen.add(status)
+            lib.ogle_cuda_clear_device_status()
+    finally:
+        lib.ogle_cuda_set_wait_limit(-1)
+        lib.ogle_cuda_clear_device_status()
+    assert -6 in seen
+    assert torch.equal(run(), want) and lib.ogle_cuda_device_status() == 0
+
+
 def test_bounded_waits_of_the_cluster_form(oracle_port):
     """Zero polls allowed: every block of a cluster gives up, all meet at the cluster's barriers, the launch returns with
     the status word set, and with the limit restored the same call gives what it gave before."""

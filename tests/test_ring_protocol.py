@@ -103,3 +103,49 @@ def test_tensor_memory_is_freed_after_the_last_multiply(name):
 
 def test_the_model_sees_an_epilogue_that_gives_up_alone():
     assert _freed_in_flight(4, False)
+
+
+def _groups_stay_together(name):
+    """Whether a thread of an epilogue group that gives up on an accumulator goes on to the group's next barrier instead of
+    leaving (waits of the cluster form, whose warps meet at the block's barrier only, are no group's)."""
+    text = open(os.path.join(KERNELS, name)).read()
+    waits = [m.start() for m in re.finditer(r"wait_\w+\(&bar_acc_full\[as\]", text)]
+    assert waits
+    return not any("break;" in text[at:at + re.search(r"group_sync\w*\(|group_and\(|bar\.sync", text[at:]).start()] for at in waits)
+
+
+def _stuck(tiles, stay):
+    """Whether some warps of a group can wait at a barrier that others never come to. Each warp sees a tile's accumulator come
+    or gives up on it by itself, and then comes to the barrier all the same or leaves."""
+    start = ((0, "waits"),) * 4                           # (tile, waits | at the barrier | left) of each warp
+    seen, todo = {start}, [start]
+    while todo:
+        warps = todo.pop()
+        nxt = []
+        for i, (tile, at) in enumerate(warps):
+            put = lambda s: warps[:i] + (s,) + warps[i + 1:]
+            if at == "waits" and tile < tiles:
+                nxt.append(put((tile, "at the barrier")))
+                if not stay:
+                    nxt.append(put((tile, "left")))
+            elif at == "waits":
+                nxt.append(put((tile, "left")))
+        at_barrier = [w for w in warps if w[1] == "at the barrier"]
+        if len(at_barrier) == 4:
+            nxt.append(tuple((tile + 1, "waits") for tile, _ in warps))
+        elif at_barrier and not any(w[1] == "waits" for w in warps):
+            return True
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("name", TENSOR_CORE_KERNELS)
+def test_no_epilogue_group_waits_for_warps_that_gave_up(name):
+    assert not _stuck(2, _groups_stay_together(name))
+
+
+def test_the_model_sees_warps_that_leave_by_themselves():
+    assert _stuck(2, False)
