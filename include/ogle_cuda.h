@@ -135,7 +135,8 @@ typedef struct {
                                 same bits: where it could run, neither lets the taps of a 3x3 layer lie side by side. */
     int sm_pair;             /* tensor-core path: 2 = compute tiles of 256 pixels on pairs of SMs (each SM of a
                                 pair loads half of the filter tile; needs n_tile a multiple of 64 and an unsplit
-                                reduction - chosen or asked for by split = 1 - else ignored), 1 = one SM per tile, 0 = chosen by the library.
+                                reduction - chosen or asked for by split = 1 - else ignored, as it is by layers whose taps
+                                lie side by side: see n_tile), 1 = one SM per tile, 0 = chosen by the library.
                                 Results do not depend on it bit for bit. */
 } OgleConvParams;
 

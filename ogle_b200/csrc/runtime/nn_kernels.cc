@@ -261,8 +261,10 @@ public:
     // deep its operand ring is and how long a tile's epilogue takes; which width wins depends on the batch
     // (rounds of tiles over the SMs) in ways a cost model only approximates. Every width gives the same bits
     // (the library settles the ranges of the reduction before it looks at the width), so the layer simply times the candidates on its own tensors and keeps the fastest; then, at that width, the
-    // number of ranges its reduction is split into (which does change the order of the partial sums); last, for
-    // an unsplit reduction, whether pairs of SMs should share the filter tiles (same bits again).
+    // number of ranges its reduction is split into (which does change the order of the partial sums); then, for
+    // an unsplit reduction, whether pairs of SMs should share the filter tiles (same bits again); last, channels on M (the
+    // bits of that number of ranges, but for 3x3 layers whose taps would lie side by side). Launches of taps side by side
+    // are the same whatever width or pairing is asked for: those candidates are left out.
     void Tune() override {
         OgleConvParams& p = sibling_ ? pair_params_ : params_;
         if (!filter_is_constant_ || std::string(ogle_cuda_conv2d_kernel_name(&p)) != "conv_tc2_kernel") return;
@@ -283,6 +285,10 @@ public:
             if (cudaEventSynchronize(e1) != cudaSuccess) return false;
             return cudaEventElapsedTime(ms, e0, e1) == cudaSuccess;
         };
+        auto taps_side_by_side = [] {
+            OgleContraction c;
+            return ogle_cuda_last_contraction(&c) == OGLE_OK && c.form == 6;
+        };
         float auto_ms = 0.f, best_ms = 0.f;
         p.n_tile = 0;
         p.split = 0;
@@ -291,7 +297,8 @@ public:
         if (time_it(&auto_ms)) {
             best_ms = auto_ms;
             int best_tile = 0, best_split = 0, best_pair = 0;
-            for (int bn = 32; bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
+            const bool beside = taps_side_by_side();
+            for (int bn = 32; !beside && bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
                 float ms;
                 p.n_tile = bn;
                 if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_tile = bn; }
@@ -300,17 +307,20 @@ public:
             static const int splits[] = {1, 2, 3, 4, 6, 8, 12, 16};          // then the reduction split at that width
             for (int k : splits) {
                 float ms;
+                if (k == 1 && beside) continue;
                 p.split = k;
                 if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_split = k; }
             }
             p.split = best_split;
             int pair_tile = best_tile;
-            for (int bn = 64; bn <= 256 && bn <= kmax; bn += 64) {           // SM pairs, unsplit, at the widths that halve
+            for (int bn = 64; !beside && bn <= 256 && bn <= kmax; bn += 64) {           // SM pairs, unsplit, at the widths that halve
                 float ms;
                 p.n_tile = bn;
                 p.split = 1;
                 p.sm_pair = 2;
-                if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_pair = 2; pair_tile = bn; }
+                const bool timed = time_it(&ms);
+                if (taps_side_by_side()) break;              // (split by default, and timed unsplit above)
+                if (timed && ms < best_ms) { best_ms = ms; best_pair = 2; pair_tile = bn; }
             }
             if (best_pair) { best_tile = pair_tile; best_split = 1; }
             // at most 128 output channels: the accumulator kept transposed (filters on the multiply's 128-row side)

@@ -54,6 +54,24 @@ def test_single_conv_session_round_trip(oracle_port):
         sess.close()
 
 
+def test_tuning_leaves_out_what_taps_side_by_side_ignore():
+    """A layer whose launch is the same at every width and on SM pairs is not timed at those: four candidates of four launches
+    less than a 5x5 layer on the same tensors, at least."""
+    from ogle_b200 import _lib, models, session
+    lib = _lib.cuda_lib()
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((64, 28, 28, 64), dtype=np.float32)
+    launches = []
+    for k in (3, 5):
+        sess = session.FBOSession()
+        sess.LoadGraph(models.single_conv(x.shape, rng.standard_normal((64, 64, k, k), dtype=np.float32), np.zeros(64, np.float32), 1, k // 2, 1, 1))
+        before = lib.ogle_cuda_launch_count()
+        sess.Run({"input": x})
+        launches.append(lib.ogle_cuda_launch_count() - before)
+        sess.close()
+    assert launches[0] <= launches[1] - 16
+
+
 def test_unknown_operator_and_bad_file_are_errors_not_aborts():
     from ogle_b200 import dlx, session
     s = dlx.Scope()
