@@ -82,7 +82,8 @@ int ogle_cuda_set_overlapped_launches(int on);
  * zeros before the first. */
 typedef struct {
     int form;        /* 1 whole tiles; 2 ranges of the reduction combined through memory; 3 ranges added up inside a
-                        cluster; 4 tiles on pairs of SMs; 5 channels on M; 6 taps of a filter row side by side */
+                        cluster; 4 tiles on pairs of SMs; 5 channels on M; 6 taps of a filter row side by side; 7 whole tiles
+                        of an RGB stem, its filters kept in shared memory */
     int ranges;      /* ranges of the reduction (1 = not split) */
     int n_tile;      /* output channels of a tile */
     int overlapped;  /* 1: allowed to start its set-up while the launch before it drains */

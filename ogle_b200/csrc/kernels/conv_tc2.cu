@@ -1219,7 +1219,7 @@ int launch_tc_v2(TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi, cons
     t.epi_share = t.total_work <= 4 * sms || chunks > 2 ? 1 : 0;
     const unsigned grid = (unsigned)(t.total_work < sms ? t.total_work : sms);
     const bool overlapped = overlapped_launches_enabled(t.overlapped);
-    note_contraction(t.cluster ? 3 : (t.split_k > 1 ? 2 : (t.taps ? 6 : 1)), t.split_k, t.BN, overlapped);
+    note_contraction(t.cluster ? 3 : (t.split_k > 1 ? 2 : (t.taps ? 6 : (keep ? 7 : 1))), t.split_k, t.BN, overlapped);
     if (t.cluster) {
         // every block one work item; the blocks of a tile are consecutive, and a cluster
         cudaLaunchConfig_t cfg = {};

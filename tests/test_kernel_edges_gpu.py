@@ -534,6 +534,93 @@ def test_taps_by_shape_alone(shape):
     assert (ops.last_contraction().form == 6) == (form == 6)
 
 
+WHOLE_CODE = """
+import torch
+from ogle_b200 import _lib, ops
+g = torch.Generator(device="cuda").manual_seed(11)
+rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+# 3x3 layers of stride 1 which by themselves would lie with their taps side by side: in whole tiles of every width and on
+# pairs of SMs, rows of an image, several images and pieces of a row to a tile
+for N, H, W, C, K in [(2, 38, 38, 64, 256), (6, 60, 64, 40, 256), (2, 75, 75, 20, 64), (1, 150, 150, 32, 96), (40, 28, 28, 64, 130), (200, 7, 9, 70, 128)]:
+    x = torch.zeros((N, H, W, ops.up4(C)), device="cuda")
+    x[..., :C] = rand(N, H, W, C)
+    w, b = rand(K, C, 3, 3) / (9 * C) ** 0.5, rand(K)
+    want = torch.nn.functional.conv2d(x[..., :C].permute(0, 3, 1, 2).double(), w.double(), b.double(), padding=1).permute(0, 2, 3, 1)
+    for math in (ops.MATH_TF32X3, ops.MATH_TF32):
+        p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, math)
+        p.split, p.channels_on_m = 1, 1
+        packed = ops.conv2d_prepack(p, w)
+        outs = []
+        for n_tile, pair in [(bn, 1) for bn in range(32, 257, 32) if bn <= (K + 31) // 32 * 32] + [(bn, 2) for bn in (64, 128, 192, 256) if bn <= (K + 31) // 32 * 32]:
+            p.n_tile, p.sm_pair = n_tile, pair
+            outs.append(ops.conv2d(p, x, packed, b, workspace=None))
+            assert (ops.last_contraction().form, ops.last_contraction().n_tile) == (1 if pair == 1 else 4, n_tile), (N, K, n_tile, pair, ops.last_contraction().form)
+            assert torch.equal(outs[0], outs[-1]), (N, H, C, K, math, n_tile, pair)
+        # (the bound of the taps' test)
+        assert float((outs[0][..., :K].double() - want).norm()) <= (2e-6 + 6e-9 * 9 * C if math == ops.MATH_TF32X3 else 1e-3) * float(want.norm())
+assert _lib.cuda_lib().ogle_cuda_device_status() == 0
+"""
+
+
+def test_whole_tiles_and_pairs_of_layers_that_take_taps():
+    """The form switched off (the switch is read once per process), so that the others are compared on such layers too."""
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", WHOLE_CODE], cwd=root, env=dict(os.environ, OGLE_TC_TAPS="0"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("shape", [(64, 28, 28, 64, 64), (16, 40, 30, 200, 96), (128, 14, 14, 256, 128)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_taps_are_as_near_to_64_bits_as_whole_tiles(shape, math):
+    """A third of the length of a sum in tensor memory: split-mode results are nearer (1.8e-6 of the norm and 3.4e-6 at 576
+    elements); in one pass the operands' ten bits are all there is to see."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K = shape
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x = torch.rand((N, H, W, C), generator=g, device="cuda")
+    w = torch.randn((K, C, 3, 3), generator=g, device="cuda") / (9 * C) ** 0.5 + 0.02
+    want = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), w.double(), padding=1).permute(0, 2, 3, 1)
+    p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, False, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    p.split = 1
+    packed = ops.conv2d_prepack(p, w)
+    errors, forms = [], []
+    for p.channels_on_m in (0, 1):                                    # (1: whole tiles)
+        errors.append(float((ops.conv2d(p, x, packed, workspace=None)[..., :K].double() - want).norm() / want.norm()))
+        forms.append(ops.last_contraction().form)
+    assert forms[1] in (1, 4) and (forms[0] == 6 or math == "MATH_TF32")
+    assert errors[0] <= (0.8 if math == "MATH_TF32X3" else 1.001) * errors[1], errors
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_taps_keep_non_finite_values_in_their_windows(bad, math):
+    """At the ends of rows and images, at the ends of tiles of 126 pixels and of warps: the values whose window holds one are
+    not finite, all others are what they were."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, C, K = 40, 31, 33, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, w = torch.randn((N, H, W, C), generator=g, device="cuda"), torch.randn((K, C, 3, 3), generator=g, device="cuda") / 24.0
+    p = ops.conv_params(N, H, W, C, K, 3, 1, 1, 1, 1, False, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    p.split = 1
+    packed = ops.conv2d_prepack(p, w)
+    clean = ops.conv2d(p, x, packed, workspace=None)
+    assert ops.last_contraction().form == 6
+    flat = x.view(-1, C)
+    M = N * H * W
+    places = [W - 1, 2 * W, H * W - 1, H * W, M - 1, 0, 5 * H * W + 10 * W - 1, 125 + 126 * 40, 126 * 60, 126 * 80 + 31, 126 * 100 + 32, 126 * 120 + 95]
+    hit = torch.zeros(M, device="cuda")
+    for i in places:
+        flat[i, 7] = bad
+        hit[i] = 1.0
+    hit = torch.nn.functional.max_pool2d(hit.view(N, 1, H, W), 3, 1, 1).view(N, H, W) > 0
+    got = ops.conv2d(p, x, packed, workspace=None)
+    assert not torch.isfinite(got[hit]).any()
+    assert torch.equal(got[~hit], clean[~hit])
+
+
 ON_M_CODE = """
 import torch
 from ogle_b200 import _lib, ops
@@ -697,6 +784,8 @@ def test_kept_filters_and_windows_of_rgb_stems(shape):
     assert float((got[..., :K].double() - want).norm()) <= 3e-6 * float(want.norm())
     if k == 3:
         return                                                        # (the direct kernel's)
+    # all filters, two windows and the staging slabs in 224 KB, and one filter tile
+    assert ops.last_contraction().form == (7 if K <= 64 else 1)
     assert torch.equal(ops.conv2d_residual(p, x, packed, b, torch.zeros_like(got)), got)
     try:
         lib.ogle_cuda_set_wait_limit(0)
