@@ -496,7 +496,6 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         t.g_bytes = (t.g_iw * t.g_ih * 16 + 1023) / 1024 * 1024;
         const cuuint32_t es[4] = {1, 1, 1, 1};
         if (t.g_iw > 128) {
-            t.g_pixels = 1;
             const cuuint64_t dims[4] = {4, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.N};
             const cuuint64_t str[3] = {16, (cuuint64_t)a.W * 16, (cuuint64_t)a.W * 16 * a.H};
             const cuuint32_t box[4] = {4, (cuuint32_t)t.g_iw, (cuuint32_t)t.g_ih, 1};

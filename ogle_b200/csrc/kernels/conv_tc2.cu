@@ -385,7 +385,7 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 // gather form: the tile's input window
                 auto load_window = [&](uint32_t to, uint64_t* bar) {
-                    if (a.g_pixels) tma_load_4d(to, &tmA, bar, 0, ax, ay, an);
+                    if (a.g_iw > 128) tma_load_4d(to, &tmA, bar, 0, ax, ay, an);
                     else tma_load_4d(to, &tmA, bar, 2 * ax, ay, an, 0);
                 };
                 // position of the first chunk: filter row, filter column, channel offset

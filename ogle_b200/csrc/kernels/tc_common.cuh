@@ -73,9 +73,9 @@ struct TcArgs {
     // build the 128 x 32 operand of the chunk from it, row r = window values of output pixel r
     // at reduction indices k = (ky * g_k + kx) * g_C + c, zero padded to a multiple of 32
     // (chunks_per_tap chunks; kernel = 1 in this form). g_C = input channels, g_k = filter
-    // size, g_bytes = window bytes rounded up to 1 KB (its slot at the end of every stage). g_pixels: the window's map has
-    // pixels as an extent of their own (windows more than 128 wide), not rows of them.
-    int gather, g_iw, g_ih, g_C, g_bytes, g_k, g_pixels;
+    // size, g_bytes = window bytes rounded up to 1 KB (its slot at the end of every stage). The map of windows more than 128
+    // pixels wide has pixels as an extent of their own, that of narrower ones rows of them.
+    int gather, g_iw, g_ih, g_C, g_bytes, g_k;
     // Residual operand (one-SM form, reduction unsplit or split inside a cluster): res[pixel * res_ld + channel] is added to the
     // convolution's value (after the bias, before the activation) - a residual block's Add and activation in
     // the convolution's own pass. Null = none.
