@@ -13,6 +13,7 @@ bool conv_tc_supported(const ConvArgs& a, int variant);
 bool conv_tc_gather_supported(const ConvArgs& a, int variant);
 bool dw_tma_supported(const ConvArgs& a);
 bool conv_smallc_supported(const ConvArgs& a);
+const char* conv_igemm_name(const ConvArgs& a);
 
 // Destination-indexed packing of an OIHW filter into the three sections of the
 // packed blob (see FilterLayout).
@@ -254,7 +255,7 @@ const char* ogle_cuda_conv2d_kernel_name(const OgleConvParams* p) {
     }
     if (variant == CONV_GROUPED) return "grouped_kernel";
     if (variant == CONV_GENERAL && conv_smallc_supported(a)) return "conv3x3_smallc_kernel";
-    return "conv_igemm_kernel";
+    return conv_igemm_name(a);
 }
 
 int ogle_cuda_conv2d_pair_supported(const OgleConvParams* p) {

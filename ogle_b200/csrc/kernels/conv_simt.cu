@@ -168,6 +168,19 @@ bool conv_smallc_supported(const ConvArgs& a);
 int launch_conv_smallc(const ConvArgs& a, const float* x, const float* w_tap_major, const float* bias, float* y,
                        cudaStream_t s);
 
+static IgemmArgs igemm_args(const ConvArgs& a, const float* x, const float* w, const float* bias, float* y) {
+    IgemmArgs g = {};
+    g.x = x; g.w = w; g.bias = bias; g.y = y;
+    g.M = a.M; g.H = a.H; g.W = a.W; g.Ho = a.Ho; g.Wo = a.Wo; g.Cs = a.Cs;
+    g.kernel = a.kernel; g.stride = a.stride; g.pad = a.pad; g.dil = a.dil;
+    g.Cp = a.Cp; g.R = a.kernel * a.kernel * a.Cp;
+    g.ldb = a.Kp; g.n_b = a.Kp; g.N = a.K; g.n_store = a.Kp;
+    g.ldy = a.Ks; g.yoff = a.koff;
+    g.act = a.act; g.lo = a.lo; g.hi = a.hi;
+    g.alpha = 1.f; g.beta = 1.f; g.bias_mode = a.has_bias ? 2 : 0;
+    return g;
+}
+
 int launch_conv_simt(const ConvArgs& a, int variant, const float* x, const float* w,
                      const float* bias, float* y, cudaStream_t s) {
     if (variant == CONV_DEPTHWISE) {
@@ -207,16 +220,19 @@ int launch_conv_simt(const ConvArgs& a, int variant, const float* x, const float
         }
         return OGLE_OK;
     }
-    IgemmArgs g = {};
-    g.x = x; g.w = w; g.bias = bias; g.y = y;
-    g.M = a.M; g.H = a.H; g.W = a.W; g.Ho = a.Ho; g.Wo = a.Wo; g.Cs = a.Cs;
-    g.kernel = a.kernel; g.stride = a.stride; g.pad = a.pad; g.dil = a.dil;
-    g.Cp = a.Cp; g.R = a.kernel * a.kernel * a.Cp;
-    g.ldb = a.Kp; g.n_b = a.Kp; g.N = a.K; g.n_store = a.Kp;
-    g.ldy = a.Ks; g.yoff = a.koff;
-    g.act = a.act; g.lo = a.lo; g.hi = a.hi;
-    g.alpha = 1.f; g.beta = 1.f; g.bias_mode = a.has_bias ? 2 : 0;
-    return launch_igemm(g, false, s);
+    return launch_igemm(igemm_args(a, x, w, bias, y), false, s);
+}
+
+const char* conv_igemm_name(const ConvArgs& a) {
+    const long pixels = (long)a.H * a.W;
+    ConvArgs part = a;                               // of a batch that goes in groups, the first
+    if (pixels * a.N >= 0x7fffffffL) {
+        part.N = pixels < 0x7fffffffL ? (int)(0x7fffffffL / pixels) : 1;
+        part.M = (long)part.N * a.Ho * a.Wo;
+    }
+    const char* name = "";
+    launch_igemm(igemm_args(part, nullptr, nullptr, nullptr, nullptr), false, nullptr, &name);
+    return name;
 }
 
 }  // namespace ogle

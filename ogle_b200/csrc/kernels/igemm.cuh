@@ -27,6 +27,7 @@ struct IgemmArgs {
     int ldc;
 };
 
-int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s);
+// name: not null = nothing is launched (y is null), and *name says which kernel would be.
+int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s, const char** name = nullptr);
 
 }  // namespace ogle

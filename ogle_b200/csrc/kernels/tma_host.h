@@ -65,10 +65,10 @@ inline bool make_map_pixels(CUtensorMap* m, const void* ptr, int W, int H, int N
 // `pixels` consecutive positions of the window's first tap, which walk the image from `lower` to its far edge plus `upper`
 // ({w, h} each), row after row and image after image; positions outside the image read zero.
 inline bool make_map_im2col(CUtensorMap* m, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
-                            const int* lower, const int* upper, int channels, int pixels) {
+                            const int* lower, const int* upper, int channels, int pixels, int stride = 1) {
     EncodeIm2colFn fn = encode_im2col_fn();
     if (!fn) return false;
-    const cuuint32_t es[4] = {1, 1, 1, 1};
+    const cuuint32_t es[4] = {1, (cuuint32_t)stride, (cuuint32_t)stride, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides_bytes, lower, upper, (cuuint32_t)channels,
               (cuuint32_t)pixels, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;

@@ -253,6 +253,36 @@ def test_fp32_contraction_forms(m, k, n, trans_b):
     assert (got[:, n:] == 0).all()
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride, pad, dilation: tiles of 128 and of 64 pixels, alone and over clusters of 2, 4, 5, 6 and 8;
+    # channels that end inside a step, columns and pixels inside a tile, strides, dilations, padding wider than the window
+    (5, 60, 45, 54, 374, 3, 1, 0, 2), (4, 43, 38, 115, 286, 1, 1, 1, 1), (2, 43, 41, 262, 214, 3, 1, 3, 1), (3, 48, 27, 296, 367, 1, 1, 0, 1),
+    (4, 44, 14, 157, 237, 3, 1, 0, 1), (4, 43, 26, 25, 183, 5, 1, 1, 1), (6, 45, 30, 57, 33, 3, 1, 0, 1), (1, 6, 27, 355, 62, 5, 2, 4, 2),
+    (4, 10, 22, 309, 87, 5, 3, 4, 2), (4, 41, 43, 106, 389, 5, 2, 2, 1), (2, 56, 55, 154, 86, 5, 1, 5, 2), (3, 45, 30, 25, 219, 5, 1, 2, 2),
+    (5, 59, 21, 315, 92, 3, 1, 3, 2), (2, 30, 42, 121, 113, 3, 1, 3, 1), (3, 13, 18, 286, 362, 5, 1, 2, 1)])
+def test_fp32_contraction_by_the_copy_engine(shape):
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    N, H, W, ci, K, k, s, pd, d = shape
+    g = torch.Generator(device="cuda").manual_seed(ci + K)
+    x = torch.zeros((N, H, W, ops.up4(ci)), device="cuda")
+    x[..., :ci] = torch.randn((N, H, W, ci), generator=g, device="cuda")
+    w, b = torch.randn((K, ci, k, k), generator=g, device="cuda"), torch.randn(K, generator=g, device="cuda")
+    p = ops.conv_params(N, H, W, ci, K, k, s, pd, d, 1, True, ops.ACT_CLIP, -3.0, 40.0, ops.MATH_FP32)
+    if k == 1 and pd == 0:
+        p.min_value = 0.0           # (a pointwise clip is to [0, max])
+    assert _lib.cuda_lib().ogle_cuda_conv2d_kernel_name(C.byref(p)) == b"conv_igemm_tma_kernel"
+    got = ops.conv2d(p, x, ops.conv2d_prepack(p, w), b)
+    x64 = x[..., :ci].permute(0, 3, 1, 2).double()
+    conv = lambda u, v, c: torch.nn.functional.conv2d(u, v, c, s, pd, d).permute(0, 2, 3, 1)
+    want = conv(x64, w.double(), b.double()).clamp(p.min_value, 40.0)
+    # every partial sum rounded once: at most (terms) * 2^-24 of the sum of the terms' magnitudes
+    bound = (k * k * ci + 4) * 2.0 ** -24 * conv(x64.abs(), w.double().abs(), b.double().abs())
+    assert ((got[..., :K].double() - want).abs() <= bound).all()
+    assert (got[..., K:] == 0).all()
+
+
 def test_fp32_gemm_of_many_columns():
     """Up to 65535 column tiles of 64."""
     import torch
@@ -968,7 +998,7 @@ for N, H, C, K, k in ((1, 19, 512, 512, 1), (16, 38, 256, 512, 1), (4, 20, 64, 2
 @pytest.mark.parametrize("case", [
     # C, K, kernel, stride, group, math, size
     (64, 64, 3, 1, 64, 2, 40), (50, 50, 5, 2, 50, 2, 40), (64, 64, 3, 1, 64, 2, 3), (64, 64, 7, 1, 64, 2, 40), (64, 32, 3, 1, 4, 2, 40),
-    (3, 32, 3, 2, 1, 2, 40), (64, 64, 1, 1, 1, 0, 40), (64, 64, 1, 1, 1, 2, 40)])
+    (3, 32, 3, 2, 1, 2, 40), (64, 64, 1, 1, 1, 0, 40), (64, 64, 1, 1, 1, 2, 40), (256, 256, 3, 1, 1, 0, 40)])
 def test_kernel_names_are_those_of_the_sources(case):
     """What a profile is filtered by is the name of a kernel that exists."""
     import ctypes as C
