@@ -195,7 +195,8 @@ __device__ __forceinline__ void cluster_sync() {
 // Cluster form: this block's band of the tile's rows, summed over the partial tiles of the cluster in rank order (the
 // order the slices of the scratch form are added in: the same bits), then bias, residual operand and activation, and
 // plain coalesced stores. The band's columns are dealt out as float4s, a row's neighbours to neighbouring threads.
-__device__ __forceinline__ void cluster_reduce(const TcArgs& a, uint32_t partial, const float* __restrict__ bias) {
+// s_bias: the tile's columns' (with beta), staged while the accumulator was being computed.
+__device__ __forceinline__ void cluster_reduce(const TcArgs& a, uint32_t partial, const float* s_bias, const float* __restrict__ bias) {
     const int ranks = a.split_k, tile = (int)blockIdx.x / ranks, rank = (int)blockIdx.x - tile * ranks;
     const TileCoord tc_ = tile_coord(a, tile);
     const int nbase = tc_.n_tile * a.BN;
@@ -220,6 +221,8 @@ __device__ __forceinline__ void cluster_reduce(const TcArgs& a, uint32_t partial
         const int real = second ? a.K - a.split_col : (a.split_col > 0 ? a.K1 : a.K);
         if (lcol >= real) continue;                        // between the two outputs
         const uint32_t at = partial + (uint32_t)((q >> 3) * kStagingBytes + row * 128 + (((q & 7) ^ (row & 7)) << 4));
+        float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.res) res = __ldg(reinterpret_cast<const float4*>(a.res + pixel * a.res_ld + lcol));
         float4 part[8];
 #pragma unroll
         for (int p = 0; p < 8; ++p)
@@ -228,14 +231,12 @@ __device__ __forceinline__ void cluster_reduce(const TcArgs& a, uint32_t partial
 #pragma unroll
         for (int p = 1; p < 8; ++p)
             if (p < ranks) { v[0] += part[p].x; v[1] += part[p].y; v[2] += part[p].z; v[3] += part[p].w; }
-        float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.res) res = __ldg(reinterpret_cast<const float4*>(a.res + pixel * a.res_ld + lcol));
         const float rr[4] = {res.x, res.y, res.z, res.w};
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             if (lcol + l < real) {
                 if (a.bias_mode == 1) v[l] = fmaf(a.beta, __ldg(bias + pixel * a.ldc + lcol + l), a.alpha * v[l]);
-                else v[l] = fmaf(a.alpha, v[l], a.bias_mode == 2 ? a.beta * __ldg(bias + col + l) : 0.f);
+                else v[l] = fmaf(a.alpha, v[l], s_bias[q * 4 + l]);
                 if (a.res) v[l] += rr[l];
                 v[l] = apply_act(v[l], a.act, a.lo, a.hi);
             } else {
@@ -815,6 +816,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         // One work item per block: its raw sums go to the operand ring, which the last multiply has left, slab by slab
         // in the swizzle of the staging slabs; both groups take part.
         const int row = (warp & 3) * 32 + lane;
+        if (warp < 6) {
+            const int nbase = tile_coord(a, (int)blockIdx.x / a.split_k).n_tile * a.BN;
+            for (int i = threadIdx.x - 64; i < a.BN; i += 128)
+                s_bias[0][i] = a.bias_mode == 2 && nbase + i < a.K ? a.beta * __ldg(bias + nbase + i) : 0.f;
+        }
         bool ok = wait_or_abort(&bar_acc_full[0], 0u, abort_flag, a.spin_limit);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { record_error(err_flag, 4); s_abort = 1; }
@@ -1050,9 +1056,11 @@ conv_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         // word says so); none leaves while another may still read its partial tile.
         __syncwarp();
         cluster_sync();
-        cluster_reduce(a, base, bias);
+        cluster_reduce(a, base, s_bias[0], bias);
+        // (what was read has been used, and nobody reads what was written: no order to be kept, and no wait for the stores)
         __syncwarp();
-        cluster_sync();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     }
 }
 
