@@ -7,7 +7,8 @@
 // once and nothing is staged in global memory.
 // What bounds it is the number of instructions: 1024 images x 1917 anchors x 21 classes, top 200, took
 // 428 us with a radix selection over registers and a radix sort of the survivors (238 k warp
-// instructions per image); counting into the bins that the sort needs anyway took it to 192 us.
+// instructions per image); counting into the bins that the sort needs anyway took it to 192 us, kernels that know how many
+// pieces a row of logits has to 155 with the decode (logits in and results out take 47 at the HBM rate).
 #include <cstring>
 
 #include "common.cuh"
@@ -62,7 +63,8 @@ __device__ __forceinline__ unsigned hist_get(const unsigned* hist, unsigned bin)
 //  - Where that bin holds too many (scores that all lie close together), the candidates above it are ranked as they
 //    are and the bin itself is counted again over its own range, nine bits finer, and so on; at single keys the
 //    rest are equal scores, taken in index order.
-template <typename Emit>
+// kFour: four scores of a thread find their places at once, where registers allow it (1024 x 1917 x 21: 158 us, 154).
+template <bool kFour, typename Emit>
 __device__ __forceinline__ int warp_topk(const float* vals, int Ap, KeySpace ks, int k, unsigned* hist,
                                          unsigned short* list, Emit emit) {
     const int lane = threadIdx.x & 31;
@@ -127,13 +129,31 @@ __device__ __forceinline__ int warp_topk(const float* vals, int Ap, KeySpace ks,
             for (int i = lane * 4; i < Ap; i += 128) {
                 const float4 v = *reinterpret_cast<const float4*>(vals + i);
                 const float f[4] = {v.x, v.y, v.z, v.w};
+                if constexpr (kFour) {
+                    // the four places come back one behind the other, not one after the other
+                    unsigned pos[4];
+                    bool in[4];
 #pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    const unsigned key = __float_as_uint(f[l]) - ks.base;
-                    if (key - from < span) {
+                    for (int l = 0; l < 4; ++l) {
+                        const unsigned key = __float_as_uint(f[l]) - ks.base;
+                        in[l] = key - from < span;
                         const unsigned bin = (key - lo) >> shift, half = (bin & 1u) * 16u;
-                        const unsigned pos = (atomicAdd(&hist[bin >> 1], 1u << half) >> half) & 0xffffu;
-                        list[pos] = (unsigned short)(i + l);
+                        pos[l] = 0;
+                        if (in[l]) pos[l] = atomicAdd(&hist[bin >> 1], 1u << half);
+                        pos[l] = (pos[l] >> half) & 0xffffu;
+                    }
+#pragma unroll
+                    for (int l = 0; l < 4; ++l)
+                        if (in[l]) list[pos[l]] = (unsigned short)(i + l);
+                } else {
+#pragma unroll
+                    for (int l = 0; l < 4; ++l) {
+                        const unsigned key = __float_as_uint(f[l]) - ks.base;
+                        if (key - from < span) {
+                            const unsigned bin = (key - lo) >> shift, half = (bin & 1u) * 16u;
+                            const unsigned pos = (atomicAdd(&hist[bin >> 1], 1u << half) >> half) & 0xffffu;
+                            list[pos] = (unsigned short)(i + l);
+                        }
                     }
                 }
             }
@@ -217,18 +237,38 @@ __device__ __forceinline__ float at_most_one(float s) {
     return r;
 }
 
-// A row of at most 32 logits in registers by 128-bit loads, its exponentials taken once.
-__device__ __forceinline__ void load_row(const DetectArgs& a, const float* row, float (&e)[32]) {
+// A row of kQuads * 4 - 3 to kQuads * 4 logits in registers by 128-bit loads, its exponentials taken once. How many there
+// are is known when this is compiled but for the last three: with up to 32 of them told apart at run time the loops over
+// a row were a sixth of the whole selection (1024 images, 1917 anchors, 21 classes 183 us, 154 with 24; 2 classes 77, 41).
+template <int kQuads>
+__device__ __forceinline__ bool is_class(int j, int C) { return j < kQuads * 4 - 3 || j < C; }
+template <int kQuads>
+__device__ __forceinline__ void load_row(const float* row, int C, float (&e)[kQuads * 4]) {
     const float4* row4 = reinterpret_cast<const float4*>(row);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (q * 4 < a.logit_stride) v = row4[q];
+    for (int q = 0; q < kQuads; ++q) {
+        const float4 v = row4[q];
         e[q * 4 + 0] = v.x; e[q * 4 + 1] = v.y; e[q * 4 + 2] = v.z; e[q * 4 + 3] = v.w;
     }
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-        if (j < a.C) e[j] = expf(e[j]);
+    for (int j = 0; j < kQuads * 4; ++j)
+        if (is_class<kQuads>(j, C)) e[j] = expf(e[j]);
+}
+// (for the kernel that has one form for all)
+template <int kQuads> struct Quads { static constexpr int value = kQuads; };
+// f(Quads<number of 128-bit pieces of a row of C <= 32 logits>)
+template <typename F>
+__device__ __forceinline__ void by_quads(int C, F f) {
+    switch ((C + 3) >> 2) {
+        case 1: f(Quads<1>()); break;
+        case 2: f(Quads<2>()); break;
+        case 3: f(Quads<3>()); break;
+        case 4: f(Quads<4>()); break;
+        case 5: f(Quads<5>()); break;
+        case 6: f(Quads<6>()); break;
+        case 7: f(Quads<7>()); break;
+        default: f(Quads<8>()); break;
+    }
 }
 
 // Bytes [0, bytes) at p on their way into L2, a line a thread.
@@ -239,10 +279,12 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long bytes) {
 
 // Mode 1: per class. Dynamic shared memory: float scores[classes_per_pass][Ap], histograms of as many classes
 // (kHistWords words each), one list of survivors per warp (kListMax 16-bit indices).
-// kAhead: what the SM reads next is on its way into L2 while a block selects, at 71 registers a thread (a block an SM is all
+// kAhead: what the SM reads next is on its way into L2 while a block selects, at 72 to 96 registers a thread (a block an SM is all
 // it is compiled for); else 48, for launches whose shared memory and threads let more blocks onto an SM than that (below).
-template <bool kAhead>
-__global__ void __launch_bounds__(640, kAhead ? 1 : 0)
+// kPieces: 128-bit pieces of a row of logits (0: rows that are not read in such). A kernel for each, since the small ones
+// otherwise get the registers of the large ones, or spill: 1024 images, 300 anchors, 21 classes 49.6 us with one for all, 45.8.
+template <bool kAhead, int kPieces>
+__global__ void __launch_bounds__(640, kAhead ? 1 : 2)
 ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ boxes,
                   float* __restrict__ out_score, int* __restrict__ out_anchor, int* __restrict__ out_class,
                   float4* __restrict__ out_box, int* __restrict__ out_count, const DetectArgs a) {
@@ -262,7 +304,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
     const int c_lo = 1 + part * per_part, c_hi = min(a.C, c_lo + per_part);     // this block's classes
     for (int c0 = c_lo; c0 < c_hi; c0 += a.classes_per_pass) {
         const int nc = min(a.classes_per_pass, c_hi - c0);
-        for (int i = tid; i < nc * kHistWords; i += blockDim.x) hists[i] = 0;
+        for (int i = tid; i < nc * (kHistWords / 4); i += blockDim.x) reinterpret_cast<uint4*>(hists)[i] = make_uint4(0, 0, 0, 0);
         if (a.Ap > a.A)
             for (int j = tid; j < nc * 4; j += blockDim.x)
                 if (a.Ap - 4 + (j & 3) >= a.A) scores[(j >> 2) * a.Ap + a.Ap - 4 + (j & 3)] = __int_as_float(0x7fc00000);
@@ -275,19 +317,23 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
         // softmax as the reference post-process does it - exp of the raw logits, summed in class
         // order - with the per-class divide replaced by one IEEE reciprocal of the sum and a
         // multiply per class (scores within one ulp of the reference's quotient)
-        if (nc == c_hi - c_lo && a.rows_fit) {
-            for (int i = tid; i < a.A; i += blockDim.x) {
-                float e[32];
-                load_row(a, lg + (long)i * a.logit_stride, e);
-                float total = 0.f;
+        if constexpr (kPieces > 0) {
+            auto rows_of = [&](auto wanted) {
+                for (int i = tid; i < a.A; i += blockDim.x) {
+                    float e[kPieces * 4];
+                    load_row<kPieces>(lg + (long)i * a.logit_stride, a.C, e);
+                    float total = 0.f;
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < a.C) total += e[j];
-                const float inv = 1.0f / total;
+                    for (int j = 0; j < kPieces * 4; ++j)
+                        if (is_class<kPieces>(j, a.C)) total += e[j];
+                    const float inv = 1.0f / total;
 #pragma unroll
-                for (int j = 1; j < 32; ++j)
-                    if (j >= c0 && j < c0 + nc) put(j - c0, i, at_most_one(e[j] * inv));
-            }
+                    for (int j = 1; j < kPieces * 4; ++j)
+                        if (wanted(j)) put(j - c0, i, at_most_one(e[j] * inv));
+                }
+            };
+            if (nc == a.C - 1) rows_of([&](int j) { return is_class<kPieces>(j, a.C); });
+            else rows_of([&](int j) { return j >= c0 && j < c0 + nc; });
         } else {
             for (int i = tid; i < a.A; i += blockDim.x) {
                 const float* row = lg + (long)i * a.logit_stride;
@@ -304,7 +350,7 @@ ssd_detect_kernel(const float* __restrict__ logits, const float4* __restrict__ b
             const int cls = c0 + j;
             const float* vals = scores + j * a.Ap;
             const long base = (long)n * rows + (long)(cls - 1) * a.top_k;
-            const int cnt = warp_topk(vals, a.Ap, a.ks, a.top_k, hists + j * kHistWords, list, [&](int r, int an) {
+            const int cnt = warp_topk<kAhead>(vals, a.Ap, a.ks, a.top_k, hists + j * kHistWords, list, [&](int r, int an) {
                 out_score[base + r] = vals[an];
                 out_anchor[base + r] = an;
                 out_class[base + r] = cls;
@@ -347,38 +393,46 @@ ssd_detect_rule_kernel(const float* __restrict__ logits, const float4* __restric
     for (int i = a.A + tid; i < a.Ap; i += blockDim.x) scores[i] = __int_as_float(0x7fc00000);
     __syncthreads();
     grid_dependency_wait();
-    const bool fits = a.rows_fit;
-    for (int i = tid; i < a.A; i += blockDim.x) {
-        const float* row = lg + (long)i * a.logit_stride;
-        float total, max_e = 0.f;
-        int max_id = 0;
-        if (fits) {
-            float e[32];
-            load_row(a, row, e);
-            total = e[0];
-#pragma unroll
-            for (int j = 1; j < 32; ++j)
-                if (j < a.C) {
-                    total += e[j];
-                    if (max_e < e[j]) { max_e = e[j]; max_id = j; }
-                }
-        } else {
-            total = expf(row[0]);
-            for (int j = 1; j < a.C; ++j) {
-                const float e = expf(row[j]);
-                total += e;
-                if (max_e < e) { max_e = e; max_id = j; }
-            }
-        }
+    auto put = [&](int i, float max_e, float total, int max_id) {
         const float s = max_e / total;
         scores[i] = s;
         best[i] = max_id;
         const unsigned key = __float_as_uint(s) - a.ks.base;
         if (key - 1u < a.ks.max_key) hist_add(hist, key >> a.ks.shift);
+    };
+    if (a.rows_fit) {
+        by_quads(a.C, [&](auto quads) {
+            constexpr int kQuads = decltype(quads)::value;
+            for (int i = tid; i < a.A; i += blockDim.x) {
+                float e[kQuads * 4];
+                load_row<kQuads>(lg + (long)i * a.logit_stride, a.C, e);
+                float total = e[0], max_e = 0.f;
+                int max_id = 0;
+#pragma unroll
+                for (int j = 1; j < kQuads * 4; ++j)
+                    if (is_class<kQuads>(j, a.C)) {
+                        total += e[j];
+                        if (max_e < e[j]) { max_e = e[j]; max_id = j; }
+                    }
+                put(i, max_e, total, max_id);
+            }
+        });
+    } else {
+        for (int i = tid; i < a.A; i += blockDim.x) {
+            const float* row = lg + (long)i * a.logit_stride;
+            float total = expf(row[0]), max_e = 0.f;
+            int max_id = 0;
+            for (int j = 1; j < a.C; ++j) {
+                const float e = expf(row[j]);
+                total += e;
+                if (max_e < e) { max_e = e; max_id = j; }
+            }
+            put(i, max_e, total, max_id);
+        }
     }
     __syncthreads();
     if (warp == 0) {
-        const int cnt = warp_topk(scores, a.Ap, a.ks, a.top_k, hist, list, [&](int r, int an) { picked[r] = an; });
+        const int cnt = warp_topk<true>(scores, a.Ap, a.ks, a.top_k, hist, list, [&](int r, int an) { picked[r] = an; });
         if (lane == 0) s_cnt = cnt;
     }
     __syncthreads();
@@ -461,6 +515,11 @@ int ogle_cuda_ssd_decode(const float* pred, const float* anchors, float* out, in
     return finish_launch();
 }
 
+typedef void (*DetectKernel)(const float*, const float4*, float*, int*, int*, float4*, int*, const DetectArgs);
+#define DETECT_KERNELS(ahead) \
+    {ssd_detect_kernel<ahead, 0>, ssd_detect_kernel<ahead, 1>, ssd_detect_kernel<ahead, 2>, ssd_detect_kernel<ahead, 3>, \
+     ssd_detect_kernel<ahead, 4>, ssd_detect_kernel<ahead, 5>, ssd_detect_kernel<ahead, 6>, ssd_detect_kernel<ahead, 7>, ssd_detect_kernel<ahead, 8>}
+
 static int launch_detect(const OgleDetectParams* p, const float* logits, const float* boxes, const float* anchors,
                          const float* variances, float* out_score, int* out_anchor, int* out_class, float* out_box,
                          int* out_count, ogle_stream_t stream) {
@@ -508,13 +567,18 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
             if ((size_t)half * (per_class + per_warp) <= 112 * 1024) a.parts = 2;
         }
         const int classes = (fg + a.parts - 1) / a.parts;
-        const int pickers = classes < 20 ? classes : 20;             // (only they need a list)
-        const size_t warp_bytes = per_warp * (size_t)pickers;
-        const size_t block_bytes = classes * per_class + warp_bytes + 1024;
+        // Where half as many warps as classes have a thread for every row, blocks of those, twice as many to an SM, keep more
+        // of their threads busy through the softmax (1024 images, 300 anchors, 21 classes, top 100: 51.8 us, 48.0; 500
+        // anchors 74.3, 82.2, so not there).
+        int pickers = classes < 20 ? classes : 20;
+        if (p->A <= 32 * ((classes + 1) / 2) && (classes + 1) / 2 < pickers) pickers = (classes + 1) / 2;
+        const size_t block_bytes = classes * per_class + per_warp * (size_t)pickers + 1024;
         const long waiting = ((long)p->N * a.parts + kNumSMs - 1) / kNumSMs;       // blocks to an SM, and how many fit
         const long fitting = block_bytes < kSmemBudget ? (long)(kSmemBudget / block_bytes) : 1;
         const int share = (int)(20 / (waiting < fitting ? waiting : fitting));
-        threads = 32 * (pickers > share ? pickers : share);
+        if (pickers < share) pickers = share;
+        threads = 32 * pickers;
+        const size_t warp_bytes = per_warp * (size_t)(pickers < classes ? pickers : classes);      // (only who picks needs a list)
         const size_t budget = a.parts == 2 && p->N * a.parts > kNumSMs ? 112 * 1024 : kSmemBudget;
         if (per_class + warp_bytes > budget) return OGLE_ERR_UNSUPPORTED;
         size_t cpp = (budget - warp_bytes) / per_class;
@@ -526,20 +590,33 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         smem = (size_t)a.Ap * 8 + kHistWords * 4 + kMaxTopK * 6 * sizeof(int) + kListMax * sizeof(unsigned short);
         if (smem > kSmemRule) return OGLE_ERR_UNSUPPORTED;
     }
-    static thread_local int attr_set_for_device = -1, regs[2];
+    static const DetectKernel per_class_kernels[2][9] = {DETECT_KERNELS(false), DETECT_KERNELS(true)};
+    const int pieces = a.rows_fit ? (a.C + 3) >> 2 : 0;
+    static thread_local int known_device = -1, regs[2][9];           // (0: not asked yet)
+    static thread_local bool rule_set;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_set_for_device != dev) {
-        cudaFuncAttributes fa;
-        cudaError_t e = cudaFuncSetAttribute(ssd_detect_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_detect_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
-        if (e == cudaSuccess)
+    if (known_device != dev) {
+        memset(regs, 0, sizeof(regs));
+        rule_set = false;
+        known_device = dev;
+    }
+    if (p->mode == 0 ? !rule_set : regs[0][pieces] == 0) {
+        cudaError_t e = cudaSuccess;
+        if (p->mode == 0) {
             e = cudaFuncSetAttribute(ssd_detect_rule_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemRule);
-        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, ssd_detect_kernel<false>);
-        if (e == cudaSuccess) { regs[0] = fa.numRegs; e = cudaFuncGetAttributes(&fa, ssd_detect_kernel<true>); }
+        } else {
+            int asked[2];
+            for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+                cudaFuncAttributes fa;
+                e = cudaFuncSetAttribute(per_class_kernels[i][pieces], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+                if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, per_class_kernels[i][pieces]);
+                if (e == cudaSuccess) asked[i] = fa.numRegs;
+            }
+            if (e == cudaSuccess) { regs[0][pieces] = asked[0]; regs[1][pieces] = asked[1]; }
+        }
         if (e != cudaSuccess) { set_last_error(e); return OGLE_ERR_CUDA; }
-        regs[1] = fa.numRegs;
-        attr_set_for_device = dev;
+        if (p->mode == 0) rule_set = true;
     }
     bool wide = false;
     if (p->mode == 1) {
@@ -553,13 +630,13 @@ static int launch_detect(const OgleDetectParams* p, const float* logits, const f
         if (blocks > waiting) blocks = waiting;
         int fit[2];
         for (int i = 0; i < 2; ++i) {
-            const int warps = 4 * (16384 / ((regs[i] + 7) / 8 * 8 * 32)) / (threads / 32);
+            const int warps = 4 * (16384 / ((regs[i][pieces] + 7) / 8 * 8 * 32)) / (threads / 32);
             fit[i] = blocks < warps ? blocks : warps;
         }
         wide = fit[1] >= fit[0];
         a.ahead = p->N > kNumSMs ? kNumSMs * fit[1] / a.parts : 0;
     }
-    const auto kernel = p->mode != 1 ? ssd_detect_rule_kernel : (wide ? ssd_detect_kernel<true> : ssd_detect_kernel<false>);
+    const DetectKernel kernel = p->mode != 1 ? ssd_detect_rule_kernel : per_class_kernels[wide ? 1 : 0][pieces];
     launch_overlapped(kernel, dim3(p->N * a.parts), dim3(threads), smem,
                       (cudaStream_t)stream, logits, reinterpret_cast<const float4*>(boxes), out_score, out_anchor, out_class,
                       reinterpret_cast<float4*>(out_box), out_count, a);

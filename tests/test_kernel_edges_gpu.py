@@ -78,6 +78,16 @@ def test_detect_selection_edges(oracle_port, anchors, classes, top_k, spread):
         _check_per_class(oracle_port, logits, boxes, thr, top_k, (classes + 3) // 4 * 4)
 
 
+@pytest.mark.parametrize("classes", [2, 4, 5, 8, 9, 12, 13, 16, 17, 20, 21, 24, 25, 28, 29, 32])
+def test_detect_rows_of_every_length(oracle_port, classes):
+    """A kernel for each number of 128-bit pieces in a row of logits, the last of them full and with one value: all classes
+    in one block of as many warps as classes and of half as many, half of the classes a block, classes in two passes."""
+    rng = np.random.default_rng(classes)
+    for images, anchors in ((2, 70), (1, 500), (150, 90), (1, 3000)):
+        logits = (rng.standard_normal((images, anchors, classes)) * 2).astype(np.float32)
+        _check_per_class(oracle_port, logits, rng.random((images, anchors, 4), dtype=np.float32), 0.02, 20, (classes + 3) // 4 * 4)
+
+
 @pytest.mark.parametrize("anchors,classes,spread,thr", [(1917, 2, 3.0, 0.3), (1917, 21, 1e-3, 0.01), (333, 5, 0.0, 0.1), (40, 33, 2.0, -1.0)])
 def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
     """The reference detector's rule, decoded by the caller and decoded on the way, over the same edges."""
