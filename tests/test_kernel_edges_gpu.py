@@ -968,6 +968,38 @@ def test_clusters_do_not_take_longer_ranges(shape, math):
     assert err <= 1.05 * run(planned)[1] + 1e-8
 
 
+@pytest.mark.parametrize("m,k,n,bias_mode", [
+    # a row, two, up to four and up to eight; one to eight warps to a column, four columns to a warp; reductions and columns
+    # that end inside a step, a piece, the pack's padding
+    (1, 512, 1000, 2), (1, 5, 3, 1), (1, 131, 9473, 2), (1, 4099, 10, 0), (2, 1030, 77, 2), (2, 33, 4801, 0), (3, 129, 130, 1),
+    (4, 2049, 300, 2), (3, 3001, 2200, 0), (5, 64, 9, 1), (8, 700, 1001, 2), (7, 97, 6000, 2)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_products_of_few_rows(m, k, n, bias_mode, math):
+    """Against 64 bits with B as the pack holds it, whose every product is rounded only as the sum is."""
+    import torch
+    from ogle_b200 import ops
+    mode = getattr(ops, math)
+    if mode == ops.MATH_TF32 and (m, k) == (3, 3001):
+        pytest.skip("so many products of one pass are the tensor cores'")
+    g = torch.Generator(device="cuda").manual_seed(m * k + n)
+    pad = lambda t, v: torch.nn.functional.pad(t, (0, ops.up4(t.shape[-1]) - t.shape[-1]), value=v)
+    a, b = torch.randn((m, k), generator=g, device="cuda"), torch.randn((n, k), generator=g, device="cuda")
+    c = torch.randn((n,) if bias_mode == 2 else (m, n), generator=g, device="cuda")
+    before = ops.last_contraction()
+    got = ops.gemm_packed(pad(a, float("nan")), ops.gemm_pack_b(pad(b, float("nan")), m, k, n, 1, mode),      # (NaN: never to be read)
+                          None if bias_mode == 0 else pad(c, 0.0), m, k, n, 1, 0.5, 2.0 if bias_mode else 0.0, bias_mode, mode)
+    after = ops.last_contraction()
+    assert (before.form, before.ranges, before.n_tile) == (after.form, after.ranges, after.n_tile)             # no tensor-core launch
+    hi = (b.view(torch.int32) & ~0x1fff).view(torch.float32)
+    held = (hi.double() + ((b - hi).bfloat16().double() if mode == ops.MATH_TF32X3 else 0.0)).t()
+    bias = 2.0 * c.double() if bias_mode else torch.zeros((), dtype=torch.float64, device="cuda")
+    want = 0.5 * (a.double() @ held) + bias
+    # every partial sum rounded once: at most k * 2^-24 of the sum of the terms' magnitudes
+    bound = (k + 8) * 2.0 ** -24 * (0.5 * (a.abs().double() @ held.abs()) + bias.abs())
+    assert ((got[:, :n].double() - want).abs() <= bound).all()
+    assert (got[:, n:] == 0).all()
+
+
 @pytest.mark.parametrize("name,value", [("OGLE_TC_PAIR", "1"), ("OGLE_TC_PAIR", "0"), ("OGLE_TC_BN", "64"), ("OGLE_TC_BN", "192")])
 def test_forced_forms_are_the_ones_that_run(name, value):
     """The switches for measurements are read once per process: convolutions, with and without a residual operand, and
