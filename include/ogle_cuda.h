@@ -78,14 +78,14 @@ int ogle_cuda_device_status_detail(void);
  * Captured CUDA graphs keep what was in force when they were captured. */
 int ogle_cuda_set_overlapped_launches(int on);
 
-/* How the calling thread's latest tensor-core contraction (a convolution or gemm) was laid out, for tests and reports;
+/* How the calling thread's latest contraction with packed filters (a convolution or gemm) was laid out, for tests and reports;
  * zeros before the first. */
 typedef struct {
     int form;        /* 1 whole tiles; 2 ranges of the reduction combined through memory; 3 ranges added up inside a
                         cluster; 4 tiles on pairs of SMs; 5 channels on M; 6 taps of a filter row side by side; 7 whole tiles
-                        of an RGB stem, its filters kept in shared memory */
+                        of an RGB stem, its filters kept in shared memory; 8 few rows, on the CUDA cores */
     int ranges;      /* ranges of the reduction (1 = not split) */
-    int n_tile;      /* output channels of a tile */
+    int n_tile;      /* output channels of a tile (form 8: of a warp) */
     int overlapped;  /* 1: allowed to start its set-up while the launch before it drains */
 } OgleContraction;
 int ogle_cuda_last_contraction(OgleContraction* out);

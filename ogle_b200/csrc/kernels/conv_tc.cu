@@ -22,6 +22,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "few_rows.cuh"
 #include "tc_common.cuh"
 #include "tma_host.h"
 
@@ -424,6 +425,15 @@ splitk_reduce_kernel(const float4* __restrict__ ws, int slices, long slice_q, in
 // ws / ws_bytes: scratch for a split reduction of more than two ranges (or of a layer with an
 // activation), may be null. ws_needed != null: plan only - no tensor maps, no launch - and report the
 // scratch size this layer would like.
+// Whether a convolution has so few pixels that the CUDA cores are quicker (few_rows.cu), and the caller leaves that open:
+// a fixed 3 us instead of 6 to 8, but by the multiply-add (in graphs: 9 pixels, 256 -> 128 pointwise 6.4 -> 3.8 us, 4 pixels
+// of 3x3 256 -> 150 9.3 -> 4.6, 8 of them 9.5 -> 5.8; 16 pixels of 3x3 69 -> 271, 2.7 M products, 7.9 -> 8.5).
+static bool few_rows(const ConvArgs& a) {
+    if (a.n_tile || a.split || a.on_m || a.pair || filter_compact(a.C, a.kernel, 1)) return false;
+    const double products = (double)a.M * a.K * a.kernel * a.kernel * a.C;
+    return (a.M <= 32 && products <= 1.5e6) || (a.M <= 8 && products <= 3e6);
+}
+
 int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x, const float* w_hi,
                    const float* w_lo, const float* bias, float* y, cudaStream_t s, float* y2, int K1,
                    int split_col, void* ws, size_t ws_bytes, size_t* ws_needed, const float* residual, int res_ld) {
@@ -437,6 +447,18 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
             return OGLE_ERR_UNSUPPORTED;
         t.split_col = split_col;
         t.K1 = K1;
+    }
+    if (!plan_only && few_rows(a)) {
+        FewRowsArgs r = {};
+        r.x = x; r.hi = w_hi; r.lo = math_mode == OGLE_MATH_TF32X3 ? w_lo : nullptr; r.bias = bias; r.res = residual;
+        r.y = y + a.koff; r.y2 = y2;
+        r.M = (int)a.M; r.N = a.K; r.C = a.C; r.Cp32 = (a.C + 31) / 32 * 32; r.kernel = a.kernel;
+        r.H = a.H; r.W = a.W; r.Ho = a.Ho; r.Wo = a.Wo; r.stride = a.stride; r.pad = a.pad; r.dil = a.dil;
+        r.ldx = a.Cs; r.ldy = y2 ? up4(K1) : a.Ks; r.ldy2 = y2 ? up4(a.K - split_col) : 0; r.res_ld = res_ld;
+        r.split_col = y2 ? split_col : 0; r.N1 = K1;
+        r.alpha = 1.f; r.beta = 1.f; r.bias_mode = a.has_bias ? 2 : 0;
+        r.act = a.act; r.lo_clip = a.lo; r.hi_clip = a.hi;
+        return launch_few_rows(r, s);
     }
     // channel extents and row strides of the output tensor(s)
     const int kp_a = y2 ? up4(K1) : a.Kp, ks_a = y2 ? up4(K1) : a.Ks;

@@ -1,0 +1,27 @@
+// Arguments of the contraction of few rows with packed filters (few_rows.cu).
+#pragma once
+#include "conv_args.cuh"
+
+namespace ogle {
+
+// D[m][n] = sum over taps and channels of A and B. B as the tensor-core kernels take it: `hi` [>= N rows][kernel^2][Cp32],
+// `lo` the cross section beside it (null: one pass, `hi` alone). A is a matrix of M rows of C elements, ldx floats apart
+// (kernel 1, H 0), or the windows of a convolution over pixels of ldx floats.
+struct FewRowsArgs {
+    const float *x, *hi, *lo, *bias, *res;
+    float *y, *y2;
+    int M, N;                          // rows; columns (stacked, with two outputs)
+    int C, Cp32, kernel;
+    int H, W, Ho, Wo, stride, pad, dil;
+    int ldx, ldy, ldy2, ldc, res_ld;   // floats a row (of y, y2 from their first column on)
+    int split_col, N1;                 // two outputs: columns [0, N1) to y, [split_col, N) to y2 (split_col 0: one)
+    float alpha, beta;
+    int bias_mode;                     // 0 none, 1 matrix [M][ldc], 2 row [N]
+    int act;
+    float lo_clip, hi_clip;
+    int kw;                            // set by the launch
+};
+
+int launch_few_rows(FewRowsArgs a, cudaStream_t s);
+
+}  // namespace ogle

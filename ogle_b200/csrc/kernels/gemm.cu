@@ -3,6 +3,7 @@
 // go to the tcgen05 path when the shape allows it.
 #include <cuda_bf16.h>
 
+#include "few_rows.cuh"
 #include "igemm.cuh"
 
 namespace ogle {
@@ -59,110 +60,6 @@ gemm_pack_b_kernel(const float* __restrict__ B, float* __restrict__ hi, __nv_bfl
             *reinterpret_cast<uint2*>(cross + chunk * 2 + 32 + kk) = all;
         }
     }
-}
-
-// A product of a few rows and a packed B: bound by fetching B once, and, at a few megabytes of it, by the launch and a trip
-// to L2, of which the tensor-core kernel makes several (1 x 512 x 1000, waited for: 30 us a call, 22). A warp takes kCols columns, 128 reduction
-// elements a step, every lane four of each; where the columns do not fill the GPU, kw warps share them and a reduction.
-// Multiply-adds are fp32 on the operand as the pack holds it - its high part, in split mode plus the bfloat16 of the rest,
-// an exact sum -: nothing is dropped that the tensor-core passes keep.
-struct RowsArgs {
-    const float *A, *hi, *bias;
-    const __nv_bfloat16* cross;
-    float* Y;
-    int M, K, N, lda, ldy, ldc, Kp32;
-    float alpha, beta;
-    int bias_mode, kw;
-};
-
-template <int kRows, int kCols, bool kSplit>
-__global__ void __launch_bounds__(256)
-gemm_rows_kernel(const RowsArgs a) {
-    __shared__ float s_part[8][kRows * kCols];
-    grid_dependency_trigger();
-    grid_dependency_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int group = warp / a.kw, part = warp - group * a.kw, groups = 8 / a.kw;
-    const int n0 = ((int)blockIdx.x * groups + group) * kCols, m0 = (int)blockIdx.y * kRows;
-    const int Np = (a.N + 3) / 4 * 4;
-    float acc[kRows][kCols];
-#pragma unroll
-    for (int m = 0; m < kRows; ++m)
-#pragma unroll
-        for (int c = 0; c < kCols; ++c) acc[m][c] = 0.f;
-    if (n0 < Np) {                                   // (rows of the pack past N are zeros, up to a multiple of 128)
-#pragma unroll(kRows * kCols == 1 ? 8 : (kRows * kCols <= 4 ? 4 : 2))
-        for (int k = part * 128 + lane * 4; k < a.Kp32; k += a.kw * 128) {
-            float b[kCols][4];
-#pragma unroll
-            for (int c = 0; c < kCols; ++c) {
-                const long row = (long)(n0 + c) * a.Kp32;
-                const float4 h = __ldg(reinterpret_cast<const float4*>(a.hi + row + k));
-                b[c][0] = h.x; b[c][1] = h.y; b[c][2] = h.z; b[c][3] = h.w;
-                if (kSplit) {
-                    const uint2 l = __ldg(reinterpret_cast<const uint2*>(a.cross + (row + (k & ~31)) * 2 + (k & 31)));
-                    b[c][0] += __uint_as_float(l.x << 16); b[c][1] += __uint_as_float(l.x & 0xffff0000u);
-                    b[c][2] += __uint_as_float(l.y << 16); b[c][3] += __uint_as_float(l.y & 0xffff0000u);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < kRows; ++m) {
-                float v[4] = {0.f, 0.f, 0.f, 0.f};
-                if (m0 + m < a.M) {
-                    const float* from = a.A + (long)(m0 + m) * a.lda + k;
-                    if (k + 4 <= a.K) {
-                        const float4 q = *reinterpret_cast<const float4*>(from);
-                        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-                    } else {                         // what lies past the end of a row is not to be read
-#pragma unroll
-                        for (int l = 0; l < 3; ++l)
-                            if (k + l < a.K) v[l] = from[l];
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < kCols; ++c)
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) acc[m][c] = fmaf(v[l], b[c][l], acc[m][c]);
-            }
-        }
-    }
-    float mine = 0.f;                                // lane m * kCols + c keeps that sum
-#pragma unroll
-    for (int m = 0; m < kRows; ++m)
-#pragma unroll
-        for (int c = 0; c < kCols; ++c) {
-            float v = acc[m][c];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (lane == m * kCols + c) mine = v;
-        }
-    if (a.kw > 1) {
-        if (lane < kRows * kCols) s_part[warp][lane] = mine;
-        __syncthreads();
-        if (part != 0) return;
-        if (lane < kRows * kCols)
-            for (int p = 1; p < a.kw; ++p) mine += s_part[warp + p][lane];
-    }
-    const int m = m0 + lane / kCols, n = n0 + lane % kCols;
-    if (lane >= kRows * kCols || m >= a.M || n >= Np) return;
-    float v = 0.f;                                   // padded columns are zero
-    if (n < a.N) {
-        if (a.bias_mode == 1) v = fmaf(a.beta, a.bias[(long)m * a.ldc + n], a.alpha * mine);
-        else v = fmaf(a.alpha, mine, a.bias_mode == 2 ? a.beta * a.bias[n] : 0.f);
-    }
-    a.Y[(long)m * a.ldy + n] = v;
-}
-
-template <int kRows>
-static int launch_rows(const RowsArgs& a, bool split, bool overlapped, cudaStream_t s) {
-    // four columns a warp where one each is more than the GPU holds at once
-    const bool wide = a.N > 8 * 8 * kNumSMs / 2;
-    const int per_block = 8 / a.kw * (wide ? 4 : 1);
-    const dim3 grid((unsigned)((up4(a.N) + per_block - 1) / per_block), (unsigned)((a.M + kRows - 1) / kRows));
-    auto kernel = wide ? (split ? gemm_rows_kernel<kRows, 4, true> : gemm_rows_kernel<kRows, 4, false>)
-                       : (split ? gemm_rows_kernel<kRows, 1, true> : gemm_rows_kernel<kRows, 1, false>);
-    launch_overlapped_if(overlapped_launches_enabled(overlapped), kernel, grid, dim3(256), 0, s, a);
-    return finish_launch();
 }
 
 }  // namespace ogle
@@ -222,21 +119,19 @@ static int gemm_packed(const OgleGemmParams* pp, const float* A, const void* pac
     const size_t half = (size_t(Np128) * Kp32 * sizeof(float) + 255) / 256 * 256;
     const float* hi = static_cast<const float*>(packed_b);
     const float* lo = reinterpret_cast<const float*>(static_cast<const char*>(packed_b) + half);
-    // A row at a time is always quicker without the tensor cores (1 x 4096 x 4096 70 us, 31; in one pass 19, 13); up to eight rows while there is
-    // little to multiply (4 x 679 x 2536 13.9 us, 13.1; 3 x 2516 x 2240 in one pass 14.9, 19.1), further where split-mode
-    // reductions are too long to be cut (2 x 3430 x 700 42 us, 13; 3 x 3784 x 3257 62, 52). Not behind a packing pass, whose
-    // B it would wait for no less.
+    // A row at a time is always quicker without the tensor cores (in graphs: 1 x 512 x 1000 8.6 -> 3.2 us; 1 x 4096 x 4096 70 ->
+    // 31, in one pass 19 -> 13), up to eight rows while there is little to multiply (8 x 512 x 1000 8.7 -> 5.0; 6 x 911 x
+    // 1257 9.5 -> 13), further where split-mode reductions are too long to be cut (2 x 3430 x 700 42 -> 13, 3 x 3784 x 3257
+    // 62 -> 52). Not behind a packing pass, whose B it would wait for no less.
     const bool split = p.math_mode == OGLE_MATH_TF32X3;
     const double products = (double)p.M * p.N * p.K;
-    if (!overlapped && (p.M == 1 || (p.M <= 8 && products <= 8e6) || (split && p.M <= 4 && p.K >= 2048 && products <= 4e7))) {
-        RowsArgs r = {A, hi, C, reinterpret_cast<const __nv_bfloat16*>(lo), Y, p.M, p.K, p.N, p.lda, p.ldy, p.ldc, Kp32, p.alpha, p.beta, p.bias_mode, 1};
-        const long warps = up4(p.N);
-        while (r.kw < 8 && warps * r.kw * 2 <= 8 * kNumSMs * 2 && Kp32 >= r.kw * 256) r.kw *= 2;
-        cudaStream_t s = (cudaStream_t)stream;
-        if (p.M == 1) return launch_rows<1>(r, split, overlapped, s);
-        if (p.M == 2) return launch_rows<2>(r, split, overlapped, s);
-        if (p.M <= 4) return launch_rows<4>(r, split, overlapped, s);
-        return launch_rows<8>(r, split, overlapped, s);
+    if (!overlapped && (p.M == 1 || (p.M <= 8 && products <= 6e6) || (split && p.M <= 4 && p.K >= 2048 && products <= 4e7))) {
+        FewRowsArgs r = {};
+        r.x = A; r.hi = hi; r.lo = split ? lo : nullptr; r.bias = C; r.y = Y;
+        r.M = p.M; r.N = p.N; r.C = p.K; r.Cp32 = Kp32; r.ldx = p.lda; r.ldy = p.ldy; r.ldc = p.ldc;
+        r.kernel = 1;
+        r.alpha = p.alpha; r.beta = p.beta; r.bias_mode = p.bias_mode;
+        return launch_few_rows(r, (cudaStream_t)stream);
     }
     return launch_gemm_tc_packed(p, A, hi, lo, C, Y, (cudaStream_t)stream, overlapped);
 }

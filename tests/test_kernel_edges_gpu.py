@@ -985,11 +985,9 @@ def test_products_of_few_rows(m, k, n, bias_mode, math):
     pad = lambda t, v: torch.nn.functional.pad(t, (0, ops.up4(t.shape[-1]) - t.shape[-1]), value=v)
     a, b = torch.randn((m, k), generator=g, device="cuda"), torch.randn((n, k), generator=g, device="cuda")
     c = torch.randn((n,) if bias_mode == 2 else (m, n), generator=g, device="cuda")
-    before = ops.last_contraction()
     got = ops.gemm_packed(pad(a, float("nan")), ops.gemm_pack_b(pad(b, float("nan")), m, k, n, 1, mode),      # (NaN: never to be read)
                           None if bias_mode == 0 else pad(c, 0.0), m, k, n, 1, 0.5, 2.0 if bias_mode else 0.0, bias_mode, mode)
-    after = ops.last_contraction()
-    assert (before.form, before.ranges, before.n_tile) == (after.form, after.ranges, after.n_tile)             # no tensor-core launch
+    assert ops.last_contraction().form == 8
     hi = (b.view(torch.int32) & ~0x1fff).view(torch.float32)
     held = (hi.double() + ((b - hi).bfloat16().double() if mode == ops.MATH_TF32X3 else 0.0)).t()
     bias = 2.0 * c.double() if bias_mode else torch.zeros((), dtype=torch.float64, device="cuda")
@@ -998,6 +996,57 @@ def test_products_of_few_rows(m, k, n, bias_mode, math):
     bound = (k + 8) * 2.0 ** -24 * (0.5 * (a.abs().double() @ held.abs()) + bias.abs())
     assert ((got[:, :n].double() - want).abs() <= bound).all()
     assert (got[:, n:] == 0).all()
+
+
+@pytest.mark.parametrize("shape", [
+    # N, H, W, C, K, kernel, stride, pad, dilation: a pixel, two, some, several images; channels that end inside a piece;
+    # padding, strides and dilations that leave taps outside the image
+    (1, 1, 1, 256, 150, 3, 1, 1, 1), (1, 2, 1, 45, 33, 1, 1, 0, 1), (2, 1, 1, 130, 7, 5, 1, 2, 1), (1, 3, 3, 128, 220, 3, 2, 1, 1),
+    (5, 2, 3, 50, 61, 3, 1, 1, 1), (1, 5, 4, 97, 65, 3, 2, 3, 2), (32, 1, 1, 64, 36, 1, 1, 0, 1), (8, 2, 2, 128, 222, 3, 2, 1, 1)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+@pytest.mark.parametrize("output", ["alone", "slice", "residual", "pair"])
+def test_convolutions_of_few_pixels(shape, math, output):
+    """Against 64 bits with the filters as the pack holds them, whose every product is rounded only as the sum is: by
+    itself, into a slice of a wider tensor, with a residual operand, as two convolutions in one."""
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    N, H, W, ci, K, k, s, pd, d = shape
+    mode = getattr(ops, math)
+    g = torch.Generator(device="cuda").manual_seed(ci + K)
+    x = torch.zeros((N, H, W, ops.up4(ci)), device="cuda")
+    x[..., :ci] = torch.randn((N, H, W, ci), generator=g, device="cuda")
+    filters = [torch.randn((n, ci, k, k), generator=g, device="cuda") for n in ((K, 5) if output == "pair" else (K,))]
+    biases = [torch.randn(w.shape[0], generator=g, device="cuda") for w in filters]
+    p = ops.conv_params(N, H, W, ci, K, k, s, pd, d, 1, True, ops.ACT_RELU, 0.0, 0.0, mode)
+    pixels = (N, p.out_hwc[0], p.out_hwc[1])
+    res = torch.randn(pixels + (ops.up4(K),), generator=g, device="cuda")
+    if output == "pair":
+        gots = ops.conv2d_pair(x, filters[0], biases[0], filters[1], biases[1], N, H, W, ci, k, s, pd, d, ops.ACT_RELU, math_mode=mode)
+    elif output == "residual":
+        gots = [ops.conv2d_residual(p, x, ops.conv2d_prepack(p, filters[0]), biases[0], res)]
+    elif output == "slice":
+        p.out_channel_offset, p.out_channel_stride = 8, ops.up4(K) + 12
+        wide = torch.full(pixels + (ops.up4(K) + 12,), 7.0, device="cuda")
+        packed = ops.conv2d_prepack(p, filters[0])
+        _lib.check(_lib.cuda_lib().ogle_cuda_conv2d(C.byref(p), ops._p(x), ops._p(packed), ops._p(biases[0]), ops._p(wide), ops._stream()), "conv2d")
+        assert (wide[..., :8] == 7).all() and (wide[..., 8 + ops.up4(K):] == 7).all()
+        gots = [wide[..., 8:8 + ops.up4(K)]]
+    else:
+        gots = [ops.conv2d(p, x, ops.conv2d_prepack(p, filters[0]), biases[0])]
+    assert ops.last_contraction().form == 8
+    x64 = x[..., :ci].permute(0, 3, 1, 2).double()
+    conv = lambda u, v: torch.nn.functional.conv2d(u, v, None, s, pd, d).permute(0, 2, 3, 1)
+    for got, w, b in zip(gots, filters, biases):
+        hi = (w.view(torch.int32) & ~0x1fff).view(torch.float32)
+        held = hi.double() + ((w - hi).bfloat16().double() if mode == ops.MATH_TF32X3 else 0.0)
+        other = b.double() + (res[..., :K].double() if output == "residual" else 0.0)
+        want = (conv(x64, held) + other).clamp(min=0)
+        # every partial sum rounded once: at most (terms) * 2^-24 of the sum of the terms' magnitudes
+        bound = (k * k * ci + 8) * 2.0 ** -24 * (conv(x64.abs(), held.abs()) + b.abs().double() + (res[..., :K].abs().double() if output == "residual" else 0.0))
+        n = w.shape[0]
+        assert ((got[..., :n].double() - want).abs() <= bound).all()
+        assert (got[..., n:ops.up4(n)] == 0).all()
 
 
 @pytest.mark.parametrize("name,value", [("OGLE_TC_PAIR", "1"), ("OGLE_TC_PAIR", "0"), ("OGLE_TC_BN", "64"), ("OGLE_TC_BN", "192")])
