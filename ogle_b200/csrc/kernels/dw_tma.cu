@@ -3,8 +3,8 @@
 //
 // One block per SM slot walks a list of tiles. A tile is th x tw output pixels of
 // one image for a slab of 32 channels (16 where 32 would leave much of the last slab
-// empty; channels past the tensor arrive as zeros and are not stored); tw is the map's width up to 16, half of it up to
-// 32 (19 is 10 + 9), a third up to 48, else 32 or, at stride 2, 16. Its input window, halo included, is ONE TMA box
+// empty; channels past the tensor arrive as zeros and are not stored), chosen by an estimate
+// (choose_shape). Its input window, halo included, is ONE TMA box
 // [IH rows][IW cols][channels of the slab]; pixels outside the image arrive as zeros,
 // which is the convolution's padding. A ring of two to four shared-memory stages: while
 // the block computes tile i from one stage, the TMA engine fills the others with the next tiles, so
@@ -15,7 +15,8 @@
 // shared-memory reads are conflict-free (slabs of 16 at stride 2 are not: two wavefronts).
 // The 32 pixel slots of a block (64 with slabs of 16) are split into row groups of tw.
 // Widths that are no multiple of 32 channels, and 5x5 windows, ran on kernels that fetch every
-// tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 25 us here (16 us floor).
+// tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 22 us here (16 us floor).
+#include <cmath>
 #include <cstdlib>
 
 #include "tc_common.cuh"
@@ -226,12 +227,69 @@ int slab_quads(const ConvArgs& a) {
     return 6 * full <= 7 * half ? 8 : 4;
 }
 
-// Tile shape for a map: full-width tiles when the map is at most 16 wide, equal parts up to 48; the rows per
-// thread (one of the compiled RPG values) that leaves the fewest idle output rows.
+// Whether tiles of th x tw pixels leave room for two stages; t's shape and stages.
+bool fit_tile(const ConvArgs& a, int quads, int tw, int rpg, DwTiles* t) {
+    const int S = a.stride, KS = a.kernel, groups = 256 / quads / tw, th = rpg * groups;
+    const int iw = (tw - 1) * S + KS, ih = (th - 1) * S + KS;
+    if (iw > 256 || ih > 256) return false;
+    const size_t tile = ((size_t)ih * iw * quads * 16 + 127) / 128 * 128;
+    if (2 * tile + 128 > (size_t)kDwSmemMax) return false;
+    t->tw = tw; t->th = th; t->row_groups = groups; t->iw = iw; t->ih = ih;
+    // as many tiles in flight as fit: HBM latency x bandwidth needs ~90 KB per SM
+    const int st = (int)((size_t)(kDwSmemMax - 128) / tile);
+    t->stages = st > kDwMaxStages ? kDwMaxStages : st;
+    return true;
+}
+
+// Tile shape at stride 1: equal parts of the map's width, or one of a few widths that fill a block's pixel slots, and the
+// rows a thread computes, by an estimate of the time: rounds of tiles over the resident blocks, of which each takes a fixed
+// time, its rows' multiply-adds and its copies, partly beside one another; or the time at the HBM rate, which rings of fewer
+// than four stages do not reach. Fitted to 60 layers, 4 us to 170, with every width and row count timed: 5 % faster on
+// average than choose_shape_by_rows, 3 % off the best; 16 x 75 x 75 x 144
+// 24.3 -> 22.4 us (tiles of 15 keep 30 of 32 slots busy where 32, 32 and 11 kept 25), 64 x 75 x 75 x 128 64 -> 59,
+// 22 x 83 x 99 x 345 101 -> 86.
+int choose_shape_stride1(const ConvArgs& a, int quads, DwTiles* t) {
+    static const int kRows3[] = {10, 8, 7, 5, 4, 2}, kRows5[] = {4, 2};
+    const int* rows = a.kernel == 5 ? kRows5 : kRows3;
+    const int nrows = a.kernel == 5 ? 2 : 6;
+    const int slab = quads * 4, cblocks = (a.Kp + slab - 1) / slab;
+    int resident = kNumSMs * (a.kernel == 3 ? 2 : 1);
+    if (cblocks <= resident) resident -= resident % cblocks;
+    const double hbm = 8.0 * a.N * a.Ho * a.Wo * a.Kp / 6.0e6;
+    const char* env_tw = getenv("OGLE_DW_TW");
+    const char* env_rows = getenv("OGLE_DW_RPG");
+    const int force_rows = env_rows ? atoi(env_rows) : 0;
+    int best = 0;
+    double best_us = 0.0;
+    auto consider = [&](int tw) {
+        for (int i = 0; i < nrows; ++i) {
+            DwTiles s;
+            if ((force_rows && rows[i] != force_rows) || !fit_tile(a, quads, tw, rows[i], &s)) continue;
+            const double tiles = (double)((a.Wo + tw - 1) / tw) * ((a.Ho + s.th - 1) / s.th) * cblocks * a.N;
+            const double rounds = ceil(tiles / resident);
+            const double compute = 1.47 + 0.088 * rows[i] * (a.kernel == 3 ? 1.0 : 3.8), copy = 0.0023 * s.ih * s.iw * quads / 8;
+            const double work = rounds * (compute > copy ? compute + 0.37 * copy : copy + 0.37 * compute);
+            const double memory = s.stages < 4 ? 1.24 * hbm : hbm;
+            const double us = work > memory ? work + 0.33 * memory : memory + 0.33 * work;
+            if (!best || us < best_us) { best = rows[i]; best_us = us; *t = s; }
+        }
+    };
+    if (env_tw && atoi(env_tw) >= 1 && atoi(env_tw) <= 32) {
+        consider(atoi(env_tw) < a.Wo ? atoi(env_tw) : a.Wo);
+        return best;
+    }
+    for (int tw = a.Wo < 32 ? a.Wo : 32; tw >= 5; --tw) {
+        const int parts = (a.Wo + tw - 1) / tw;
+        if ((a.Wo + parts - 1) / parts == tw || tw == 8 || tw == 10 || tw == 16 || tw == 32) consider(tw);
+    }
+    return best;
+}
+
+// Tile shape at stride 2, and of large tensors: full-width tiles when the map is at most 16 wide, equal parts up to 48, else
+// 32 or, at stride 2, 16 pixels; the rows per thread (one of the compiled RPG values) that leaves the fewest idle output rows.
 // Returns the chosen RPG, or 0 when no shape fits two stages in kDwSmemMax.
-int choose_shape(const ConvArgs& a, DwTiles* t) {
-    const int S = a.stride, KS = a.kernel, CB = slab_quads(a);
-    const int slots = 256 / CB;                      // output pixels a block computes at once
+int choose_shape_by_rows(const ConvArgs& a, int quads, DwTiles* t) {
+    const int S = a.stride, KS = a.kernel;
     int tw = a.Wo <= 32 ? a.Wo : (S == 1 ? 32 : 16);
     // Widths that would leave many of the 32 pixel slots of a block idle are cut into equal parts
     // (measured at batch 256: 19 -> 2 x 10 is 6 % faster, 38 -> 3 x 13 is 18 % faster than 32 + 6)
@@ -239,35 +297,52 @@ int choose_shape(const ConvArgs& a, DwTiles* t) {
     else if (a.Wo > 32 && a.Wo <= 48) tw = (a.Wo + 2) / 3;
     if (const char* e = getenv("OGLE_DW_TW")) { const int v = atoi(e); if (v >= 1 && v <= 32) tw = v < a.Wo ? v : a.Wo; }
     const int force_rpg = getenv("OGLE_DW_RPG") ? atoi(getenv("OGLE_DW_RPG")) : 0;
-    const int groups = slots / tw;
     static const int kRpg1[] = {10, 8, 7, 5, 4, 2}, kRpg2[] = {7, 5, 4, 2}, kRpg5[] = {4, 2};
     const int* cand = KS == 5 ? kRpg5 : (S == 1 ? kRpg1 : kRpg2);
     const int ncand = KS == 5 ? 2 : (S == 1 ? 6 : 4);
     int best = 0;
     long best_cost = -1;
     for (int i = 0; i < ncand; ++i) {
-        const int rpg = cand[i], th = rpg * groups;
-        if (force_rpg && rpg != force_rpg) continue;
-        const int iw = (tw - 1) * S + KS, ih = (th - 1) * S + KS;
-        if (iw > 256 || ih > 256) continue;
-        const size_t tile = ((size_t)ih * iw * CB * 16 + 127) / 128 * 128;
-        if (2 * tile + 128 > (size_t)kDwSmemMax) continue;
-        const long tiles_y = (a.Ho + th - 1) / th;
+        const int rpg = cand[i];
+        DwTiles s;
+        if ((force_rpg && rpg != force_rpg) || !fit_tile(a, quads, tw, rpg, &s)) continue;
+        const long tiles_y = (a.Ho + s.th - 1) / s.th;
         // rows computed (idle ones included) plus a charge per tile for its halo rows
-        long cost = tiles_y * (th * S + KS - 1);
+        long cost = tiles_y * (s.th * S + KS - 1);
         // a single channel slab: neighbouring blocks then work on neighbouring
         // tiles of the same rows, and a ring of three shallower tiles measured 20 % faster
         // than two deep ones on the 150x150 map
-        if (a.Kp <= CB * 4 && 3 * tile + 128 > (size_t)kDwSmemMax) cost *= 2;
-        if (best_cost < 0 || cost < best_cost) {
-            best_cost = cost; best = rpg;
-            t->tw = tw; t->th = th; t->row_groups = groups; t->iw = iw; t->ih = ih;
-            // as many tiles in flight as fit: HBM latency x bandwidth needs ~90 KB per SM
-            int st = (int)((size_t)(kDwSmemMax - 128) / tile);
-            t->stages = st > kDwMaxStages ? kDwMaxStages : st;
-        }
+        if (a.Kp <= quads * 4 && s.stages < 3) cost *= 2;
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = rpg; *t = s; }
     }
     return best;
+}
+
+// The shape for a layer, and the rows a thread computes (0: none fits). The last few layers' are kept, by their sizes:
+// to weigh some eighty shapes takes as long as the launch.
+int choose_shape(const ConvArgs& a, DwTiles* t) {
+    struct Known { int N, H, W, Kp, K, kernel, stride, pad, rows; DwTiles t; };
+    static thread_local Known known[8];
+    static thread_local int next = 0;
+    const bool forced = getenv("OGLE_DW_TW") || getenv("OGLE_DW_RPG");
+    if (!forced)
+        for (const Known& k : known)
+            if (k.kernel == a.kernel && k.stride == a.stride && k.pad == a.pad && k.N == a.N && k.H == a.H && k.W == a.W && k.Kp == a.Kp && k.K == a.K) {
+                *t = k.t;
+                return k.rows;
+            }
+    const int quads = slab_quads(a);
+    // Tensors that do not stay in L2 are bound by HBM, by what the estimate does not see (256 x 38 x 38 x 256: 127 us in
+    // parts of 13, 146 in what it takes), unless tiles of 32 hang far over the map's edge (27 x 127 x 70 x 160 56 -> 52).
+    int rows = choose_shape_by_rows(a, quads, t);
+    const bool large = 8.0 * a.N * a.Ho * a.Wo * a.Kp > 160e6;
+    if (a.stride == 1 && !(rows && large && (double)a.Wo * a.Ho >= 0.72 * (double)(((a.Wo + t->tw - 1) / t->tw) * t->tw) *
+                                                                  (((a.Ho + t->th - 1) / t->th) * t->th)))
+        rows = choose_shape_stride1(a, quads, t);
+    if (forced) return rows;
+    known[next] = {a.N, a.H, a.W, a.Kp, a.K, a.kernel, a.stride, a.pad, rows, *t};
+    next = (next + 1) & 7;
+    return rows;
 }
 
 }  // namespace

@@ -29,6 +29,19 @@ def test_depthwise_any_width(oracle_port, channels, kernel, stride, size):
     close(run_case_cuda(case), oracle_port.conv2d(x, w, b, stride, kernel // 2, 1, channels, 1, 0.5, 6.0))
 
 
+@pytest.mark.parametrize("size", [(75, 75), (31, 66), (17, 99), (9, 151), (150, 12), (4, 127), (33, 8)])
+@pytest.mark.parametrize("images,channels,kernel", [(1, 40, 3), (12, 64, 3), (3, 20, 5)])
+def test_depthwise_tile_shapes(oracle_port, size, images, channels, kernel):
+    """Stride 1: parts of the width from 5 to 32 pixels, every row count, tiles that hang over the right and lower edges."""
+    from gpu_ops import run_case_cuda
+    rng = np.random.default_rng(size[1] + channels)
+    x = rng.standard_normal((images,) + size + (channels,), dtype=np.float32)
+    w = rng.standard_normal((channels, 1, kernel, kernel), dtype=np.float32) * np.float32(0.3)
+    b = rng.standard_normal(channels, dtype=np.float32)
+    case = dict(op="conv2d", x=x, w=w, bias=b, stride=1, pad=kernel // 2, dilation=1, group=channels, act=2, lo=0.0, hi=6.0)
+    close(run_case_cuda(case), oracle_port.conv2d(x, w, b, 1, kernel // 2, 1, channels, 2, 0.0, 6.0))
+
+
 @pytest.mark.parametrize("channels", [1, 6, 12, 20, 129, 1028])
 def test_batchnorm_any_width_is_exact(oracle_port, channels):
     from gpu_ops import run_case_cuda
