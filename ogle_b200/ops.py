@@ -35,6 +35,10 @@ def last_contraction():
     return out
 
 
+# Results are made by new_empty(sizes...) of an fp32 input: 1.3 us of a thread that issues small calls back to back, where
+# torch.empty(shape, dtype, device) takes 2.4 (one product of a row with a packed B: 9.2 us -> 8.0 in all).
+
+
 def up4(v):
     return (v + 3) // 4 * 4
 
@@ -111,7 +115,7 @@ def conv2d(p, x4, packed, bias=None, out=None, workspace="auto"):
     ks = p.out_channel_stride or up4(K)
     if out is None:
         out = torch.zeros((p.N, Ho, Wo, ks), dtype=torch.float32, device="cuda") if ks != up4(K) else \
-            torch.empty((p.N, Ho, Wo, ks), dtype=torch.float32, device="cuda")
+            x4.new_empty(p.N, Ho, Wo, ks)
     if isinstance(workspace, str):
         workspace = conv_workspace(p)
     check(_lib.cuda_lib().ogle_cuda_conv2d_ws(C.byref(p), _p(x4), _p(packed), _p(bias), _p(out), _p(workspace),
@@ -124,7 +128,7 @@ def conv2d_residual(p, x4, packed, bias, residual4, out=None):
     _require_cuda(x4, packed, bias, residual4)
     Ho, Wo, K = p.out_hwc
     if out is None:
-        out = torch.empty((p.N, Ho, Wo, up4(K)), dtype=torch.float32, device="cuda")
+        out = x4.new_empty(p.N, Ho, Wo, up4(K))
     check(_lib.cuda_lib().ogle_cuda_conv2d_residual(C.byref(p), _p(x4), _p(packed), _p(bias), _p(residual4),
                                                     residual4.shape[-1], _p(out), _stream()), "conv2d_residual")
     return out
@@ -172,7 +176,7 @@ def pool_params(N, H, W, Cc, kernel, stride, pad, type_):
 def pool(p, x4):
     _require_cuda(x4)
     Ho, Wo, Cc = p.out_hwc
-    out = torch.empty((p.N, Ho, Wo, up4(Cc)), dtype=torch.float32, device="cuda")
+    out = x4.new_empty(p.N, Ho, Wo, up4(Cc))
     check(_lib.cuda_lib().ogle_cuda_pool(C.byref(p), _p(x4), _p(out), _stream()), "pool")
     return out
 
@@ -220,7 +224,7 @@ def gemm(A4, B4, C4, M, K, N, transB=0, alpha=1.0, beta=1.0, bias_mode=0, math_m
     p.ldc = C4.shape[-1] if (C4 is not None and bias_mode == 1) else 0
     p.ldy = up4(N)
     p.math_mode = math_mode
-    out = torch.empty((M, up4(N)), dtype=torch.float32, device="cuda")
+    out = A4.new_empty(M, up4(N))
     check(_lib.cuda_lib().ogle_cuda_gemm(C.byref(p), _p(A4), _p(B4), _p(C4), _p(out), _stream()), "gemm")
     return out
 
@@ -251,7 +255,7 @@ def gemm_packed(A4, packed_b, C4, M, K, N, transB=0, alpha=1.0, beta=1.0, bias_m
     _require_cuda(A4, packed_b, C4)
     p = _gemm_params(A4, A4, C4, M, K, N, transB, alpha, beta, bias_mode, math_mode)
     p.ldb = 0
-    out = torch.empty((M, up4(N)), dtype=torch.float32, device="cuda")
+    out = A4.new_empty(M, up4(N))
     check(_lib.cuda_lib().ogle_cuda_gemm_packed(C.byref(p), _p(A4), _p(packed_b), _p(C4), _p(out), _stream()), "gemm_packed")
     return out
 
@@ -262,8 +266,8 @@ def gemm_ws(A4, B4, C4, M, K, N, transB=0, alpha=1.0, beta=1.0, bias_mode=0, mat
     p = _gemm_params(A4, B4, C4, M, K, N, transB, alpha, beta, bias_mode, math_mode)
     lib = _lib.cuda_lib()
     if workspace is None:
-        workspace = torch.empty(lib.ogle_cuda_gemm_packed_b_bytes(C.byref(p)) // 4, dtype=torch.float32, device="cuda")
-    out = torch.empty((M, up4(N)), dtype=torch.float32, device="cuda")
+        workspace = A4.new_empty(lib.ogle_cuda_gemm_packed_b_bytes(C.byref(p)) // 4)
+    out = A4.new_empty(M, up4(N))
     check(lib.ogle_cuda_gemm_ws(C.byref(p), _p(A4), _p(B4), _p(C4), _p(out), _p(workspace), workspace.numel() * 4,
                                 _stream()), "gemm_ws")
     return out
@@ -290,7 +294,7 @@ def concat(xs4, shapes, axis):
     out_shape[axis] = sum(s[axis] for s in shapes)
     for i, s in enumerate(shapes):
         p.in_shapes[i][:] = [1] * (4 - rank) + list(s)
-    out = torch.empty(out_shape[:-1] + [up4(out_shape[-1])], dtype=torch.float32, device="cuda")
+    out = xs4[0].new_empty(*out_shape[:-1], up4(out_shape[-1]), dtype=torch.float32)
     ptrs = (C.c_void_p * len(xs4))(*[x.data_ptr() for x in xs4])
     check(_lib.cuda_lib().ogle_cuda_concat(C.byref(p), ptrs, _p(out), _stream()), "concat")
     return out, out_shape
@@ -316,7 +320,7 @@ def reshape(x4, in_shape, out_shape):
 def nchw_to_nhwc4(x_nchw):
     _require_cuda(x_nchw)
     N, Cc, H, W = x_nchw.shape
-    out = torch.empty((N, H, W, up4(Cc)), dtype=torch.float32, device="cuda")
+    out = x_nchw.new_empty(N, H, W, up4(Cc))
     check(_lib.cuda_lib().ogle_cuda_nchw_to_nhwc4(_p(x_nchw), _p(out), N, Cc, H, W, _stream()), "nchw_to_nhwc4")
     return out
 
@@ -373,14 +377,13 @@ def ssd_detect(logits, boxes, num_classes, mode, score_thr, top_k, nms_thr=0.0, 
     p.N, p.A, p.C, p.logit_stride, p.mode = N, A, num_classes, ls, mode
     p.score_thr, p.top_k, p.nms_thr, p.image_w, p.image_h = score_thr, top_k, nms_thr, image_w, image_h
     rows = top_k if mode == 0 else (num_classes - 1) * top_k
-    score = torch.empty((N, rows), dtype=torch.float32, device="cuda")
-    anchor = torch.empty((N, rows), dtype=torch.int32, device="cuda")
-    cls = torch.empty((N, rows), dtype=torch.int32, device="cuda")
-    box = torch.empty((N, rows, 4), dtype=torch.float32, device="cuda")
-    count = torch.empty((N,) if mode == 0 else (N, num_classes - 1), dtype=torch.int32, device="cuda")
-    check(_lib.cuda_lib().ogle_cuda_ssd_detect(C.byref(p), _p(logits), _p(boxes), _p(score),
-                                               C.c_void_p(anchor.data_ptr()), C.c_void_p(cls.data_ptr()),
-                                               _p(box), C.c_void_p(count.data_ptr()), _stream()), "ssd_detect")
+    score = logits.new_empty(N, rows)
+    anchor = logits.new_empty(N, rows, dtype=torch.int32)
+    cls = torch.empty_like(anchor)
+    box = logits.new_empty(N, rows, 4)
+    count = anchor.new_empty(N) if mode == 0 else anchor.new_empty(N, num_classes - 1)
+    check(_lib.cuda_lib().ogle_cuda_ssd_detect(C.byref(p), _p(logits), _p(boxes), _p(score), _p(anchor), _p(cls), _p(box),
+                                               _p(count), _stream()), "ssd_detect")
     return score, anchor, cls, box, count
 
 
