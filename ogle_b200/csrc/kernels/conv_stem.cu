@@ -6,14 +6,22 @@
 //
 //  * persistent blocks walk a list of tiles (rows x columns of one image); the input
 //    window of a tile, halo included, is ONE TMA box of 16-byte pixels whose out-of-image
-//    part arrives as zeros (the padding); two stages, so the next tile loads while this
-//    one is computed;
+//    part arrives as zeros (the padding); three stages, each filled again by the last warp
+//    that is through with it, so that no warp waits for another: one's loads and stores fall
+//    into another's multiply-adds (with a barrier a tile: 285 us where this takes 262);
 //  * a warp owns a run of PL*PXT output pixels of one row, PL = 32 / (K/8) pixel lanes x
-//    K/8 channel groups: a thread accumulates PXT pixels (interleaved across the lanes,
-//    which makes the shared-memory reads conflict-free) x 8 channels in registers;
-//  * per filter tap the thread reads its 8x3 weights once (128-bit shared loads) and one
-//    float4 per pixel: about one load per eleven multiply-adds, no bounds checks and no
-//    address arithmetic in the inner loop.
+//    K/8 channel groups: a thread accumulates PXT pixels x 8 channels in registers. The
+//    eight are two fours K/2 apart: the channel groups of a pixel write whole 32-byte
+//    sectors (as eight in a row each store wrote half of one: 314 us -> 294 at 32 channels,
+//    125 -> 100 at 64);
+//  * per filter tap the thread reads its 8x3 weights once (128-bit shared loads). Its
+//    pixels lie side by side where that costs no bank conflicts, so that a row of the
+//    window is read once for the three taps across it (294 -> 285): 87 shared loads to 540
+//    two-wide multiply-adds, no bounds checks and no address arithmetic in the inner loop.
+//
+// Times are of 256 images of 300 x 300, 3 -> 32 channels, stride 2: 314 us -> 262, of which HBM
+// wants 169 and the fp32 pipes 147 (53 % busy at 285 us). Smaller tiles for few images gain under
+// 1 us (8 images 13.1) and lose 4 % and more from 16 images on.
 #include "tc_common.cuh"
 #include "tma_host.h"
 
@@ -49,17 +57,29 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return d;
 }
 
+// One more warp has finished reading; how many had before it. Its reads come before, the caller's copies behind.
+__device__ __forceinline__ unsigned through(unsigned* count) {
+    unsigned old;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(count)) : "memory");
+    return old;
+}
+
 // KP: the padded output channel count when it is known at compile time (32, the usual stem), so that
-// every shared-memory offset inside the tap loops is an immediate; 0 = read it from the arguments.
+// every shared-memory offset inside the tap loops is an immediate (64: 343 us -> 316, 64 images of 224 x 224);
+// 0 = read it from the arguments.
 template <int S, int PXT, int CIN, int KP>
 __global__ void __launch_bounds__(256, 2)
 conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __restrict__ w, const float* __restrict__ bias,
                       float* __restrict__ y, const ConvArgs a, const StemTiles tl, int* err_flag) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kStemStages];
-    // weights [9][CIN][Kp] + bias [Kp], then the two input stages (128-byte aligned)
+    __shared__ unsigned s_done[kStemStages];         // warps that are through with a stage
+    // weights [9][CIN][Kp] + bias [Kp], then the input stages (128-byte aligned)
     float* s_w = reinterpret_cast<float*>(smem_raw);
     const int Kp = KP ? KP : a.Kp;
+    // A thread's pixels side by side: five of them (an odd number of 16-byte pixels, or of pairs, between lanes), or four at
+    // stride 1 with at most eight lanes across. Four at stride 2 put lanes 128 bytes apart: 32 images of 256 x 256 34.3 -> 40.1.
+    constexpr bool kRun = PXT % 2 != 0 || (S == 1 && KP >= 32);
     const int kgroups = KP ? KP / 8 : tl.kgroups;
     const int pls = KP ? 32 / (KP / 8) : tl.pl;           // pixel lanes per warp
     const int wn = 9 * CIN * Kp;
@@ -71,22 +91,10 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
 
     grid_dependency_trigger();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStemStages; ++i) mbar_init(&bar_full[i], 1);
+        for (int i = 0; i < kStemStages; ++i) { mbar_init(&bar_full[i], 1); s_done[i] = 0; }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     grid_dependency_wait();         // nothing from global memory before this point
-    for (int i = threadIdx.x; i < wn; i += blockDim.x) {
-        const int k = i % Kp, c = (i / Kp) % CIN, tap = i / (Kp * CIN);
-        s_w[i] = c < a.C ? w[(tap * a.Cp + c) * Kp + k] : 0.f;     // tap-major packed filter
-    }
-    for (int i = threadIdx.x; i < Kp; i += blockDim.x) s_w[wn + i] = (a.has_bias && i < a.K) ? bias[i] : 0.f;
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kg = lane % kgroups, pl = lane / kgroups;
-    const int seg = warp % tl.segs, row = warp / tl.segs;
-    const bool active = row < tl.rows;
-    const float* wk = s_w + kg * 8;
     const int tile_px = tl.segs * tl.seg_px;        // output columns per tile
 
     // tile index -> (column tile, row tile, image), 32-bit (a 64-bit division costs as much as
@@ -99,32 +107,38 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
         tma_load_4d(base + (uint32_t)stage * stage_pitch, &tmX, &bar_full[stage], 0, (int)tx * tile_px * S - a.pad,
                     (int)ty * tl.rows * S - a.pad, (int)n);
     };
-
     const uint32_t total = (uint32_t)tl.total;
-    const bool full_k = kg * 8 + 8 <= a.K;           // every lane of this thread's eight is a real channel
-    // ring of kStemStages input tiles: the tiles of the next kStemStages - 1 rounds are in flight
-    // while one is being used
+    // ring of kStemStages input tiles: those of the next rounds are in flight while one is being used
     if (threadIdx.x == 0)
-        for (int i = 0; i < kStemStages - 1; ++i)
+        for (int i = 0; i < kStemStages; ++i)
             if (blockIdx.x + (uint32_t)i * gridDim.x < total) issue(blockIdx.x + (uint32_t)i * gridDim.x, i);
-    uint32_t it = 0;
+    for (int i = threadIdx.x; i < wn; i += blockDim.x) {
+        const int k = i % Kp, c = (i / Kp) % CIN, tap = i / (Kp * CIN);
+        s_w[i] = c < a.C ? w[(tap * a.Cp + c) * Kp + k] : 0.f;     // tap-major packed filter
+    }
+    for (int i = threadIdx.x; i < Kp; i += blockDim.x) s_w[wn + i] = (a.has_bias && i < a.K) ? bias[i] : 0.f;
+    __syncthreads();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kg = lane % kgroups, pl = lane / kgroups;
+    const int seg = warp % tl.segs, row = warp / tl.segs;
+    const bool active = row < tl.rows;
+    const float* wk = s_w + kg * 4;
+    const int half = Kp / 2;
+    const bool full_k = half + kg * 4 + 4 <= a.K;    // every lane of this thread's eight is a real channel
+    // a rectified value is one clipped to [0, inf)
+    const float lo = a.act == OGLE_ACT_CLIP ? a.lo : 0.f, hi = a.act == OGLE_ACT_CLIP ? a.hi : INFINITY;
+    const int pitch = (kRun ? 1 : pls) * a.Ks;
     int stage = 0;
     uint32_t phase = 0;
-    for (uint32_t tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
-        // the stage refilled here was last read by tile it-1, finished before the barrier at the loop's end
-        {
-            const uint32_t ahead = tile + (uint32_t)(kStemStages - 1) * gridDim.x;
-            int refill = stage + kStemStages - 1;
-            if (refill >= kStemStages) refill -= kStemStages;
-            if (threadIdx.x == 0 && ahead < total) issue(ahead, refill);
-        }
+    for (uint32_t tile = blockIdx.x; tile < total; tile += gridDim.x) {
         const uint32_t tq = tile / tiles_x;
         const int tx = (int)(tile - tq * tiles_x);
         const int n = (int)(tq / tiles_y);
         const int ty = (int)(tq - (uint32_t)n * tiles_y);
         if (!mbar_wait(&bar_full[stage], phase)) {
-            if (threadIdx.x == 0) record_error(err_flag, 8);
-            break;   // uniform: every thread waits on the same barrier with the same bound
+            if (lane == 0) record_error(err_flag, 8);
+            break;
         }
         if (active) {
             const float4* tile_s = stage0 + (size_t)stage * (stage_pitch / 16);
@@ -133,29 +147,46 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
             unsigned long long acc2[PXT][4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                const unsigned long long b = pack2(s_w[wn + kg * 8 + 2 * m], s_w[wn + kg * 8 + 2 * m + 1]);
+                const float* bk = wk + wn + (m >> 1) * half + (m & 1) * 2;
+                const unsigned long long b = pack2(bk[0], bk[1]);
 #pragma unroll
                 for (int i = 0; i < PXT; ++i) acc2[i][m] = b;
             }
-            const int lc = seg * tl.seg_px + pl;                      // first local output column of this thread
+            const int lc = seg * tl.seg_px + (kRun ? pl * PXT : pl);      // first local output column of this thread
             const float4* prow = tile_s + (size_t)(row * S) * tl.iw + lc * S;
-            const int step = pls * S;                                 // input columns between this thread's pixels
+            const int step = kRun ? S : pls * S;                          // input columns between this thread's pixels
 #pragma unroll
             for (int ky = 0; ky < 3; ++ky) {
+                float win[kRun ? (PXT - 1) * S + 3 : 1][CIN];
+                if (kRun) {
+#pragma unroll
+                    for (int j = 0; j < (PXT - 1) * S + 3; ++j) {
+                        const float4 q = prow[ky * tl.iw + j];
+                        const float u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int c = 0; c < CIN; ++c) win[j][c] = u[c];
+                    }
+                }
 #pragma unroll
                 for (int kx = 0; kx < 3; ++kx) {
                     unsigned long long f2[CIN][4];
 #pragma unroll
                     for (int c = 0; c < CIN; ++c) {
                         const ulonglong2 f0 = *reinterpret_cast<const ulonglong2*>(wk + ((ky * 3 + kx) * CIN + c) * Kp);
-                        const ulonglong2 f1 = *reinterpret_cast<const ulonglong2*>(wk + ((ky * 3 + kx) * CIN + c) * Kp + 4);
+                        const ulonglong2 f1 = *reinterpret_cast<const ulonglong2*>(wk + ((ky * 3 + kx) * CIN + c) * Kp + half);
                         f2[c][0] = f0.x; f2[c][1] = f0.y; f2[c][2] = f1.x; f2[c][3] = f1.y;
                     }
                     const float4* p = prow + ky * tl.iw + kx;
 #pragma unroll
                     for (int i = 0; i < PXT; ++i) {
-                        const float4 q = p[i * step];
-                        const float u[4] = {q.x, q.y, q.z, q.w};
+                        float u[4] = {};
+                        if (kRun) {
+#pragma unroll
+                            for (int c = 0; c < CIN; ++c) u[c] = win[kRun ? i * S + kx : 0][c];
+                        } else {
+                            const float4 q = p[i * step];
+                            u[0] = q.x; u[1] = q.y; u[2] = q.z; u[3] = q.w;
+                        }
 #pragma unroll
                         for (int c = 0; c < CIN; ++c) {
                             const unsigned long long uu = pack2(u[c], u[c]);
@@ -172,26 +203,37 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
                 for (int m = 0; m < 4; ++m) unpack2(acc2[i][m], acc[i][2 * m], acc[i][2 * m + 1]);
             const int oy = ty * tl.rows + row;
             if (oy < a.Ho) {
-                float* yrow = y + (((long)n * a.Ho + oy) * a.Wo) * a.Ks + a.koff + kg * 8;
+                float* dst = y + (((long)n * a.Ho + oy) * a.Wo + tx * tile_px + lc) * a.Ks + a.koff + kg * 4;
+                if (a.act != OGLE_ACT_NONE) {
 #pragma unroll
-                for (int i = 0; i < PXT; ++i) {
-                    const int ox = tx * tile_px + lc + i * pls;
-                    if (ox >= a.Wo) continue;
-                    float v[8];
+                    for (int i = 0; i < PXT; ++i)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = apply_act(acc[i][j], a.act, a.lo, a.hi);
-                    if (!full_k) {
+                        for (int j = 0; j < 8; ++j) acc[i][j] = fminf(fmaxf(acc[i][j], lo), hi);
+                }
+                if (!full_k) {
+#pragma unroll
+                    for (int i = 0; i < PXT; ++i)
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
-                            if (kg * 8 + j >= a.K) v[j] = 0.f;       // padded lanes stay zero
-                    }
-                    float* dst = yrow + (long)ox * a.Ks;
+                            if (kg * 4 + (j & 3) + (j >> 2) * half >= a.K) acc[i][j] = 0.f;       // padded lanes stay zero
+                }
+#pragma unroll
+                for (int i = 0; i < PXT; ++i, dst += pitch) {
+                    const int ox = tx * tile_px + lc + i * (kRun ? 1 : pls);
+                    if (ox >= a.Wo) continue;
+                    const float* v = acc[i];
                     *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-                    *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                    *reinterpret_cast<float4*>(dst + half) = make_float4(v[4], v[5], v[6], v[7]);
                 }
             }
         }
-        __syncthreads();
+        // the last warp to finish a tile has its stage filled again: no warp waits for another
+        __syncwarp();
+        if (lane == 0 && through(&s_done[stage]) == blockDim.x / 32 - 1) {
+            s_done[stage] = 0;
+            const uint32_t ahead = tile + (uint32_t)kStemStages * gridDim.x;
+            if (ahead < total) issue(ahead, stage);
+        }
         if (++stage == kStemStages) { stage = 0; phase ^= 1u; }
     }
 }
@@ -265,6 +307,10 @@ int launch_c(const ConvArgs& a, const StemTiles& tl, const float* x, const float
     if (a.Kp == 32) {
         if (a.C == 3) return launch<S, PXT, 3, 32>(a, tl, x, w, bias, y, s);
         return launch<S, PXT, 4, 32>(a, tl, x, w, bias, y, s);
+    }
+    if (a.Kp == 64) {
+        if (a.C == 3) return launch<S, PXT, 3, 64>(a, tl, x, w, bias, y, s);
+        return launch<S, PXT, 4, 64>(a, tl, x, w, bias, y, s);
     }
     if (a.C == 3) return launch<S, PXT, 3, 0>(a, tl, x, w, bias, y, s);
     return launch<S, PXT, 4, 0>(a, tl, x, w, bias, y, s);

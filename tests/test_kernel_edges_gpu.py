@@ -1099,6 +1099,38 @@ for N, H, C, K, k in ((1, 19, 512, 512, 1), (16, 38, 256, 512, 1), (4, 20, 64, 2
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, channels, K, stride: fewer tiles than stages, stages filled over and over, warps without a row, widths at which a
+    # thread has five pixels and four, both ends of the channel counts that are known at compile time and are not
+    (1, 9, 11, 3, 32, 2), (3, 3, 300, 3, 32, 1), (70, 90, 150, 3, 32, 2), (40, 64, 64, 4, 29, 1), (30, 64, 64, 3, 32, 2), (25, 112, 112, 3, 64, 2),
+    (9, 75, 61, 4, 62, 1), (6, 40, 64, 1, 64, 1), (12, 90, 250, 3, 16, 1), (5, 60, 200, 2, 7, 1), (2, 1, 500, 3, 64, 1)])
+def test_direct_stems_whose_warps_run_free(shape):
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    N, H, W, ch, K, s = shape
+    g = torch.Generator(device="cuda").manual_seed(W + K)
+    x = torch.zeros((N, H, W, 4), device="cuda")
+    x[..., :ch] = torch.randn((N, H, W, ch), generator=g, device="cuda")
+    w, b = torch.randn((K, ch, 3, 3), generator=g, device="cuda"), torch.randn(K, generator=g, device="cuda")
+
+    def conv64(x, w, b):
+        return torch.nn.functional.conv2d(x[..., :ch].permute(0, 3, 1, 2).double(), w.double(), b.double(), s, 1).permute(0, 2, 3, 1)
+
+    want, size = conv64(x, w, b), conv64(x.abs(), w.abs(), b.abs())
+    for act, clamp in ((ops.ACT_NONE, (None, None)), (ops.ACT_RELU, (0.0, None)), (ops.ACT_CLIP, (-1.0, 2.5))):
+        p = ops.conv_params(N, H, W, ch, K, 3, s, 1, 1, 1, True, act, -1.0, 2.5, ops.MATH_FP32, 0, ops.up4(K) + 8, 4)
+        assert _lib.cuda_lib().ogle_cuda_conv2d_kernel_name(C.byref(p)) == b"conv3x3_smallc_kernel"
+        out = torch.full((N, want.shape[1], want.shape[2], ops.up4(K) + 8), -7.0, device="cuda")
+        ops.conv2d(p, x, ops.conv2d_prepack(p, w), b, out, workspace=None)
+        ref = want if act == ops.ACT_NONE else want.clamp(*clamp)
+        # 9 * ch + 1 roundings of partial sums no larger than the sum of sizes
+        assert bool(((out[..., 4:4 + K].double() - ref).abs() <= (9 * ch + 1) * 2.0 ** -24 * size).all())
+        assert bool((out[..., :4] == -7.0).all()) and bool((out[..., 4 + ops.up4(K):] == -7.0).all())
+        assert bool((out[..., 4 + K:4 + ops.up4(K)] == 0.0).all())
+    assert _lib.cuda_lib().ogle_cuda_device_status() == 0
+
+
 @pytest.mark.parametrize("case", [
     # C, K, kernel, stride, group, math, size
     (64, 64, 3, 1, 64, 2, 40), (50, 50, 5, 2, 50, 2, 40), (64, 64, 3, 1, 64, 2, 3), (64, 64, 7, 1, 64, 2, 40), (64, 32, 3, 1, 4, 2, 40),
