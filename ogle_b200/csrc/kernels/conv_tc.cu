@@ -38,6 +38,9 @@ int launch_tc_pair(tc::TcArgs& t, const CUtensorMap& mA, const CUtensorMap& mBhi
                    const CUtensorMap& mY, const CUtensorMap& mY2, long m_tiles, const float* bias, int* err_flag,
                    cudaStream_t s);
 
+int launch_conv_window(const ConvArgs& a, int passes, bool row_tiles, const float* x, const float* w, const float* bias, float* y,
+                       const float* residual, int res_ld, cudaStream_t s);
+
 const int* tc_cluster_capacity();      // [k], 2 <= k <= 8: clusters of k blocks that can be resident at once
 
 __device__ int g_tc_error = 0;   // first error seen by any block (0 = none)
@@ -434,6 +437,25 @@ static bool few_rows(const ConvArgs& a) {
     return (a.M <= 32 && products <= 1.5e6) || (a.M <= 8 && products <= 3e6);
 }
 
+// Whether a stem of 5 x 5 or 7 x 7 filters takes its windows as they are (conv_window.cu): one tile of channels, and maps that
+// its tiles of 8 x 16 pixels (or, at stride 1, 128 x 1) cover about as well as the gather form's best shape. In graphs, 7 x 7 / 2, 3 -> 64 channels, one
+// pass: 1 image of 224 x 224 8.2 us gathered, 7.2 so, 8 24.1 and 14.5, 128 279 and 135; split mode 32 images 69.3 and 62.1,
+// 128 257 and 226. With 49 channels and more and three values to gather it is no better up to eight rounds of tiles (1 image
+// 7.7 and 8.6, 8 20.9 and 21.0, 16 34.1 and 33.6), with fewer channels from the first on (3 x 200 x 120 -> 48 20.9 and 14.6).
+static double window_tiles(const ConvArgs& a, bool* row_tiles) {
+    const double tall = (double)((a.Wo + 7) / 8) * ((a.Ho + 15) / 16), flat = (double)((a.Wo + 127) / 128) * a.Ho;
+    *row_tiles = a.stride == 1 && flat < tall;
+    return *row_tiles ? flat : tall;
+}
+static bool window_form(const ConvArgs& a, int variant, bool split_mode) {
+    int tw, th;
+    bool row_tiles;
+    if (a.kernel == 3 || a.K > 64 || a.n_tile || !conv_tc_gather_supported(a, variant) || !gather_tile(a, true, &tw, &th)) return false;
+    const double gathered = (double)((a.Wo + tw - 1) / tw) * ((a.Ho + th - 1) / th), windows = window_tiles(a, &row_tiles);
+    if (split_mode && a.kernel == 7 && a.C == 3 && a.K > 48 && windows * a.N <= 8.0 * kNumSMs) return false;
+    return windows <= 1.3 * gathered && windows * a.N < 0x7fffffff - 2 * kNumSMs;
+}
+
 int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x, const float* w_hi,
                    const float* w_lo, const float* bias, float* y, cudaStream_t s, float* y2, int K1,
                    int split_col, void* ws, size_t ws_bytes, size_t* ws_needed, const float* residual, int res_ld) {
@@ -459,6 +481,13 @@ int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x
         r.alpha = 1.f; r.beta = 1.f; r.bias_mode = a.has_bias ? 2 : 0;
         r.act = a.act; r.lo_clip = a.lo; r.hi_clip = a.hi;
         return launch_few_rows(r, s);
+    }
+    if (!plan_only && !y2 && window_form(a, variant, math_mode == OGLE_MATH_TF32X3)) {
+        // (the tap-major section of the packed filter lies in front of the one that w_hi points to)
+        const float* taps_first = w_hi - filter_layout(a.K, a.C, a.kernel, 1, a.Cp).off_hi / sizeof(float);
+        bool row_tiles;
+        window_tiles(a, &row_tiles);
+        return launch_conv_window(a, math_mode == OGLE_MATH_TF32X3 ? 3 : 1, row_tiles, x, taps_first, bias, y, residual, res_ld, s);
     }
     // channel extents and row strides of the output tensor(s)
     const int kp_a = y2 ? up4(K1) : a.Kp, ks_a = y2 ? up4(K1) : a.Ks;

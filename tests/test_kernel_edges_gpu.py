@@ -1131,6 +1131,48 @@ def test_direct_stems_whose_warps_run_free(shape):
     assert _lib.cuda_lib().ogle_cuda_device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, W, channels, K, kernel, stride, padding: tiles that hang over both edges, fewer and more than a round of blocks, channel
+    # counts around a multiply's and a slab's width, paddings of either parity, tiles of a row
+    (1, 32, 32, 3, 16, 7, 2, 3), (9, 113, 75, 3, 17, 7, 2, 2), (2, 64, 60, 4, 48, 7, 1, 3), (40, 70, 70, 3, 40, 5, 1, 2), (3, 64, 80, 1, 64, 5, 2, 0),
+    (4, 61, 47, 2, 33, 5, 1, 1), (40, 120, 120, 3, 64, 7, 2, 3), (5, 47, 63, 1, 1, 7, 1, 0), (6, 90, 40, 4, 32, 5, 2, 1), (2, 77, 200, 2, 64, 7, 2, 3),
+    (9, 1, 300, 3, 50, 5, 1, 2), (4, 3, 1024, 4, 64, 7, 1, 3)])
+@pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
+def test_stems_whose_window_is_the_operand(shape, math):
+    """Against 64 bits, in a slice of a wider tensor, with a residual operand, beside an infinite pixel and with lanes behind
+    the channels that are not numbers."""
+    import torch
+    from ogle_b200 import _lib, ops
+    N, H, W, ch, K, k, s, pad = shape
+    g = torch.Generator(device="cuda").manual_seed(W + K)
+    x = torch.full((N, H, W, 4), float("nan"), device="cuda")
+    x[..., :ch] = torch.randn((N, H, W, ch), generator=g, device="cuda")
+    w, b = torch.randn((K, ch, k, k), generator=g, device="cuda") / (ch * k * k) ** 0.5, torch.randn(K, generator=g, device="cuda")
+    p = ops.conv_params(N, H, W, ch, K, k, s, pad, 1, 1, True, ops.ACT_CLIP, -0.5, 1.5, getattr(ops, math), 0, ops.up4(K) + 8, 4)
+    packed = ops.conv2d_prepack(p, w)
+    want = torch.nn.functional.conv2d(x[..., :ch].permute(0, 3, 1, 2).double(), w.double(), b.double(), s, pad).permute(0, 2, 3, 1)
+    # at most 196 products and sums of fp32 grade, or of operands with ten mantissa bits
+    bound = (3e-6 if math == "MATH_TF32X3" else 1e-3) * float(want.norm())
+    out = torch.full(want.shape[:3] + (ops.up4(K) + 8,), -7.0, device="cuda")
+    ops.conv2d(p, x, packed, b, out, workspace=None)
+    assert ops.last_contraction().form == 7
+    assert float((out[..., 4:4 + K].double() - want.clamp(-0.5, 1.5)).norm()) <= bound
+    assert bool((out[..., :4] == -7.0).all()) and bool((out[..., 4 + ops.up4(K):] == -7.0).all())
+    assert bool((out[..., 4 + K:4 + ops.up4(K)] == 0.0).all())
+    p = ops.conv_params(N, H, W, ch, K, k, s, pad, 1, 1, True, ops.ACT_NONE, 0.0, 0.0, getattr(ops, math))
+    res = torch.randn(want.shape[:3] + (ops.up4(K),), generator=g, device="cuda")
+    plain, got = ops.conv2d(p, x, packed, b, workspace=None), ops.conv2d_residual(p, x, packed, b, res)
+    assert torch.equal(got[..., :K], plain[..., :K] + res[..., :K]) and bool((got[..., K:] == 0.0).all())
+    # an infinite pixel reaches the outputs whose windows hold it and no others
+    y0, x0 = H // 2, W // 2
+    x[0, y0, x0, 0] = float("inf")
+    hit = torch.nn.functional.conv2d((x[:, :, :, 0] == float("inf")).double()[:, None], torch.ones((1, 1, k, k), device="cuda").double(), None, s, pad)[:, 0] > 0
+    again = ops.conv2d(p, x, packed, b, workspace=None)
+    assert torch.equal(again[~hit], plain[~hit])
+    assert not bool(torch.isfinite(again[hit][:, :K]).any())
+    assert _lib.cuda_lib().ogle_cuda_device_status() == 0
+
+
 @pytest.mark.parametrize("case", [
     # C, K, kernel, stride, group, math, size
     (64, 64, 3, 1, 64, 2, 40), (50, 50, 5, 2, 50, 2, 40), (64, 64, 3, 1, 64, 2, 3), (64, 64, 7, 1, 64, 2, 40), (64, 32, 3, 1, 4, 2, 40),
