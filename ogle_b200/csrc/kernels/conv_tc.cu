@@ -428,11 +428,12 @@ splitk_reduce_kernel(const float4* __restrict__ ws, int slices, long slice_q, in
 // ws / ws_bytes: scratch for a split reduction of more than two ranges (or of a layer with an
 // activation), may be null. ws_needed != null: plan only - no tensor maps, no launch - and report the
 // scratch size this layer would like.
-// Whether a convolution has so few pixels that the CUDA cores are quicker (few_rows.cu), and the caller leaves that open:
+// Whether a convolution has so few pixels that the CUDA cores are quicker (few_rows.cu), and the caller leaves the ranges of
+// the reduction open (a tile width, pairs of SMs or channels on M say how tiles are laid out, and there are none):
 // a fixed 3 us instead of 6 to 8, but by the multiply-add (in graphs: 9 pixels, 256 -> 128 pointwise 6.4 -> 3.8 us, 4 pixels
 // of 3x3 256 -> 150 9.3 -> 4.6, 8 of them 9.5 -> 5.8; 16 pixels of 3x3 69 -> 271, 2.7 M products, 7.9 -> 8.5).
 static bool few_rows(const ConvArgs& a) {
-    if (a.n_tile || a.split || a.on_m || a.pair || filter_compact(a.C, a.kernel, 1)) return false;
+    if (a.split || filter_compact(a.C, a.kernel, 1)) return false;
     const double products = (double)a.M * a.K * a.kernel * a.kernel * a.C;
     return (a.M <= 32 && products <= 1.5e6) || (a.M <= 8 && products <= 3e6);
 }
@@ -450,7 +451,7 @@ static double window_tiles(const ConvArgs& a, bool* row_tiles) {
 static bool window_form(const ConvArgs& a, int variant, bool split_mode) {
     int tw, th;
     bool row_tiles;
-    if (a.kernel == 3 || a.K > 64 || a.n_tile || !conv_tc_gather_supported(a, variant) || !gather_tile(a, true, &tw, &th)) return false;
+    if (a.kernel == 3 || a.K > 64 || !conv_tc_gather_supported(a, variant) || !gather_tile(a, true, &tw, &th)) return false;
     const double gathered = (double)((a.Wo + tw - 1) / tw) * ((a.Ho + th - 1) / th), windows = window_tiles(a, &row_tiles);
     if (split_mode && a.kernel == 7 && a.C == 3 && a.K > 48 && windows * a.N <= 8.0 * kNumSMs) return false;
     return windows <= 1.3 * gathered && windows * a.N < 0x7fffffff - 2 * kNumSMs;

@@ -22,8 +22,8 @@
 // Large layers run at 46-47 TFLOP/s (3x3 256 -> 256 at 38 x 38 x 32 images: 1658 -> 1183 us); packed and scalar
 // multiply-adds measure within 5 % of each other there, so it is the FP32 pipe and its operand reads, not issue slots
 // or shared memory (42 % busy), that set the pace. At 8 images the gain is in filling the SMs: ResNet's 512-channel
-// 3x3 layers at 7 x 7 were 32 blocks (407 us, now 69), the 256-channel ones at 14 x 14 205 us, now 55; the network
-// 3010 -> 957 us.
+// 3x3 layers at 7 x 7 were 32 blocks (407 us, then 69), the 256-channel ones at 14 x 14 205 us, then 55; the network
+// 3010 -> 942 us, and 882 with conv_igemm_tma_kernel.
 #include "igemm.cuh"
 #include "tc_common.cuh"
 #include "tma_host.h"

@@ -264,7 +264,7 @@ public:
     // number of ranges its reduction is split into (which does change the order of the partial sums); then, for
     // an unsplit reduction, whether pairs of SMs should share the filter tiles (same bits again); last, channels on M (the
     // bits of that number of ranges, but for 3x3 layers whose taps would lie side by side). Launches of taps side by side
-    // are the same whatever width or pairing is asked for: those candidates are left out.
+    // are the same whatever width or pairing is asked for, those of few rows whatever width: those candidates are left out.
     void Tune() override {
         OgleConvParams& p = sibling_ ? pair_params_ : params_;
         if (!filter_is_constant_ || std::string(ogle_cuda_conv2d_kernel_name(&p)) != "conv_tc2_kernel") return;
@@ -285,10 +285,11 @@ public:
             if (cudaEventSynchronize(e1) != cudaSuccess) return false;
             return cudaEventElapsedTime(ms, e0, e1) == cudaSuccess;
         };
-        auto taps_side_by_side = [] {
+        auto ran_as = [](int form) {
             OgleContraction c;
-            return ogle_cuda_last_contraction(&c) == OGLE_OK && c.form == 6;
+            return ogle_cuda_last_contraction(&c) == OGLE_OK && c.form == form;
         };
+        auto taps_side_by_side = [&] { return ran_as(6); };
         float auto_ms = 0.f, best_ms = 0.f;
         p.n_tile = 0;
         p.split = 0;
@@ -297,8 +298,8 @@ public:
         if (time_it(&auto_ms)) {
             best_ms = auto_ms;
             int best_tile = 0, best_split = 0, best_pair = 0;
-            const bool beside = taps_side_by_side();
-            for (int bn = 32; !beside && bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
+            const bool beside = taps_side_by_side(), few_rows = ran_as(8);
+            for (int bn = 32; !beside && !few_rows && bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
                 float ms;
                 p.n_tile = bn;
                 if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_tile = bn; }

@@ -1047,6 +1047,11 @@ def test_convolutions_of_few_pixels(shape, math, output):
         gots = [wide[..., 8:8 + ops.up4(K)]]
     else:
         gots = [ops.conv2d(p, x, ops.conv2d_prepack(p, filters[0]), biases[0])]
+        # (no tiles: how they are to be laid out does not matter)
+        for name, value in (("n_tile", 32), ("sm_pair", 1), ("channels_on_m", 1)):
+            setattr(p, name, value)
+            assert torch.equal(ops.conv2d(p, x, ops.conv2d_prepack(p, filters[0]), biases[0]), gots[0])
+            setattr(p, name, 0)
     assert ops.last_contraction().form == 8
     x64 = x[..., :ci].permute(0, 3, 1, 2).double()
     conv = lambda u, v: torch.nn.functional.conv2d(u, v, None, s, pd, d).permute(0, 2, 3, 1)
@@ -1163,6 +1168,9 @@ def test_stems_whose_window_is_the_operand(shape, math):
     res = torch.randn(want.shape[:3] + (ops.up4(K),), generator=g, device="cuda")
     plain, got = ops.conv2d(p, x, packed, b, workspace=None), ops.conv2d_residual(p, x, packed, b, res)
     assert torch.equal(got[..., :K], plain[..., :K] + res[..., :K]) and bool((got[..., K:] == 0.0).all())
+    p.n_tile = 32
+    assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), plain)
+    p.n_tile = 0
     # an infinite pixel reaches the outputs whose windows hold it and no others
     y0, x0 = H // 2, W // 2
     x[0, y0, x0, 0] = float("inf")
