@@ -184,8 +184,8 @@ conv_window_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 else tma_load_4d(to, &tmX, &bar_raw_full[s], 0, x, y, n);
                 ++issued;
             }
-            if (!ok)                 // what is in flight lands before the block ends
-                for (int i = issued < 2 ? 0 : issued - 2; i < issued; ++i) (void)mbar_wait(&bar_raw_full[i & 1], (uint32_t)(i >> 1) & 1u);
+            // what is in flight lands before the block ends: others may have given up on it after the last was asked for
+            for (int i = issued < 2 ? 0 : issued - 2; i < issued; ++i) (void)mbar_wait(&bar_raw_full[i & 1], (uint32_t)(i >> 1) & 1u);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ multiplies

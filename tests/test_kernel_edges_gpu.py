@@ -850,7 +850,7 @@ def test_kept_filters_and_windows_of_rgb_stems(shape):
     assert torch.equal(ops.conv2d(p, x, packed, b, workspace=None), got)
 
 
-@pytest.mark.parametrize("form", ["whole", "whole, alternate tiles", "whole, residual", "taps", "taps, residual", "kept", "scratch", "cluster", "pairs",
+@pytest.mark.parametrize("form", ["whole", "whole, alternate tiles", "whole, residual", "taps", "taps, residual", "kept", "window", "scratch", "cluster", "pairs",
                                   "channels on M", "channels on M, turns"])
 @pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
 def test_waits_that_run_out_for_some(form, math):
@@ -862,6 +862,7 @@ def test_waits_that_run_out_for_some(form, math):
     # N, H, C, K, kernel, stride
     N, H, C, K, k, s = {"whole": (16, 40, 96, 160, 1, 1), "whole, alternate tiles": (64, 40, 32, 64, 1, 1), "whole, residual": (16, 40, 96, 160, 3, 2),
                         "taps": (64, 28, 64, 64, 3, 1), "taps, residual": (64, 28, 64, 32, 3, 1), "kept": (20, 112, 3, 64, 7, 2),
+                        "window": (20, 112, 2, 64, 7, 2),
                         "scratch": (8, 10, 512, 100, 3, 1), "cluster": (1, 19, 256, 256, 1, 1), "pairs": (16, 40, 96, 256, 1, 1),
                         "channels on M": (32, 28, 64, 64, 3, 1), "channels on M, turns": (32, 28, 64, 128, 3, 1)}[form]
     g = torch.Generator(device="cuda").manual_seed(K)

@@ -149,3 +149,53 @@ def test_no_epilogue_group_waits_for_warps_that_gave_up(name):
 
 def test_the_model_sees_warps_that_leave_by_themselves():
     assert _stuck(2, False)
+
+
+def _window_copies_waited_for():
+    """When the window kernel's copying thread waits, at its end, for the copies it has asked for."""
+    text = open(os.path.join(KERNELS, "conv_window.cu")).read()
+    role = text[text.index("-- copies"):text.index("-- multiplies")]
+    drain = re.search(r"(if \(!ok\)[^\n]*\n\s*)?for \(int i = issued[^\n]*mbar_wait\(&bar_raw_full", role)
+    return "never" if not drain else "when it gave up" if drain.group(1) else "always"
+
+
+def _lands_in_a_block_that_ended(tiles, stages, waits):
+    """Whether a copy can land after the block's roles have left. One role asks for a tile's copy once the tile a ring before
+    it has been read; the other reads tiles in order as they land. Each gives up wherever it waits, or goes on."""
+    start = (0, 0, 0, "runs", "runs")                     # asked for, landed, read, the copying role, the reading one
+    seen, todo = {start}, [start]
+    while todo:
+        asked, landed, read, copying, reading = todo.pop()
+        if copying == reading == "left" and landed < asked:
+            return True
+        nxt = []
+        if landed < asked:
+            nxt.append((asked, landed + 1, read, copying, reading))
+        if copying == "runs":
+            if asked == tiles:
+                nxt.append((asked, landed, read, "waits" if waits == "always" else "left", reading))
+            elif asked < read + stages:
+                nxt.append((asked + 1, landed, read, copying, reading))
+            else:
+                nxt.append((asked, landed, read, "left" if waits == "never" else "waits", reading))
+        if copying == "waits" and landed == asked:
+            nxt.append((asked, landed, read, "left", reading))
+        if reading == "runs":
+            if read < landed:
+                nxt.append((asked, landed, read + 1, copying, "runs" if read + 1 < tiles else "left"))
+            else:
+                nxt.append((asked, landed, read, copying, "left"))
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
+def test_no_window_lands_in_a_block_that_ended(tiles):
+    assert not _lands_in_a_block_that_ended(tiles, 2, _window_copies_waited_for())
+
+
+def test_the_model_sees_readers_that_give_up_alone():
+    assert _lands_in_a_block_that_ended(1, 2, "when it gave up")
