@@ -54,21 +54,6 @@ struct WindowArgs {
     uint32_t spin_limit;
 };
 
-__device__ __forceinline__ bool wait_turn(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit) {
-    const uint32_t addr = smem_u32(bar);
-    for (uint32_t spin = 0; spin < limit; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
-        if ((spin & 255u) == 255u && *abort_flag) return false;
-    }
-    return false;
-}
-
 // K-major operand of pieces of 8 rows x 16 bytes: `lead` bytes to the next piece along the reduction, `next8` to the next eight rows.
 __device__ __forceinline__ uint64_t plain_desc(uint32_t lead, uint32_t next8) {
     return (uint64_t)(lead >> 4) << 16 | (uint64_t)(next8 >> 4) << 32 | (uint64_t)1 << 46;

@@ -309,6 +309,7 @@ constexpr int kTmaBN = 64, kTmaTX = 4, kTmaK = 32, kTmaStages = 2;
 struct IgemmTile {
     int im2col;                      // 0: the rows of A follow one another
     int chunks, per_tap;             // steps of kTmaK reduction elements: all, and of one filter tap
+    uint32_t spin_limit;             // polls of a wait before it gives up
 };
 
 template <int TY>
@@ -319,6 +320,9 @@ conv_igemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     constexpr uint32_t kBytesA = BM * 128, kBytesB = kTmaK * BN * 4, kStage = kBytesA + kBytesB;
     extern __shared__ __align__(1024) unsigned char ring[];
     __shared__ __align__(8) uint64_t full[kTmaStages];
+    // the tile's first pixel; whether somebody gave up, and the step at which thread 0, which asks for the copies, did (here
+    // and not in its registers, which all are short of: eight of them went to the stack)
+    __shared__ int s_at[3], s_abort, s_stop;
     const int tid = threadIdx.x, tx = tid % kTmaTX, ty = tid / kTmaTX;
     const long m0 = (long)blockIdx.x * BM;
     const int n0 = blockIdx.y * BN, splits = gridDim.z, rank = blockIdx.z;
@@ -326,15 +330,17 @@ conv_igemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const uint32_t base = smem_addr(ring);
     if (tid == 0) {
         for (int i = 0; i < kTmaStages; ++i) tc::mbar_init(&full[i], 1);
+        s_abort = 0;
+        s_stop = count;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    int ax = 0, ay = 0, an = 0, ky = 0, kx = 0, cc = 0;       // thread 0: position of the tile's first pixel, next step
+    int ky = 0, kx = 0, cc = 0;                                // thread 0: next step
     if (tid == 0) {
-        const long line = m0 / a.Wo;
-        ax = (int)(m0 - line * a.Wo) * a.stride - a.pad;
-        an = (int)(line / a.Ho);
-        ay = (int)(line - (long)an * a.Ho) * a.stride - a.pad;
+        const long line = m0 / a.Wo, an = line / a.Ho;
+        s_at[0] = (int)(m0 - line * a.Wo) * a.stride - a.pad;
+        s_at[1] = (int)(line - an * a.Ho) * a.stride - a.pad;
+        s_at[2] = (int)an;
         const int tap = first / tl.per_tap;
         cc = first - tap * tl.per_tap;
         ky = tap / a.kernel;
@@ -343,7 +349,7 @@ conv_igemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     auto issue = [&](int stage) {
         const uint32_t to = base + (uint32_t)stage * kStage;
         tc::mbar_expect_tx(&full[stage], kStage);
-        if (tl.im2col) tc::tma_load_im2col(to, &tmA, &full[stage], cc * kTmaK, ax, ay, an, kx * a.dil, ky * a.dil);
+        if (tl.im2col) tc::tma_load_im2col(to, &tmA, &full[stage], cc * kTmaK, s_at[0], s_at[1], s_at[2], kx * a.dil, ky * a.dil);
         else tc::tma_load_2d(to, &tmA, &full[stage], cc * kTmaK, (int)m0);
         tc::tma_load_3d(to + kBytesA, &tmB, &full[stage], n0, cc * kTmaK, ky * a.kernel + kx);
         if (++cc == tl.per_tap) { cc = 0; if (++kx == a.kernel) { kx = 0; ++ky; } }
@@ -359,7 +365,12 @@ conv_igemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     int stage = 0;
     uint32_t phase = 0;
     for (int t = 0; t < count; ++t) {
-        if (came && !tc::mbar_wait(&full[stage], phase)) { came = false; tc::record_error(err_flag, 8); }
+        if (came && !tc::wait_turn(&full[stage], phase, &s_abort, tl.spin_limit)) {
+            came = false;                                      // (a thread that gives up goes on to the barriers all the same)
+            s_abort = 1;
+            if (tid == 0) s_stop = t;
+            tc::record_error(err_flag, 8);
+        }
         const float* sa = reinterpret_cast<const float*>(ring + stage * kStage) + ty * 32;
         const float* sb = reinterpret_cast<const float*>(ring + stage * kStage + kBytesA) + tx * 4;
 #pragma unroll
@@ -386,11 +397,11 @@ conv_igemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
         }
         __syncthreads();                                       // everyone is done with the stage
-        if (tid == 0 && t + kTmaStages < count) issue(stage);
+        if (tid == 0 && came && t + kTmaStages < count) issue(stage);
         if (++stage == kTmaStages) { stage = 0; phase ^= 1u; }
     }
-    if (!came && tid == 0)                                     // no copy may land in a block that has retired
-        for (int t = count > kTmaStages ? count - kTmaStages : 0; t < count; ++t)
+    if (tid == 0)                                              // no copy may land in a block that has retired
+        for (int t = s_stop; t < count && t < s_stop + kTmaStages; ++t)
             tc::mbar_wait(&full[t % kTmaStages], (uint32_t)(t / kTmaStages) & 1u);
 
     if (splits == 1) {
@@ -503,6 +514,7 @@ int launch_igemm_tma(const IgemmArgs& a, const TmaPlan& plan, cudaStream_t s) {
     tl.per_tap = (a.Cp + kTmaK - 1) / kTmaK;
     tl.chunks = a.kernel * a.kernel * tl.per_tap;
     tl.im2col = a.kernel == 1 && a.stride == 1 && a.pad == 0 ? 0 : 1;
+    tl.spin_limit = tc::role_wait_limit();
     const int BM = plan.ty * 4;
     CUtensorMap mA, mB;
     if (!tl.im2col) {

@@ -114,6 +114,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return false;
 }
 
+// Wait for a role's turn: gives up after `limit` polls, or once another role has.
+__device__ __forceinline__ bool wait_turn(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit) {
+    const uint32_t addr = smem_u32(bar);
+    for (uint32_t spin = 0; spin < limit; ++spin) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+        if (done) return true;
+        if ((spin & 255u) == 255u && *abort_flag) return false;
+    }
+    return false;
+}
+
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint64_t* bar,
                                             int c0, int c1, int c2, int c3) {
     asm volatile(

@@ -306,6 +306,41 @@ def test_fp32_contraction_by_the_copy_engine(shape):
     assert (got[..., K:] == 0).all()
 
 
+@pytest.mark.parametrize("shape", [
+    # N, H, C, K, kernel, stride: the fp32 contraction by the copy engine in one piece, over clusters, of a matrix
+    (16, 40, 96, 160, 3, 1), (8, 14, 256, 256, 3, 1), (32, 56, 96, 200, 1, 1)])
+def test_fp32_waits_that_run_out(shape):
+    """Limits at which some threads or blocks give up and others do not: the launch returns, with the status set or with the
+    result, and the next one is right again."""
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    lib = _lib.cuda_lib()
+    N, H, ci, K, k, s = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *d: torch.randn(d, generator=g, device="cuda")
+    x, w, b = torch.zeros((N, H, H, ops.up4(ci)), device="cuda"), rand(K, ci, k, k) / (ci * k * k) ** 0.5, rand(K)
+    x[..., :ci] = rand(N, H, H, ci)
+    p = ops.conv_params(N, H, H, ci, K, k, s, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_FP32)
+    assert lib.ogle_cuda_conv2d_kernel_name(C.byref(p)) == b"conv_igemm_tma_kernel"
+    packed = ops.conv2d_prepack(p, w)
+    want = ops.conv2d(p, x, packed, b)
+    seen = set()
+    try:
+        for limit in [0, 1, 2, 3, 4, 6, 8, 11, 16, 23, 32, 64, 128, 256, 1024, 4096] * 2:
+            lib.ogle_cuda_set_wait_limit(limit)
+            got = ops.conv2d(p, x, packed, b)
+            status = lib.ogle_cuda_device_status()
+            assert status == -6 or (status == 0 and torch.equal(got, want)), (limit, status)
+            seen.add(status)
+            lib.ogle_cuda_clear_device_status()
+    finally:
+        lib.ogle_cuda_set_wait_limit(-1)
+        lib.ogle_cuda_clear_device_status()
+    assert -6 in seen
+    assert torch.equal(ops.conv2d(p, x, packed, b), want) and lib.ogle_cuda_device_status() == 0
+
+
 def test_fp32_gemm_of_many_columns():
     """Up to 65535 column tiles of 64."""
     import torch

@@ -199,3 +199,58 @@ def test_no_window_lands_in_a_block_that_ended(tiles):
 
 def test_the_model_sees_readers_that_give_up_alone():
     assert _lands_in_a_block_that_ended(1, 2, "when it gave up")
+
+
+def _fp32_ring():
+    """What thread 0 of the fp32 contraction does once its wait has run out: whether it asks for further copies, and whether
+    it then waits for those in flight from the step that did not come on."""
+    text = open(os.path.join(KERNELS, "igemm.cu")).read()
+    body = text[text.index("conv_igemm_tma_kernel("):]
+    asks = re.search(r"if \(tid == 0 && ([^;]*)t \+ kTmaStages < count\) issue", body).group(1)
+    return "came" not in asks, re.search(r"for \(int t = s_stop; t < count && t < s_stop \+ kTmaStages", body) is not None
+
+
+def _copy_behind_a_copy(count, stages, asks_on, waits_from_stop):
+    """Whether thread 0, which asks for a step's copy two steps ahead and may give up at any wait, can ask for a stage that a
+    copy is still on its way to, or leave with one in flight. A wait succeeds by its phase's parity."""
+    start = (0, None, tuple(1 if i < count else 0 for i in range(stages)), (0,) * stages, None)
+    seen, todo = {start}, [start]
+    while todo:
+        t, stop, asked, landed, drain = todo.pop()
+        nxt = []
+        for i in range(stages):
+            if landed[i] < asked[i]:
+                nxt.append((t, stop, asked, landed[:i] + (landed[i] + 1,) + landed[i + 1:], drain))
+        came = lambda step: landed[step % stages] % 2 != step // stages % 2
+        if t < count:
+            for gave_up in ([False] if stop is None and came(t) else []) + [True]:
+                now = t if stop is None and gave_up else stop
+                ask, i = asked, t % stages
+                if (now is None or asks_on) and t + stages < count:
+                    if asked[i] > landed[i]:
+                        return True
+                    ask = asked[:i] + (asked[i] + 1,) + asked[i + 1:]
+                nxt.append((t + 1, now, ask, landed, None))
+        else:
+            first = count if stop is None else stop if waits_from_stop else max(0, count - stages)
+            last = min(count, first + stages)
+            at = first if drain is None else drain
+            if at >= last:
+                if asked != landed:
+                    return True
+            elif came(at):
+                nxt.append((t, stop, asked, landed, at + 1))
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 6, 7])
+def test_fp32_ring_after_a_wait_that_ran_out(count):
+    assert not _copy_behind_a_copy(count, 2, *_fp32_ring())
+
+
+def test_the_model_sees_copies_asked_for_after_giving_up():
+    assert _copy_behind_a_copy(6, 2, True, True) and _copy_behind_a_copy(6, 2, False, False)
