@@ -61,13 +61,14 @@ const char* ogle_cuda_build_info(void);
 uint64_t ogle_cuda_launch_count(void);
 /* Last CUDA error string seen by this library on the calling thread. */
 const char* ogle_cuda_last_error(void);
-/* Device-side status word of the tensor-core kernels: 0, or the code of the first
+/* Device-side status word of the kernels that wait for copies or multiplies: 0, or the code of the first
  * bounded wait that gave up (the launch then produced no valid output). Reading
  * synchronises the device; clear resets it. */
 int ogle_cuda_device_status(void);
 int ogle_cuda_clear_device_status(void);
 /* The raw status word: which wait gave up (1 producer, 2 MMA issuer, 3 operand split,
- * 4 epilogue, 5 accumulator hand-back); 0 when none did. Synchronises the device. */
+ * 4 epilogue, 5 accumulator hand-back; 6 depthwise, 8 direct stem or fp32 contraction); 0 when none did. Synchronises the
+ * device. */
 int ogle_cuda_device_status_detail(void);
 /* Programmatic dependent launches for the kernels launched after this call (process-wide): each kernel's
  * prologue (barrier set-up, tensor-memory allocation, descriptor prefetch) may then run while its predecessor
@@ -90,8 +91,9 @@ typedef struct {
 } OgleContraction;
 int ogle_cuda_last_contraction(OgleContraction* out);
 
-/* How many times a role of the tensor-core kernels polls for its turn before it gives up, for
- * the launches that follow on any stream (process-wide). polls < 0 restores the default (2^22,
+/* How many times a role of the tensor-core kernels polls for its turn before it gives up, or, for its operands, a thread
+ * of the fp32 contraction by the copy engine or a warp of the direct RGB stem, for the launches that follow on any stream
+ * (process-wide). polls < 0 restores the default (2^22,
  * tens of milliseconds); 0 makes every such wait give up at once. It exists to exercise the
  * give-up path without a fault: a launch whose waits run out writes no valid output, sets the
  * status word, waits for its own copies and multiplies in flight (those waits keep the full

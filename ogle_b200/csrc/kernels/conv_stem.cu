@@ -40,6 +40,7 @@ struct StemTiles {
     int tiles_x, tiles_y;
     int iw, ih;                      // input window of a tile
     int total;                       // tiles; 32-bit so that the per-tile index arithmetic is
+    uint32_t spin_limit;             // polls of a wait before it gives up
 };
 
 // Two fp32 values in one 64-bit register, and the packed multiply-add of sm_100.
@@ -74,6 +75,8 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kStemStages];
     __shared__ unsigned s_done[kStemStages];         // warps that are through with a stage
+    __shared__ unsigned s_asked[kStemStages];        // copies asked for (a stage without a tile has none)
+    __shared__ int s_abort;                          // a warp gave up
     // weights [9][CIN][Kp] + bias [Kp], then the input stages (128-byte aligned)
     float* s_w = reinterpret_cast<float*>(smem_raw);
     const int Kp = KP ? KP : a.Kp;
@@ -91,7 +94,8 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
 
     grid_dependency_trigger();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStemStages; ++i) { mbar_init(&bar_full[i], 1); s_done[i] = 0; }
+        for (int i = 0; i < kStemStages; ++i) { mbar_init(&bar_full[i], 1); s_done[i] = 0; s_asked[i] = 1; }
+        s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     grid_dependency_wait();         // nothing from global memory before this point
@@ -136,8 +140,14 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
         const int tx = (int)(tile - tq * tiles_x);
         const int n = (int)(tq / tiles_y);
         const int ty = (int)(tq - (uint32_t)n * tiles_y);
-        if (!mbar_wait(&bar_full[stage], phase)) {
-            if (lane == 0) record_error(err_flag, 8);
+        if (!__all_sync(0xffffffffu, wait_turn(&bar_full[stage], phase, &s_abort, tl.spin_limit))) {
+            s_abort = 1;
+            if (lane == 0) {
+                record_error(err_flag, 8);
+                // What this warp has asked for lands before it leaves; what others ask for from now on they wait for themselves.
+                for (int i = 0; i < kStemStages; ++i)
+                    if (blockIdx.x + (uint32_t)i * gridDim.x < total) mbar_wait(&bar_full[i], (s_asked[i] - 1) & 1u);
+            }
             break;
         }
         if (active) {
@@ -232,7 +242,7 @@ conv3x3_smallc_kernel(const __grid_constant__ CUtensorMap tmX, const float* __re
         if (lane == 0 && through(&s_done[stage]) == blockDim.x / 32 - 1) {
             s_done[stage] = 0;
             const uint32_t ahead = tile + (uint32_t)kStemStages * gridDim.x;
-            if (ahead < total) issue(ahead, stage);
+            if (ahead < total) { issue(ahead, stage); ++s_asked[stage]; }
         }
         if (++stage == kStemStages) { stage = 0; phase ^= 1u; }
     }
@@ -330,6 +340,7 @@ int launch_conv_smallc(const ConvArgs& a, const float* x, const float* w_tap_maj
                        cudaStream_t s) {
     StemTiles t = {};
     const int pxt = choose_pxt(a, &t);
+    t.spin_limit = role_wait_limit();
     if (a.stride == 1) {
         if (pxt == 5) return launch_c<1, 5>(a, t, x, w_tap_major, bias, y, s);
         if (pxt == 4) return launch_c<1, 4>(a, t, x, w_tap_major, bias, y, s);

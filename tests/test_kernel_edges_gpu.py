@@ -307,8 +307,9 @@ def test_fp32_contraction_by_the_copy_engine(shape):
 
 
 @pytest.mark.parametrize("shape", [
-    # N, H, C, K, kernel, stride: the fp32 contraction by the copy engine in one piece, over clusters, of a matrix
-    (16, 40, 96, 160, 3, 1), (8, 14, 256, 256, 3, 1), (32, 56, 96, 200, 1, 1)])
+    # N, H, C, K, kernel, stride: the fp32 contraction by the copy engine in one piece, over clusters, of a matrix;
+    # the direct stem with more tiles than stages, and fewer
+    (16, 40, 96, 160, 3, 1), (8, 14, 256, 256, 3, 1), (32, 56, 96, 200, 1, 1), (64, 150, 3, 32, 3, 2), (2, 20, 3, 64, 3, 1)])
 def test_fp32_waits_that_run_out(shape):
     """Limits at which some threads or blocks give up and others do not: the launch returns, with the status set or with the
     result, and the next one is right again."""
@@ -322,7 +323,7 @@ def test_fp32_waits_that_run_out(shape):
     x, w, b = torch.zeros((N, H, H, ops.up4(ci)), device="cuda"), rand(K, ci, k, k) / (ci * k * k) ** 0.5, rand(K)
     x[..., :ci] = rand(N, H, H, ci)
     p = ops.conv_params(N, H, H, ci, K, k, s, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_FP32)
-    assert lib.ogle_cuda_conv2d_kernel_name(C.byref(p)) == b"conv_igemm_tma_kernel"
+    assert lib.ogle_cuda_conv2d_kernel_name(C.byref(p)) == (b"conv3x3_smallc_kernel" if ci == 3 else b"conv_igemm_tma_kernel")
     packed = ops.conv2d_prepack(p, w)
     want = ops.conv2d(p, x, packed, b)
     seen = set()

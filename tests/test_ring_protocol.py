@@ -254,3 +254,48 @@ def test_fp32_ring_after_a_wait_that_ran_out(count):
 
 def test_the_model_sees_copies_asked_for_after_giving_up():
     assert _copy_behind_a_copy(6, 2, True, True) and _copy_behind_a_copy(6, 2, False, False)
+
+
+def _stem_warps_wait():
+    """Whether a warp of the direct stem that gives up waits for the copies that were asked for before it leaves."""
+    text = open(os.path.join(KERNELS, "conv_stem.cu")).read()
+    body = text[text.index("conv3x3_smallc_kernel("):]
+    gives_up = body[body.index("s_abort = 1;"):]
+    return re.search(r"mbar_wait\(&bar_full\[i\], \(s_asked\[i\] - 1\) & 1u\)", gives_up[:gives_up.index("break;")]) is not None
+
+
+def _stem_copies_outlive(tiles, stages, warps, give_up_waits):
+    """Whether a copy can land after the block. Every warp reads all tiles in order, each as it lands, or gives up by itself
+    and waits for what has been asked for by then; the last to have read a stage's tile asks for its next."""
+    start = ((0,) * warps, (-1,) * warps, 0)              # tiles read; -1 runs, 1 left, -2 - x gives up and waits for x; tiles landed (a bit each)
+    seen, todo = {start}, [start]
+    while todo:
+        read, how, landed = todo.pop()
+        asked = sum(1 << t for t in range(tiles) if t < stages or t - stages < min(read))
+        if all(h == 1 for h in how) and landed != asked:
+            return True
+        nxt = [(read, how, landed | 1 << t) for t in range(tiles) if asked >> t & 1 and not landed >> t & 1]
+        for i in range(warps):
+            put = lambda h: how[:i] + (h,) + how[i + 1:]
+            if how[i] == -1 and read[i] == tiles:
+                nxt.append((read, put(1), landed))
+            elif how[i] == -1:
+                nxt.append((read, put(-2 - asked if give_up_waits else 1), landed))
+                if landed >> read[i] & 1:
+                    nxt.append((read[:i] + (read[i] + 1,) + read[i + 1:], how, landed))
+            elif how[i] < -1 and (-2 - how[i]) & ~landed == 0:
+                nxt.append((read, put(1), landed))
+        for s in nxt:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return False
+
+
+@pytest.mark.parametrize("tiles", [1, 3, 6])
+def test_no_stem_copy_lands_in_a_block_that_ended(tiles):
+    assert not _stem_copies_outlive(tiles, 3, 2, _stem_warps_wait())
+
+
+def test_the_model_sees_a_stem_warp_that_gives_up():
+    assert _stem_copies_outlive(6, 3, 2, False)
