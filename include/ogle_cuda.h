@@ -84,7 +84,8 @@ int ogle_cuda_set_overlapped_launches(int on);
 typedef struct {
     int form;        /* 1 whole tiles; 2 ranges of the reduction combined through memory; 3 ranges added up inside a
                         cluster; 4 tiles on pairs of SMs; 5 channels on M; 6 taps of a filter row side by side; 7 whole tiles
-                        of an RGB stem, its filters kept in shared memory; 8 few rows, on the CUDA cores */
+                        of an RGB stem, its filters kept in shared memory; 8 few rows, on the CUDA cores; 9 an RGB stem
+                        whose input window is the operand */
     int ranges;      /* ranges of the reduction (1 = not split) */
     int n_tile;      /* output channels of a tile (form 8: of a warp) */
     int overlapped;  /* 1: allowed to start its set-up while the launch before it drains */

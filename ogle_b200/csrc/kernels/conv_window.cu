@@ -380,8 +380,7 @@ int launch(const ConvArgs& a, int passes, const float* x, const float* w, const 
     }
     const int blocks = t.total < kNumSMs ? t.total : kNumSMs;
     const bool overlapped = overlapped_launches_enabled();
-    // (with a residual operand it goes by the number of the whole tiles of one SM, as the gather form there does)
-    note_contraction(residual ? 1 : 7, 1, t.np, overlapped);
+    note_contraction(9, 1, t.np, overlapped);
     launch_overlapped_if(overlapped, conv_window_kernel<kK, kS, kTileW>, dim3((unsigned)blocks), dim3(kThreadsW), smem, s, mX, mY, w, bias, t,
                          error_flag_ptr());
     return finish_launch();
