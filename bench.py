@@ -291,7 +291,7 @@ def classify_layers(rows, costs, peaks, passes_equiv):
         bound = None
         if byts:
             t_hbm = byts / (peaks["hbm_gbs"] * 1e9)
-            t_ten = flops / (tensor_peak * 1e12) if (tensor_peak and "tc" in key) else 0.0
+            t_ten = flops / (tensor_peak * 1e12) if (tensor_peak and ("tc" in key or key == "conv_window_kernel")) else 0.0
             bound = "tensor" if t_ten > t_hbm else "hbm"
         for k in ((key, None), (key, bound)) if bound else ((key, None),):
             f = fam.setdefault(k, dict(ms=0.0, launches=0, flops=0, bytes=0))

@@ -192,8 +192,10 @@ size_t ogle_cuda_conv2d_workspace_bytes(const OgleConvParams* p);
 int ogle_cuda_conv2d_ws(const OgleConvParams* p, const float* x, const void* packed_filter, const float* bias,
                         float* y, void* workspace, size_t workspace_bytes, ogle_stream_t stream);
 
-/* Name of the device kernel that ogle_cuda_conv2d launches for these parameters
- * (for profiles and reports; "" when the parameters are invalid). */
+/* Name of the device kernel that ogle_cuda_conv2d (ogle_cuda_conv2d_pair, given the stacked filters' parameters) launches
+ * for these parameters (for profiles and reports; "" when the parameters are invalid). "conv_tc2_kernel" stands for all
+ * tensor-core forms of conv_tc2.cu and its two variants, conv_tc2_pair_kernel and conv_tc2_t_kernel, among which the scratch
+ * lent decides too: OgleContraction tells those apart. */
 const char* ogle_cuda_conv2d_kernel_name(const OgleConvParams* p);
 
 /* Two convolutions that read the same input with the same window (kernel, stride,

@@ -14,6 +14,7 @@ bool conv_tc_gather_supported(const ConvArgs& a, int variant);
 bool dw_tma_supported(const ConvArgs& a);
 bool conv_smallc_supported(const ConvArgs& a);
 const char* conv_igemm_name(const ConvArgs& a);
+const char* conv_tc_name(const ConvArgs& a, int variant, int math_mode);
 
 // Destination-indexed packing of an OIHW filter into the three sections of the
 // packed blob (see FilterLayout).
@@ -248,7 +249,7 @@ size_t ogle_cuda_conv2d_workspace_bytes(const OgleConvParams* p) {
 const char* ogle_cuda_conv2d_kernel_name(const OgleConvParams* p) {
     ConvArgs a; int variant;
     if (fill_args(p, &a, &variant) != OGLE_OK) return "";
-    if (served_by_tc(p, a, variant)) return "conv_tc2_kernel";
+    if (served_by_tc(p, a, variant)) return conv_tc_name(a, variant, p->math_mode);
     if (variant == CONV_DEPTHWISE) {
         if (dw_tma_supported(a)) return "dw_tma_kernel";
         return (a.kernel == 3 && a.dil == 1 && (a.stride == 1 || a.stride == 2)) ? "dw3x3_kernel" : "dw_generic_kernel";

@@ -457,6 +457,12 @@ static bool window_form(const ConvArgs& a, int variant, bool split_mode) {
     return windows <= 1.3 * gathered && windows * a.N < 0x7fffffff - 2 * kNumSMs;
 }
 
+// The kernel that launch_conv_tc runs for a layer (the tensor-core forms by one name); with two outputs none has a window.
+const char* conv_tc_name(const ConvArgs& a, int variant, int math_mode) {
+    if (few_rows(a)) return "few_rows_kernel";
+    return window_form(a, variant, math_mode == OGLE_MATH_TF32X3) ? "conv_window_kernel" : "conv_tc2_kernel";
+}
+
 int launch_conv_tc(const ConvArgs& a, int variant, int math_mode, const float* x, const float* w_hi,
                    const float* w_lo, const float* bias, float* y, cudaStream_t s, float* y2, int K1,
                    int split_col, void* ws, size_t ws_bytes, size_t* ws_needed, const float* residual, int res_ld) {

@@ -162,10 +162,14 @@ public:
         params_.min_value = min_; params_.max_value = max_;
         params_.math_mode = context_->math_mode();
         OGLE_CUDA_OK(ogle_cuda_conv2d_infer(&params_));
-        // family (the reference's shader name) : device kernel that serves it
-        const size_t colon = kernel_fname_.find(':');
-        kernel_fname_ = kernel_fname_.substr(0, colon) + ":" + ogle_cuda_conv2d_kernel_name(&params_);
+        NameKernel();
         output_shapes[0] = {image_shape[0], params_.out_hwc[0], params_.out_hwc[1], filter_shape[0]};
+    }
+
+    // family (the reference's shader name) : device kernel that serves it
+    void NameKernel() {
+        const size_t colon = kernel_fname_.find(':');
+        kernel_fname_ = kernel_fname_.substr(0, colon) + ":" + ogle_cuda_conv2d_kernel_name(sibling_ ? &pair_params_ : &params_);
     }
 
     // Two convolutions over one feature map with the same window and constant filters run as
@@ -214,6 +218,7 @@ public:
         EnsureWorkspace(ogle_cuda_conv2d_pair_workspace_bytes(&f, K1, split));
         sibling_ = o;
         kernel_name_ += "+" + o->kernel_name_;
+        NameKernel();
         return true;
     }
 
@@ -231,8 +236,7 @@ public:
         if (ogle_cuda_conv2d_infer(&q) != OGLE_OK) return false;
         params_ = q;
         placed_ = dst;
-        const size_t colon = kernel_fname_.find(':');
-        kernel_fname_ = kernel_fname_.substr(0, colon) + ":" + ogle_cuda_conv2d_kernel_name(&params_);
+        NameKernel();
         return true;
     }
 
@@ -267,7 +271,7 @@ public:
     // are the same whatever width or pairing is asked for, those of few rows whatever width: those candidates are left out.
     void Tune() override {
         OgleConvParams& p = sibling_ ? pair_params_ : params_;
-        if (!filter_is_constant_ || std::string(ogle_cuda_conv2d_kernel_name(&p)) != "conv_tc2_kernel") return;
+        if (!filter_is_constant_ || !ogle_cuda_conv2d_residual_supported(&p)) return;      // (the tensor-core path's layers)
         cudaStream_t s = reinterpret_cast<cudaStream_t>(context_->stream());
         cudaEvent_t e0, e1;
         if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return;
@@ -349,6 +353,7 @@ public:
             tuned_split_ = best_split;
             tuned_pair_ = best_pair;
         }
+        NameKernel();                        // (a reduction split by request is no few-pixel launch)
         workspace_for();
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);

@@ -177,7 +177,8 @@ def main():
             p = ops._gemm_params(A4, B4, None, M, K, N, 0, 1.0, 1.0, 0, mode)
             if mode == ops.MATH_FP32:
                 call = lambda: lib.ogle_cuda_gemm(C.byref(p), ops._p(A4), ops._p(B4), None, ops._p(out), ops._stream())
-                kernel = "conv_igemm_tma_kernel"
+                # (the product is the pointwise convolution of M pixels)
+                kernel = lib.ogle_cuda_conv2d_kernel_name(C.byref(ops.conv_params(1, M, 1, K, N, 1, math_mode=mode))).decode()
             else:
                 packed = ops.gemm_pack_b(B4, M, K, N, 0, mode)     # B is a constant (weights): packed once
                 call = lambda: lib.ogle_cuda_gemm_packed(C.byref(p), ops._p(A4), ops._p(packed), None, ops._p(out), ops._stream())

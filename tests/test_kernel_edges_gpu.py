@@ -1248,6 +1248,30 @@ def test_kernel_names_are_those_of_the_sources(case):
     assert name in kernels
 
 
+@pytest.mark.parametrize("case", [
+    # images, size, C, K, kernel, stride, split asked for, name: both sides of what decides between the tensor-core path's kernels
+    (1, 3, 256, 128, 1, 1, 0, "few_rows_kernel"), (1, 3, 256, 128, 1, 1, 2, "conv_tc2_kernel"), (32, 1, 64, 700, 1, 1, 0, "few_rows_kernel"),
+    (33, 1, 64, 600, 1, 1, 0, "conv_tc2_kernel"), (2, 2, 128, 300, 3, 1, 0, "few_rows_kernel"), (2, 2, 128, 330, 3, 1, 0, "conv_tc2_kernel"),
+    (2, 64, 3, 48, 7, 2, 0, "conv_window_kernel"), (2, 64, 3, 49, 7, 2, 0, "conv_tc2_kernel"), (2, 64, 2, 64, 7, 2, 0, "conv_window_kernel"),
+    (2, 64, 3, 65, 5, 1, 0, "conv_tc2_kernel"), (80, 120, 3, 64, 7, 2, 0, "conv_window_kernel")])
+@pytest.mark.parametrize("residual", [False, True])
+def test_kernel_names_say_what_runs(case, residual):
+    import ctypes as C
+    import torch
+    from ogle_b200 import _lib, ops
+    N, size, ci, k, f, s, split, name = case
+    p = ops.conv_params(N, size, size, ci, k, f, s, f // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_TF32X3)
+    p.split = split
+    assert _lib.cuda_lib().ogle_cuda_conv2d_kernel_name(C.byref(p)).decode() == name
+    x, b = torch.zeros((N, size, size, ops.up4(ci)), device="cuda"), torch.ones(k, device="cuda")
+    packed = ops.conv2d_prepack(p, torch.zeros((k, ci, f, f), device="cuda"))
+    y = ops.conv2d(p, x, packed, b)
+    if residual:
+        ops.conv2d_residual(p, x, packed, b, torch.zeros_like(y))
+    form = ops.last_contraction().form
+    assert {8: "few_rows_kernel", 9: "conv_window_kernel"}.get(form, "conv_tc2_kernel") == name
+
+
 @pytest.mark.parametrize("env,overlapped", [(None, 1), ("0", 0), ("1", 1)])
 def test_products_overlap_their_packing_pass_unless_told_otherwise(env, overlapped):
     """gemm_ws in all its forms - clusters, pairs of SMs, whole tiles - asks for it; OGLE_PDL, read once per process, wins."""

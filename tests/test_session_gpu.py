@@ -575,6 +575,26 @@ def test_sharded_detector_fed_frames_equals_fed_tensors(oracle_port):
         assert np.array_equal(got[0][key], got[1][key]), key
 
 
+def test_profile_books_small_maps_under_their_kernel():
+    """One image's late heads, pairs among them, have so few pixels that the CUDA cores serve them; where the tuning prefers
+    ranges of the reduction on the tensor cores, the profile says so."""
+    from ogle_b200 import models, session
+    model, _ = models.mobilenet_v1_ssd(batch=1, num_classes=21, seed=8, weight_std=0.02)
+    x = np.zeros((1, 300, 300, 3), np.float32)
+    for tune in (0, 1):
+        sess = session.FBOSession()
+        sess.set_option("math_mode", 2)
+        sess.set_option("tune", tune)
+        sess.LoadGraph(model)
+        sess.Run({"input": x})
+        kernels = {name: kernel.split(":")[1] for name, type_, kernel, _ in sess.Profile({"input": x}) if type_ == "Conv"}
+        if not tune:
+            assert any("+" in name and kernel == "few_rows_kernel" for name, kernel in kernels.items()), kernels
+        assert set(kernels.values()) <= {"few_rows_kernel", "conv_tc2_kernel", "dw_tma_kernel", "dw3x3_kernel", "dw_generic_kernel",
+                                         "conv3x3_smallc_kernel"}
+        sess.close()
+
+
 def test_profile_tool_reports_per_type_table(tmp_path):
     """ogle_profile (the headless counterpart of nn/profile_main.cc): loads a dlx file, runs it and
     prints the per-node-type table; --json gives the same numbers for scripts."""
