@@ -125,8 +125,9 @@ typedef struct {
                                 sm_pair); a caller may time the candidates and keep the fastest. Many-tile 3x3
                                 layers of stride 1 have tiles of 32 or 64 channels whatever is asked for, the
                                 taps of a filter row side by side; layers of a few pixels (form 8 of
-                                OgleContraction, unless split is asked for) and 5x5 and 7x7 stems of up to 64
-                                channels have none. */
+                                OgleContraction) have none unless split is asked for, and 5x5 and 7x7 stems of up
+                                to 64 channels whose window is the operand (form 9) never: those ignore split,
+                                channels_on_m and sm_pair too. */
     int split;               /* tensor-core path: ranges the reduction is split into (1 = not split, up to
                                 16); 0 = chosen by the library. Two to eight ranges of a launch of few tiles
                                 are added up inside a cluster of SMs; any other number, and launches of more

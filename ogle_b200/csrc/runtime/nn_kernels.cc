@@ -268,7 +268,8 @@ public:
     // number of ranges its reduction is split into (which does change the order of the partial sums); then, for
     // an unsplit reduction, whether pairs of SMs should share the filter tiles (same bits again); last, channels on M (the
     // bits of that number of ranges, but for 3x3 layers whose taps would lie side by side). Launches of taps side by side
-    // are the same whatever width or pairing is asked for, those of few rows whatever width: those candidates are left out.
+    // are the same whatever width or pairing is asked for, those of few rows whatever width, stems with the window as operand
+    // whatever is asked for: those candidates are left out.
     void Tune() override {
         OgleConvParams& p = sibling_ ? pair_params_ : params_;
         if (!filter_is_constant_ || !ogle_cuda_conv2d_residual_supported(&p)) return;      // (the tensor-core path's layers)
@@ -302,8 +303,8 @@ public:
         if (time_it(&auto_ms)) {
             best_ms = auto_ms;
             int best_tile = 0, best_split = 0, best_pair = 0;
-            const bool beside = taps_side_by_side(), few_rows = ran_as(8);
-            for (int bn = 32; !beside && !few_rows && bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
+            const bool beside = taps_side_by_side(), few_rows = ran_as(8), fixed = ran_as(9);
+            for (int bn = 32; !beside && !few_rows && !fixed && bn <= 256 && bn <= kmax; bn += 32) {          // tile widths, the library's split rule
                 float ms;
                 p.n_tile = bn;
                 if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_tile = bn; }
@@ -312,13 +313,13 @@ public:
             static const int splits[] = {1, 2, 3, 4, 6, 8, 12, 16};          // then the reduction split at that width
             for (int k : splits) {
                 float ms;
-                if (k == 1 && beside) continue;
+                if (fixed || (k == 1 && beside)) continue;
                 p.split = k;
                 if (time_it(&ms) && ms < best_ms) { best_ms = ms; best_split = k; }
             }
             p.split = best_split;
             int pair_tile = best_tile;
-            for (int bn = 64; !beside && bn <= 256 && bn <= kmax; bn += 64) {           // SM pairs, unsplit, at the widths that halve
+            for (int bn = 64; !beside && !fixed && bn <= 256 && bn <= kmax; bn += 64) {           // SM pairs, unsplit, at the widths that halve
                 float ms;
                 p.n_tile = bn;
                 p.split = 1;
@@ -330,7 +331,7 @@ public:
             if (best_pair) { best_tile = pair_tile; best_split = 1; }
             // at most 128 output channels: the accumulator kept transposed (filters on the multiply's 128-row side)
             int best_on_m = 0;
-            if (p.out_hwc[2] <= 128) {
+            if (p.out_hwc[2] <= 128 && !fixed) {
                 float ms;
                 p.n_tile = 0;
                 p.split = 1;

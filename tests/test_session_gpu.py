@@ -575,6 +575,27 @@ def test_sharded_detector_fed_frames_equals_fed_tensors(oracle_port):
         assert np.array_equal(got[0][key], got[1][key]), key
 
 
+@pytest.mark.parametrize("channels,timed", [(2, 4), (16, 40)])
+def test_tuning_leaves_out_what_a_stem_ignores(channels, timed):
+    """A stem whose window is the operand ignores width, ranges, SM pairs and channels on M: its tuning launches it four times
+    to see that, and times nothing else. (A layer that can be tuned, for comparison: many more.)"""
+    from ogle_b200 import _lib, models, session
+    lib = _lib.cuda_lib()
+    w = np.full((64, channels, 7, 7), 0.01, np.float32)
+    launches = []
+    for tune in (0, 1):
+        sess = session.FBOSession()
+        sess.set_option("math_mode", 2)
+        sess.set_option("tune", tune)
+        model = models.single_conv((2, 96, 96, channels), w, None, 2, 3)
+        before = lib.ogle_cuda_launch_count()
+        sess.LoadGraph(model)
+        sess.Run({"input": np.zeros((2, 96, 96, channels), np.float32)})
+        launches.append(lib.ogle_cuda_launch_count() - before)
+        sess.close()
+    assert launches[1] - launches[0] == timed if channels == 2 else launches[1] - launches[0] >= timed
+
+
 def test_profile_books_small_maps_under_their_kernel():
     """One image's late heads, pairs among them, have so few pixels that the CUDA cores serve them; where the tuning prefers
     ranges of the reduction on the tensor cores, the profile says so."""
