@@ -318,19 +318,26 @@ int choose_shape_by_rows(const ConvArgs& a, int quads, DwTiles* t) {
     return best;
 }
 
-// The shape for a layer, and the rows a thread computes (0: none fits). The last few layers' are kept, by their sizes:
-// to weigh some eighty shapes takes as long as the launch.
+// The shape for a layer, and the rows a thread computes (0: none fits). Those of the last layers are kept, by their sizes:
+// to weigh some eighty shapes takes the host 0.45 us. There is room for a few networks' layers: a network runs its layers in
+// turn, and fewer places than it has (eight, of MobileNet's nine) would all have changed hands when they come round again.
+// A layer lies in one of four places.
 int choose_shape(const ConvArgs& a, DwTiles* t) {
     struct Known { int N, H, W, Kp, K, kernel, stride, pad, rows; DwTiles t; };
-    static thread_local Known known[8];
-    static thread_local int next = 0;
+    constexpr int kKnown = 64, kPlaces = 4;
+    static thread_local Known known[kKnown];
+    static thread_local unsigned next = 0;
     const bool forced = getenv("OGLE_DW_TW") || getenv("OGLE_DW_RPG");
-    if (!forced)
-        for (const Known& k : known)
-            if (k.kernel == a.kernel && k.stride == a.stride && k.pad == a.pad && k.N == a.N && k.H == a.H && k.W == a.W && k.Kp == a.Kp && k.K == a.K) {
-                *t = k.t;
-                return k.rows;
-            }
+    unsigned at = 0;
+    for (int v : {a.N, a.H, a.W, a.K, a.kernel, a.stride, a.pad}) at = (at ^ (unsigned)v) * 2654435761u;
+    at >>= 26;                       // (the upper six bits)
+    for (unsigned i = 0; !forced && i < kPlaces; ++i) {
+        const Known& k = known[(at + i) % kKnown];
+        if (k.kernel == a.kernel && k.stride == a.stride && k.pad == a.pad && k.N == a.N && k.H == a.H && k.W == a.W && k.Kp == a.Kp && k.K == a.K) {
+            *t = k.t;
+            return k.rows;
+        }
+    }
     const int quads = slab_quads(a);
     // Tensors that do not stay in L2 are bound by HBM, by what the estimate does not see (256 x 38 x 38 x 256: 127 us in
     // parts of 13, 146 in what it takes), unless tiles of 32 hang far over the map's edge (27 x 127 x 70 x 160 56 -> 52).
@@ -340,8 +347,10 @@ int choose_shape(const ConvArgs& a, DwTiles* t) {
                                                                   (((a.Ho + t->th - 1) / t->th) * t->th)))
         rows = choose_shape_stride1(a, quads, t);
     if (forced) return rows;
-    known[next] = {a.N, a.H, a.W, a.Kp, a.K, a.kernel, a.stride, a.pad, rows, *t};
-    next = (next + 1) & 7;
+    unsigned place = at + next++ % kPlaces;
+    for (unsigned i = 0; i < kPlaces; ++i)
+        if (!known[(at + i) % kKnown].kernel) { place = at + i; break; }          // (a free one)
+    known[place % kKnown] = {a.N, a.H, a.W, a.Kp, a.K, a.kernel, a.stride, a.pad, rows, *t};
     return rows;
 }
 

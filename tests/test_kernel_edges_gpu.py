@@ -42,6 +42,31 @@ def test_depthwise_tile_shapes(oracle_port, size, images, channels, kernel):
     close(run_case_cuda(case), oracle_port.conv2d(x, w, b, 1, kernel // 2, 1, channels, 2, 0.0, 6.0))
 
 
+def test_depthwise_shapes_of_a_network_are_weighed_once():
+    """A pass over the thirteen depthwise layers of a network takes the host no longer a layer than one of them over and over;
+    layers that it has not seen lately take longer."""
+    import ctypes as C
+    import time
+    from ogle_b200 import _lib, ops
+    name = _lib.cuda_lib().ogle_cuda_conv2d_kernel_name
+    layers = [(150, 32, 1), (150, 64, 2), (75, 128, 1), (75, 128, 2), (38, 256, 1), (38, 256, 2), (19, 512, 1), (19, 512, 2), (10, 1024, 1),
+              (75, 144, 1), (56, 96, 1), (28, 192, 1), (14, 384, 1)]
+    of = lambda images: [C.byref(ops.conv_params(images, h, h, c, c, 3, s, 1, 1, c, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_TF32X3)) for h, c, s in layers]
+
+    def took(calls):
+        best = 1e9
+        for _ in range(200):
+            t = time.perf_counter()
+            for p in calls:
+                name(p)
+            best = min(best, (time.perf_counter() - t) / len(calls))
+        return best
+
+    network = of(1)
+    one, turns, unseen = took([p for p in network for _ in range(4)]), took(network * 4), took([p for n in range(2, 34) for p in of(n)])
+    assert turns - one <= 0.5 * (unseen - one), (one, turns, unseen)
+
+
 @pytest.mark.parametrize("channels", [1, 6, 12, 20, 129, 1028])
 def test_batchnorm_any_width_is_exact(oracle_port, channels):
     from gpu_ops import run_case_cuda
