@@ -45,8 +45,7 @@ few_rows_kernel(const FewRowsArgs a) {
     if (n0 < Np) {                                   // (rows of the pack past N are zeros, up to a multiple of 128)
         const int total = taps * a.Cp32;
         const __nv_bfloat16* cross = reinterpret_cast<const __nv_bfloat16*>(a.lo);
-#pragma unroll(kRows * kCols == 1 ? 8 : (kRows * kCols <= 4 ? 4 : 2))
-        for (int k = part * 128 + lane * 4; k < total; k += a.kw * 128) {
+        auto step = [&](int k) {
             float b[kCols][4];
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
@@ -92,6 +91,22 @@ few_rows_kernel(const FewRowsArgs a) {
 #pragma unroll
                     for (int l = 0; l < 4; ++l) acc[r][c] = fmaf(v[l], b[c][l], acc[r][c]);
             }
+        };
+        // Several rows: all lanes take as many steps, but for one by itself at the end. In one loop to the end of the reduction
+        // some lanes went once more through its unrolled part while the others took its remainder, one after the other:
+        // 4 x 448 x 1500 8.7 us (8.3 on the tensor cores), 5.9 so; 6 x 864 x 700 8.9 -> 6.1; 260 convolutions of few pixels 3 %.
+        // (One row has less in its steps, and the last by itself costs more: a pixel of 5x5 607 -> 40 5.9 us, 7.0 that way. In
+        // long reductions it is one of many: 2 x 3092 x 2558 16.1, 17.0 that way; with four columns a warp both loops want the
+        // registers of two blocks: 8 x 64 x 5000 3.9, 5.7.)
+        constexpr int kAtOnce = kRows * kCols == 1 ? 8 : (kRows * kCols <= 4 ? 4 : 2);
+        if (kRows > 1 && kCols == 1 && total < 2048) {
+            int k0 = part * 128;
+#pragma unroll(kAtOnce)
+            for (; k0 + 128 <= total; k0 += a.kw * 128) step(k0 + lane * 4);
+            if (k0 + lane * 4 < total) step(k0 + lane * 4);
+        } else {
+#pragma unroll(kAtOnce)
+            for (int k = part * 128 + lane * 4; k < total; k += a.kw * 128) step(k);
         }
     }
     float mine = 0.f;                                // lane r * kCols + c keeps that sum

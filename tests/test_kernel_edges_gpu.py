@@ -161,6 +161,19 @@ def test_reference_rule_edges(oracle_port, anchors, classes, spread, thr):
         assert (anchor[n, k:] == -1).all()
 
 
+def _in_a_graph(fn, launches=20):
+    """Replays of that many launches, for what takes the device less than the host takes to ask for it."""
+    import torch
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        fn()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(launches):
+                fn()
+    return graph.replay
+
+
 def _median_us(fn):
     import torch
     times = []
@@ -1056,7 +1069,7 @@ def test_clusters_do_not_take_longer_ranges(shape, math):
     # a row, two, up to four and up to eight; one to eight warps to a column, four columns to a warp; reductions and columns
     # that end inside a step, a piece, the pack's padding
     (1, 512, 1000, 2), (1, 5, 3, 1), (1, 131, 9473, 2), (1, 4099, 10, 0), (2, 1030, 77, 2), (2, 33, 4801, 0), (3, 129, 130, 1),
-    (4, 2049, 300, 2), (3, 3001, 2200, 0), (5, 64, 9, 1), (8, 700, 1001, 2), (7, 97, 6000, 2)])
+    (4, 2049, 300, 2), (4, 448, 1500, 2), (8, 864, 700, 0), (3, 3001, 2200, 0), (5, 64, 9, 1), (8, 700, 1001, 2), (7, 97, 6000, 2)])
 @pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
 def test_products_of_few_rows(m, k, n, bias_mode, math):
     """Against 64 bits with B as the pack holds it, whose every product is rounded only as the sum is."""
@@ -1082,11 +1095,28 @@ def test_products_of_few_rows(m, k, n, bias_mode, math):
     assert (got[:, n:] == 0).all()
 
 
+def test_few_rows_whose_reduction_ends_inside_a_step():
+    """A reduction of three and a half steps takes no longer than one of four (1.4 of it when lanes took turns)."""
+    import torch
+    from ogle_b200 import ops
+
+    def took(k):
+        g = torch.Generator(device="cuda").manual_seed(k)
+        a, b = torch.randn((4, k), generator=g, device="cuda"), torch.randn((k, 1500), generator=g, device="cuda")
+        packed = ops.gemm_pack_b(b, 4, k, 1500, 0, ops.MATH_TF32X3)
+        call = lambda: ops.gemm_packed(a, packed, None, 4, k, 1500, 0, 1.0, 1.0, 0, ops.MATH_TF32X3)
+        call()
+        assert ops.last_contraction().form == 8
+        return _median_us(_in_a_graph(call))
+
+    assert took(448) <= 1.15 * took(512)
+
+
 @pytest.mark.parametrize("shape", [
     # N, H, W, C, K, kernel, stride, pad, dilation: a pixel, two, some, several images; channels that end inside a piece;
     # padding, strides and dilations that leave taps outside the image
     (1, 1, 1, 256, 150, 3, 1, 1, 1), (1, 2, 1, 45, 33, 1, 1, 0, 1), (2, 1, 1, 130, 7, 5, 1, 2, 1), (1, 3, 3, 128, 220, 3, 2, 1, 1),
-    (5, 2, 3, 50, 61, 3, 1, 1, 1), (1, 5, 4, 97, 65, 3, 2, 3, 2), (32, 1, 1, 64, 36, 1, 1, 0, 1), (8, 2, 2, 128, 222, 3, 2, 1, 1)])
+    (5, 2, 3, 50, 61, 3, 1, 1, 1), (1, 1, 4, 448, 200, 1, 1, 0, 1), (1, 5, 4, 97, 65, 3, 2, 3, 2), (32, 1, 1, 64, 36, 1, 1, 0, 1), (8, 2, 2, 128, 222, 3, 2, 1, 1)])
 @pytest.mark.parametrize("math", ["MATH_TF32X3", "MATH_TF32"])
 @pytest.mark.parametrize("output", ["alone", "slice", "residual", "pair"])
 def test_convolutions_of_few_pixels(shape, math, output):
