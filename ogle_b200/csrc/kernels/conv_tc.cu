@@ -432,10 +432,20 @@ splitk_reduce_kernel(const float4* __restrict__ ws, int slices, long slice_q, in
 // the reduction open (a tile width, pairs of SMs or channels on M say how tiles are laid out, and there are none):
 // a fixed 3 us instead of 6 to 8, but by the multiply-add (in graphs: 9 pixels, 256 -> 128 pointwise 6.4 -> 3.8 us, 4 pixels
 // of 3x3 256 -> 150 9.3 -> 4.6, 8 of them 9.5 -> 5.8; 16 pixels of 3x3 69 -> 271, 2.7 M products, 7.9 -> 8.5).
+// Not where a reduction is short for its columns: blocks that the GPU does not hold at once (three to an SM) take one and a half
+// to five us more, and 64 elements take the tensor cores 5.0 (6.2 with more than 512 columns). 24 pixels 64 -> 700, 528 blocks,
+// 6.4 -> 5.8, 32 of 64 -> 512 4.9 -> 5.8, of 33 -> 1366 6.4 -> 11.2; two steps a warp 6 of 164 -> 2342 7.3 -> 8.1; 128 elements
+// 7 of 2785 columns 7.1 -> 6.4, and longer ones have no more columns than that.
 static bool few_rows(const ConvArgs& a) {
     if (a.split || filter_compact(a.C, a.kernel, 1)) return false;
     const double products = (double)a.M * a.K * a.kernel * a.kernel * a.C;
-    return (a.M <= 32 && products <= 1.5e6) || (a.M <= 8 && products <= 3e6);
+    if (!((a.M <= 32 && products <= 1.5e6) || (a.M <= 8 && products <= 3e6))) return false;
+    const int total = a.kernel * a.kernel * ((a.C + 31) / 32 * 32), rows = few_rows_rows(a.M);
+    const int per_block = 8 / few_rows_warps(a.K, total) * few_rows_cols(a.K);
+    const long blocks = (long)div_up(up4(a.K), per_block) * div_up(a.M, rows);
+    if (rows < 4 || blocks <= 3 * kNumSMs) return true;
+    if (total <= 64) return a.K > 512 && blocks <= 560;
+    return total <= 128 || total >= 256;
 }
 
 // Whether a stem of 5 x 5 or 7 x 7 filters takes its windows as they are (conv_window.cu): one tile of channels, and maps that

@@ -152,19 +152,15 @@ void (*kernel_for(const FewRowsArgs& a))(FewRowsArgs) {
 }  // namespace
 
 int launch_few_rows(FewRowsArgs a, cudaStream_t s) {
-    const int total = a.kernel * a.kernel * a.Cp32;
-    a.kw = 1;
-    while (a.kw < 8 && (long)up4(a.N) * a.kw * 2 <= 16 * kNumSMs && total >= a.kw * 256) a.kw *= 2;
-    const int rows = a.M == 1 ? 1 : (a.M == 2 ? 2 : 4);
-    // four columns a warp where one each is more than the GPU holds at once
-    const bool wide = a.N > 32 * kNumSMs;
-    const int per_block = 8 / a.kw * (wide ? 4 : 1);
+    a.kw = few_rows_warps(a.N, a.kernel * a.kernel * a.Cp32);
+    const int rows = few_rows_rows(a.M), cols = few_rows_cols(a.N), per_block = 8 / a.kw * cols;
+    const bool wide = cols > 1;
     const dim3 grid((unsigned)((up4(a.N) + per_block - 1) / per_block), (unsigned)((a.M + rows - 1) / rows));
     const auto kernel = rows == 1   ? (wide ? kernel_for<1, 4>(a) : kernel_for<1, 1>(a))
                         : rows == 2 ? (wide ? kernel_for<2, 4>(a) : kernel_for<2, 1>(a))
                                     : (wide ? kernel_for<4, 4>(a) : kernel_for<4, 1>(a));
     const bool overlapped = overlapped_launches_enabled();
-    note_contraction(8, a.kw, wide ? 4 : 1, overlapped);
+    note_contraction(8, a.kw, cols, overlapped);
     launch_overlapped_if(overlapped, kernel, grid, dim3(256), 0, s, a);
     return finish_launch();
 }

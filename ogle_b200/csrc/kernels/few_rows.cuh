@@ -24,4 +24,15 @@ struct FewRowsArgs {
 
 int launch_few_rows(FewRowsArgs a, cudaStream_t s);
 
+// Warps that share a column and a reduction of `total` elements: as many as fill the GPU, with two steps each.
+inline int few_rows_warps(int N, int total) {
+    int kw = 1;
+    while (kw < 8 && (long)up4(N) * kw * 2 <= 16 * kNumSMs && total >= kw * 256) kw *= 2;
+    return kw;
+}
+// Columns of a warp: four where one each is more than the GPU holds at once.
+inline int few_rows_cols(int N) { return N > 32 * kNumSMs ? 4 : 1; }
+// Rows of a warp.
+inline int few_rows_rows(long M) { return M == 1 ? 1 : (M == 2 ? 2 : 4); }
+
 }  // namespace ogle

@@ -122,10 +122,13 @@ static int gemm_packed(const OgleGemmParams* pp, const float* A, const void* pac
     // A row at a time is always quicker without the tensor cores (in graphs: 1 x 512 x 1000 8.6 -> 3.2 us; 1 x 4096 x 4096 70 ->
     // 31, in one pass 19 -> 13), up to eight rows while there is little to multiply (8 x 512 x 1000 8.7 -> 5.0; 6 x 911 x
     // 1257 9.5 -> 13), further where split-mode reductions are too long to be cut (2 x 3430 x 700 42 -> 13, 3 x 3784 x 3257
-    // 62 -> 52). Not behind a packing pass, whose B it would wait for no less.
+    // 62 -> 52), or nearly so: from 2660 elements on ranges in clusters would move the result too far (choose_cluster). Below,
+    // four rows over columns that give each SM less than two blocks of a warp a column are no better off (4 x 2500 x 1500
+    // 19.4 -> 22), nor is a warp of four columns (3 x 2500 x 5000 26 -> 41). Not behind a packing pass, whose B it would wait for no less.
     const bool split = p.math_mode == OGLE_MATH_TF32X3;
     const double products = (double)p.M * p.N * p.K;
-    if (!overlapped && (p.M == 1 || (p.M <= 8 && products <= 6e6) || (split && p.M <= 4 && p.K >= 2048 && products <= 4e7))) {
+    const bool cut = p.K <= 2660 && (few_rows_cols(p.N) > 1 || (p.M == 4 && p.N < 16 * kNumSMs && few_rows_warps(p.N, Kp32) == 1));
+    if (!overlapped && (p.M == 1 || (p.M <= 8 && products <= 6e6) || (split && p.M <= 4 && p.K >= 2048 && products <= 4e7 && !cut))) {
         FewRowsArgs r = {};
         r.x = A; r.hi = hi; r.lo = split ? lo : nullptr; r.bias = C; r.y = Y;
         r.M = p.M; r.N = p.N; r.C = p.K; r.Cp32 = Kp32; r.ldx = p.lda; r.ldy = p.ldy; r.ldc = p.ldc;

@@ -1065,6 +1065,22 @@ def test_clusters_do_not_take_longer_ranges(shape, math):
     assert err <= 1.05 * run(planned)[1] + 1e-8
 
 
+@pytest.mark.parametrize("m,k,n,form", [
+    # reductions that clusters can still cut, and longer ones; columns for a warp each, for several and for four a warp
+    (4, 2500, 1500, 3), (4, 2500, 3000, 8), (4, 2500, 1000, 8), (4, 2700, 1500, 8), (3, 2500, 1500, 8), (2, 2500, 5000, 3), (2, 2700, 5000, 8), (1, 2500, 5000, 8)])
+def test_long_products_of_few_rows(m, k, n, form):
+    """Which kernel serves them, and as exactly as either does."""
+    import torch
+    from ogle_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m * k + n)
+    a, b = torch.randn((m, k), generator=g, device="cuda"), torch.randn((k, n), generator=g, device="cuda")
+    got = ops.gemm_packed(a, ops.gemm_pack_b(b, m, k, n, 0, ops.MATH_TF32X3), None, m, k, n, 0, 1.0, 1.0, 0, ops.MATH_TF32X3)
+    assert ops.last_contraction().form == form
+    want = a.double() @ b.double()
+    # products of fp32 grade; sums in tensor memory lose 6e-9 of the norm per element
+    assert float((got.double() - want).norm()) <= (2e-5 if form == 3 else 5e-6) * float(want.norm())
+
+
 @pytest.mark.parametrize("m,k,n,bias_mode", [
     # a row, two, up to four and up to eight; one to eight warps to a column, four columns to a warp; reductions and columns
     # that end inside a step, a piece, the pack's padding
@@ -1305,8 +1321,10 @@ def test_kernel_names_are_those_of_the_sources(case):
 
 @pytest.mark.parametrize("case", [
     # images, size, C, K, kernel, stride, split asked for, name: both sides of what decides between the tensor-core path's kernels
-    (1, 3, 256, 128, 1, 1, 0, "few_rows_kernel"), (1, 3, 256, 128, 1, 1, 2, "conv_tc2_kernel"), (32, 1, 64, 700, 1, 1, 0, "few_rows_kernel"),
-    (33, 1, 64, 600, 1, 1, 0, "conv_tc2_kernel"), (2, 2, 128, 300, 3, 1, 0, "few_rows_kernel"), (2, 2, 128, 330, 3, 1, 0, "conv_tc2_kernel"),
+    (1, 3, 256, 128, 1, 1, 0, "few_rows_kernel"), (1, 3, 256, 128, 1, 1, 2, "conv_tc2_kernel"), (32, 1, 64, 400, 1, 1, 0, "few_rows_kernel"),
+    (33, 1, 64, 400, 1, 1, 0, "conv_tc2_kernel"), (32, 1, 64, 512, 1, 1, 0, "conv_tc2_kernel"), (24, 1, 64, 700, 1, 1, 0, "few_rows_kernel"),
+    (32, 1, 33, 1366, 1, 1, 0, "conv_tc2_kernel"), (8, 1, 128, 2900, 1, 1, 0, "few_rows_kernel"), (6, 1, 164, 2342, 1, 1, 0, "conv_tc2_kernel"),
+    (2, 1, 64, 3000, 1, 1, 0, "few_rows_kernel"), (2, 2, 128, 300, 3, 1, 0, "few_rows_kernel"), (2, 2, 128, 330, 3, 1, 0, "conv_tc2_kernel"),
     (2, 64, 3, 48, 7, 2, 0, "conv_window_kernel"), (2, 64, 3, 49, 7, 2, 0, "conv_tc2_kernel"), (2, 64, 2, 64, 7, 2, 0, "conv_window_kernel"),
     (2, 64, 3, 65, 5, 1, 0, "conv_tc2_kernel"), (80, 120, 3, 64, 7, 2, 0, "conv_window_kernel")])
 @pytest.mark.parametrize("residual", [False, True])
