@@ -453,6 +453,10 @@ static bool few_rows(const ConvArgs& a) {
 // pass: 1 image of 224 x 224 8.2 us gathered, 7.2 so, 8 24.1 and 14.5, 128 279 and 135; split mode 32 images 69.3 and 62.1,
 // 128 257 and 226. With 49 channels and more and three values to gather it is no better up to eight rounds of tiles (1 image
 // 7.7 and 8.6, 8 20.9 and 21.0, 16 34.1 and 33.6), with fewer channels from the first on (3 x 200 x 120 -> 48 20.9 and 14.6).
+// One input channel is a quarter of what the window's pixels carry, and 25 or 49 values a row are soon gathered: where whole
+// slabs of outputs leave the gather form without ragged ends it is the better one in split mode (7x7, 3 images of 112 x 70 -> 64
+// 7.3 and 8.6, 5 of 241 x 143 at stride 1 26.3 and 29.4; 5x5 between 0.90 and 1.07 of it), in one pass up to a round of 7x7 tiles
+// (86 x 193 -> 64 7.0 and 7.8; 20 images of 38 x 114 15.9 and 14.6).
 static double window_tiles(const ConvArgs& a, bool* row_tiles) {
     const double tall = (double)((a.Wo + 7) / 8) * ((a.Ho + 15) / 16), flat = (double)((a.Wo + 127) / 128) * a.Ho;
     *row_tiles = a.stride == 1 && flat < tall;
@@ -464,6 +468,7 @@ static bool window_form(const ConvArgs& a, int variant, bool split_mode) {
     if (a.kernel == 3 || a.K > 64 || !conv_tc_gather_supported(a, variant) || !gather_tile(a, true, &tw, &th)) return false;
     const double gathered = (double)((a.Wo + tw - 1) / tw) * ((a.Ho + th - 1) / th), windows = window_tiles(a, &row_tiles);
     if (split_mode && a.kernel == 7 && a.C == 3 && a.K > 48 && windows * a.N <= 8.0 * kNumSMs) return false;
+    if (a.C == 1 && a.K % 32 == 0 && a.kernel == 7 && (split_mode || (windows < gathered ? windows : gathered) * a.N <= kNumSMs)) return false;
     return windows <= 1.3 * gathered && windows * a.N < 0x7fffffff - 2 * kNumSMs;
 }
 

@@ -1326,7 +1326,8 @@ def test_kernel_names_are_those_of_the_sources(case):
     (32, 1, 33, 1366, 1, 1, 0, "conv_tc2_kernel"), (8, 1, 128, 2900, 1, 1, 0, "few_rows_kernel"), (6, 1, 164, 2342, 1, 1, 0, "conv_tc2_kernel"),
     (2, 1, 64, 3000, 1, 1, 0, "few_rows_kernel"), (2, 2, 128, 300, 3, 1, 0, "few_rows_kernel"), (2, 2, 128, 330, 3, 1, 0, "conv_tc2_kernel"),
     (2, 64, 3, 48, 7, 2, 0, "conv_window_kernel"), (2, 64, 3, 49, 7, 2, 0, "conv_tc2_kernel"), (2, 64, 2, 64, 7, 2, 0, "conv_window_kernel"),
-    (2, 64, 3, 65, 5, 1, 0, "conv_tc2_kernel"), (80, 120, 3, 64, 7, 2, 0, "conv_window_kernel")])
+    (2, 64, 3, 65, 5, 1, 0, "conv_tc2_kernel"), (80, 120, 3, 64, 7, 2, 0, "conv_window_kernel"),
+    (3, 90, 1, 64, 7, 2, 0, "conv_tc2_kernel"), (3, 90, 1, 60, 7, 2, 0, "conv_window_kernel"), (3, 90, 1, 32, 5, 2, 0, "conv_window_kernel")])
 @pytest.mark.parametrize("residual", [False, True])
 def test_kernel_names_say_what_runs(case, residual):
     import ctypes as C
