@@ -625,8 +625,11 @@ int launch_igemm(const IgemmArgs& a, bool trans_b, cudaStream_t s, const char** 
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = k;
-            // (two or three blocks an SM come out ahead of what they are counted as above)
-            us = 0.41 * (blocks < 2.7 ? 2.7 : blocks) * ((steps + k - 1) / k + 6.0);
+            // (Two or three blocks an SM come out ahead of what they are counted as above, and so do five and a part, of which the
+            // last two run beside each other alone: 3 images of 40 x 28, 3x3 87 -> 220, 5.7 blocks, 40.1 us where six take
+            // 46.7, and the other form 43.8. Five images of 61 x 23, 3x3 315 -> 92, 5.95 blocks, 155 and 117.)
+            const double exact = (double)(tiles * k) / kNumSMs;
+            us = 0.41 * (blocks < 2.7 ? 2.55 : (exact > 5.0 && exact < 5.75 ? exact + 0.1 : blocks)) * ((steps + k - 1) / k + 6.0);
         }
     }
     const int rc = by_copy_engine(us, best);

@@ -318,8 +318,8 @@ def test_fp32_contraction_forms(m, k, n, trans_b):
     # N, H, W, C, K, kernel, stride, pad, dilation: tiles of 128 and of 64 pixels, alone and over clusters of 2, 4, 5, 6 and 8;
     # channels that end inside a step, columns and pixels inside a tile, strides, dilations, padding wider than the window
     (5, 60, 45, 54, 374, 3, 1, 0, 2), (4, 43, 38, 115, 286, 1, 1, 1, 1), (2, 43, 41, 262, 214, 3, 1, 3, 1), (3, 48, 27, 296, 367, 1, 1, 0, 1),
-    (4, 44, 14, 157, 237, 3, 1, 0, 1), (4, 43, 26, 25, 183, 5, 1, 1, 1), (6, 45, 30, 57, 33, 3, 1, 0, 1), (1, 6, 27, 355, 62, 5, 2, 4, 2),
-    (4, 10, 22, 309, 87, 5, 3, 4, 2), (4, 41, 43, 106, 389, 5, 2, 2, 1), (2, 56, 55, 154, 86, 5, 1, 5, 2), (3, 45, 30, 25, 219, 5, 1, 2, 2),
+    (4, 44, 14, 157, 237, 3, 1, 0, 1), (7, 43, 26, 25, 183, 5, 1, 1, 1), (6, 45, 30, 57, 33, 3, 1, 0, 1), (1, 6, 27, 703, 62, 5, 2, 4, 2),
+    (4, 10, 22, 701, 87, 5, 3, 4, 2), (3, 41, 43, 106, 389, 5, 2, 2, 1), (2, 56, 55, 154, 86, 5, 1, 5, 2), (7, 45, 30, 25, 219, 5, 1, 2, 2),
     (5, 59, 21, 315, 92, 3, 1, 3, 2), (2, 30, 42, 121, 113, 3, 1, 3, 1), (3, 13, 18, 286, 362, 5, 1, 2, 1)])
 def test_fp32_contraction_by_the_copy_engine(shape):
     import ctypes as C
@@ -1344,6 +1344,19 @@ def test_kernel_names_say_what_runs(case, residual):
         ops.conv2d_residual(p, x, packed, b, torch.zeros_like(y))
     form = ops.last_contraction().form
     assert {8: "few_rows_kernel", 9: "conv_window_kernel"}.get(form, "conv_tc2_kernel") == name
+
+
+@pytest.mark.parametrize("shape,name", [
+    # N, H, W, C, K, kernel, stride: two blocks an SM and fewer, six, and others, on either side of the two forms' times
+    ((3, 40, 28, 87, 220, 3, 1), "conv_igemm_kernel"), ((55, 24, 5, 49, 139, 5, 2), "conv_igemm_kernel"), ((1, 7, 14, 578, 55, 3, 1), "conv_igemm_kernel"),
+    ((8, 38, 6, 53, 423, 3, 1), "conv_igemm_kernel"), ((8, 56, 56, 64, 64, 3, 1), "conv_igemm_tma_kernel"), ((8, 28, 28, 128, 256, 3, 2), "conv_igemm_tma_kernel"),
+    ((5, 63, 25, 315, 92, 3, 1), "conv_igemm_tma_kernel"), ((1, 7, 10, 698, 304, 3, 2), "conv_igemm_tma_kernel"), ((8, 7, 7, 512, 512, 3, 1), "conv_igemm_tma_kernel"), ((32, 38, 38, 256, 256, 3, 1), "conv_igemm_tma_kernel")])
+def test_fp32_contraction_takes_the_faster_form(shape, name):
+    import ctypes as C
+    from ogle_b200 import _lib, ops
+    N, H, W, ci, K, k, s = shape
+    p = ops.conv_params(N, H, W, ci, K, k, s, k // 2, 1, 1, True, ops.ACT_RELU, 0.0, 0.0, ops.MATH_FP32)
+    assert _lib.cuda_lib().ogle_cuda_conv2d_kernel_name(C.byref(p)).decode() == name
 
 
 @pytest.mark.parametrize("env,overlapped", [(None, 1), ("0", 0), ("1", 1)])
