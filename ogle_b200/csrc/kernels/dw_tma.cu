@@ -15,7 +15,7 @@
 // shared-memory reads are conflict-free (slabs of 16 at stride 2 are not: two wavefronts).
 // The 32 pixel slots of a block (64 with slabs of 16) are split into row groups of tw.
 // Widths that are no multiple of 32 channels, and 5x5 windows, ran on kernels that fetch every
-// tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 22 us here (16 us floor).
+// tap through L1: 16 x 75 x 75 x 144 channels took 39 us there and 23.5 us here (16 us floor).
 #include <cmath>
 #include <cstdlib>
 
@@ -241,21 +241,35 @@ bool fit_tile(const ConvArgs& a, int quads, int tw, int rpg, DwTiles* t) {
     return true;
 }
 
-// Tile shape at stride 1: equal parts of the map's width, or one of a few widths that fill a block's pixel slots, and the
-// rows a thread computes, by an estimate of the time: rounds of tiles over the resident blocks, of which each takes a fixed
+// Output pixels of all tiles of a map, those past its edges included.
+double covered(const ConvArgs& a, const DwTiles& t) {
+    return (double)((a.Wo + t.tw - 1) / t.tw) * t.tw * ((a.Ho + t.th - 1) / t.th) * t.th;
+}
+
+// Estimate of a launch's time (us) at stride 1: rounds of tiles over the resident blocks, of which each takes a fixed
 // time, its rows' multiply-adds and its copies, partly beside one another; or the time at the HBM rate, which rings of fewer
-// than four stages do not reach. Fitted to 60 layers, 4 us to 170, with every width and row count timed: 5 % faster on
-// average than choose_shape_by_rows, 3 % off the best; 16 x 75 x 75 x 144
-// 24.3 -> 22.4 us (tiles of 15 keep 30 of 32 slots busy where 32, 32 and 11 kept 25), 64 x 75 x 75 x 128 64 -> 59,
-// 22 x 83 x 99 x 345 101 -> 86.
-int choose_shape_stride1(const ConvArgs& a, int quads, DwTiles* t) {
-    static const int kRows3[] = {10, 8, 7, 5, 4, 2}, kRows5[] = {4, 2};
-    const int* rows = a.kernel == 5 ? kRows5 : kRows3;
-    const int nrows = a.kernel == 5 ? 2 : 6;
+// than four stages do not reach.
+double stride1_us(const ConvArgs& a, int quads, const DwTiles& t, int rows) {
     const int slab = quads * 4, cblocks = (a.Kp + slab - 1) / slab;
     int resident = kNumSMs * (a.kernel == 3 ? 2 : 1);
     if (cblocks <= resident) resident -= resident % cblocks;
     const double hbm = 8.0 * a.N * a.Ho * a.Wo * a.Kp / 6.0e6;
+    const double tiles = (double)((a.Wo + t.tw - 1) / t.tw) * ((a.Ho + t.th - 1) / t.th) * cblocks * a.N;
+    const double rounds = ceil(tiles / resident);
+    const double compute = 1.47 + 0.088 * rows * (a.kernel == 3 ? 1.0 : 3.8), copy = 0.0023 * t.ih * t.iw * quads / 8;
+    const double work = rounds * (compute > copy ? compute + 0.37 * copy : copy + 0.37 * compute);
+    const double memory = t.stages < 4 ? 1.24 * hbm : hbm;
+    return work > memory ? work + 0.33 * memory : memory + 0.33 * work;
+}
+
+// Tile shape at stride 1: equal parts of the map's width, or one of a few widths that fill a block's pixel slots, and the
+// rows a thread computes, by the estimate. Fitted to 60 layers, 4 us to 170, with every width and row count timed: 5 % faster
+// on average than choose_shape_by_rows, 3 % off the best; 16 x 75 x 75 x 144 25.2 -> 23.5 us (tiles of 15 keep 30 of 32
+// slots busy where 32, 32 and 11 kept 25), 64 x 75 x 75 x 128 64 -> 59, 22 x 83 x 99 x 345 101 -> 86.
+int choose_shape_stride1(const ConvArgs& a, int quads, DwTiles* t) {
+    static const int kRows3[] = {10, 8, 7, 5, 4, 2}, kRows5[] = {4, 2};
+    const int* rows = a.kernel == 5 ? kRows5 : kRows3;
+    const int nrows = a.kernel == 5 ? 2 : 6;
     const char* env_tw = getenv("OGLE_DW_TW");
     const char* env_rows = getenv("OGLE_DW_RPG");
     const int force_rows = env_rows ? atoi(env_rows) : 0;
@@ -265,12 +279,7 @@ int choose_shape_stride1(const ConvArgs& a, int quads, DwTiles* t) {
         for (int i = 0; i < nrows; ++i) {
             DwTiles s;
             if ((force_rows && rows[i] != force_rows) || !fit_tile(a, quads, tw, rows[i], &s)) continue;
-            const double tiles = (double)((a.Wo + tw - 1) / tw) * ((a.Ho + s.th - 1) / s.th) * cblocks * a.N;
-            const double rounds = ceil(tiles / resident);
-            const double compute = 1.47 + 0.088 * rows[i] * (a.kernel == 3 ? 1.0 : 3.8), copy = 0.0023 * s.ih * s.iw * quads / 8;
-            const double work = rounds * (compute > copy ? compute + 0.37 * copy : copy + 0.37 * compute);
-            const double memory = s.stages < 4 ? 1.24 * hbm : hbm;
-            const double us = work > memory ? work + 0.33 * memory : memory + 0.33 * work;
+            const double us = stride1_us(a, quads, s, rows[i]);
             if (!best || us < best_us) { best = rows[i]; best_us = us; *t = s; }
         }
     };
@@ -343,9 +352,19 @@ int choose_shape(const ConvArgs& a, DwTiles* t) {
     // parts of 13, 146 in what it takes), unless tiles of 32 hang far over the map's edge (27 x 127 x 70 x 160 56 -> 52).
     int rows = choose_shape_by_rows(a, quads, t);
     const bool large = 8.0 * a.N * a.Ho * a.Wo * a.Kp > 160e6;
-    if (a.stride == 1 && !(rows && large && (double)a.Wo * a.Ho >= 0.72 * (double)(((a.Wo + t->tw - 1) / t->tw) * t->tw) *
-                                                                  (((a.Ho + t->th - 1) / t->th) * t->th)))
-        rows = choose_shape_stride1(a, quads, t);
+    if (a.stride == 1 && !(rows && large && (double)a.Wo * a.Ho >= 0.72 * covered(a, *t))) {
+        // Where the two are estimated alike, and this one neither hangs less over the map's edge nor keeps as many of a block's
+        // pixel slots busy, it is not the better one (12 x 9 x 45 x 832 in parts of 15 8.3 us, of 23, estimated 1 % better, 9.5;
+        // 10 x 41 x 27 x 807 of 14 15.4, of 27 17.5). Of 360 layers ten are 5 to 13 % slower than by the other rule, the
+        // geometric mean of all is 0.91.
+        DwTiles other;
+        const int other_rows = choose_shape_stride1(a, quads, &other);
+        if (!rows || (other_rows && (covered(a, other) <= 0.97 * covered(a, *t) || other.tw * other.row_groups >= t->tw * t->row_groups ||
+                                     stride1_us(a, quads, other, other_rows) < 0.984 * stride1_us(a, quads, *t, rows)))) {
+            rows = other_rows;
+            *t = other;
+        }
+    }
     if (forced) return rows;
     unsigned place = at + next++ % kPlaces;
     for (unsigned i = 0; i < kPlaces; ++i)

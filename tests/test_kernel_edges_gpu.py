@@ -42,6 +42,25 @@ def test_depthwise_tile_shapes(oracle_port, size, images, channels, kernel):
     close(run_case_cuda(case), oracle_port.conv2d(x, w, b, 1, kernel // 2, 1, channels, 2, 0.0, 6.0))
 
 
+@pytest.mark.parametrize("shape,width", [((12, 9, 45, 832), 15), ((10, 41, 27, 807), 14), ((8, 15, 47, 800), 16)])
+def test_depthwise_shapes_estimated_alike(shape, width, monkeypatch):
+    """Maps that another width, of a time estimated within 1.5 %, took 12-15 % longer for: not slower than in the named one."""
+    import torch
+    from ogle_b200 import ops
+    N, H, W, ch = shape
+    g = torch.Generator(device="cuda").manual_seed(ch)
+    x = torch.zeros((N, H, W, ops.up4(ch)), device="cuda")
+    x[..., :ch] = torch.randn((N, H, W, ch), generator=g, device="cuda")
+    p = ops.conv_params(N, H, W, ch, ch, 3, 1, 1, 1, ch, False, ops.ACT_RELU, 0.0, 0.0, ops.MATH_FP32)
+    packed, y = ops.conv2d_prepack(p, torch.randn((ch, 1, 3, 3), generator=g, device="cuda")), torch.empty_like(x)
+    took = []
+    for forced in (False, True):
+        if forced:
+            monkeypatch.setenv("OGLE_DW_TW", str(width))
+        took.append(_median_us(_in_a_graph(lambda: ops.conv2d(p, x, packed, None, y, workspace=None))))
+    assert took[0] <= 1.06 * took[1], took
+
+
 def test_depthwise_shapes_of_a_network_are_weighed_once():
     """A pass over the thirteen depthwise layers of a network takes the host no longer a layer than one of them over and over;
     layers that it has not seen lately take longer."""
