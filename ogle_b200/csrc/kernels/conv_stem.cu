@@ -8,7 +8,7 @@
 //    window of a tile, halo included, is ONE TMA box of 16-byte pixels whose out-of-image
 //    part arrives as zeros (the padding); three stages, each filled again by the last warp
 //    that is through with it, so that no warp waits for another: one's loads and stores fall
-//    into another's multiply-adds (with a barrier a tile: 285 us where this takes 262);
+//    into another's multiply-adds (with a barrier a tile: 285 us where this takes 265);
 //  * a warp owns a run of PL*PXT output pixels of one row, PL = 32 / (K/8) pixel lanes x
 //    K/8 channel groups: a thread accumulates PXT pixels x 8 channels in registers. The
 //    eight are two fours K/2 apart: the channel groups of a pixel write whole 32-byte
@@ -19,7 +19,7 @@
 //    window is read once for the three taps across it (294 -> 285): 87 shared loads to 540
 //    two-wide multiply-adds, no bounds checks and no address arithmetic in the inner loop.
 //
-// Times are of 256 images of 300 x 300, 3 -> 32 channels, stride 2: 314 us -> 262, of which HBM
+// Times are of 256 images of 300 x 300, 3 -> 32 channels, stride 2: 314 us -> 265, of which HBM
 // wants 169 and the fp32 pipes 147 (53 % busy at 285 us). Smaller tiles for few images gain under
 // 1 us (8 images 13.1) and lose 4 % and more from 16 images on.
 #include "tc_common.cuh"

@@ -482,7 +482,8 @@ int launch_tma(const IgemmArgs& a, const CUtensorMap& mA, const CUtensorMap& mB,
 // from 3e7 to 2e10 operations all but a dozen that take over 40 us took within 5 % of the estimate.
 struct TmaPlan { int ty, splits; double us; };
 
-// least: ranges the reduction has in the other form; with fewer, sums are longer and errors larger (by up to a quarter).
+// least: ranges the reduction has in the other form; with fewer, sums are longer and errors larger (by up to a quarter). At the
+// same number the longest may be up to 24 elements longer than there, since a step is 32 elements of one tap.
 TmaPlan plan_tma(const IgemmArgs& a, int least) {
     const int chunks = a.kernel * a.kernel * ((a.Cp + kTmaK - 1) / kTmaK);
     TmaPlan best = {0, 1, 1e30};
